@@ -526,8 +526,8 @@ struct FrameJob {
   unsigned long long *counters;  // [0] nodes evaluated, [1] near the liquidus, [2] fallbacks
 };
 
-__device__ __forceinline__ void node_xyz(const FrameJob &j, int64_t n, double &x, double &y, double &z) {
-  const int64_t I = n % j.nodes[0], J = (n / j.nodes[0]) % j.nodes[1], K = n / ((int64_t)j.nodes[0] * j.nodes[1]);
+__device__ __forceinline__ void node_xyz(const FrameJob &j, int64_t I, int64_t J, int64_t K, double &x, double &y,
+                                         double &z) {
   x = (j.origin[0] + j.spacing * (double)I) * j.length_scale;
   y = (j.origin[1] + j.spacing * (double)J) * j.length_scale;
   z = (j.origin[2] + j.spacing * (double)K) * j.length_scale;
@@ -542,7 +542,7 @@ __global__ void scan_frames_kernel(FrameJob j) {
     const int f = j.f0 + (int)(q / j.nnodes);
     const int64_t n = q % j.nnodes;
     double x, y, z;
-    node_xyz(j, n, x, y, z);
+    node_xyz(j, n % j.nodes[0], (n / j.nodes[0]) % j.nodes[1], n / ((int64_t)j.nodes[0] * j.nodes[1]), x, y, z);
     j.ring[(int64_t)(f % j.slots) * j.nnodes + n] = scan_field(j.src, x, y, z, frame_time(j, f));
   }
 }
@@ -557,28 +557,72 @@ __global__ void fill_frames_kernel(FrameJob j) {
   }
 }
 
-// Query q of a model-frame job: its node (or -1 outside the grid) and frame.
-__device__ __forceinline__ int64_t frame_query(const FrameJob &j, int64_t q, int &f) {
-  const int64_t boxn = (int64_t)j.box[0] * j.box[1] * j.box[2];
-  f = j.f0 + (int)(q / boxn);
-  const int64_t l = q % boxn;
-  const int bi = (int)(l % j.box[0]), bj = (int)((l / j.box[0]) % j.box[1]),
-            bk = (int)(l / ((int64_t)j.box[0] * j.box[1]));
-  double xl, yl, dir;
-  scan_position(j.src, frame_time(j, f), xl, yl, dir);
-  const double xmin = dir > 0 ? xl + j.win_lo[0] : xl - j.win_hi[0];
-  const double ymin = yl + j.win_lo[1];
-  const double zmin = j.src.z_top - j.win_hi[2];
-  const int i0 = (int)floor((xmin / j.length_scale - j.origin[0]) / j.spacing);
-  const int j0 = (int)floor((ymin / j.length_scale - j.origin[1]) / j.spacing);
-  const int k0 = (int)floor((zmin / j.length_scale - j.origin[2]) / j.spacing);
-  const int I = i0 + bi, J = j0 + bj, K = k0 + bk;
-  if (I < 0 || I >= j.nodes[0] || J < 0 || J >= j.nodes[1] || K < 0 || K >= j.nodes[2]) return -1;
+// What the model's queries of one frame share: the frame's time, where the
+// source is and which way it moves, and the FE nodes the model answers for:
+// the window around the source (job.box nodes from its lower corner) clipped
+// to the grid. `first` = queries of the job's frames before this one.
+struct FrameBox {
+  double t, xl, yl, dir;
+  int lo[3], n[3];
+  int64_t first;
+};
+
+// Frames one launch answers for: their boxes live in shared memory.
+constexpr int kJobFrames = 64;
+
+__device__ __forceinline__ void frame_box(const FrameJob &j, int f, FrameBox &b) {
+  b.t = frame_time(j, f);
+  scan_position(j.src, b.t, b.xl, b.yl, b.dir);
+  const double low[3] = {b.dir > 0 ? b.xl + j.win_lo[0] : b.xl - j.win_hi[0], b.yl + j.win_lo[1],
+                         j.src.z_top - j.win_hi[2]};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int i0 = (int)floor((low[a] / j.length_scale - j.origin[a]) / j.spacing);
+    const int64_t end = min((int64_t)j.nodes[a], (int64_t)i0 + j.box[a]);
+    b.lo[a] = max(i0, 0);
+    b.n[a] = end > b.lo[a] ? (int)(end - b.lo[a]) : 0;
+  }
+}
+
+// Boxes of the job's frames into shared memory (every thread of the block);
+// returns the job's query count. The callers synchronise afterwards by the
+// barrier this ends with.
+__device__ int64_t frame_boxes(const FrameJob &j, FrameBox *boxes) {
+  if ((int)threadIdx.x < j.nf) frame_box(j, j.f0 + (int)threadIdx.x, boxes[threadIdx.x]);
+  __syncthreads();
+  int64_t total = 0;
+  for (int k = 0; k < j.nf; ++k) {
+    if (threadIdx.x == 0) boxes[k].first = total;
+    total += (int64_t)boxes[k].n[0] * boxes[k].n[1] * boxes[k].n[2];
+  }
+  __syncthreads();
+  return total;
+}
+
+// Query q of the job: the index of its frame's box and its node.
+__device__ __forceinline__ int64_t frame_query(const FrameJob &j, const FrameBox *boxes, int64_t q, int &k, int &I,
+                                               int &J, int &K) {
+  int lo = 0, hi = j.nf - 1;  // the last frame whose first query is at most q (empty frames share theirs)
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (boxes[mid].first <= q) lo = mid; else hi = mid - 1;
+  }
+  k = lo;
+  const FrameBox &b = boxes[k];
+  const int64_t l = q - b.first;
+  const int64_t row = l / b.n[0], slab = row / b.n[1];
+  I = b.lo[0] + (int)(l - row * b.n[0]);
+  J = b.lo[1] + (int)(row - slab * b.n[1]);
+  K = b.lo[2] + (int)slab;
   return ((int64_t)K * j.nodes[1] + J) * j.nodes[0] + I;
 }
 
 // ---------------------------------------------------------------------------
 // Fused inference: the whole network on 128-query tiles, persistent.
+// Frames: only nodes inside both the source's window and the grid are
+// queries (a raster over a 60 x 60 x 40-cell block has 0.5% of its windows'
+// nodes inside the grid: with all of them evaluated, 1,484 frames took 250 ms,
+// now a few; the whole run of that raster 458 -> 207 ms).
 // Shared memory: activations H (128 x 256 bf16, four 64-column blocks of
 // 16 KB) and one layer's weights (256 x 256 bf16, four blocks of 32 KB).
 // 512 threads: warp w reads TMEM lanes 32 (w % 4) (its rows) and handles the
@@ -612,11 +656,14 @@ __global__ void __launch_bounds__(kInferThreads, 1)
   __shared__ __align__(16) float s_wh[kSurOut][kSurHid];
   __shared__ float s_bh[kSurOut];
   __shared__ float s_head[kInferGroups][128][2];
+  __shared__ float s_raw[SRC == kSrcFrames ? 128 : 1][kSurIn];
+  __shared__ FrameBox s_box[SRC == kSrcFrames ? kJobFrames : 1];
   const CUtensorMap *tW[4] = {&tW0, &tW1, &tW2, &tW3};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q4 = warp & 3, grp = warp >> 2, row = q4 * 32 + lane;
-  const int64_t ntiles = (a.nq + 127) / 128;
+  const int64_t nq = SRC == kSrcFrames ? frame_boxes(a.job, s_box) : a.nq;
+  const int64_t ntiles = (nq + 127) / 128;
   const SurParamLayout L;
 
   for (int i = threadIdx.x; i < kSurLayers * kSurHid; i += blockDim.x)
@@ -652,22 +699,41 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 
   for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
     const int64_t qi = tile * 128 + row;
-    bool valid = qi < a.nq;
+    const bool valid = qi < nq;
     float raw[kSurIn] = {0, 0, 0, 0, 0};
-    int f = 0;
+    int fk = 0;
     int64_t node = -1;
     double nx = 0, ny = 0, nz = 0;
     if (SRC == kSrcArray) {
       if (valid)
 #pragma unroll
         for (int i = 0; i < kSurIn; ++i) raw[i] = a.raw[qi * kSurIn + i];
-    } else if (valid) {
-      node = frame_query(a.job, qi, f);
-      valid = node >= 0;
-      if (valid) {
-        node_xyz(a.job, node, nx, ny, nz);
-        scan_inputs(a.job.src, nx, ny, nz, frame_time(a.job, f), raw);
+    } else {
+      // The first group works out the rows' nodes and raw inputs (along-track
+      // offset from the source, positive ahead of it, lateral offset, depth
+      // below the top surface, in m; power, W; speed, m/s) for all four groups,
+      // with the frame's source position at hand: an FP64 instruction holds its
+      // scheduler for 64 cycles on GB300, and about 110 of them in every one of
+      // the 16 warps (position, window corner and divisions per row) were most
+      // of a tile's 13.6 us.
+      if (grp == 0) {
+        if (valid) {
+          int I, J, K;
+          node = frame_query(a.job, s_box, qi, fk, I, J, K);
+          node_xyz(a.job, I, J, K, nx, ny, nz);
+          const FrameBox &fb = s_box[fk];
+          raw[0] = (float)((nx - fb.xl) * fb.dir);
+          raw[1] = (float)(ny - fb.yl);
+          raw[2] = (float)(a.job.src.z_top - nz);
+          raw[3] = (float)a.job.src.power;
+          raw[4] = (float)a.job.src.speed;
+        }
+#pragma unroll
+        for (int i = 0; i < kSurIn; ++i) s_raw[row][i] = raw[i];
       }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < kSurIn; ++i) raw[i] = s_raw[row][i];
     }
     // Fourier features: this group's 16 phases, sines at column j, cosines at 64 + j
     for (int j0 = grp * (kSurFreq / kInferGroups); j0 < (grp + 1) * (kSurFreq / kInferGroups); j0 += 8) {
@@ -771,8 +837,8 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         const bool fb = near && e > a.job.thresh;
         if (valid) {
           double out = (double)T;
-          if (fb) out = scan_field(a.job.src, nx, ny, nz, frame_time(a.job, f));
-          a.job.ring[(int64_t)(f % a.job.slots) * a.job.nnodes + node] = out;
+          if (fb) out = scan_field(a.job.src, nx, ny, nz, s_box[fk].t);
+          a.job.ring[(int64_t)((a.job.f0 + fk) % a.job.slots) * a.job.nnodes + node] = out;
         }
         const unsigned nv = __popc(__ballot_sync(0xffffffffu, valid));
         const unsigned nn = __popc(__ballot_sync(0xffffffffu, near));
@@ -1219,18 +1285,24 @@ void produce_frames(ThermalModel *model, sur::FrameJob job, cudaStream_t s) {
   }
   if (!job.counters) job.counters = model->counters;
   InferArgs ia{};
-  ia.nq = (int64_t)job.box[0] * job.box[1] * job.box[2] * job.nf;
-  ia.job = job;
   ia.error = model->err;
   CUtensorMap tw[kSurLayers];
   for (int l = 0; l < kSurLayers; ++l) tw[l] = tmap_bf16(model->Wb[l], kSurHid, SurParamLayout::in_dim(l), 256);
   int sms = 0;
   SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, model->device));
   SCK(cudaFuncSetAttribute(mlp_infer_kernel<kSrcFrames>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem));
-  const int64_t tiles = (ia.nq + 127) / 128;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sms));
-  mlp_infer_kernel<kSrcFrames><<<grid, kInferThreads, kInferSmem, s>>>(tw[0], tw[1], tw[2], tw[3], model->dev(), ia);
-  SCK(cudaGetLastError());
+  const int f_end = job.f0 + job.nf;
+  for (int f = job.f0; f < f_end; f += kJobFrames) {
+    ia.job = job;
+    ia.job.f0 = f;
+    ia.job.nf = std::min(kJobFrames, f_end - f);
+    // most queries the frames can have: a window clipped to the grid each
+    int64_t most = ia.job.nf;
+    for (int a = 0; a < 3; ++a) most *= std::min<int64_t>(job.box[a], job.nodes[a]);
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((most + 127) / 128, sms));
+    mlp_infer_kernel<kSrcFrames><<<grid, kInferThreads, kInferSmem, s>>>(tw[0], tw[1], tw[2], tw[3], model->dev(), ia);
+    SCK(cudaGetLastError());
+  }
 }
 
 }  // namespace amca

@@ -48,17 +48,4 @@ __host__ __device__ inline double scan_field(const ScanSource &s, double x, doub
   return (s.t_cap < T) ? s.t_cap : T;
 }
 
-// The model's raw inputs for a point: along-track offset (m, positive ahead of
-// the source), lateral offset (m), depth below the top surface (m), power (W),
-// speed (m/s).
-__host__ __device__ inline void scan_inputs(const ScanSource &s, double x, double y, double z, double t, float in[5]) {
-  double xl, yl, dir;
-  scan_position(s, t, xl, yl, dir);
-  in[0] = (float)((x - xl) * dir);
-  in[1] = (float)(y - yl);
-  in[2] = (float)(s.z_top - z);
-  in[3] = (float)s.power;
-  in[4] = (float)s.speed;
-}
-
 }  // namespace amca

@@ -191,3 +191,48 @@ def test_realm_runs_on_model_frames(A, trained):
     a, b = out["model"], out["fe"]
     assert abs(a["grains"] - b["grains"]) <= max(3, 0.25 * b["grains"]), out
     assert abs(a["mean_size_cells"] - b["mean_size_cells"]) <= 0.25 * b["mean_size_cells"], out
+
+
+@pytest.mark.parametrize("cells,tracks,f0,nf", [
+    ((100, 60, 40), 2, 0, 3),      # the source before the block: the window hangs over three faces
+    ((100, 60, 40), 1, 200, 1),    # inside the block
+    ((37, 23, 11), 2, 330, 5),     # few nodes: the last tile nearly empty, frames on both tracks
+    ((100, 60, 40), 1, 0, 131),    # more frames than one launch answers for
+    ((300, 200, 180), 1, 100, 2),  # a grid larger than the window across and in depth
+])
+def test_model_frames_equal_the_model_at_the_window_nodes(A, cells, tracks, f0, nf):
+    """Every node of the grid inside the window holds the model's temperature of its raw inputs, every other the
+    ambient temperature (the same kernel body on the same float32 inputs: equal bit for bit)."""
+    spec = decks.thermal_spec()
+    m = A.ThermalModel(**spec)
+    sc = decks.scan_of(cells, 2.0e-6, tracks=tracks, hatch=4.0e-5, margin_end=1.0e-4)
+    nf = min(nf, sc["frames"] - f0)
+    got, _, counts = m.frames(A.Scan.of(**sc), f0, nf, 1700.0, 150.0, 1e30)
+    h = sc["spacing"] * sc["length_scale"]
+    box = [int(np.ceil((spec["window_hi"][a] - spec["window_lo"][a]) / h)) + 2 for a in range(3)]
+    total = 0
+    for k in range(nf):
+        t = (f0 + k) * sc["frame_dt"] * sc["time_scale"]
+        tr = min(max(int(t / sc["track_time"]), 0), tracks - 1) if tracks > 1 else 0
+        tl = t - tr * sc["track_time"] if tracks > 1 else t
+        d = -1.0 if tr % 2 else 1.0
+        xl = sc["x_turn"] - sc["speed"] * tl if tr % 2 else sc["x_start"] + sc["speed"] * tl
+        yl = sc["y_line"] + tr * sc["hatch"]
+        low = [xl + spec["window_lo"][0] if d > 0 else xl - spec["window_hi"][0], yl + spec["window_lo"][1],
+               sc["z_top"] - spec["window_hi"][2]]
+        rng = []
+        for a in range(3):
+            i0 = int(np.floor((low[a] / sc["length_scale"] - sc["origin"][a]) / sc["spacing"]))
+            rng.append(np.arange(max(i0, 0), max(min(i0 + box[a], sc["nodes"][a]), max(i0, 0))))
+        want = np.full(sc["nodes"][::-1], sc["t0"])
+        if all(len(r) for r in rng):
+            x, y, z = ((sc["origin"][a] + sc["spacing"] * rng[a]) * sc["length_scale"] for a in range(3))
+            Z, Y, X = np.meshgrid(z, y, x, indexing="ij")
+            raw = np.stack([((X - xl) * d).ravel(), (Y - yl).ravel(), (sc["z_top"] - Z).ravel(),
+                            np.full(X.size, sc["power"]), np.full(X.size, sc["speed"])], 1).astype(np.float32)
+            T, _ = m.eval(raw)
+            want[np.ix_(rng[2], rng[1], rng[0])] = T.astype(np.float64).reshape(X.shape)
+            total += X.size
+        assert np.array_equal(got[k], want.ravel()), (k, f0 + k)
+    assert counts[0] == total
+    m.close()
