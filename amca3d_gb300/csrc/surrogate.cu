@@ -3,18 +3,19 @@
 // FE-coupled path that use it or the synthetic field it learns.
 //
 // Kernels:
-//   mlp_gemm_kernel<EPI>  one hidden layer's GEMM over a batch, D = A B^T with
-//                         bf16 operands loaded by TMA (128-byte swizzle), FP32
-//                         accumulators in TMEM, and a fused epilogue:
-//                         bias + SiLU (forward; row and transposed copies for
-//                         the weight gradients), bias + SiLU + FP32 head +
-//                         loss gradients (last layer), SiLU' (backward), or a
-//                         split-K partial (weight gradients).
+//   mlp_step_kernel       training: forward, loss and backward through the
+//                         activations of a 128-row tile, persistent; bf16
+//                         operands in shared memory, FP32 accumulators in TMEM.
+//   mlp_wgrad_kernel      training: weight gradients over pieces of the batch,
+//                         operands MN-major straight from the row-major
+//                         activations.
+//   mlp_chain_kernel      training: bias and head gradients, column sums.
+//   mlp_update_kernel     training: the pieces' sum and Adam.
 //   mlp_infer_kernel      the whole network per 128-query tile, persistent:
 //                         Fourier features written into shared memory, four
 //                         MMA layers with their weights streamed by TMA while
 //                         the previous epilogue runs, the head in FP32.
-//   plus feature encoding, reductions, Adam, data generation and the frame
+//   plus data generation and the frame
 //   generators (multi-track field, model frames with fallback).
 // Every wait (mbarrier) is bounded; a wait that runs out sets *error and the
 // block returns after releasing its TMEM.
@@ -46,8 +47,6 @@ using bf16 = __nv_bfloat16;
 constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s: every mbarrier wait
 constexpr int kErrWait = 1;
 
-enum { kEpiFwd = 0, kEpiHead = 1, kEpiBwd = 2, kEpiPartial = 3 };
-
 // fast reciprocal (MUFU) on an argument kept below 2^126 (z >= -80)
 __device__ __forceinline__ float sigmoid(float z) { return __fdividef(1.0f, 1.0f + __expf(-fmaxf(z, -80.0f))); }
 __device__ __forceinline__ float silu(float z) { return z * sigmoid(z); }
@@ -68,55 +67,382 @@ __device__ __forceinline__ void phases(const SurModelDev &m, const float raw[kSu
   sincospif(2.0f * f, &sv, &cv);
 }
 
-// ---------------------------------------------------------------------------
-// Layer GEMM with fused epilogues (training). D[M x N] = A[M x K] * B[N x K]^T.
-// Block: 256 threads; thread 0 issues the TMA loads and the MMAs; afterwards
-// warp w reads TMEM lanes 32 (w % 4) .. +31 (rows) and columns of half w / 4.
-// ---------------------------------------------------------------------------
-constexpr int kStages = 4;
-
-struct GemmArgs {
-  int M, N, K;
-  int kb_per_split;        // 64-wide K blocks per block (split-K over gridDim.z)
-  const float *bias;       // [N]
-  bf16 *out_row;           // [M x N]  H (forward) or dZ (backward)
-  bf16 *out_t;             // [N x M]  transposed copy
-  bf16 *head_t;            // [N x M]  last layer: its activations, transposed (head weight gradients)
-  bf16 *z_row;             // [M x N]  pre-activation (forward)
-  const bf16 *z_in;        // [M x N]  pre-activation of this output (backward)
-  float *partial;          // [splits x M x N] (split-K)
-  // last layer
-  const float *Wh, *bh;    // head (2 x N, 2)
-  const float *target;     // [M] normalised temperature
-  float *pred;             // [M x 2] mu, s
-  float *dpred;            // [M x 2] dL/dmu, dL/ds
-  float *loss;             // [M]
-  float inv_batch, lambda_s;
-  int *error;
-};
-
 __device__ __forceinline__ uint8_t *align1024(uint8_t *p) {
   return (uint8_t *)(((uintptr_t)p + 1023) & ~(uintptr_t)1023);
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(256, 1)
-    mlp_gemm_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, GemmArgs a) {
+// ---------------------------------------------------------------------------
+// Training. A step is four kernels:
+//   mlp_step_kernel    forward, loss and the pre-activation gradients dZ of a
+//                      128-row tile, layer by layer in shared memory;
+//   mlp_wgrad_kernel   weight gradients dZ_l^T X_l over pieces of the batch;
+//   mlp_chain_kernel   bias and head gradients, column sums over the batch;
+//   mlp_update_kernel  the sums over the pieces, and Adam.
+// Only what the gradients contract over the whole batch goes through memory:
+// the layer inputs X_l, the head's input and dZ_l, row-major bf16, 4.4 KB a
+// row. The weight gradients read them as MN-major operands, so no transposed
+// copy of an activation or a weight exists. Before (a GEMM per layer and
+// direction, each epilogue storing a row-major and a transposed copy, the
+// transposed one 2 bytes at a time, one-block-per-column bias and head sums):
+// 505 us for a step of 32,768 rows; now 188 us (alone and from a cold cache:
+// 105, 32, 32 and 22 us; the chains run beside the weight gradients, a step's
+// set-up beside the update before it). Every sum keeps its order: the trained
+// parameters are the same bits.
+// ---------------------------------------------------------------------------
+constexpr int kTrainThreads = 512, kTrainGroups = 4, kTrainCols = kSurHid / kTrainGroups;
+constexpr uint32_t kTrainSmem = 64u * 1024u + 128u * 1024u + 1024u;
+
+// Tensor maps of a training step: bf16 weights [out][in] (box 64 x 256), the
+// batch's layer inputs (X[0]: features) and dZ, each [rows][columns].
+struct TrainMaps {
+  CUtensorMap W[kSurLayers], X_out[kSurLayers + 1], dZ_out[kSurLayers];  // boxes of 128 rows (X[4]: the head's input)
+  CUtensorMap X_in[kSurLayers], dZ_in[kSurLayers];  // boxes of kWgradRows rows
+};
+
+struct StepArgs {
+  int64_t n;                  // rows, a multiple of 128
+  const float *raw, *target;  // samples: raw inputs (5 each) and normalised temperature
+  uint64_t nsamples, start, perm;  // row q is sample (start + q) * perm mod nsamples
+  uint4 *zs;                  // bf16 pre-activations of layers 0..2, in the order of the threads that use them
+  float *pred, *loss;         // [n x 2] mu, s; [n]
+  float2 *dpred;              // [n] dL/dmu, dL/ds
+  float inv_batch, lambda_s;
+  int *error;
+};
+
+__device__ __forceinline__ uint64_t sample_of(const StepArgs &a, uint64_t q) {
+  const uint64_t i = a.start + q;
+  if (__umul64hi(i, a.perm) == 0) return (i * a.perm) % a.nsamples;
+  return (uint64_t)(((unsigned __int128)i * a.perm) % a.nsamples);
+}
+
+// Forward and backward of 128-row tiles, persistent, one block per SM. Shared
+// memory: the tile's current activations or dZ (128 x 256 bf16) and one layer's
+// weights (256 x 256 bf16, streamed by TMA while the previous epilogue runs;
+// the backward pass reads the same [out][in] tiles as MN-major B operands). 512 threads: warp w reads TMEM lanes
+// 32 (w % 4) (its rows) and the 64-column group w / 4. An epilogue is bound by
+// its two MUFU operations per element (2.1 us a tile and layer), a layer's MMAs
+// take 1.35 us.
+// Head gradients: dL/dmu and dL/ds of a row are split into three bf16 terms
+// each, which hold all 24 bits of an FP32 value, so H4^T dpred runs on the
+// tensor cores with exact products and FP32 sums; it accumulates in TMEM over
+// the block's tiles.
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    mlp_step_kernel(const __grid_constant__ TrainMaps tm, SurModelDev md, StepArgs a) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t *smem = align1024(smem_raw);
-  __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
+  uint8_t *H = align1024(smem_raw);
+  uint8_t *Wsm = H + 64 * 1024;
+  __shared__ __align__(8) uint64_t wbar, mbar;
   __shared__ uint32_t tmem_base;
   __shared__ int s_abort;
-  __shared__ float s_head[2][128][2];
+  __shared__ __align__(16) float s_bias[kSurLayers][kSurHid];
+  __shared__ __align__(16) float s_wh[kSurOut][kSurHid];
+  __shared__ float s_bh[kSurOut];
+  __shared__ float s_head[kTrainGroups][128][2];
+  __shared__ float s_raw[128][kSurIn], s_y[128], s_dp[128][2];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int N = a.N;
-  const uint32_t a_bytes = 128u * 128u, b_bytes = (uint32_t)N * 128u, stage_bytes = a_bytes + b_bytes;
-  const int m0 = blockIdx.x * 128;
-  const int kb0 = blockIdx.z * a.kb_per_split, nk = a.kb_per_split;
+  const int q4 = warp & 3, grp = warp >> 2, row = q4 * 32 + lane;
+  const int64_t ntiles = a.n / 128;
+  const SurParamLayout L;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    umma::mbar_init(umma::smem_u32(&wbar), 1);
+    umma::mbar_init(umma::smem_u32(&mbar), 1);
+    umma::mbar_fence_init();
+    s_abort = 0;
+  }
+  if (warp == 0) umma::tmem_alloc(umma::smem_u32(&tmem_base), 256);
+  // the parameters may still be in the making (the previous step's update)
+  umma::wait_prerequisites();
+  for (int i = threadIdx.x; i < kSurLayers * kSurHid; i += blockDim.x)
+    s_bias[i / kSurHid][i % kSurHid] = md.p[L.b[i / kSurHid] + i % kSurHid];
+  for (int i = threadIdx.x; i < kSurOut * kSurHid; i += blockDim.x) s_wh[i / kSurHid][i % kSurHid] = md.p[L.Wh + i];
+  if (threadIdx.x < kSurOut) s_bh[threadIdx.x] = md.p[L.bh + threadIdx.x];
+  umma::tc_fence_before();
+  __syncthreads();
+  umma::tc_fence_after();
+  const uint32_t tmem = tmem_base;
+  const uint32_t trow = tmem + ((uint32_t)(q4 * 32) << 16);
+  constexpr uint32_t id_fwd = umma::idesc_bf16_f32(128, kSurHid);
+  constexpr uint32_t id_bwd = umma::idesc_bf16_f32(128, kSurHid, false, true);
+
+  bool w_pending = false;  // thread 0: a weight load is in flight, and the phase it completes
+  uint32_t wph = 0;
+  auto load_w = [&](int l) {
+    const int kbs = SurParamLayout::in_dim(l) / 64;
+    const uint32_t bar = umma::smem_u32(&wbar);
+    umma::mbar_expect_tx(bar, (uint32_t)kbs * 32u * 1024u);
+    for (int kb = 0; kb < kbs; ++kb) umma::tma_load_2d(umma::smem_u32(Wsm + kb * 32 * 1024), &tm.W[l], bar, kb * 64, 0);
+    w_pending = true;
+  };
+  auto weights_in = [&]() {
+    if (!umma::mbar_wait(umma::smem_u32(&wbar), wph, kWaitNs)) return false;
+    w_pending = false;
+    wph ^= 1u;
+    return true;
+  };
+  auto store_tile = [&](const CUtensorMap &t, int kbs, int64_t tile) {
+    for (int kb = 0; kb < kbs; ++kb) umma::tma_store_2d(&t, umma::smem_u32(H + kb * 16 * 1024), kb * 64, (int)(tile * 128));
+    umma::bulk_commit();
+  };
+  if (threadIdx.x == 0) load_w(0);
+  uint32_t mph = 0;
+  bool ok = true;
+  // every MMA issued by thread 0 has completed (bounded), in all threads
+  auto mma_done = [&]() {
+    const bool mok = umma::mbar_wait(umma::smem_u32(&mbar), mph, kWaitNs);
+    mph ^= 1u;
+    ok = __syncthreads_and(mok ? 1 : 0) != 0 && !s_abort;
+    umma::tc_fence_after();
+    return ok;
+  };
+  // what was written to shared memory is visible to the tensor cores and TMA
+  auto publish = [&]() {
+    umma::fence_async_smem();
+    umma::tc_fence_before();
+    __syncthreads();
+  };
+
+  for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    if (grp == 0) {
+      const uint64_t i = sample_of(a, (uint64_t)(tile * 128 + row));
+#pragma unroll
+      for (int k = 0; k < kSurIn; ++k) s_raw[row][k] = a.raw[i * kSurIn + k];
+      s_y[row] = a.target[i];
+    }
+    if (threadIdx.x == 0) umma::bulk_wait_read();  // the previous tile's last store has left H
+    __syncthreads();
+    {
+      float raw[kSurIn];
+#pragma unroll
+      for (int k = 0; k < kSurIn; ++k) raw[k] = s_raw[row][k];
+      for (int j0 = grp * (kSurFreq / kTrainGroups); j0 < (grp + 1) * (kSurFreq / kTrainGroups); j0 += 8) {
+        __align__(16) bf16 sb[8], cb[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          float sv, cv;
+          phases(md, raw, j0 + t, sv, cv);
+          sb[t] = __float2bfloat16_rn(sv);
+          cb[t] = __float2bfloat16_rn(cv);
+        }
+        *(uint4 *)(H + umma::sw128_offset(row, j0, 128)) = *(const uint4 *)sb;
+        *(uint4 *)(H + umma::sw128_offset(row, kSurFreq + j0, 128)) = *(const uint4 *)cb;
+      }
+    }
+    publish();
+    if (threadIdx.x == 0) store_tile(tm.X_out[0], kSurEnc / 64, tile);
+    uint4 *zt = a.zs + tile * (3 * (kTrainCols / 8) * kTrainThreads) + threadIdx.x;
+
+    // --- forward ---
+    for (int l = 0; l < kSurLayers; ++l) {
+      if (threadIdx.x == 0) {
+        if (!weights_in()) {
+          s_abort = 1;
+        } else {
+          umma::tc_fence_after();
+          const int kbs = SurParamLayout::in_dim(l) / 64;
+          for (int kb = 0; kb < kbs; ++kb) {
+            const uint32_t ha = umma::smem_u32(H + kb * 16 * 1024), wa = umma::smem_u32(Wsm + kb * 32 * 1024);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma::mma_bf16(tmem, umma::sdesc_sw128(ha + 32u * k), umma::sdesc_sw128(wa + 32u * k), id_fwd,
+                             (kb | k) != 0 ? 1u : 0u);
+          }
+        }
+        umma::mma_commit(umma::smem_u32(&mbar));
+        umma::bulk_wait_read();  // H may be rewritten once its store has read it
+      }
+      if (!mma_done()) break;
+      // the weights are free again (the last layer's stay for the backward pass)
+      if (threadIdx.x == 0 && l < kSurLayers - 1) load_w(l + 1);
+      if (l < kSurLayers - 1) {
+        for (int c0 = grp * kTrainCols; c0 < (grp + 1) * kTrainCols; c0 += 32) {
+          float v[32];
+          umma::tmem_ld32(trow + c0, v);
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            __align__(16) bf16 zb[8], hb[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+              const float z = v[j + t] + s_bias[l][c0 + j + t];
+              zb[t] = __float2bfloat16_rn(z);
+              hb[t] = __float2bfloat16_rn(silu(z));
+            }
+            zt[(l * (kTrainCols / 8) + (c0 % kTrainCols + j) / 8) * kTrainThreads] = *(const uint4 *)zb;
+            *(uint4 *)(H + umma::sw128_offset(row, c0 + j, 128)) = *(const uint4 *)hb;
+          }
+        }
+        publish();
+        if (threadIdx.x == 0) store_tile(tm.X_out[l + 1], kSurHid / 64, tile);
+      }
+    }
+    if (!ok) break;
+
+    // --- head: mu and s are summed column by column in each half (groups 0, 1
+    // and 2, 3), the second group of a half going on where the first ended ---
+    float mu = 0.0f, s = 0.0f;
+    for (int pass = 0; pass < 2; ++pass) {
+      if ((grp & 1) == pass) {
+        if (pass) {
+          mu = s_head[grp - 1][row][0];
+          s = s_head[grp - 1][row][1];
+        }
+        for (int c0 = grp * kTrainCols; c0 < (grp + 1) * kTrainCols; c0 += 32) {
+          float v[32];
+          umma::tmem_ld32(trow + c0, v);
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            __align__(16) bf16 hb[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+              const float h = silu(v[j + t] + s_bias[kSurLayers - 1][c0 + j + t]);
+              hb[t] = __float2bfloat16_rn(h);
+              mu = fmaf(h, s_wh[0][c0 + j + t], mu);
+              s = fmaf(h, s_wh[1][c0 + j + t], s);
+            }
+            *(uint4 *)(H + umma::sw128_offset(row, c0 + j, 128)) = *(const uint4 *)hb;
+          }
+        }
+        s_head[grp][row][0] = mu;
+        s_head[grp][row][1] = s;
+      }
+      publish();
+    }
+    if (threadIdx.x == 0) {  // the head's input, for its gradients; read before dZ replaces it
+      store_tile(tm.X_out[kSurLayers], kSurHid / 64, tile);
+      umma::bulk_wait_read();
+    }
+    if (grp == 1) {
+      mu = s_head[1][row][0] + s_head[3][row][0] + s_bh[0];
+      s = s_head[1][row][1] + s_head[3][row][1] + s_bh[1];
+      s = fminf(fmaxf(s, -12.0f), 4.0f);
+      const float r = mu - s_y[row];
+      const float e2 = __expf(-2.0f * s);
+      // mean squared error on mu; the error head learns log |mu - y| (Gaussian
+      // negative log-likelihood with mu held fixed), weighted by lambda_s
+      const float dmu = r * a.inv_batch;
+      const float ds = a.lambda_s * (1.0f - e2 * r * r) * a.inv_batch;
+      const int64_t m = tile * 128 + row;
+      *(float2 *)(a.pred + 2 * m) = make_float2(mu, s);
+      a.loss[m] = 0.5f * r * r;
+      s_dp[row][0] = dmu;
+      s_dp[row][1] = ds;
+      a.dpred[m] = make_float2(dmu, ds);
+    }
+    __syncthreads();
+    {  // dZ of the last layer
+      const float dmu = s_dp[row][0], ds = s_dp[row][1];
+      for (int c0 = grp * kTrainCols; c0 < (grp + 1) * kTrainCols; c0 += 32) {
+        float v[32];
+        umma::tmem_ld32(trow + c0, v);
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          __align__(16) bf16 gb[8];
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+            const float dh = dmu * s_wh[0][c0 + j + t] + ds * s_wh[1][c0 + j + t];
+            gb[t] = __float2bfloat16_rn(dh * silu_grad(v[j + t] + s_bias[kSurLayers - 1][c0 + j + t]));
+          }
+          *(uint4 *)(H + umma::sw128_offset(row, c0 + j, 128)) = *(const uint4 *)gb;
+        }
+      }
+    }
+    publish();
+    if (threadIdx.x == 0) store_tile(tm.dZ_out[kSurLayers - 1], kSurHid / 64, tile);
+
+    // --- backward: dZ_{l-1} = (dZ_l W_l) SiLU'(z_{l-1}) ---
+    for (int l = kSurLayers - 1; l > 0; --l) {
+      if (threadIdx.x == 0) {
+        if (l < kSurLayers - 1 && !weights_in()) {
+          s_abort = 1;
+        } else {
+          umma::tc_fence_after();
+          for (int k = 0; k < 16; ++k)
+            umma::mma_bf16(tmem, umma::sdesc_sw128(umma::smem_u32(H + (k >> 2) * 16 * 1024) + 32u * (k & 3)),
+                           umma::sdesc_sw128_mn(umma::smem_u32(Wsm) + 2048u * k, 32 * 1024), id_bwd, k != 0 ? 1u : 0u);
+        }
+        umma::mma_commit(umma::smem_u32(&mbar));
+        umma::bulk_wait_read();
+      }
+      uint4 zq[kTrainCols / 8];  // in flight while the MMAs run
+#pragma unroll
+      for (int c = 0; c < kTrainCols / 8; ++c) zq[c] = zt[((l - 1) * (kTrainCols / 8) + c) * kTrainThreads];
+      if (!mma_done()) break;
+      if (threadIdx.x == 0) {
+        if (l > 1) load_w(l - 1);
+        else if (tile + gridDim.x < ntiles) load_w(0);
+      }
+#pragma unroll
+      for (int h = 0; h < kTrainCols / 32; ++h) {
+        const int c0 = grp * kTrainCols + 32 * h;
+        float v[32];
+        umma::tmem_ld32(trow + c0, v);
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          const bf16 *zb = (const bf16 *)&zq[4 * h + j / 8];
+          __align__(16) bf16 gb[8];
+#pragma unroll
+          for (int t = 0; t < 8; ++t)
+            gb[t] = __float2bfloat16_rn(v[j + t] * silu_grad(__bfloat162float(zb[t])));
+          *(uint4 *)(H + umma::sw128_offset(row, c0 + j, 128)) = *(const uint4 *)gb;
+        }
+      }
+      publish();
+      if (threadIdx.x == 0) store_tile(tm.dZ_out[l - 1], kSurHid / 64, tile);
+    }
+  }
+  if (threadIdx.x == 0) {
+    if (!ok) {
+      atomicCAS(a.error, 0, kErrWait);
+      if (w_pending) umma::mbar_wait(umma::smem_u32(&wbar), wph, kWaitNs);  // let a load in flight land
+    }
+    umma::bulk_wait();
+  }
+  umma::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) umma::tmem_free(tmem, 256);
+}
+
+// Weight gradients of one piece of the batch: block (item, piece) computes rows
+// 128 h .. +127 and `width` columns of dZ_l^T X_l over the piece's rows, both
+// operands MN-major tiles of 32 rows loaded by TMA (4-stage ring). Two blocks
+// per SM (96 KB and 256 TMEM columns each), so that one's stores run under the
+// other's MMAs.
+// The piece's sums go to memory as float4s in the order of the threads, which
+// the update kernel reads back coalesced. The pieces are the longest equal
+// ones that divide the batch into at most 64 of at least 512 rows (an odd
+// number of rows / 128 divides into few or none); where that leaves SMs idle
+// the columns are split too.
+constexpr int kWgradThreads = 256, kWgradStages = 4, kWgradRows = 32;
+constexpr uint32_t kWgradBox = kWgradRows * 128u;  // 64 columns of a stage's rows
+constexpr uint32_t kWgradStage = (2u + 4u) * kWgradBox;
+constexpr uint32_t kWgradSmem = kWgradStages * kWgradStage + 1024u;
+// floats of a piece: the weights of row half h of layer l from wgrad_offset(2 l + h)
+constexpr int64_t kPiece = (int64_t)kSurHid * (kSurEnc + 3 * kSurHid);
+__host__ __device__ constexpr int64_t wgrad_offset(int lh) {
+  return lh < 2 ? (int64_t)lh * 128 * kSurEnc : (int64_t)kSurHid * kSurEnc + (int64_t)(lh - 2) * 128 * kSurHid;
+}
+__host__ __device__ constexpr int wgrad_items(int width) {
+  return 2 * (width < kSurEnc ? kSurEnc / width : 1) + 6 * (kSurHid / width);
+}
+
+__global__ void __launch_bounds__(kWgradThreads, 2)
+    mlp_wgrad_kernel(const __grid_constant__ TrainMaps tm, int width, int per, float *partial, int *error) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = align1024(smem_raw);
+  __shared__ __align__(8) uint64_t full[kWgradStages], empty[kWgradStages], done;
+  __shared__ uint32_t tmem_base;
+  __shared__ int s_abort;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // item: (layer, column slice, row half), the first layer's first
+  const int n0 = 2 * (width < kSurEnc ? kSurEnc / width : 1), per_layer = 2 * (kSurHid / width);
+  const int x = blockIdx.x, l = x < n0 ? 0 : 1 + (x - n0) / per_layer;
+  const int in_layer = l == 0 ? x : (x - n0) % per_layer, h = in_layer & 1;
+  const int N = min(width, SurParamLayout::in_dim(l)), col0 = (in_layer >> 1) * N;
+  const int kb0 = blockIdx.y * per, nk = per;  // blocks of kWgradRows rows
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kWgradStages; ++s) {
       umma::mbar_init(umma::smem_u32(&full[s]), 1);
       umma::mbar_init(umma::smem_u32(&empty[s]), 1);
     }
@@ -131,288 +457,242 @@ __global__ void __launch_bounds__(256, 1)
   const uint32_t tmem = tmem_base;
 
   if (threadIdx.x == 0) {
-    umma::tma_prefetch_desc(&tA);
-    umma::tma_prefetch_desc(&tB);
-    const uint32_t idesc = umma::idesc_bf16_f32(128, N);
+    const uint32_t idesc = umma::idesc_bf16_f32(128, N, true, true);
+    const uint32_t bytes = (2u + (uint32_t)(N / 64)) * kWgradBox;
     auto load = [&](int s, int kb) {
-      const uint32_t sa = umma::smem_u32(smem + (size_t)s * stage_bytes), bar = umma::smem_u32(&full[s]);
-      umma::mbar_expect_tx(bar, stage_bytes);
-      umma::tma_load_2d(sa, &tA, bar, (kb0 + kb) * 64, m0);
-      umma::tma_load_2d(sa + a_bytes, &tB, bar, (kb0 + kb) * 64, 0);
+      const uint32_t sa = umma::smem_u32(smem + s * kWgradStage), bar = umma::smem_u32(&full[s]);
+      const int r = (kb0 + kb) * kWgradRows;
+      umma::mbar_expect_tx(bar, bytes);
+      for (int c = 0; c < 2; ++c) umma::tma_load_2d(sa + c * kWgradBox, &tm.dZ_in[l], bar, h * 128 + c * 64, r);
+      for (int c = 0; c < N / 64; ++c) umma::tma_load_2d(sa + (2 + c) * kWgradBox, &tm.X_in[l], bar, col0 + c * 64, r);
     };
     int loaded = 0;
-    for (int s = 0; s < kStages && s < nk; ++s, ++loaded) load(s, s);
+    for (; loaded < kWgradStages && loaded < nk; ++loaded) load(loaded, loaded);
     bool ok = true;
-    for (int kb = 0; kb < nk && ok; ++kb) {
-      const int s = kb % kStages;
-      if (!umma::mbar_wait(umma::smem_u32(&full[s]), (uint32_t)((kb / kStages) & 1), kWaitNs)) {
+    for (int kb = 0; kb < nk; ++kb) {
+      const int s = kb % kWgradStages;
+      if (!umma::mbar_wait(umma::smem_u32(&full[s]), (uint32_t)((kb / kWgradStages) & 1), kWaitNs)) {
         ok = false;
         break;
       }
       umma::tc_fence_after();
-      const uint32_t sa = umma::smem_u32(smem + (size_t)s * stage_bytes), sb = sa + a_bytes;
+      const uint32_t sa = umma::smem_u32(smem + s * kWgradStage), sb = sa + 2u * kWgradBox;
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        umma::mma_bf16(tmem, umma::sdesc_sw128(sa + 32u * k), umma::sdesc_sw128(sb + 32u * k), idesc,
-                       (kb | k) != 0 ? 1u : 0u);
+      for (int k = 0; k < kWgradRows / 16; ++k)
+        umma::mma_bf16(tmem, umma::sdesc_sw128_mn(sa + 2048u * k, kWgradBox),
+                       umma::sdesc_sw128_mn(sb + 2048u * k, kWgradBox), idesc, (kb | k) != 0 ? 1u : 0u);
       umma::mma_commit(umma::smem_u32(&empty[s]));
-      // refill the stage of the previous K block (its MMAs were issued one iteration earlier)
-      const int kr = kb - 1 + kStages;
-      if (kb >= 1 && kr < nk) {
-        const int sp = (kb - 1) % kStages;
-        if (!umma::mbar_wait(umma::smem_u32(&empty[sp]), (uint32_t)(((kb - 1) / kStages) & 1), kWaitNs)) {
+      // refill the stage of the previous block (its MMAs were issued one iteration earlier)
+      if (kb >= 1 && loaded < nk) {
+        const int sp = (kb - 1) % kWgradStages;
+        if (!umma::mbar_wait(umma::smem_u32(&empty[sp]), (uint32_t)(((kb - 1) / kWgradStages) & 1), kWaitNs)) {
           ok = false;
           break;
         }
-        load(sp, kr);
-        ++loaded;
+        load(sp, loaded++);
       }
     }
     if (!ok) {
       s_abort = 1;
-      atomicCAS(a.error, 0, kErrWait);
+      atomicCAS(error, 0, kErrWait);
       // let every load still in flight land before the block exits
       for (int kb = 0; kb < loaded; ++kb)
-        umma::mbar_wait(umma::smem_u32(&full[kb % kStages]), (uint32_t)((kb / kStages) & 1), kWaitNs);
+        umma::mbar_wait(umma::smem_u32(&full[kb % kWgradStages]), (uint32_t)((kb / kWgradStages) & 1), kWaitNs);
     }
-    umma::mma_commit(umma::smem_u32(&done));  // arrives once every MMA issued above has completed
+    umma::mma_commit(umma::smem_u32(&done));
   }
   const bool done_ok = umma::mbar_wait(umma::smem_u32(&done), 0, kWaitNs);
   const bool all_ok = __syncthreads_and(done_ok ? 1 : 0) != 0;
-  if (!done_ok) atomicCAS(a.error, 0, kErrWait);
+  if (!done_ok) atomicCAS(error, 0, kErrWait);
   umma::tc_fence_after();
-
   if (all_ok && !s_abort) {
-    const int q = warp & 3, half = warp >> 2;
-    const int row = q * 32 + lane, m = m0 + row;
+    const int q = warp & 3, half = warp >> 2, row = q * 32 + lane;
     const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
-    const int cols = N / 2, cbeg = half * cols;
-    if (EPI == kEpiPartial) {
-      float *dst = a.partial + ((size_t)blockIdx.z * a.M + m) * N;
-      for (int c0 = cbeg; c0 < cbeg + cols; c0 += 32) {
-        float v[32];
-        umma::tmem_ld32(trow + c0, v);
+    float4 *w = (float4 *)(partial + (int64_t)blockIdx.y * kPiece + wgrad_offset(2 * l + h));
+    for (int c0 = half * (N / 2); c0 < (half + 1) * (N / 2); c0 += 32) {
+      float v[32];
+      umma::tmem_ld32(trow + c0, v);
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) *(float4 *)(dst + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-      }
-    } else if (EPI == kEpiFwd) {
-      for (int c0 = cbeg; c0 < cbeg + cols; c0 += 32) {
-        float v[32];
-        umma::tmem_ld32(trow + c0, v);
-        __align__(16) bf16 zb[32], hb[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float z = v[j] + a.bias[c0 + j];
-          const float h = silu(z);
-          zb[j] = __float2bfloat16_rn(z);
-          hb[j] = __float2bfloat16_rn(h);
-          a.out_t[(size_t)(c0 + j) * a.M + m] = hb[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-          *(uint4 *)(a.z_row + (size_t)m * N + c0 + j) = *(const uint4 *)&zb[j];
-          *(uint4 *)(a.out_row + (size_t)m * N + c0 + j) = *(const uint4 *)&hb[j];
-        }
-      }
-    } else if (EPI == kEpiBwd) {
-      for (int c0 = cbeg; c0 < cbeg + cols; c0 += 32) {
-        float v[32];
-        umma::tmem_ld32(trow + c0, v);
-        __align__(16) bf16 zb[32], gb[32];
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) *(uint4 *)&zb[j] = *(const uint4 *)(a.z_in + (size_t)m * N + c0 + j);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          gb[j] = __float2bfloat16_rn(v[j] * silu_grad(__bfloat162float(zb[j])));
-          a.out_t[(size_t)(c0 + j) * a.M + m] = gb[j];
-        }
-        if (a.out_row) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) *(uint4 *)(a.out_row + (size_t)m * N + c0 + j) = *(const uint4 *)&gb[j];
-        }
-      }
-    } else {  // kEpiHead: last hidden layer, FP32 head, loss gradients, then dZ of this layer
-      float mu = 0.0f, s = 0.0f;
-      for (int c0 = cbeg; c0 < cbeg + cols; c0 += 32) {
-        float v[32];
-        umma::tmem_ld32(trow + c0, v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float h = silu(v[j] + a.bias[c0 + j]);
-          a.head_t[(size_t)(c0 + j) * a.M + m] = __float2bfloat16_rn(h);
-          mu = fmaf(h, a.Wh[c0 + j], mu);
-          s = fmaf(h, a.Wh[N + c0 + j], s);
-        }
-      }
-      s_head[half][row][0] = mu;
-      s_head[half][row][1] = s;
-      __syncthreads();
-      mu = s_head[0][row][0] + s_head[1][row][0] + a.bh[0];
-      s = s_head[0][row][1] + s_head[1][row][1] + a.bh[1];
-      s = fminf(fmaxf(s, -12.0f), 4.0f);
-      const float y = a.target[m];
-      const float r = mu - y;
-      const float e2 = __expf(-2.0f * s);
-      // mean squared error on mu; the error head learns log |mu - y| (Gaussian
-      // negative log-likelihood with mu held fixed), weighted by lambda_s
-      const float dmu = r * a.inv_batch;
-      const float ds = a.lambda_s * (1.0f - e2 * r * r) * a.inv_batch;
-      if (half == 0) {
-        a.pred[2 * (size_t)m] = mu;
-        a.pred[2 * (size_t)m + 1] = s;
-        a.dpred[2 * (size_t)m] = dmu;
-        a.dpred[2 * (size_t)m + 1] = ds;
-        a.loss[m] = 0.5f * r * r;
-      }
-      for (int c0 = cbeg; c0 < cbeg + cols; c0 += 32) {
-        float v[32];
-        umma::tmem_ld32(trow + c0, v);
-        __align__(16) bf16 gb[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float dh = dmu * a.Wh[c0 + j] + ds * a.Wh[N + c0 + j];
-          gb[j] = __float2bfloat16_rn(dh * silu_grad(v[j] + a.bias[c0 + j]));
-          a.out_t[(size_t)(c0 + j) * a.M + m] = gb[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) *(uint4 *)(a.out_row + (size_t)m * N + c0 + j) = *(const uint4 *)&gb[j];
-      }
+      for (int j = 0; j < 32; j += 4)
+        w[((col0 + c0 + j) / 4) * 128 + row] = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     }
   }
   umma::tc_fence_before();
   __syncthreads();
   if (warp == 0) umma::tmem_free(tmem, 256);
+  umma::wait_prerequisites();  // the update kernel, next in the stream, needs the chains too
 }
 
-}  // namespace sur
-}  // namespace amca
-
-namespace amca {
-namespace sur {
-
-// ---------------------------------------------------------------------------
-// Training helpers
-// ---------------------------------------------------------------------------
-
-// E[m][0..127] and its transpose from raw inputs (rows past n are zero).
-__global__ void encode_kernel(SurModelDev md, const float *raw, int64_t n, int64_t M, bf16 *E, bf16 *Et) {
-  const int64_t total = M * kSurFreq;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = q / kSurFreq;
-    const int j = (int)(q % kSurFreq);
-    float sv = 0.0f, cv = 0.0f;
-    if (m < n) {
-      float r[kSurIn];
-#pragma unroll
-      for (int i = 0; i < kSurIn; ++i) r[i] = raw[m * kSurIn + i];
-      phases(md, r, j, sv, cv);
-    }
-    const bf16 s = __float2bfloat16_rn(sv), c = __float2bfloat16_rn(cv);
-    E[m * kSurEnc + j] = s;
-    E[m * kSurEnc + kSurFreq + j] = c;
-    Et[(int64_t)j * M + m] = s;
-    Et[(int64_t)(kSurFreq + j) * M + m] = c;
-  }
-}
-
-// out[r] = sum over the `splits` partials of element r; a deterministic
-// split-K reduction.
-__global__ void reduce_partials_kernel(const float *partial, int splits, int64_t count, float *out) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < count; r += (int64_t)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += partial[(int64_t)z * count + r];
-    out[r] = s;
-  }
-}
-
-// out[r] = sum_m X[r][m] for a [rows x M] bf16 matrix (bias gradients from the
-// transposed dZ); one block per row, fixed reduction order.
-__global__ void row_sum_kernel(const bf16 *X, int64_t M, float *out) {
-  __shared__ float red[256];
-  const bf16 *x = X + (int64_t)blockIdx.x * M;
-  float s = 0.0f;
-  for (int64_t m = threadIdx.x; m < M; m += blockDim.x) s += __bfloat162float(x[m]);
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[blockIdx.x] = red[0];
-}
-
-// Head gradients: gWh[j][c] = sum_m dpred[m][j] H[c][m], gbh[j] = sum_m dpred[m][j];
-// one block per column c (plus one block for the biases).
-__global__ void head_grad_kernel(const bf16 *Ht, const float *dpred, int64_t M, int N, float *gWh, float *gbh) {
-  __shared__ float red[2][256];
-  const int c = blockIdx.x;
-  float s0 = 0.0f, s1 = 0.0f;
-  for (int64_t m = threadIdx.x; m < M; m += blockDim.x) {
-    const float h = c < N ? __bfloat162float(Ht[(int64_t)c * M + m]) : 1.0f;
-    s0 += dpred[2 * m] * h;
-    s1 += dpred[2 * m + 1] * h;
-  }
-  red[0][threadIdx.x] = s0;
-  red[1][threadIdx.x] = s1;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      red[0][threadIdx.x] += red[0][threadIdx.x + w];
-      red[1][threadIdx.x] += red[1][threadIdx.x + w];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    if (c < N) {
-      gWh[c] = red[0][0];
-      gWh[N + c] = red[1][0];
-    } else {
-      gbh[0] = red[0][0];
-      gbh[1] = red[1][0];
-    }
-  }
-}
-
-// Adam step over every parameter; refreshes the bf16 copies ([out][in] and,
-// for layers 1.., the transposed [in][out] copy the backward GEMMs read).
-struct AdamArgs {
-  float *p, *m, *v;
-  const float *g;
+// Column sums of the batch in 256 interleaved chains: chain t of column c adds
+// rows t, t + 256, t + 512, ... in order. Sets 0..3 are the bias gradients
+// (the rows of dZ_l), 4 and 5 the head's (rows of its input times dL/dmu and
+// dL/ds), and the head's own biases (dL/dmu, dL/ds themselves) go to chainb.
+// The update kernel adds the chains pairwise, t and t + 128 first. A thread has
+// four columns, a warp 256 bytes of a row; 64 blocks a matrix read the batch
+// once, most of it from L2 (one block per column over a transposed copy
+// before).
+constexpr int kChains = 256, kChainSets = kSurLayers + kSurOut, kChainThreads = 256, kChainCols = 4;
+struct ChainArgs {
+  const bf16 *dZ[kSurLayers], *H;
+  const float2 *dpred;
   int64_t n;
-  float lr, beta1, beta2, eps, bc1, bc2;
-  bf16 *Wb[kSurLayers], *Wtb[kSurLayers];
-  int64_t Woff[kSurLayers];
+  float *chain;   // [kChainSets][kChains][kSurHid]
+  float *chainb;  // [kChains][kSurOut]
 };
 
-__device__ __forceinline__ void store_bf16_copies(const AdamArgs &a, int64_t i, float p) {
+constexpr int kChainBatch = 16;  // rows whose loads are in flight before any is added
+
+__global__ void __launch_bounds__(kChainThreads) mlp_chain_kernel(ChainArgs a) {
+  umma::launch_dependents();  // the weight gradients need nothing of this kernel
+  constexpr int per_row = kSurHid / kChainCols;  // threads on one row
+  const int t = blockIdx.x * (kChainThreads / per_row) + threadIdx.x / per_row;
+  const int c = threadIdx.x % per_row * kChainCols;
+  const int set = blockIdx.y;
+  const bool head = set == kSurLayers;
+  const bf16 *src = (head ? a.H : set == 0 ? a.dZ[0] : set == 1 ? a.dZ[1] : set == 2 ? a.dZ[2] : a.dZ[3]) + c;
+  float s0[kChainCols] = {}, s1[kChainCols] = {}, b0 = 0.0f, b1 = 0.0f;
+  for (int64_t m0 = t; m0 < a.n; m0 += kChains * kChainBatch) {
+    uint2 u[kChainBatch];
+    float2 d[kChainBatch];
 #pragma unroll
-  for (int l = 0; l < kSurLayers; ++l) {
-    const int K = SurParamLayout::in_dim(l);
-    const int64_t o = i - a.Woff[l];
-    if (o >= 0 && o < (int64_t)kSurHid * K) {
-      a.Wb[l][o] = __float2bfloat16_rn(p);
-      if (a.Wtb[l]) a.Wtb[l][(o % K) * kSurHid + o / K] = __float2bfloat16_rn(p);
+    for (int k = 0; k < kChainBatch; ++k) {
+      const int64_t m = m0 + k * kChains;
+      u[k] = m < a.n ? *(const uint2 *)(src + m * kSurHid) : make_uint2(0u, 0u);
     }
+    if (head) {
+#pragma unroll
+      for (int k = 0; k < kChainBatch; ++k) {
+        const int64_t m = m0 + k * kChains;
+        d[k] = m < a.n ? a.dpred[m] : make_float2(0.0f, 0.0f);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kChainBatch; ++k) {
+      if (m0 + k * kChains >= a.n) break;
+      const __nv_bfloat162 *b = (const __nv_bfloat162 *)&u[k];
+      const float h[kChainCols] = {__low2float(b[0]), __high2float(b[0]), __low2float(b[1]), __high2float(b[1])};
+      if (!head) {
+#pragma unroll
+        for (int i = 0; i < kChainCols; ++i) s0[i] += h[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < kChainCols; ++i) {
+          s0[i] += d[k].x * h[i];
+          s1[i] += d[k].y * h[i];
+        }
+        b0 += d[k].x;
+        b1 += d[k].y;
+      }
+    }
+  }
+  float *out = a.chain + ((int64_t)set * kChains + t) * kSurHid + c;
+  *(float4 *)out = make_float4(s0[0], s0[1], s0[2], s0[3]);
+  if (head) {
+    *(float4 *)(out + kChains * kSurHid) = make_float4(s1[0], s1[1], s1[2], s1[3]);
+    if (c == 0) *(float2 *)(a.chainb + kSurOut * t) = make_float2(b0, b1);
   }
 }
 
-__global__ void adam_kernel(AdamArgs a) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float g = a.g[i];
-    const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * g;
-    const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * g * g;
-    a.m[i] = m;
-    a.v[i] = v;
-    const float p = a.p[i] - a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
-    a.p[i] = p;
-    store_bf16_copies(a, i, p);
+// Gradients summed over the pieces in order, or from the chains. ADAM: then the
+// parameter's Adam step and its bf16 copy; otherwise the gradient is stored.
+// The first kWeightBlocks blocks have two weights per thread, the
+// others 32 columns of a chain set (the last one the head's biases). Bound by
+// reading the pieces (59 MB at 64 of them).
+struct AdamArgs {
+  float *p, *m, *v, *g;
+  float lr, beta1, beta2, eps, bc1, bc2;
+  bf16 *Wb[kSurLayers];
+};
+
+template <bool ADAM>
+__device__ __forceinline__ float update_param(const AdamArgs &a, int64_t i, float g) {
+  if (!ADAM) {
+    a.g[i] = g;
+    return 0.0f;
   }
+  const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * g;
+  const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * g * g;
+  a.m[i] = m;
+  a.v[i] = v;
+  const float p = a.p[i] - a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
+  a.p[i] = p;
+  return p;
+}
+
+constexpr int kUpdateThreads = 256;
+constexpr int kWeightBlocks = (int)(kPiece / 2 / kUpdateThreads);
+constexpr int kUpdateBlocks = kWeightBlocks + kChainSets * kSurHid / 32 + 1;
+static_assert(kPiece % (2 * kUpdateThreads) == 0, "whole blocks of weights");
+
+// x[t] + x[t + 128], then + 64, ... + 8: the pairwise sum of the 32 chains
+// t = w, w + 8, w + 16, ... (i-th value: t = w + 8 i)
+template <int N>
+__device__ __forceinline__ float pair_sum(const float *x) {
+  if constexpr (N == 32) return x[0];
+  else return pair_sum<2 * N>(x) + pair_sum<2 * N>(x + N);
+}
+
+template <bool ADAM>
+__global__ void __launch_bounds__(kUpdateThreads)
+    mlp_update_kernel(AdamArgs a, const float *partial, int pieces, const float *chain, const float *chainb) {
+  umma::launch_dependents();  // the next step's blocks set up meanwhile
+  const SurParamLayout L;
+  if (blockIdx.x < kWeightBlocks) {
+    const int i = blockIdx.x * kUpdateThreads + threadIdx.x;
+    const float2 *src = (const float2 *)partial + i;
+    float2 s = make_float2(0.0f, 0.0f);
+    for (int z0 = 0; z0 < pieces; z0 += 16) {
+      float2 q[16];
+#pragma unroll
+      for (int z = 0; z < 16; ++z)
+        q[z] = z0 + z < pieces ? __ldcs(src + (z0 + z) * (kPiece / 2)) : make_float2(0.0f, 0.0f);
+#pragma unroll
+      for (int z = 0; z < 16; ++z) {
+        if (z0 + z >= pieces) break;
+        s.x += q[z].x;
+        s.y += q[z].y;
+      }
+    }
+    int lh = 0;
+    while (lh + 1 < 2 * kSurLayers && 2 * i >= wgrad_offset(lh + 1)) ++lh;
+    const int l = lh >> 1, K = l == 0 ? kSurEnc : kSurHid;
+    const int o = 2 * i - (int)wgrad_offset(lh);  // ((column / 4) * 128 + row) * 4 + column % 4
+    const int at = ((lh & 1) * 128 + (o >> 2) % 128) * K + (o >> 9) * 4 + (o & 3);
+    const int64_t first = l == 0 ? 0 : L.W[1] + (l - 1) * (L.W[2] - L.W[1]);
+    const float px = update_param<ADAM>(a, first + at, s.x), py = update_param<ADAM>(a, first + at + 1, s.y);
+    if (ADAM) {
+      bf16 *wb = l == 0 ? a.Wb[0] : l == 1 ? a.Wb[1] : l == 2 ? a.Wb[2] : a.Wb[3];
+      *(__nv_bfloat162 *)(wb + at) = __floats2bfloat162_rn(px, py);
+    }
+    return;
+  }
+  __shared__ float red[8][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = (blockIdx.x - kWeightBlocks) * 32 + lane;  // column of all chain sets
+  const bool last = blockIdx.x == kUpdateBlocks - 1;
+  const int set = j / kSurHid, c = j % kSurHid;
+  const float *src = last ? chainb + lane : chain + (int64_t)set * kChains * kSurHid + c;
+  const int stride = last ? kSurOut : kSurHid;
+  float x[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) x[i] = !last || lane < kSurOut ? src[(w + 8 * i) * stride] : 0.0f;
+  red[w][lane] = pair_sum<1>(x);
+  __syncthreads();
+  if (w != 0 || (last && lane >= kSurOut)) return;
+  const float g = ((red[0][lane] + red[4][lane]) + (red[2][lane] + red[6][lane])) +
+                  ((red[1][lane] + red[5][lane]) + (red[3][lane] + red[7][lane]));
+  update_param<ADAM>(a, last ? L.bh + lane : set < kSurLayers ? L.b[0] + c + (set ? L.b[1] - L.b[0] + (set - 1) * (L.b[2] - L.b[1]) : 0)
+                                                             : L.Wh + (set - kSurLayers) * kSurHid + c, g);
 }
 
 // bf16 copies of every layer's weights from the master parameters.
 __global__ void refresh_bf16_kernel(AdamArgs a) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x)
-    store_bf16_copies(a, i, a.p[i]);
+  const SurParamLayout L;
+  for (int l = 0; l < kSurLayers; ++l) {
+    const int64_t n = (int64_t)kSurHid * SurParamLayout::in_dim(l);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+      a.Wb[l][i] = __float2bfloat16_rn(a.p[L.W[l] + i]);
+  }
 }
 
 // acc[0] += sum of loss[0..n)
@@ -489,18 +769,6 @@ __global__ void make_data_kernel(DataSpec ds, int64_t first, int64_t n, float *r
     raw[q * kSurIn + 4] = (float)s.speed;
     const double yv = (T - ds.t_shift) / ds.t_scale;
     target[q] = (float)(ds.log_out ? log(yv) : yv);
-  }
-}
-
-// Batch rows from the data set through an affine permutation:
-// row q = data[(start + q) * perm_a mod n], perm_a coprime to n.
-__global__ void gather_batch_kernel(const float *raw, const float *target, int64_t nsamples, int64_t start, int64_t nb,
-                                    uint64_t perm_a, float *braw, float *btarget) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nb; q += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t i = (uint64_t)(((unsigned __int128)(uint64_t)(start + q) * perm_a) % (uint64_t)nsamples);
-#pragma unroll
-    for (int k = 0; k < kSurIn; ++k) braw[q * kSurIn + k] = raw[i * kSurIn + k];
-    btarget[q] = target[i];
   }
 }
 
@@ -904,19 +1172,26 @@ CUtensorMap tmap_bf16(const void *base, int64_t rows, int64_t cols, int box_rows
   return m;
 }
 
-template <int EPI>
-void launch_gemm(const CUtensorMap &tA, const CUtensorMap &tB, GemmArgs a, int splits, cudaStream_t s) {
-  const size_t smem = (size_t)kStages * (16384 + (size_t)a.N * 128) + 1024;
-  SCK(cudaFuncSetAttribute(mlp_gemm_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (a.M % 128 || (a.N != 128 && a.N != 256) || a.K % (64 * splits))
-    throw std::invalid_argument("layer GEMM: M must be a multiple of 128, N 128 or 256, K a multiple of 64 x splits");
-  a.kb_per_split = a.K / 64 / splits;
-  mlp_gemm_kernel<EPI><<<dim3(a.M / 128, 1, splits), 256, smem, s>>>(tA, tB, a);
-  SCK(cudaGetLastError());
-}
-
 int grid_1d(int64_t n, int threads = 256) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads, 152 * 16));
+}
+
+// A launch whose blocks may start while the kernel before it in the stream
+// still runs (once all of its blocks have let them: launch_dependents); it
+// waits by itself (wait_prerequisites) before it needs that kernel's results.
+template <typename... P, typename... A>
+void launch_early(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  SCK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
 }
 
 uint64_t gcd64(uint64_t a, uint64_t b) {
@@ -942,7 +1217,7 @@ struct ThermalModel {
   float in_shift[kSurIn], in_scale[kSurIn], t_shift = 0, t_scale = 1;
   // device
   float *fourier = nullptr, *p = nullptr, *m1 = nullptr, *m2 = nullptr, *g = nullptr;
-  bf16 *Wb[kSurLayers] = {}, *Wtb[kSurLayers] = {};
+  bf16 *Wb[kSurLayers] = {};
   int *err = nullptr;
   unsigned long long *counters = nullptr;
   float *ds_raw = nullptr, *ds_target = nullptr;
@@ -951,12 +1226,13 @@ struct ThermalModel {
   int64_t seen = 0;
   // batch buffers
   int64_t nb = 0;
-  int splits = 1;
-  float *braw = nullptr, *by = nullptr, *pred = nullptr, *dpred = nullptr, *loss = nullptr, *partial = nullptr;
-  bf16 *E = nullptr, *Et = nullptr, *Z[kSurLayers] = {}, *Hr[kSurLayers] = {}, *Ht[kSurLayers + 1] = {};
-  bf16 *dZ[kSurLayers] = {}, *dZt[kSurLayers] = {};
-  CUtensorMap tmA_fwd[kSurLayers], tmB_fwd[kSurLayers], tmA_dw[kSurLayers], tmB_dw[kSurLayers], tmA_dh[kSurLayers],
-      tmB_dh[kSurLayers];
+  int blocks = 0;                        // of the step kernel
+  int pieces = 0, per = 0, width = 256;  // of the weight gradients: pieces, their kWgradRows-row blocks, column slice
+  float *braw = nullptr, *by = nullptr, *pred = nullptr, *loss = nullptr, *partial = nullptr;
+  sur::ChainArgs chains;
+  float2 *dpred = nullptr;
+  uint4 *zs = nullptr;
+  sur::TrainMaps maps;
   std::vector<void *> allocs, batch_allocs;
 
   template <typename T>
@@ -1000,12 +1276,7 @@ struct ThermalModel {
     a.m = m1;
     a.v = m2;
     a.g = g;
-    a.n = L.total;
-    for (int l = 0; l < kSurLayers; ++l) {
-      a.Wb[l] = Wb[l];
-      a.Wtb[l] = Wtb[l];
-      a.Woff[l] = L.W[l];
-    }
+    for (int l = 0; l < kSurLayers; ++l) a.Wb[l] = Wb[l];
     return a;
   }
   void check_error() {
@@ -1062,8 +1333,9 @@ struct ThermalModel {
     for (int l = 0; l < kSurLayers; ++l) {
       const int K = SurParamLayout::in_dim(l);
       Wb[l] = alloc<bf16>((size_t)kSurHid * K);
-      if (l > 0) Wtb[l] = alloc<bf16>((size_t)kSurHid * K);
     }
+    SCK(cudaFuncSetAttribute(sur::mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sur::kTrainSmem));
+    SCK(cudaFuncSetAttribute(sur::mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sur::kWgradSmem));
     err = alloc<int>(1);
     counters = alloc<unsigned long long>(4);
     SCK(cudaMemcpyAsync(fourier, fourier_h, sizeof fourier_h, cudaMemcpyHostToDevice, stream));
@@ -1094,105 +1366,73 @@ struct ThermalModel {
     batch_allocs.clear();
     nb = 0;
     const int64_t kblocks = n / 64;
-    // split-K of the weight-gradient GEMMs: at most 64 splits of at least 8 K blocks
-    splits = 1;
-    while (splits < 64 && kblocks % (splits * 2) == 0 && kblocks / (splits * 2) >= 8) splits *= 2;
+    // pieces of the weight gradients: at most 64, of at least 8 blocks of 64 rows each, all alike
+    pieces = 1;
+    while (pieces < 64 && kblocks % (pieces * 2) == 0 && kblocks / (pieces * 2) >= 8) pieces *= 2;
+    per = (int)(n / sur::kWgradRows / pieces);
+    int sms = 0;
+    SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    width = kSurHid;
+    while (width > 64 && sur::wgrad_items(width) * pieces < sms) width /= 2;
+    blocks = (int)std::min<int64_t>(n / 128, sms);
     braw = balloc<float>((size_t)n * kSurIn);
     by = balloc<float>((size_t)n);
     pred = balloc<float>((size_t)n * 2);
-    dpred = balloc<float>((size_t)n * 2);
     loss = balloc<float>((size_t)n);
-    partial = balloc<float>((size_t)splits * kSurHid * kSurHid);
-    E = balloc<bf16>((size_t)n * kSurEnc);
-    Et = balloc<bf16>((size_t)n * kSurEnc);
-    Ht[0] = Et;
-    for (int l = 0; l < kSurLayers; ++l) {
-      Z[l] = balloc<bf16>((size_t)n * kSurHid);
-      Hr[l] = balloc<bf16>((size_t)n * kSurHid);  // Hr[l] = H_{l+1} rows
-      Ht[l + 1] = balloc<bf16>((size_t)n * kSurHid);
-      dZ[l] = balloc<bf16>((size_t)n * kSurHid);
-      dZt[l] = balloc<bf16>((size_t)n * kSurHid);
-    }
+    dpred = balloc<float2>((size_t)n);
+    partial = balloc<float>((size_t)pieces * sur::kPiece);
+    zs = balloc<uint4>((size_t)n / 128 * 3 * (sur::kTrainCols / 8) * sur::kTrainThreads);
     for (int l = 0; l < kSurLayers; ++l) {
       const int K = SurParamLayout::in_dim(l);
-      // forward: A = layer input rows [n x K], B = W_l [256 x K]
-      tmA_fwd[l] = sur::tmap_bf16(l == 0 ? (const void *)E : (const void *)Hr[l - 1], n, K, 128);
-      tmB_fwd[l] = sur::tmap_bf16(Wb[l], kSurHid, K, 256);
-      // weight gradient: A = dZ_l^T [256 x n], B = input^T [K x n]
-      tmA_dw[l] = sur::tmap_bf16(dZt[l], kSurHid, n, 128);
-      tmB_dw[l] = sur::tmap_bf16(Ht[l], K, n, K);
-      // input gradient (l >= 1): A = dZ_l [n x 256], B = W_l^T [K x 256]
-      if (l > 0) {
-        tmA_dh[l] = sur::tmap_bf16(dZ[l], n, kSurHid, 128);
-        tmB_dh[l] = sur::tmap_bf16(Wtb[l], K, kSurHid, 256);
-      }
+      const bf16 *X = balloc<bf16>((size_t)n * K), *dZ = balloc<bf16>((size_t)n * kSurHid);
+      chains.dZ[l] = dZ;
+      maps.W[l] = sur::tmap_bf16(Wb[l], kSurHid, K, 256);
+      maps.X_out[l] = sur::tmap_bf16(X, n, K, 128);
+      maps.X_in[l] = sur::tmap_bf16(X, n, K, sur::kWgradRows);
+      maps.dZ_out[l] = sur::tmap_bf16(dZ, n, kSurHid, 128);
+      maps.dZ_in[l] = sur::tmap_bf16(dZ, n, kSurHid, sur::kWgradRows);
     }
+    chains.H = balloc<bf16>((size_t)n * kSurHid);
+    maps.X_out[kSurLayers] = sur::tmap_bf16(chains.H, n, kSurHid, 128);
+    chains.dpred = dpred;
+    chains.n = n;
+    chains.chain = balloc<float>((size_t)sur::kChainSets * sur::kChains * kSurHid);
+    chains.chainb = balloc<float>((size_t)sur::kChains * kSurOut);
     nb = n;
   }
 
-  // Forward and backward over the batch in braw / by; gradients into g.
-  void forward_backward() {
+  // Forward and backward over the nb rows that are samples (start + q) * perm
+  // mod nsamples, q = 0.., of raw / target; the gradients' pieces are left for
+  // update().
+  void forward_backward(const float *raw, const float *target, int64_t nsamples, int64_t start, uint64_t perm) {
     using namespace sur;
-    const int64_t n = nb;
-    const SurModelDev md = dev();
-    SCK(cudaMemsetAsync(err, 0, sizeof(int), stream));
-    encode_kernel<<<grid_1d(n * kSurFreq), 256, 0, stream>>>(md, braw, n, n, E, Et);
+    StepArgs a{};
+    a.n = nb;
+    a.raw = raw;
+    a.target = target;
+    a.nsamples = (uint64_t)nsamples;
+    a.start = (uint64_t)start;
+    a.perm = perm;
+    a.zs = zs;
+    a.pred = pred;
+    a.loss = loss;
+    a.dpred = dpred;
+    a.inv_batch = 1.0f / (float)nb;
+    a.lambda_s = 0.1f;
+    a.error = err;
+    launch_early(mlp_step_kernel, dim3(blocks), kTrainThreads, kTrainSmem, stream, maps, dev(), a);
+    mlp_chain_kernel<<<dim3(kChains * (kSurHid / kChainCols) / kChainThreads, kSurLayers + 1), kChainThreads, 0, stream>>>(
+        chains);
     SCK(cudaGetLastError());
-    for (int l = 0; l < kSurLayers; ++l) {
-      GemmArgs a{};
-      a.M = (int)n;
-      a.N = kSurHid;
-      a.K = SurParamLayout::in_dim(l);
-      a.bias = p + L.b[l];
-      a.error = err;
-      if (l < kSurLayers - 1) {
-        a.z_row = Z[l];
-        a.out_row = Hr[l];
-        a.out_t = Ht[l + 1];
-        launch_gemm<kEpiFwd>(tmA_fwd[l], tmB_fwd[l], a, 1, stream);
-      } else {
-        a.head_t = Ht[l + 1];
-        a.out_row = dZ[l];
-        a.out_t = dZt[l];
-        a.Wh = p + L.Wh;
-        a.bh = p + L.bh;
-        a.target = by;
-        a.pred = pred;
-        a.dpred = dpred;
-        a.loss = loss;
-        a.inv_batch = 1.0f / (float)n;
-        a.lambda_s = 0.1f;
-        launch_gemm<kEpiHead>(tmA_fwd[l], tmB_fwd[l], a, 1, stream);
-      }
-    }
-    head_grad_kernel<<<kSurHid + 1, 256, 0, stream>>>(Ht[kSurLayers], dpred, n, kSurHid, g + L.Wh, g + L.bh);
+    launch_early(mlp_wgrad_kernel, dim3(wgrad_items(width), pieces), kWgradThreads, kWgradSmem, stream, maps, width, per,
+                 partial, err);
+  }
+
+  // The summed gradients into g.
+  void gradients() {
+    sur::mlp_update_kernel<false><<<sur::kUpdateBlocks, sur::kUpdateThreads, 0, stream>>>(adam_args(), partial, pieces,
+                                                                                         chains.chain, chains.chainb);
     SCK(cudaGetLastError());
-    for (int l = kSurLayers - 1; l >= 0; --l) {
-      const int K = SurParamLayout::in_dim(l);
-      row_sum_kernel<<<kSurHid, 256, 0, stream>>>(dZt[l], n, g + L.b[l]);
-      SCK(cudaGetLastError());
-      GemmArgs w{};
-      w.M = kSurHid;
-      w.N = K;
-      w.K = (int)n;
-      w.partial = partial;
-      w.error = err;
-      launch_gemm<kEpiPartial>(tmA_dw[l], tmB_dw[l], w, splits, stream);
-      reduce_partials_kernel<<<grid_1d((int64_t)kSurHid * K), 256, 0, stream>>>(partial, splits,
-                                                                                 (int64_t)kSurHid * K, g + L.W[l]);
-      SCK(cudaGetLastError());
-      if (l > 0) {
-        GemmArgs b{};
-        b.M = (int)n;
-        b.N = K;
-        b.K = kSurHid;
-        b.z_in = Z[l - 1];
-        b.out_row = l > 1 ? dZ[l - 1] : nullptr;
-        b.out_t = dZt[l - 1];
-        b.error = err;
-        launch_gemm<kEpiBwd>(tmA_dh[l], tmB_dh[l], b, 1, stream);
-      }
-    }
   }
 
   void adam(float lr) {
@@ -1204,7 +1444,8 @@ struct ThermalModel {
     a.eps = 1e-8f;
     a.bc1 = (float)(1.0 - std::pow(0.9, (double)adam_t));
     a.bc2 = (float)(1.0 - std::pow(0.999, (double)adam_t));
-    sur::adam_kernel<<<sur::grid_1d(L.total), 256, 0, stream>>>(a);
+    sur::mlp_update_kernel<true><<<sur::kUpdateBlocks, sur::kUpdateThreads, 0, stream>>>(a, partial, pieces,
+                                                                                        chains.chain, chains.chainb);
     SCK(cudaGetLastError());
   }
 
@@ -1424,16 +1665,14 @@ int amca_thermal_train(amca_thermal *h, int64_t samples, int steps, int batch, d
     DeviceBuffers tmp;
     double *acc = (double *)tmp.get(2 * sizeof(double));
     SCK(cudaMemsetAsync(acc, 0, 2 * sizeof(double), m.stream));
+    SCK(cudaMemsetAsync(m.err, 0, sizeof(int), m.stream));
     const int edge = std::max(1, steps / 20);
     const int warm = std::max(1, steps / 50);
     SCK(cudaStreamSynchronize(m.stream));
     const auto t0 = std::chrono::steady_clock::now();
     for (int s = 0; s < steps; ++s) {
-      amca::sur::gather_batch_kernel<<<amca::sur::grid_1d(m.nb), 256, 0, m.stream>>>(
-          m.ds_raw, m.ds_target, m.ds_n, m.seen % m.ds_n, m.nb, a, m.braw, m.by);
-      SCK(cudaGetLastError());
+      m.forward_backward(m.ds_raw, m.ds_target, m.ds_n, m.seen % m.ds_n, a);
       m.seen += m.nb;
-      m.forward_backward();
       const double frac = s < warm ? (double)(s + 1) / warm : (double)(s - warm) / std::max(1, steps - warm);
       const double lr = s < warm ? lr_max * frac : lr_min + 0.5 * (lr_max - lr_min) * (1.0 + std::cos(M_PI * frac));
       m.adam((float)lr);
@@ -1501,7 +1740,9 @@ int amca_thermal_gradients(amca_thermal *h, const float *raw, const float *targe
     m.set_batch(n);
     SCK(cudaMemcpyAsync(m.braw, raw, (size_t)n * amca::kSurIn * 4, cudaMemcpyHostToDevice, m.stream));
     SCK(cudaMemcpyAsync(m.by, target, (size_t)n * 4, cudaMemcpyHostToDevice, m.stream));
-    m.forward_backward();
+    SCK(cudaMemsetAsync(m.err, 0, sizeof(int), m.stream));
+    m.forward_backward(m.braw, m.by, n, 0, 1);
+    m.gradients();
     SCK(cudaMemcpyAsync(grad, m.g, (size_t)m.L.total * 4, cudaMemcpyDeviceToHost, m.stream));
     if (pred) SCK(cudaMemcpyAsync(pred, m.pred, (size_t)n * 2 * 4, cudaMemcpyDeviceToHost, m.stream));
     SCK(cudaStreamSynchronize(m.stream));

@@ -23,6 +23,11 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
+// Programmatic dependent launch: lets the next kernel of the stream start its
+// blocks; waits until the kernels before this one have completed.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- mbarrier -------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -68,6 +73,18 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, uint
       : "memory");
 }
 
+// 2-D tiled store of a shared-memory box to (x = inner coordinate, y = row);
+// part of this thread's current bulk group.
+__device__ __forceinline__ void tma_store_2d(const void *tmap, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"((uint64_t)tmap),
+               "r"(x), "r"(y), "r"(src)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// every committed bulk store of this thread has read its shared memory / has completed
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 __device__ __forceinline__ void tma_prefetch_desc(const void *tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)tmap) : "memory");
 }
@@ -105,11 +122,27 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr) {
   return d;
 }
 
+// Descriptor of an MN-major operand (its M or N index contiguous in memory, K
+// the row index) in the same tiles: 64 M/N elements per 128-byte row, one row
+// per K index. A K step of 16 starts 2048 bytes (16 rows) after the previous
+// one; the 8-row groups of a step lie 1024 bytes apart (stride offset, bits
+// 32-45) and the next 64 M/N elements `block_bytes` further on (leading offset,
+// bits 16-29).
+__device__ __forceinline__ uint64_t sdesc_sw128_mn(uint32_t saddr, uint32_t block_bytes) {
+  uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)(block_bytes >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
 // Instruction descriptor of tcgen05.mma.kind::f16: D in FP32 (bits 4-5 = 1),
-// A and B bf16 (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0),
-// N >> 3 in bits 17-22, M >> 4 in bits 24-28.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// A and B bf16 (bits 7-9 = 1, 10-12 = 1), A MN-major in bit 15, B MN-major in
+// bit 16 (0: K-major), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool a_mn = false, bool b_mn = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u) |
+         ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // ---- MMA ------------------------------------------------------------------

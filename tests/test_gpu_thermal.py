@@ -236,3 +236,32 @@ def test_model_frames_equal_the_model_at_the_window_nodes(A, cells, tracks, f0, 
         assert np.array_equal(got[k], want.ravel()), (k, f0 + k)
     assert counts[0] == total
     m.close()
+
+
+@pytest.mark.parametrize("n", [128, 1152, 4224, 19584])
+def test_gradients_at_the_edges_of_the_batch_pieces(A, n):
+    """One tile; two pieces of nine 64-row blocks; pieces of which the last is short; one tile more than the GPU's
+    152 blocks take at once. Against the restatement with the same bf16 rounding points, within the bounds of
+    test_gradients_match_the_fp64_restatement (bf16 has 8 bits: 2^-9 a value, and flips of roundings between
+    layers)."""
+    spec = decks.thermal_spec()
+    m = A.ThermalModel(**spec)
+    p = m.params().astype(np.float64)
+    raw = window_inputs(spec, n, seed=n)
+    y = fe_target(spec, raw).astype(np.float32)
+    g, pred = m.gradients(raw, y)
+    g_ref, mu, s, _ = TO.forward_backward(p, raw, y.astype(np.float64), enc_of(m), bf16_points=True)
+    assert np.max(np.abs(pred[:, 0] - mu)) < 2e-2 * max(1.0, np.max(np.abs(mu)))
+    assert np.max(np.abs(pred[:, 1] - s)) < 2e-2 * max(1.0, np.max(np.abs(s)))
+    for k, (o, shp) in TO.layout().items():
+        sz = int(np.prod(shp))
+        a, b = g[o:o + sz].astype(np.float64), g_ref[o:o + sz]
+        rel = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)
+        assert rel < 3e-2, (k, rel)
+    # a step of training is Adam on the same sums: with the batch's own samples drawn in the set's order every
+    # parameter moves by at most the learning rate (Adam's first step is lr * g / (|g| + eps)), against its gradient
+    before = m.params()
+    m.train(samples=n, steps=1, batch=n, lr_max=1e-3, lr_min=1e-3)
+    moved = m.params() - before
+    assert np.max(np.abs(moved)) <= 1e-3 * (1 + 1e-4) + 1e-7 and np.mean(np.abs(moved) > 0.9e-3) > 0.5
+    m.close()
