@@ -54,9 +54,124 @@ struct Grid {
   double x0, y0, z0, h;
 };
 
-// get_cell_center: x0 + h*(I - 0.5) with the ghost-inclusive index I.
-AMCA_HD double centre_coord(double o, double h, int I) { return o + h * (I - 0.5); }
+// FP64 on GB300: an FP64 instruction (arithmetic, comparison or conversion)
+// holds a warp's scheduler for about 64 cycles however many lanes take part
+// (divide: 560), against 1 for an integer or FP32 one. The helpers below do
+// exact FP64 bookkeeping with integer operations on the bits instead; all of
+// them return what the FP64 operation named in their comment returns.
+AMCA_HD long long f64_bits(double x) {
+#if defined(__CUDA_ARCH__)
+  return __double_as_longlong(x);
+#else
+  long long b;
+  memcpy(&b, &x, sizeof b);
+  return b;
+#endif
+}
+AMCA_HD double bits_f64(long long b) {
+#if defined(__CUDA_ARCH__)
+  return __longlong_as_double(b);
+#else
+  double x;
+  memcpy(&x, &b, sizeof x);
+  return x;
+#endif
+}
+AMCA_HD uint32_t f32_bits(float x) {
+#if defined(__CUDA_ARCH__)
+  return __float_as_uint(x);
+#else
+  uint32_t b;
+  memcpy(&b, &x, sizeof b);
+  return b;
+#endif
+}
+AMCA_HD float bits_f32(uint32_t b) {
+#if defined(__CUDA_ARCH__)
+  return __uint_as_float(b);
+#else
+  float x;
+  memcpy(&x, &b, sizeof x);
+  return x;
+#endif
+}
+AMCA_HD int f64_exponent(double x) { return (int)((unsigned long long)f64_bits(x) >> 52) & 0x7ff; }  // biased
 
+// (double)I - 0.5: a double near 1.5 * 2^51 has a unit of 0.5, so its low bits
+// count half cells; one subtraction instead of a conversion and one.
+AMCA_HD double cells_minus_half(int I) { return bits_f64(0x4328000000000000ll + 2ll * I) - 3377699720527872.5; }
+
+// get_cell_center: x0 + h*(I - 0.5) with the ghost-inclusive index I.
+AMCA_HD double centre_coord(double o, double h, int I) { return o + h * cells_minus_half(I); }
+
+// x rounded to float towards zero (within 2^-23 of x): x is 0 or normal as a
+// float, or rounds as the conversion does.
+AMCA_HD float f64_to_f32_rz(double x) {
+  const unsigned long long b = (unsigned long long)f64_bits(x);
+  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+  if (e - 897u < 253u)
+    return bits_f32((uint32_t)(b >> 32 & 0x80000000u) | ((uint32_t)(b >> 29) - (896u << 23) & 0x7fffffffu));
+  return (b << 1) == 0 ? 0.0f : (float)x;
+}
+// (float)x for x whose float is positive and normal with room to round up
+AMCA_HD float pos_f64_to_f32_rn(double x) {
+  const unsigned long long b = (unsigned long long)f64_bits(x);
+  return bits_f32((uint32_t)((b + 0x0fffffffull + (b >> 29 & 1ull)) >> 29) - (896u << 23));
+}
+// (double)x for x positive and normal
+AMCA_HD double pos_f32_to_f64(float x) {
+  return bits_f64(((long long)f32_bits(x) << 29) + (896ll << 52));
+}
+// x < y; neither is NaN, nor are they zeros of different signs
+AMCA_HD bool f64_less(double x, double y) {
+  const long long a = f64_bits(x), b = f64_bits(y);
+  return (a ^ (a >> 63 & 0x7fffffffffffffffll)) < (b ^ (b >> 63 & 0x7fffffffffffffffll));
+}
+// 0.5 * x, exact unless x is subnormal or the smallest normal
+AMCA_HD double f64_half(double x) {
+  if (f64_exponent(x) - 2u < 0x7fcu) return bits_f64(f64_bits(x) - (1ll << 52));
+  return 0.5 * x;
+}
+AMCA_HD double f64_fma(double a, double b, double c) {
+#if defined(__CUDA_ARCH__)
+  return __fma_rn(a, b, c);
+#else
+  return fma(a, b, c);
+#endif
+}
+
+// x / 3, correctly rounded (the quotient-correction step of P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990): y = RN(1/3) is within 2^-54 relative of 1/3, so q0 = RN(x y) is within
+// 1 ulp of x/3, the residual x - 3 q0 is exact, and q0 plus residual * y differs
+// from x/3 by less than 2^-50 ulp, while no x/3 lies nearer than 1/6 ulp to a
+// rounding midpoint. x is 0 or its exponent leaves room for the residual.
+AMCA_HD double f64_third(double x) {
+  const double y = 0x1.5555555555555p-2;
+  const double q = x * y;
+  return f64_fma(f64_fma(-3.0, q, x), y, q);
+}
+// y within 2^-46 relative of 1 / b for a double b that holds a float: one
+// Newton step from the FP32 reciprocal.
+AMCA_HD double recip_of_f32(float b, double bd) {
+  const double y0 = pos_f32_to_f64(1.0f / b);
+  return f64_fma(y0, f64_fma(-bd, y0, 1.0), y0);
+}
+// x / b, correctly rounded, for that b and y: q0 is within 2^-46 of x / b, so
+// the residual has under 32 significant bits and is exact, and q0 + residual *
+// y is within 2^-92 of x / b; b has 24 bits, so no x / b lies within 2^-78
+// relative of a rounding midpoint. x is 0 or its exponent leaves room.
+AMCA_HD double div_by_f32(double x, double bd, double y) {
+  const double q = x * y;
+  return f64_fma(f64_fma(-bd, q, x), y, q);
+}
+
+AMCA_HD void cell_ijk(const Grid &g, int32_t id, int &I, int &J, int &K) {
+  K = id / g.nxyg;
+  const int r = id - K * g.nxyg;
+  J = r / g.nxg;
+  I = r - J * g.nxg;
+}
 AMCA_HD void cell_ijk(const Grid &g, int64_t id, int &I, int &J, int &K) {
   K = (int)(id / g.nxyg);
   int r = (int)(id - (int64_t)K * g.nxyg);
@@ -151,19 +266,6 @@ AMCA_HD int corner_axis(int c) { return c < 4 ? (c & 1) : 2; }
 AMCA_HD double dmin_ref(double a, double b) { return (b < a) ? b : a; }  // std::min
 AMCA_HD double dmax_ref(double a, double b) { return (a < b) ? b : a; }  // std::max
 
-// Octahedron::capture_cell: the new, decentred envelope for a captured cell.
-// gc = cell centre - parent centre (FP64). Writes the new centre offset
-// (global frame) into out[0..2] and the new half-diagonal into out[3].
-// Helpers that keep exact FP64 bookkeeping off the narrow FP64 pipe.
-AMCA_HD long long f64_bits(double x) {
-#if defined(__CUDA_ARCH__)
-  return __double_as_longlong(x);
-#else
-  long long b;
-  memcpy(&b, &x, sizeof b);
-  return b;
-#endif
-}
 // plus_zero(x) == x + 0.0 (a zero of either sign becomes +0).
 AMCA_HD double plus_zero(double x) {
   const long long b = f64_bits(x);
@@ -183,7 +285,7 @@ AMCA_HD double corner_length(int c, double length) { return (c == 2 || c == 3 ||
 // taken as sign flips; every such rewrite is bit-identical: a sum accumulated
 // from +0.0 does not depend on the signs of its zero terms (+0 + -0 = +0,
 // x + -0 = x), and squares and products of zeros are zeros.
-AMCA_HD void capture_f64(const double *l2g, double gcx, double gcy, double gcz, double length, double h,
+AMCA_HD void capture_f64_general(const double *l2g, double gcx, double gcy, double gcz, double length, double h,
                          double trunc_coeff, double out[4]) {
   double cx = plus_zero(gcx * l2g[0]);  // 0 + p
   double cy = plus_zero(gcx * l2g[1]);
@@ -283,6 +385,101 @@ AMCA_HD void capture_f64(const double *l2g, double gcx, double gcy, double gcz, 
   // (mag * c_i) / (length * T) for the corner S1 = c: non-zero on S1's axis
   // only; the rotated offset o_k = sum_i comp_i * l2g[i + 3k] is that term + 0
   const double comp = mag * c1v / (length * kTheodorus);
+  out[0] = plus_zero(comp * l2g[a0 + 0]);
+  out[1] = plus_zero(comp * l2g[a0 + 3]);
+  out[2] = plus_zero(comp * l2g[a0 + 6]);
+  out[3] = Lnew;
+}
+
+// The face quadrant of a point (the signs of its components, -0 positive).
+AMCA_HD int quadrant(double cx, double cy, double cz) {
+  const bool px = nonneg(cx), py = nonneg(cy);
+  const int q = px ? (py ? 0 : 3) : (py ? 1 : 2);
+  return nonneg(cz) ? q : q + 4;
+}
+
+#if defined(__CUDA_ARCH__)
+__device__ __noinline__ inline void capture_f64_slow(const double *l2g, double gcx, double gcy, double gcz,
+                                                     double length, double h, double trunc_coeff, double out[4]) {
+  capture_f64_general(l2g, gcx, gcy, gcz, length, h, trunc_coeff, out);
+}
+#else
+inline void capture_f64_slow(const double *l2g, double gcx, double gcy, double gcz, double length, double h,
+                             double trunc_coeff, double out[4]) {
+  capture_f64_general(l2g, gcx, gcy, gcz, length, h, trunc_coeff, out);
+}
+#endif
+
+// Octahedron::capture_cell: the new, decentred envelope for a captured cell.
+// gc = cell centre - parent centre (FP64). Writes the new centre offset
+// (global frame) into out[0..2] and the new half-diagonal into out[3].
+//
+// capture_f64_general with fewer FP64 instructions (about 60 instead of 140;
+// they are what a claim phase with new envelopes spends its time on), the same
+// bits in every case. Beyond the helpers above:
+//  - the corners in order of distance: dist_i - dist_j = 2 L (|pA_j| - |pA_i|)
+//    up to 2^-46 L^2 of rounding (each corner lies on the side of its axis that
+//    pA is on), so FP32 magnitudes that differ by more than 2^-19 L order them;
+//  - the edge products share S1A's term, and a sum of two terms accumulated
+//    from +0.0 is plus_zero of one plus the other in either order;
+//  - both edge quotients divide by the same n12, a float.
+// A point outside the envelope, corners too near a tie and magnitudes near the
+// ends of the exponent range go the general way.
+AMCA_HD void capture_f64(const double *l2g, double gcx, double gcy, double gcz, double length, double h,
+                         double trunc_coeff, double out[4]) {
+  double c[3];
+  for (int i = 0; i < 3; ++i) c[i] = (plus_zero(gcx * l2g[i]) + gcy * l2g[3 + i]) + gcz * l2g[6 + i];
+  const double interception = fabs(c[0]) + fabs(c[1]) + fabs(c[2]);
+  const int quad = quadrant(c[0], c[1], c[2]);
+  const double perp = length - interception;
+  const int ep = f64_exponent(perp), el = f64_exponent(length);
+  // lengths between 2^-50 and 2^50; perp positive (or +0) and not vanishing
+  bool general = el - 973u > 100u || f64_bits(perp) < 0 || (ep < 400 && f64_bits(perp) != 0);
+  const double third = f64_third(perp);
+  double pA[3];
+  for (int i = 0; i < 3; i++) pA[i] = c[i] + (nonneg(c[i]) ? third : -third);  // the face normal's signs are c's
+  float m[3];  // |pA|
+  for (int i = 0; i < 3; ++i) m[i] = fabsf(f64_to_f32_rz(pA[i]));
+  const float tie = 1.9073486328125e-06f * f64_to_f32_rz(length);  // 2^-19 L
+  // as the reference: corner 0 against 1, then the nearer of them against 2
+  const int k0 = face_corner(quad, 0), k1 = face_corner(quad, 1), k2 = face_corner(quad, 2);
+  const float f0 = corner_axis(k0) == 0 ? m[0] : m[1], f1 = corner_axis(k1) == 0 ? m[0] : m[1], f2 = m[2];
+  general = general || !(fabsf(f0 - f1) > tie);
+  int cid0 = f0 < f1 ? k1 : k0, cid1 = f0 < f1 ? k0 : k1, cid2 = k2;
+  const float near01 = f0 < f1 ? f1 : f0;
+  general = general || !(fabsf(near01 - f2) > tie);
+  if (near01 < f2) {
+    cid2 = cid0;
+    cid0 = k2;
+  }
+  const int a0 = corner_axis(cid0), a1 = corner_axis(cid1), a2 = corner_axis(cid2);
+  const double p0 = a0 == 0 ? pA[0] : (a0 == 1 ? pA[1] : pA[2]);
+  const double p1 = a1 == 0 ? pA[0] : (a1 == 1 ? pA[1] : pA[2]);
+  const double p2 = a2 == 0 ? pA[0] : (a2 == 1 ? pA[1] : pA[2]);
+  const double c1v = corner_length(cid0, length);  // S1 on its axis
+  const double t0 = plus_zero((p0 - c1v) * -c1v);
+  const double d12 = t0 + p1 * corner_length(cid1, length), d13 = t0 + p2 * corner_length(cid2, length);
+  const int e12 = f64_exponent(d12), e13 = f64_exponent(d13);
+  general = general || (e12 < 400 && (f64_bits(d12) << 1) != 0) || (e13 < 400 && (f64_bits(d13) << 1) != 0);
+  if (general) {
+    capture_f64_slow(l2g, gcx, gcy, gcz, length, h, trunc_coeff, out);
+    return;
+  }
+  const float n12f = sqrtf(pos_f64_to_f32_rn(bits_f64(f64_bits(length * length) + (1ll << 52))));
+  const double n12 = pos_f32_to_f64(n12f);
+  const double y = recip_of_f32(n12f, n12);
+  double I0 = div_by_f32(d12, n12, y), I1 = n12 - I0;
+  const double J0 = div_by_f32(d13, n12, y), J1 = n12 - J0;
+  const double tv = trunc_coeff * h;
+  if (f64_less(I0, tv) && f64_less(I1, tv)) {
+    I0 = f64_half(n12);  // == n12 / 2
+    I1 = I0;
+  }
+  const double s1 = (f64_less(tv, I0) ? tv : I0) + (f64_less(tv, I1) ? tv : I1);
+  const double s2 = (f64_less(tv, J0) ? tv : J0) + (f64_less(tv, J1) ? tv : J1);
+  const double L1 = f64_half(s1), L2 = f64_half(s2);
+  const double Lnew = (double)sqrtf(2.0f) * (f64_less(L1, L2) ? L2 : L1);
+  const double comp = (length - Lnew) * c1v / (length * kTheodorus);
   out[0] = plus_zero(comp * l2g[a0 + 0]);
   out[1] = plus_zero(comp * l2g[a0 + 3]);
   out[2] = plus_zero(comp * l2g[a0 + 6]);

@@ -465,12 +465,21 @@ __device__ __forceinline__ uint32_t liquid_neighbours(const uint32_t *solid, con
 // ---------------------------------------------------------------------------
 // The envelope list: wake keys, grown half-diagonals, liquid counts.
 // ---------------------------------------------------------------------------
+// x rounded down to float, by the bits where the float is normal (an FP64
+// conversion holds the scheduler for 64 cycles).
+__device__ __forceinline__ float f64_to_f32_rd(double x) {
+  if ((unsigned)f64_exponent(x) - 897u >= 253u) return f64_bits(x) == 0 ? 0.0f : __double2float_rd(x);
+  const float z = f64_to_f32_rz(x);
+  // below zero, down is away from it, unless nothing was dropped
+  return f64_bits(x) < 0 && (f64_bits(x) & 0x1fffffff) != 0 ? bits_f32(f32_bits(z) + 1u) : z;
+}
+
 // Whether an entry with wake key k is processed in a step whose cumulative
 // growth is `grown` (all: every live entry, to bring its record up to date).
 // Dead entries (NaN) never are. The test (double)k <= grown is made in FP32
 // (the FP64 pipe is narrow), exactly: for a float k it holds iff k is at most
 // grown rounded down to float, gf.
-__device__ __forceinline__ float wake_bound(double grown) { return __double2float_rd(grown); }
+__device__ __forceinline__ float wake_bound(double grown) { return f64_to_f32_rd(grown); }
 __device__ __forceinline__ bool woken(float k, float gf, bool all) { return all ? !isnan(k) : k <= gf; }
 
 // Wake key: the cumulative growth at which the half-diagonal L (grown up to
@@ -478,12 +487,11 @@ __device__ __forceinline__ bool woken(float k, float gf, bool all) { return all 
 // L), every rounding downwards, less 2^-30 of the magnitudes involved (L is
 // at most grown plus a few cells), which covers the rounding of the FP64 step
 // sums over the at most kWakeAll steps before the entry is looked at again
-// by a factor of thousands. One FP64 subtraction and one conversion; the rest
-// in FP32. +inf when no liquid neighbour is left. Waking early only costs a
-// test.
+// by a factor of thousands. One FP64 subtraction; the rest in FP32. +inf when
+// no liquid neighbour is left. Waking early only costs a test.
 __device__ __forceinline__ float wake_key(float t_lb, double L, double grown, float gf) {
   if (!(t_lb < INFINITY)) return INFINITY;
-  const float o = __double2float_rd(grown - L);
+  const float o = f64_to_f32_rd(grown - L);
   const float slack = 9.313225746154785e-10f * (fabsf(t_lb) + fabsf(o) + 2.0f * gf);
   return __fsub_rd(__fadd_rd(t_lb, o), slack);
 }
@@ -491,7 +499,15 @@ __device__ __forceinline__ float wake_key(float t_lb, double L, double grown, fl
 // Grain::grow (Grain.h:27) of the steps (from, to]: the same FP64 additions
 // of each step's dt * vel, in order.
 __device__ __forceinline__ double replay_growth(const double *dvh, double L, long long from, long long to) {
-  for (long long t = from + 1; t <= to; ++t) L += dvh[t & (kDvRing - 1)];
+  // eight increments loaded at once: the loads do not wait for the additions
+  for (long long t = from + 1; t <= to; t += 8) {
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = t + j <= to ? dvh[(t + j) & (kDvRing - 1)] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (t + j <= to) L += v[j];
+  }
   return L;
 }
 
@@ -968,9 +984,9 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
       gyd = out[1] + py;
       gzd = out[2] + pz;
       en.L = out[3];
-      en.dx = (float)(gxd - ccx);
-      en.dy = (float)(gyd - ccy);
-      en.dz = (float)(gzd - ccz);
+      en.dx = f64_to_f32_rz(gxd - ccx);  // the pre-test's error bound covers 2^-21 of it
+      en.dy = f64_to_f32_rz(gyd - ccy);
+      en.dz = f64_to_f32_rz(gzd - ccz);
       have_centre = true;
       act[p] = en;
       lstep[p] = (int32_t)step;
@@ -995,7 +1011,7 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
       cell_ijk(g, cell, I, J, K);
       const float dxf = en.dx, dyf = en.dy, dzf = en.dz;
       const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(dxf) + fabsf(dyf) + fabsf(dzf)) + d.coord_err;
-      const float L32 = (float)L;
+      const float L32 = f64_to_f32_rz(L);  // the pre-test's margin is 2^-14 of it
       float m32[9];
 #pragma unroll
       for (int q = 0; q < 9; ++q) m32[q] = __ldg(d.omat32 + 9 * ori + q);
@@ -1509,7 +1525,7 @@ __device__ __forceinline__ void init_field_word(uint32_t *orient, uint32_t *soli
     bool ghost = true;
     if (i < ncells) {
       int I, J, K;
-      cell_ijk(g, i, I, J, K);
+      cell_ijk(g, (int64_t)i, I, J, K);
       ghost = I == 0 || J == 0 || K == 0 || I == g.nxg - 1 || J == g.nyg - 1 || K == g.nzg - 1;
       orient[i] = ghost ? 0u : kLiquid;
       cellw[i] = kNoEntry;
@@ -1622,7 +1638,7 @@ __global__ void batch_gather_kernel(const PlainDevice *insts, int ninst, PlainCt
 __global__ void grain_field_init_kernel(int32_t *out, const uint32_t *orient, Grid g, long long ncells) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ncells; i += (long long)gridDim.x * blockDim.x) {
     int I, J, K;
-    cell_ijk(g, i, I, J, K);
+    cell_ijk(g, (int64_t)i, I, J, K);
     const bool ghost = I == 0 || J == 0 || K == 0 || I == g.nxg - 1 || J == g.nyg - 1 || K == g.nzg - 1;
     out[i] = ghost ? 0 : -1;
   }

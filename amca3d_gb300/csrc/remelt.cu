@@ -1534,7 +1534,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
       const int32_t mine = INT_MIN + sweep_pos(g, I, J, K);
       const float dxf = p.dx, dyf = p.dy, dzf = p.dz;
       const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(dxf) + fabsf(dyf) + fabsf(dzf)) + d.coord_err;
-      const float L32 = (float)L;
+      const float L32 = f64_to_f32_rz(L);  // the pre-test's margin is 2^-14 of it
       const float *m32 = p.m32;
       uint32_t cand = p.cand;
       while (cand) {
@@ -1635,9 +1635,9 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
           d.gz[nb] = nz;
           d.glen[nb] = out[3];
           d.gori[nb] = ori;
-          d.gdx[nb] = (float)(nx - ccx);
-          d.gdy[nb] = (float)(ny - ccy);
-          d.gdz[nb] = (float)(nz - ccz);
+          d.gdx[nb] = f64_to_f32_rz(nx - ccx);  // the pre-test's error bound covers 2^-21 of it
+          d.gdy[nb] = f64_to_f32_rz(ny - ccy);
+          d.gdz[nb] = f64_to_f32_rz(nz - ccz);
           if (d.grain[nb] < 0) {  // create_new_grain: id in sweep order after the step
             d.grain[nb] = kPendingGrain;
             const int di = I - wi, dj = J - wj, dk = K - wk;

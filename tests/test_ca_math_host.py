@@ -33,3 +33,15 @@ def test_ca_math_matches_reference_octahedron():
         out = subprocess.run([exe, data], check=True, capture_output=True, text=True).stdout.split()
     total, caps, bad = map(int, out)
     assert total == n and caps == int(k["captured"].sum()) and bad == 0
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_capture_equals_the_general_path_and_helpers_the_fp64_operations(tmp_path):
+    """Ordinary captures, zeros and ties, near ties, lengths over the exponent range and points on the surface:
+    capture_f64 returns capture_f64_general's bits; each helper its FP64 operation's."""
+    exe = str(tmp_path / "paths")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", os.path.join(HERE, "capture_paths.cpp"), "-o", exe],
+                   check=True)
+    out = subprocess.run([exe, "200000", "7"], check=True, capture_output=True, text=True).stdout.split("\n")
+    rows = [line.split() for line in out if line]
+    assert len(rows) == 13 and all(int(n) == 200000 and int(wrong) == 0 for _, n, wrong in rows), rows
