@@ -47,10 +47,25 @@ AMCA_HD bool is_liquid_now(uint32_t s, uint32_t parity) {
   return s == kLiquid || ((s & kClaimBit) && (((s & kParityBit) != 0) == (parity != 0)));
 }
 
+// n / d for 0 <= n < 2^31 as (n * mul) >> shift: with s = ceil(log2 d) and
+// mul = ceil(2^(31+s) / d), mul * d exceeds 2^(31+s) by less than d <= 2^s, so
+// n * mul / 2^(31+s) exceeds n / d by less than 1 / d.
+struct FastDiv {
+  uint32_t mul;
+  int shift;
+};
+inline FastDiv fast_div(int d) {
+  int s = 0;
+  while ((1ll << s) < d) ++s;
+  return {(uint32_t)(((1ull << (31 + s)) + (unsigned)d - 1) / (unsigned)d), 31 + s};
+}
+AMCA_HD int quotient(int n, FastDiv f) { return (int)(((uint64_t)(uint32_t)n * f.mul) >> f.shift); }
+
 struct Grid {
   int nx, ny, nz;     // interior cells
   int nxg, nyg, nzg;  // with the ghost layer
   int nxyg;
+  FastDiv by_x, by_xy;  // of nxg, nxyg
   double x0, y0, z0, h;
 };
 
@@ -167,9 +182,9 @@ AMCA_HD double div_by_f32(double x, double bd, double y) {
 }
 
 AMCA_HD void cell_ijk(const Grid &g, int32_t id, int &I, int &J, int &K) {
-  K = id / g.nxyg;
+  K = quotient(id, g.by_xy);
   const int r = id - K * g.nxyg;
-  J = r / g.nxg;
+  J = quotient(r, g.by_x);
   I = r - J * g.nxg;
 }
 AMCA_HD void cell_ijk(const Grid &g, int64_t id, int &I, int &J, int &K) {

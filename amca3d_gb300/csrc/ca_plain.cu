@@ -18,9 +18,9 @@
 //             capture this step; the others are not read. Their half-diagonal
 //             is brought up to date when they wake, by replaying the step
 //             increments from a ring, the same FP64 sums in the same order.
-//   deaths  : each entry keeps the count of its liquid neighbours; nucleation
-//             and captures decrement the counts of the entries around the
-//             cell. A sleeping entry whose count reaches zero leaves the list
+//   deaths  : around every nucleus and capture, the entries whose 26
+//             neighbours are all solid by then are found from the solid map.
+//             A sleeping entry left without a liquid neighbour leaves the list
 //             in this step if every capture that emptied it came from an
 //             earlier rank of generation 0, else in the next step (at its
 //             turn a neighbour was still liquid), exactly as the reference's
@@ -36,7 +36,7 @@
 //             that reaches the cell first in the reference. An envelope of
 //             generation g+1 first builds itself: the decentred octahedron of
 //             its parent (FP64), and writes its orientation into its cell.
-//             Each sets its liquid count and its next wake key.
+//             Each sets its next wake key.
 //   resolve : an envelope captures the cells whose final claim is its own;
 //             it stays active iff some neighbour was liquid at its turn and
 //             not captured by it (unclaimed, or claimed by a later rank).
@@ -437,33 +437,100 @@ __device__ __forceinline__ int nbr_delta(const Grid &g, int n, int &di, int &dj,
   return dk * g.nxyg + dj * g.nxg + di;
 }
 
-__device__ __forceinline__ void set_solid(uint32_t *solid, int cell) {
-  atomicOr(solid + (cell >> 5), 1u << (cell & 31));
+// Sets the bit of cell (I, J, K) in a brick map.
+__device__ __forceinline__ void set_bit(const PlainDevice &d, unsigned long long *map, int I, int J, int K) {
+  const int x = I + 2, y = J + 2, z = K + 2;
+  const int b = (z >> 2) * d.nbxy + (y >> 2) * d.nbx + (x >> 2), bit = (z & 3) * 16 + (y & 3) * 4 + (x & 3);
+  atomicOr((uint32_t *)map + 2 * (int64_t)b + (bit >> 5), 1u << (bit & 31));
 }
 
-// Bits of a cell bitmap for the 26 neighbours of `cell`, in the reference's
-// neighbour order (bit n of the result = neighbour n): one 64-bit window per
-// row of three cells, nine rows.
-__device__ __forceinline__ uint32_t neighbour_bits(const uint32_t *map, const Grid &g, int cell) {
+// Bricks side by side along an axis, `o` (0..4) cells into the first: the 4
+// cells of each line from there on. Along x a line is a nibble, along y a row
+// of nibbles (both stay inside the 32-bit halves of a brick), along z a plane.
+__device__ __forceinline__ uint2 along_x(uint2 lo, uint2 hi, int o) {
+  const uint32_t m = 0x11111111u * (0xfu >> o);  // cells the first brick has
+  return make_uint2((lo.x >> o & m) | (hi.x << (4 - o) & ~m), (lo.y >> o & m) | (hi.y << (4 - o) & ~m));
+}
+__device__ __forceinline__ uint2 along_y(uint2 lo, uint2 hi, int o) {
+  const uint32_t m = 0x00010001u * (0xffffu >> (4 * o));
+  return make_uint2((lo.x >> (4 * o) & m) | (hi.x << (16 - 4 * o) & ~m),
+                    (lo.y >> (4 * o) & m) | (hi.y << (16 - 4 * o) & ~m));
+}
+__device__ __forceinline__ unsigned long long along_z(uint2 lo, uint2 hi, int o) {
+  const unsigned long long l = (unsigned long long)lo.y << 32 | lo.x, h = (unsigned long long)hi.y << 32 | hi.x;
+  return o == 0 ? l : o == 4 ? h : l >> (16 * o) | h << (64 - 16 * o);
+}
+
+// Bits of a brick map for the 26 neighbours of cell (I, J, K), in the
+// reference's neighbour order (bit n of the result = neighbour n). Bricks the
+// 3 x 3 x 3 cells do not reach are not read.
+__device__ __forceinline__ uint32_t neighbour_bits(const PlainDevice &d, const unsigned long long *map, int I, int J,
+                                                   int K) {
+  const int x = I + 1, y = J + 1, z = K + 1;  // the lower corner's place in the map
+  const int ox = x & 3, oy = y & 3, oz = z & 3;
+  const uint2 *b = (const uint2 *)map + ((z >> 2) * d.nbxy + (y >> 2) * d.nbx + (x >> 2));
+  uint2 p[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    uint2 r[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      uint2 lo = make_uint2(0u, 0u), hi = lo;
+      if ((k == 0 || oz >= 2) && (j == 0 || oy >= 2)) {
+        lo = b[k * d.nbxy + j * d.nbx];
+        if (ox >= 2) hi = b[k * d.nbxy + j * d.nbx + 1];
+      }
+      r[j] = along_x(lo, hi, ox);
+    }
+    p[k] = along_y(r[0], r[1], oy);
+  }
+  const unsigned long long w = along_z(p[0], p[1], oz);
   uint32_t m27 = 0;
 #pragma unroll
-  for (int dk = -1; dk <= 1; ++dk)
+  for (int k = 0; k < 3; ++k)
 #pragma unroll
-    for (int dj = -1; dj <= 1; ++dj) {
-      const long long c0 = (long long)cell + dk * g.nxyg + dj * g.nxg - 1;  // the row's di = -1 cell
-      const long long w = c0 >> 5;
-      const unsigned long long two = ((unsigned long long)map[w + 1] << 32) | map[w];
-      m27 |= ((uint32_t)(two >> (c0 & 31)) & 7u) << ((dk + 1) * 9 + (dj + 1) * 3);
-    }
+    for (int j = 0; j < 3; ++j) m27 |= ((uint32_t)(w >> (16 * k + 4 * j)) & 7u) << (9 * k + 3 * j);
   return (m27 & 0x1fffu) | ((m27 >> 14) << 13);  // drop the centre cell (index 13 of 27)
 }
 
-__device__ __forceinline__ uint32_t liquid_neighbours(const uint32_t *solid, const Grid &g, int cell) {
-  return ~neighbour_bits(solid, g, cell) & 0x03ffffffu;
+__device__ __forceinline__ uint32_t liquid_neighbours(const PlainDevice &d, int I, int J, int K) {
+  return ~neighbour_bits(d, d.solid, I, J, K) & 0x03ffffffu;
+}
+
+// Which cells of the 3 x 3 x 3 block around interior cell (I, J, K) have no
+// liquid cell in their own 3 x 3 x 3 block: bit (dk + 1) * 16 + (dj + 1) * 4 +
+// (di + 1), the centre left out. The 5 x 5 x 5 cells lie in 2 x 2 x 2 bricks;
+// three in a row are solid where a line and the line from the next cell on
+// agree, axis by axis.
+__device__ __forceinline__ unsigned long long enclosed_around(const PlainDevice &d, int I, int J, int K) {
+  const int x = I, y = J, z = K;  // cell (I - 2, ..)'s place in the map
+  const int ox = x & 3, oy = y & 3, oz = z & 3;
+  const uint2 *b = (const uint2 *)d.solid + ((z >> 2) * d.nbxy + (y >> 2) * d.nbx + (x >> 2));
+  uint2 q[2][2][2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) q[k][j][i] = b[k * d.nbxy + j * d.nbx + i];
+  uint2 p[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    uint2 r[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint2 a = along_x(q[k][j][0], q[k][j][1], ox), c = along_x(q[k][j][0], q[k][j][1], ox + 1);
+      r[j] = make_uint2(a.x & c.x & (c.x >> 1), a.y & c.y & (c.y >> 1));
+    }
+    const uint2 a = along_y(r[0], r[1], oy), c = along_y(r[0], r[1], oy + 1);
+    p[k] = make_uint2(a.x & c.x & (c.x >> 4), a.y & c.y & (c.y >> 4));
+  }
+  const unsigned long long a = along_z(p[0], p[1], oz), c = along_z(p[0], p[1], oz + 1);
+  return a & c & (c >> 16) & 0x0000077707570777ull;
 }
 
 // ---------------------------------------------------------------------------
-// The envelope list: wake keys, grown half-diagonals, liquid counts.
+// The envelope list: wake keys, grown half-diagonals, cell words.
 // ---------------------------------------------------------------------------
 // x rounded down to float, by the bits where the float is normal (an FP64
 // conversion holds the scheduler for 64 cycles).
@@ -527,71 +594,58 @@ struct GenList {
   __device__ __forceinline__ long long at(long long r) const { return r < nw ? (long long)w[r] : base + (r - nw); }
 };
 
-// A nucleus turned `cell` solid before the walk: one liquid neighbour fewer
-// for every entry around it, and a sleeping entry left without one is
-// deactivated at its turn (a woken one decides at its turn itself). Returns
-// those entries.
-__device__ __noinline__ unsigned nucleus_neighbours(const PlainDevice &d, int cur, int cell, double grown, bool all,
-                                                    unsigned long long *stat_dec) {
-  const Grid &g = d.grid;
-  unsigned gone = 0;
-  int di, dj, dk;
-  // the 26 atomics issued before any result is used
-  uint32_t w[26];
-#pragma unroll
-  for (int nb = 0; nb < 26; ++nb) w[nb] = atomicSub(d.cellw + cell + nbr_delta(g, nb, di, dj, dk), 1u);
-  const float gf = wake_bound(grown);
-#pragma unroll
-  for (int nb = 0; nb < 26; ++nb) {
-    if (!has_entry(w[nb])) continue;
-    ++*stat_dec;
-    const int q = (int)(w[nb] >> 5);
-    if ((w[nb] & 31u) == 1u && !woken(d.key[cur][q], gf, all)) {
-      tombstone(d, cur, q, cell + nbr_delta(g, nb, di, dj, dk));
-      ++gone;
-    }
-  }
-  return gone;
-}
-
-// Zero-count events a block gathers before adding them to a zero list.
+// Envelopes without a liquid neighbour that a block gathers before adding
+// them to a zero list.
 constexpr int kZeroBuf = 512;
 __shared__ int s_zero[kZeroBuf];
 __shared__ unsigned s_nz;
 __shared__ unsigned long long s_zbase;
 
-// The liquid counts around the n cells that the previous generation captured
-// (its child records, this generation's ranks, which name the capturers'
-// list positions): one atomic decrement of the cell word of each
-// neighbour cell, whose old value says which entry (if any) lives there and
-// its count before. This generation's own entries still hold no-entry words
-// (they set theirs in the resolve phase, from the bitmap, which has these
-// captures), and a no-entry word never reaches a zero count. A decrement by
-// a later rank (capturer beyond the entry) is recorded in late[]; a count
-// reaching zero goes to the block's zero buffer (s_nz reset before), or to
-// the zero list of parity zpar once the buffer is full. Capture k goes to
-// the thread numbered k among `threads` ones; this thread is number t0. The
-// 26 atomics of a capture are issued before any result is used.
-__device__ __noinline__ void decrement_captures(const PlainDevice &d, int cur, long long n,
-                                                long long step, int zpar, long long t0, long long threads,
-                                                unsigned long long *stat_dec) {
+// Envelopes that the newly solid cells of this phase leave without a liquid
+// neighbour: those around the n captures of the previous generation (its child
+// records, this generation's ranks, which name the capturers' list positions),
+// or, in generation 0, around the step's n nuclei (the entries from position
+// `nuclei` on). The solid map has all of them and does not change in this
+// phase, so an envelope is found here exactly when its last liquid neighbour
+// is among these cells; by each of them that touches it, and the first to mark
+// its cell word puts it into the zero list of parity zpar (through the block's
+// buffer; s_nz reset before). A capture by a later entry of the list marks the
+// word kLate. This generation's own entries have no cell word yet (theirs
+// follow in the resolve phase); the nuclei's neighbours that are processed in
+// this generation find out at their turn. Cell k goes to the thread numbered
+// k among `threads` ones; this thread is number t0.
+// Before, every neighbour's cell word held a count of liquid neighbours and
+// each capture took 26 returning atomics: 2.9M of them per step of 320^3, 50
+// us of a 110 us claim phase; eight brick loads and about 120 integer
+// instructions find the same envelopes.
+__device__ __noinline__ void check_around(const PlainDevice &d, int cur, long long n, long long nuclei, int zpar,
+                                          long long t0, long long threads, unsigned long long *stat_found) {
   const Grid &g = d.grid;
   const EnvRec *act = d.act[cur];
   for (long long k = t0; k < n; k += threads) {
-    const uint32_t rec = d.child[k];
-    const int pc = (int)(rec >> 5);  // the capturer's list position
-    int di, dj, dk;
-    const int cell = act[pc].cell + nbr_delta(g, (int)(rec & 31u), di, dj, dk);
-    uint32_t w[26];
-#pragma unroll
-    for (int nb = 0; nb < 26; ++nb) w[nb] = atomicSub(d.cellw + cell + nbr_delta(g, nb, di, dj, dk), 1u);
-#pragma unroll
-    for (int nb = 0; nb < 26; ++nb) {
-      if (!has_entry(w[nb])) continue;
-      ++*stat_dec;
-      const int q = (int)(w[nb] >> 5);
-      if (pc > q) d.late[q] = (int32_t)step;
-      if ((w[nb] & 31u) != 1u) continue;
+    int pc = -1;  // the capturer's list position
+    int cell;
+    if (nuclei >= 0) {
+      cell = act[nuclei + k].cell;
+    } else {
+      const uint32_t rec = d.child[k];
+      pc = (int)(rec >> 5);
+      int di, dj, dk;
+      cell = act[pc].cell + nbr_delta(g, (int)(rec & 31u), di, dj, dk);
+    }
+    int I, J, K;
+    cell_ijk(g, cell, I, J, K);
+    unsigned long long left = enclosed_around(d, I, J, K);
+    while (left) {
+      const int bit = __ffsll((long long)left) - 1;
+      left &= left - 1;
+      const int nc = cell + ((bit >> 4) - 1) * g.nxyg + ((bit >> 2 & 3) - 1) * g.nxg + (bit & 3) - 1;
+      const uint32_t w = ld_volatile(d.cellw + nc);
+      if (!has_entry(w)) continue;
+      ++*stat_found;
+      const int q = (int)(w >> 5);
+      const uint32_t mark = kLeaving | (pc > q ? kLate : 0u);
+      if ((w & mark) == mark || (atomicOr(d.cellw + nc, mark) & kLeaving)) continue;
       const unsigned z = atomicAdd(&s_nz, 1u);
       if (z < (unsigned)kZeroBuf) {
         s_zero[z] = q;
@@ -603,7 +657,7 @@ __device__ __noinline__ void decrement_captures(const PlainDevice &d, int cur, l
   }
 }
 
-// The block's buffered zero events into the zero list of parity zpar (every
+// The block's buffered entries into the zero list of parity zpar (every
 // thread of the block).
 __device__ __noinline__ void flush_zero_buffer(const PlainDevice &d, int zpar) {
   __syncthreads();
@@ -615,18 +669,15 @@ __device__ __noinline__ void flush_zero_buffer(const PlainDevice &d, int zpar) {
 
 // Nucleus number r (in site order) of this step on `cell`: orientation,
 // envelope table entry and list record at position base_pos + r, grown from
-// the previous step on (CellularAutomataManager.cpp:262-290). Returns the
-// entries around it that leave the list at their turn.
-__device__ __forceinline__ unsigned place_nucleus(const PlainDevice &d, int cur, long long base_pos,
-                                                  long long base_orient, long long base_grain, long long r, int cell,
-                                                  long long step, double grown, bool all,
-                                                  unsigned long long *stat_dec) {
+// the previous step on (CellularAutomataManager.cpp:262-290).
+__device__ __forceinline__ void place_nucleus(const PlainDevice &d, int cur, long long base_pos, long long base_orient,
+                                              long long base_grain, long long r, int cell, long long step) {
   const int oid = (int)(base_orient + r);
   const long long gid = base_grain + r;
   int I, J, K;
   cell_ijk(d.grid, cell, I, J, K);
   d.orient[cell] = (uint32_t)oid;
-  set_solid(d.solid, cell);
+  set_bit(d, d.solid, I, J, K);
   d.gx[gid] = centre_coord(d.grid.x0, d.grid.h, I);
   d.gy[gid] = centre_coord(d.grid.y0, d.grid.h, J);
   d.gz[gid] = centre_coord(d.grid.z0, d.grid.h, K);
@@ -640,7 +691,6 @@ __device__ __forceinline__ unsigned place_nucleus(const PlainDevice &d, int cur,
   en.id = (int32_t)gid;
   d.act[cur][base_pos + r] = en;
   d.lstep[cur][base_pos + r] = (int32_t)(step - 1);
-  return nucleus_neighbours(d, cur, cell, grown, all, stat_dec);
 }
 
 // Sites are held as tiles of kBlock, one per block, when they fit: tile t =
@@ -676,12 +726,10 @@ __device__ __forceinline__ void step_rates(const PlainDevice &d, double time, do
   }
 }
 
-// Nuclei go to the list from position base_pos on; `gone` counts the
-// entries around them that leave the list at their turn.
+// Nuclei go to the list from position base_pos on.
 __device__ __noinline__ bool nucleation_phase(const PlainDevice &d, int cur, double time, long long step, long long base_pos,
-                                 long long base_orient, long long base_grain, double grown, bool all, int *s_cell,
-                                 double *s_dtc, unsigned long long *smem, unsigned long long *stat_live,
-                                 unsigned long long *stat_dec, unsigned *gone) {
+                                 long long base_orient, long long base_grain, int *s_cell, double *s_dtc,
+                                 unsigned long long *smem, unsigned long long *stat_live) {
   PlainCtrl *c = d.ctrl;
   unsigned long long *scan = d.scanA + (step & 1) * kStatusWords;
   const double T = d.T0 + d.Tdot * time;  // compute_cell_temperature (ProblemPhysics.cpp:164-169)
@@ -711,9 +759,7 @@ __device__ __noinline__ bool nucleation_phase(const PlainDevice &d, int cur, dou
     const unsigned long long ex = block_exclusive_scan(nuc, smem, &agg);
     const unsigned long long pre = block_prefix(scan, agg, smem, c);
     if (pre == ~0ull) return false;
-    if (nuc)
-      *gone += place_nucleus(d, cur, base_pos, base_orient, base_grain, (long long)(pre + ex), cell, step, grown, all,
-                             stat_dec);
+    if (nuc) place_nucleus(d, cur, base_pos, base_orient, base_grain, (long long)(pre + ex), cell, step);
     if (t_b == ntiles - 1 && threadIdx.x == 0) c->n_active_nuc[step & 1] = base_pos + (long long)(pre + agg);
     return true;
   }
@@ -744,9 +790,7 @@ __device__ __noinline__ bool nucleation_phase(const PlainDevice &d, int cur, dou
     }
     unsigned long long tot;
     const unsigned long long ex = block_exclusive_scan(nuc, smem, &tot);
-    if (nuc)
-      *gone += place_nucleus(d, cur, base_pos, base_orient, base_grain, (long long)(run + ex), cell, step, grown, all,
-                             stat_dec);
+    if (nuc) place_nucleus(d, cur, base_pos, base_orient, base_grain, (long long)(run + ex), cell, step);
     run += tot;
   }
   if (t_b == t_nb - 1 && threadIdx.x == 0) c->n_active_nuc[step & 1] = base_pos + (long long)(pre + agg);
@@ -817,8 +861,6 @@ __device__ __noinline__ bool wake_scan(const PlainDevice &d, int cur, long long 
   unsigned long long total = 0;
   unsigned long long off = warp_offset(cnt, d.scanC + (step & 1) * kStatusWords, smem, &total, c);
   if (off == ~0ull) return false;
-  // a key read again here may have turned dead since (a nucleus next to a
-  // sleeping entry), which the first pass counted as not woken all the same
 #pragma unroll 2
   for (long long t = wb; t < we; ++t) {
     const long long p0 = t * kKeyTile + 4 * lane;
@@ -838,7 +880,7 @@ __device__ __noinline__ bool wake_scan(const PlainDevice &d, int cur, long long 
 }
 
 // The live entries of list `cur` among [0, n), in order, into list cur ^ 1
-// with their keys, grow steps and liquid counts; the cell map follows. The
+// with their keys and grow steps; the cell map follows. The
 // new length goes to compact_len.
 __device__ __noinline__ bool compact_phase(const PlainDevice &d, int cur, long long n, unsigned par, unsigned long long *smem,
                               unsigned long long *stat_moved) {
@@ -866,8 +908,7 @@ __device__ __noinline__ bool compact_phase(const PlainDevice &d, int cur, long l
       d.act[nxt][q] = en;
       d.key[nxt][q] = key[p];
       d.lstep[nxt][q] = d.lstep[cur][p];
-      d.late[q] = -1;
-      d.cellw[en.cell] = ((uint32_t)q << 5) | (d.cellw[en.cell] & 31u);
+      d.cellw[en.cell] = (uint32_t)q << 5;
       ++*stat_moved;
     }
     off += __popc(bal);
@@ -887,21 +928,25 @@ __device__ __forceinline__ void flush_departures(PlainCtrl *c, long long step, u
   now = next = 0;
 }
 
-// Entries whose liquid count reached zero through the previous generation's
-// captures (zero list of parity zpar; gen0: those were generation 0's): each
-// leaves the list now or in the next step, and becomes a tombstone. One that
-// died at its own turn is one already; one processed this step outlived its
-// turn (it goes next step); a sleeping one (emptied only by generation 0)
-// goes now unless a capture by a later rank emptied it too.
-__device__ __noinline__ void zero_decisions(const PlainDevice &d, int cur, int zpar, bool gen0, long long step,
+// Entries left without a liquid neighbour (zero list of parity zpar; of: by
+// the step's nuclei (-1) or the captures of generation `of`): each leaves the
+// list now or in the next step, and becomes a tombstone. Emptied by nuclei: a
+// sleeping one goes now, one processed in generation 0 decides at its turn.
+// Emptied by captures: one that died at its own turn is a tombstone already;
+// one processed this step outlived its turn (it goes next step); a sleeping
+// one goes now if generation 0 emptied it and no capture by a later rank did
+// so too, else next step.
+__device__ __noinline__ void zero_decisions(const PlainDevice &d, int cur, int zpar, int of, long long step,
                                             unsigned *now, unsigned *next) {
   const unsigned long long nz = ld_volatile(&d.ctrl->zn[zpar]);
   for (unsigned long long i = (unsigned long long)t_b * kBlock + threadIdx.x; i < nz;
        i += (unsigned long long)t_nb * kBlock) {
     const int q = d.zlist[zpar][i];
-    if (isnan(d.key[cur][q])) continue;
-    const bool later = d.lstep[cur][q] == (int32_t)step || !gen0 || d.late[q] == (int32_t)step;
-    tombstone(d, cur, q, d.act[cur][q].cell);
+    const bool processed = d.lstep[cur][q] == (int32_t)step;
+    if (of < 0 ? processed : isnan(d.key[cur][q])) continue;
+    const int cell = d.act[cur][q].cell;
+    const bool later = of >= 0 && (processed || of > 0 || (d.cellw[cell] & kLate));
+    tombstone(d, cur, q, cell);
     if (later)
       ++*next;
     else
@@ -912,15 +957,16 @@ __device__ __noinline__ void zero_decisions(const PlainDevice &d, int cur, int z
 // ---------------------------------------------------------------------------
 // Claim: growth up to this step (generation 0) or self-construction
 // (generation >= 1), neighbour tests, atomicMin claims and the entry's next
-// wake key (its liquid count is set in the resolve phase).
+// wake key.
 // ---------------------------------------------------------------------------
-// With `dec` (generations after the first) the liquid counts around the
-// previous generation's captures are decremented in the same phase: the
-// first dec_warps warps of every block do that first and then join the
-// claims, whose dynamic hand-out balances the difference, so the memory
-// latency of the decrements overlaps the FP64 decentring of the claims.
+// With `checks` > 0 the neighbourhoods of that many newly solid cells are
+// checked in the same phase (check_around: the previous generation's captures,
+// or in generation 0 the nuclei, the last ranks): the last dec_warps warps of
+// every block do that first and then join the claims, whose dynamic hand-out
+// balances the difference (a generation of at most 32 ranks per block keeps
+// its claims on the blocks' first warps).
 __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind, long long lo, long long n, unsigned par,
-                            const GenList &list, long long step, double grown, bool dec,
+                            const GenList &list, long long step, double grown, long long checks,
                             int zpar, unsigned long long *stat_tests, unsigned long long *stat_tests64,
                             unsigned long long *stat_dec) {
   const Grid &g = d.grid;
@@ -932,18 +978,18 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
   // Claims need no order: warps or blocks take chunks of consecutive ranks
   // from a shared counter until none is left, so those that drew cheap
   // envelopes (few liquid neighbours) take more chunks.
-  if (dec) {
+  if (checks) {
     if (threadIdx.x == 0) s_nz = 0u;
     __syncthreads();
   }
   RankSched sched(n, &d.ctrl->claim_next, &d.ctrl->error, d.warp_sched);
-  // teams of the batched launch (at most 64 blocks) give the decrements more
-  // of their warps (batched_64: 77 ms at four, 81 at two; the whole GPU on
-  // one realm: 64.7 ms at two, 69 at four)
+  // teams of the batched launch (at most 64 blocks) give the checks more of
+  // their warps
   const int dw = t_nb <= 64 ? kDecWarpsTeam : d.dec_warps;
-  if (dec && (int)(threadIdx.x >> 5) < dw)
-    decrement_captures(d, cur, n, step, zpar, ((long long)t_b * dw + (threadIdx.x >> 5)) * 32 + (threadIdx.x & 31),
-                       (long long)t_nb * dw * 32, stat_dec);
+  const int cw = (int)(threadIdx.x >> 5) - (kWarps - dw);
+  if (checks && cw >= 0)
+    check_around(d, cur, checks, kind == 0 ? list.base : -1, zpar,
+                 ((long long)cw * t_nb + t_b) * 32 + (threadIdx.x & 31), (long long)t_nb * dw * 32, stat_dec);
   const int first = sched.first(), stride = sched.stride();
   long long b, e;
   while (sched.next(b, e)) {
@@ -953,9 +999,11 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
     bool have_centre = false;
     uint32_t liq = 0;
     const long long p = list.at(r);
+    int I, J, K;
     if (kind == 0) {
       en = act[p];
-      liq = liquid_neighbours(d.solid, g, en.cell);
+      cell_ijk(g, en.cell, I, J, K);
+      liq = liquid_neighbours(d, I, J, K);
       // Grain::grow (Grain.h:27) for every step since the record was last
       // grown: L + dt * vel, the product rounded once per step
       en.L = replay_growth(d.dvh, en.L, (long long)lstep[p], step);
@@ -968,16 +1016,16 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
       const uint32_t rec = d.child[r];
       const EnvRec pe = act[rec >> 5];  // the parent, by its list position
       const int pnb = (int)(rec & 31u);
-      int di, dj, dk, I, J, K;
+      int di, dj, dk;
       en.cell = pe.cell + nbr_delta(g, pnb, di, dj, dk);
       en.ori = pe.ori;
       en.id = (int32_t)(lo + r);
-      liq = liquid_neighbours(d.solid, g, en.cell);
+      cell_ijk(g, en.cell, I, J, K);
+      liq = liquid_neighbours(d, I, J, K);
       const double px = d.gx[pe.id], py = d.gy[pe.id], pz = d.gz[pe.id];
-      cell_ijk(g, pe.cell, I, J, K);
-      const double ccx = centre_coord(g.x0, g.h, I + di);
-      const double ccy = centre_coord(g.y0, g.h, J + dj);
-      const double ccz = centre_coord(g.z0, g.h, K + dk);
+      const double ccx = centre_coord(g.x0, g.h, I);
+      const double ccy = centre_coord(g.y0, g.h, J);
+      const double ccz = centre_coord(g.z0, g.h, K);
       double out[4];
       capture_f64(d.omat + 9 * pe.ori, ccx - px, ccy - py, ccz - pz, pe.L, g.h, d.trunc, out);
       gxd = out[0] + px;
@@ -1007,8 +1055,6 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
     // entry is looked at again next step
     if (liq && (__double_as_longlong(L) << 1) == 0) t_lb = -INFINITY;
     if (liq && (__double_as_longlong(L) << 1) != 0) {
-      int I, J, K;
-      cell_ijk(g, cell, I, J, K);
       const float dxf = en.dx, dyf = en.dy, dzf = en.dz;
       const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(dxf) + fabsf(dyf) + fabsf(dzf)) + d.coord_err;
       const float L32 = f64_to_f32_rz(L);  // the pre-test's margin is 2^-14 of it
@@ -1049,7 +1095,7 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
         int di, dj, dk;
         const int nc = cell + nbr_delta(g, nb, di, dj, dk);
         atomicMin(d.orient + nc, mine);
-        atomicOr(d.claimed + (nc >> 5), 1u << (nc & 31));
+        set_bit(d, d.claimed, I + di, J + dj, K + dk);
       }
     }
     // growth is uniform: the entry can contain one of the neighbours left
@@ -1062,11 +1108,11 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
   }
   *stat_tests += tests;
   *stat_tests64 += tests64;
-  if (dec) flush_zero_buffer(d, zpar);
+  if (checks) flush_zero_buffer(d, zpar);
 }
 
 // ---------------------------------------------------------------------------
-// Resolve: captures, deactivation, child records, liquid counts.
+// Resolve: captures, deactivation, child records.
 // ---------------------------------------------------------------------------
 // Mark of one rank: the captured neighbours (final claim is its own) and
 // whether it stays active, as captures | survives << 31.
@@ -1080,7 +1126,9 @@ __device__ __forceinline__ uint32_t mark_rank(const PlainDevice &d, long long r,
     // a liquid neighbour this envelope does not contain and nobody claimed
     // keeps it active without a look at the cell field
     const uint32_t other = lm & ~cm;
-    const uint32_t clm = neighbour_bits(d.claimed, g, cell);
+    int I, J, K;
+    cell_ijk(g, cell, I, J, K);
+    const uint32_t clm = neighbour_bits(d, d.claimed, I, J, K);
     surv = (other & ~clm) ? 1u : 0u;
     // claim words are read for contained cells, and for claimed ones while
     // survival is still open
@@ -1121,23 +1169,22 @@ __device__ __forceinline__ bool mark_in_resolve(const PlainDevice &d, long long 
 // Each block marks its contiguous chunk of ranks (the claim words are final
 // after the claim phase's barrier), then one look-back per block over the
 // chunk's marks gives new envelope ids (walk order) and child records; an
-// entry that does not survive its turn becomes a tombstone, one that does
-// gets its cell word (its position and the liquid neighbours it saw in the
-// claim phase). Marking reads
+// entry that does not survive its turn becomes a tombstone, a new one that
+// does gets its cell word (its position). Marking reads
 // only claim words, the claimed bitmap, its own ranks' masks and cells, none
 // of which another block's resolve writes, so no barrier separates the two
 // passes. Every captured cell turns solid for the next generation (whose
-// claim phase takes it off the liquid counts around it). The zero events
-// that the claim phase found (parity zdec, -1: none; zgen0: of generation
-// 0's captures) are decided here, and the list of parity zreset is emptied
+// claim phase checks the envelopes around it). The entries that the claim
+// phase found without a liquid neighbour (parity zdec; zof as in
+// zero_decisions) are decided here, and the list of parity zreset is emptied
 // for the next claim phase. The last block publishes the generation's
 // capture and survivor counts, which every block reads after the barrier.
 __device__ __noinline__ bool resolve_phase(const PlainDevice &d, int cur, long long n, long long step, unsigned par,
-                                           const GenList &list, int zdec, bool zgen0, int zreset,
+                                           const GenList &list, int zdec, int zof, int zreset,
                                            unsigned long long *smem,
                                            unsigned *gone_now, unsigned *gone_next) {
   PlainCtrl *c = d.ctrl;
-  if (zdec >= 0) zero_decisions(d, cur, zdec, zgen0, step, gone_now, gone_next);
+  zero_decisions(d, cur, zdec, zof, step, gone_now, gone_next);
   if (t_b == 0 && threadIdx.x == 0) c->zn[zreset] = 0ull;  // last read in the previous resolve phase
   long long b, e;
   block_chunk(n, b, e);
@@ -1175,25 +1222,24 @@ __device__ __noinline__ bool resolve_phase(const PlainDevice &d, int cur, long l
     // what the rank's entry needs, loaded before the scan (independent of it)
     const long long p = r < e ? list.at(r) : 0;
     const int cell = r < e ? d.cellr[r] : 0;
-    const uint32_t lq = r < e ? d.liq[r] : 0u;
     unsigned long long tot;
     const unsigned long long ex = block_exclusive_scan(((unsigned long long)__popc(cap) << 32) | surv, smem, &tot);
     if (r < e) {
-      if (!surv) {
+      if (!surv)
         tombstone(d, cur, p, cell);  // deactivated at its turn
-      } else {
-        // its cell word: position and the liquid neighbours it saw in the
-        // claim phase (this generation's captures come off in the next one)
-        d.cellw[cell] = ((uint32_t)p << 5) | (uint32_t)__popc(lq);
-      }
+      else if (r >= list.nw)
+        d.cellw[cell] = (uint32_t)p << 5;  // a new entry
       long long slot = (long long)((run + ex) >> 32);  // rank of the first child in the next generation
+      int I = 0, J = 0, K = 0;
+      if (cap) cell_ijk(g, cell, I, J, K);
       uint32_t bits = cap;
       while (bits) {
         const int nb = __ffs(bits) - 1;
         bits &= bits - 1;
         d.child[slot++] = ((uint32_t)p << 5) | (uint32_t)nb;  // parent's list position
         int di, dj, dk;
-        set_solid(d.solid, cell + nbr_delta(g, nb, di, dj, dk));  // solid for the next generation
+        nbr_offset(nb, di, dj, dk);
+        set_bit(d, d.solid, I + di, J + dj, K + dk);  // solid for the next generation
       }
     }
     run += tot;
@@ -1298,15 +1344,13 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
     __syncthreads();
     // the wake scan first: every block publishes its part of the scan at
     // once, while only the blocks holding sites take part in nucleation's.
-    // A nucleus may turn a sleeping entry dead after the scan passed it,
-    // which the scan's rule (dead or sleeping: not woken) already gave.
     const unsigned long long tn0 = threadIdx.x == 0 ? now_ns() : 0ull;
     if (!(ok = wake_scan(d, S.cur, S.a_len, S.step, S.grown_s, S.all != 0, smem))) break;
     const unsigned long long tn1 = threadIdx.x == 0 ? now_ns() : 0ull;
-    if (!(ok = nucleation_phase(d, S.cur, S.time, S.step, S.a_len, S.n_orient, S.grain, S.grown_s, S.all != 0, s_cell,
-                                s_dtc, smem, &live, &dec, &gone_now)))
+    if (!(ok = nucleation_phase(d, S.cur, S.time, S.step, S.a_len, S.n_orient, S.grain, s_cell, s_dtc, smem, &live)))
       break;
-    flush_departures(c, S.step, gone_now, gone_next);
+    // the list of generation 0's checks (last read in an earlier step)
+    if (timer) c->zn[1] = 0ull;
     if (threadIdx.x == 0) {
       const unsigned long long tn2 = now_ns();
       S.wake_busy += tn1 - tn0;
@@ -1356,8 +1400,8 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
         S.processed += S.n;
         S.t_work = now_ns();
       }
-      // (and the liquid counts around the previous generation's captures)
-      claim_phase(d, S.cur, S.gen ? 1 : 0, S.lo, S.n, S.gen & 1u, S.list, S.step, S.grown, S.gen > 0,
+      // (and the envelopes around the previous generation's captures, or the nuclei)
+      claim_phase(d, S.cur, S.gen ? 1 : 0, S.lo, S.n, S.gen & 1u, S.list, S.step, S.grown, S.gen ? S.n : S.nucs,
                   (int)((S.gen - 1) & 1u), &tests, &tests64, &dec);
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -1392,8 +1436,8 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
         if (threadIdx.x == 0) S.t_work = now_ns();
         __syncthreads();
       }
-      if (!(ok = resolve_phase(d, S.cur, S.n, S.step, S.gen & 1u, S.list, S.gen > 0 ? (int)((S.gen - 1) & 1u) : -1,
-                               S.gen == 1, (int)(S.gen & 1u), smem, &gone_now, &gone_next)))
+      if (!(ok = resolve_phase(d, S.cur, S.n, S.step, S.gen & 1u, S.list, (int)((S.gen - 1) & 1u), (int)S.gen - 1,
+                               (int)(S.gen & 1u), smem, &gone_now, &gone_next)))
         break;
       flush_departures(c, S.step, gone_now, gone_next);
       if (threadIdx.x == 0) {
@@ -1515,32 +1559,38 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) plain_persistent_kernel(Pl
   run_realm(sd, step_limit, smem);
 }
 
-// One bitmap word (32 cells) of the initial field: cells past the grid count
-// as solid.
-__device__ __forceinline__ void init_field_word(uint32_t *orient, uint32_t *solid, uint32_t *claimed, uint32_t *cellw,
-                                                const Grid &g, long long ncells, long long w) {
-  uint32_t bits = 0;
-  for (int b = 0; b < 32; ++b) {
-    const long long i = w * 32 + b;
-    bool ghost = true;
-    if (i < ncells) {
-      int I, J, K;
-      cell_ijk(g, (int64_t)i, I, J, K);
-      ghost = I == 0 || J == 0 || K == 0 || I == g.nxg - 1 || J == g.nyg - 1 || K == g.nzg - 1;
-      orient[i] = ghost ? 0u : kLiquid;
-      cellw[i] = kNoEntry;
-    }
-    bits |= (ghost ? 1u : 0u) << b;
+// The initial field, maps and cell words, by the threads numbered tid + k *
+// stride. A brick row is solid where its y or z lies outside the interior, else
+// in the cells whose x does.
+__device__ __forceinline__ void init_field(const PlainDevice &d, long long tid, long long stride) {
+  const Grid &g = d.grid;
+  for (long long i = tid; i < d.ncells; i += stride) {
+    int I, J, K;
+    cell_ijk(g, (int64_t)i, I, J, K);
+    const bool ghost = I == 0 || J == 0 || K == 0 || I == g.nxg - 1 || J == g.nyg - 1 || K == g.nzg - 1;
+    d.orient[i] = ghost ? 0u : kLiquid;
+    d.cellw[i] = kNoEntry;
   }
-  solid[w] = bits;
-  claimed[w] = 0u;
+  for (long long b = tid; b < d.nbricks; b += stride) {
+    const int bz = (int)(b / d.nbxy), r = (int)(b - (long long)bz * d.nbxy), by = r / d.nbx, bx = r - by * d.nbx;
+    unsigned xs = 0;
+    for (int i = 0; i < 4; ++i) {
+      const int I = 4 * bx + i - 2;
+      xs |= (I < 1 || I > g.nx ? 1u : 0u) << i;
+    }
+    unsigned long long bits = 0;
+    for (int k = 0; k < 4; ++k)
+      for (int j = 0; j < 4; ++j) {
+        const int J = 4 * by + j - 2, K = 4 * bz + k - 2;
+        bits |= (unsigned long long)(J < 1 || J > g.ny || K < 1 || K > g.nz ? 15u : xs) << (16 * k + 4 * j);
+      }
+    d.solid[b] = bits;
+    d.claimed[b] = 0ull;
+  }
 }
 
-__global__ void init_field_kernel(uint32_t *orient, uint32_t *solid, uint32_t *claimed, uint32_t *cellw, Grid g,
-                                  long long ncells) {
-  const long long nwords = solid_words(ncells);
-  for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += (long long)gridDim.x * blockDim.x)
-    init_field_word(orient, solid, claimed, cellw, g, ncells, w);
+__global__ void init_field_kernel(PlainDevice d) {
+  init_field(d, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1621,9 +1671,7 @@ __global__ void batch_reset_kernel(const PlainDevice *insts, int ninst, unsigned
     d.scanD[i] = 0ull;
     d.scanD[kStatusWords + i] = 0ull;
   }
-  const long long nwords = solid_words(d.ncells);
-  for (long long w = tid; w < nwords; w += stride)
-    init_field_word(d.orient, d.solid, d.claimed, d.cellw, d.grid, d.ncells, w);
+  init_field(d, tid, stride);
 }
 
 // out[r] = realm r's control block.
@@ -1717,8 +1765,10 @@ __global__ void noalloc_setup_kernel(PlainDevice d, long long liquid, unsigned l
 // carves the envelope table, lists, masks, look-back words and control block
 // out of it instead of calling cudaMalloc.
 // ---------------------------------------------------------------------------
-constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;  // 32 MiB
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;  // the limit on a call's counted buffers
+// Room for every call within it: a line of cells, the worst, takes 10 bytes per
+// cell more in brick maps than it is counted with, of at least 170.
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes + kNoAllocScratchBytes / 8];
 
 namespace {
 constexpr int kNoAllocMaxDevices = 64;
@@ -1730,11 +1780,14 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Byte offsets of every scratch buffer for a grid of n interior cells and s sites.
 struct NoAllocLayout {
-  size_t ctrl, check, live, omat32, scanA, gx, gy, gz, gori, gcell, act[2], key[2], lstep[2], late, cellw, wlist,
+  size_t ctrl, check, live, omat32, scanA, gx, gy, gz, gori, gcell, act[2], key[2], lstep[2], cellw, wlist,
       zlist[2], dvh, liq, con, cellr, child, solid, claimed, scanB, scanC, scanD, total;
+  // what the entry point's limit counts: the buffers above with 4 bytes per
+  // interior cell and two bitmaps of the cells instead of the brick maps
+  size_t counted;
   // n interior cells, s sites, `cells` ghost-inclusive cells; the caller
   // bounds all three (see kNoAllocMaxCells) so that no size below wraps
-  NoAllocLayout(long long n, long long s, long long cells) {
+  NoAllocLayout(long long n, long long s, long long cells, long long bricks) {
     size_t o = 0;
     auto take = [&](size_t bytes) {
       const size_t at = o;
@@ -1757,7 +1810,6 @@ struct NoAllocLayout {
       lstep[b] = take((size_t)n * 4);
       zlist[b] = take((size_t)n * 4);
     }
-    late = take((size_t)n * 4);
     wlist = take((size_t)n * 4);
     cellw = take((size_t)cells * 4);
     dvh = take((size_t)kDvRing * 8);
@@ -1765,12 +1817,14 @@ struct NoAllocLayout {
     cellr = take((size_t)n * 4);
     con = take((size_t)n * 4);
     child = take((size_t)n * 4);
-    solid = take((size_t)solid_words(cells) * 4);
-    claimed = take((size_t)solid_words(cells) * 4);
+    solid = take((size_t)bricks * 8);
+    claimed = take((size_t)bricks * 8);
     scanB = take((size_t)kStatusWords * 8);
     scanC = take((size_t)2 * kStatusWords * 8);
     scanD = take((size_t)2 * kStatusWords * 8);
     total = o;
+    counted = o - 2 * align256((size_t)bricks * 8) + align256((size_t)n * 4) +
+              2 * align256(((size_t)(cells + 31) / 32 + 2) * 4);
   }
 };
 
@@ -1820,11 +1874,12 @@ extern "C" int amca_plain_run_noalloc(int device, const amca_plain_params *p, co
     return noalloc_fail(err, errlen, AMCA_ERR_ARG, "grid too large for the static scratch", "too many interior cells");
   if (nsites > n)
     return noalloc_fail(err, errlen, AMCA_ERR_ARG, "more sites than interior cells", nullptr);
-  const NoAllocLayout lay(n, nsites, (long long)(p->nx + 2) * (p->ny + 2) * (p->nz + 2));
-  if (lay.total > kNoAllocScratchBytes) {
+  const long long nbx = brick_count(p->nx + 2), nby = brick_count(p->ny + 2), nbz = brick_count(p->nz + 2);
+  const NoAllocLayout lay(n, nsites, (long long)(p->nx + 2) * (p->ny + 2) * (p->nz + 2), nbx * nby * nbz);
+  if (lay.counted > kNoAllocScratchBytes || lay.total > sizeof g_noalloc_scratch) {
     char detail[160];
     snprintf(detail, sizeof detail, "needs %zu bytes of scratch for %lld cells and %lld sites, limit is %zu",
-             lay.total, n, (long long)nsites, kNoAllocScratchBytes);
+             lay.counted, n, (long long)nsites, kNoAllocScratchBytes);
     return noalloc_fail(err, errlen, AMCA_ERR_ARG, "grid too large for the static scratch", detail);
   }
   DeviceRestore restore;
@@ -1854,6 +1909,8 @@ extern "C" int amca_plain_run_noalloc(int device, const amca_plain_params *p, co
   g.nyg = p->ny + 2;
   g.nzg = p->nz + 2;
   g.nxyg = g.nxg * g.nyg;
+  g.by_x = fast_div(g.nxg);
+  g.by_xy = fast_div(g.nxyg);
   g.x0 = p->x0;
   g.y0 = p->y0;
   g.z0 = p->z0;
@@ -1875,6 +1932,9 @@ extern "C" int amca_plain_run_noalloc(int device, const amca_plain_params *p, co
   for (int a = 0; a < 3; ++a) cmax = fmax(cmax, fabs(o3[a]) + (n3[a] + 1) * p->h);
   d.coord_err = (float)(ldexp(cmax, -49) + 1e-30);
   d.ncells = (int64_t)g.nxyg * g.nzg;
+  d.nbx = (int)nbx;
+  d.nbxy = (int)(nbx * nby);
+  d.nbricks = (int)(nbx * nby * nbz);
   d.nsites = nsites;
   d.gcap = n;
   d.warp_sched = kWarpSched;
@@ -1900,7 +1960,6 @@ extern "C" int amca_plain_run_noalloc(int device, const amca_plain_params *p, co
     d.lstep[b] = (int32_t *)(base + lay.lstep[b]);
     d.zlist[b] = (int32_t *)(base + lay.zlist[b]);
   }
-  d.late = (int32_t *)(base + lay.late);
   d.wlist = (int32_t *)(base + lay.wlist);
   d.cellw = (uint32_t *)(base + lay.cellw);
   d.dvh = (double *)(base + lay.dvh);
@@ -1908,8 +1967,8 @@ extern "C" int amca_plain_run_noalloc(int device, const amca_plain_params *p, co
   d.cellr = (int32_t *)(base + lay.cellr);
   d.con = (uint32_t *)(base + lay.con);
   d.child = (uint32_t *)(base + lay.child);
-  d.solid = (uint32_t *)(base + lay.solid);
-  d.claimed = (uint32_t *)(base + lay.claimed);
+  d.solid = (unsigned long long *)(base + lay.solid);
+  d.claimed = (unsigned long long *)(base + lay.claimed);
   d.scanB = (unsigned long long *)(base + lay.scanB);
   d.scanC = (unsigned long long *)(base + lay.scanC);
   d.scanD = (unsigned long long *)(base + lay.scanD);
@@ -2000,7 +2059,7 @@ cudaError_t plain_barrier_selftest(int blocks, int parties, long long wait_ns, i
 }
 
 cudaError_t plain_init_field(const PlainDevice &d, cudaStream_t s) {
-  init_field_kernel<<<1024, 256, 0, s>>>(d.orient, d.solid, d.claimed, d.cellw, d.grid, d.ncells);
+  init_field_kernel<<<152 * 8, 256, 0, s>>>(d);
   return cudaGetLastError();
 }
 

@@ -3,9 +3,11 @@
 //
 // HBM layout (one realm):
 //   orient      u32[(nx+2)(ny+2)(nz+2)]  cellOrientationID_, ghost-inclusive, reference index order
-//   solid       1 bit per cell (+2 words): solid before the current generation; the
-//               claim phase's liquidity test reads this (L2-resident) instead of orient
-//   claimed     1 bit per cell (+2 words): set with every claim. A claimed cell is
+//   solid       1 bit per cell in bricks of 4 x 4 x 4 cells (one 64-bit word;
+//               L2-resident): solid before the current generation. The claim
+//               phase's liquidity test reads this instead of orient: a cell's 27-cell
+//               neighbourhood lies in at most 8 bricks, on average 3.4
+//   claimed     likewise: set with every claim. A claimed cell is
 //               captured in that generation and never liquid again, so stale bits
 //               are never looked at and the map is never cleared during a run
 //   site_*      nucleation sites sorted by cell id: cell i32, dTc f64, live u8
@@ -18,14 +20,11 @@
 //               key[2]   f32 wake key (cumulative growth at which the entry may
 //                        contain a liquid neighbour; NaN = dead)
 //               lstep[2] i32 step up to which the record's half-diagonal is grown
-//   late        i32 per entry: step of the last capture next to it by a later rank
 //   cellw       u32 per ghost-inclusive cell: list position of the live envelope
-//               on the cell << 5 | its liquid neighbours now; kNoEntry (all
-//               ones) for none, which the at most 26 decrements a cell sees
-//               while it has no envelope never bring to a zero count
+//               on the cell << 5 | kLeaving, kLate; kNoEntry (all ones) for none
 //   wlist       i32 per entry: positions woken this step, in walk order
-//   zlist[2]    i32 per entry: entries whose liquid count reached zero in a
-//               generation, by generation parity
+//   zlist[2]    i32 per entry: entries left without a liquid neighbour by a
+//               generation's captures (or the step's nuclei), by generation parity
 //   dvh         f64 ring of the growth increment of each step
 //   liq/con     per-rank neighbour masks of the generation being processed
 //   cellr       per-rank cell of the generation being processed
@@ -60,14 +59,25 @@ constexpr long long kKeyTile = 128;
 // is never a list position (the list holds fewer than kMaxCells entries).
 constexpr uint32_t kNoEntry = 0xFFFFFFFFu;
 AMCA_HD bool has_entry(uint32_t w) { return (w >> 5) != (kNoEntry >> 5); }
-// Defaults of PlainDevice::warp_sched and PlainDevice::mark_split.
+// The entry is in a zero list; one of the captures that emptied its
+// neighbourhood came from a later entry of the list.
+constexpr uint32_t kLeaving = 1u, kLate = 2u;
+
+// Brick maps (solid, claimed): cell (I, J, K) is bit (z & 3) * 16 + (y & 3) * 4
+// + (x & 3) of brick (z >> 2, y >> 2, x >> 2) at x = I + 2, y = J + 2, z = K + 2.
+// The shift and the brick past the last cell keep the 5 x 5 x 5 neighbourhood of
+// an interior cell inside the map; what lies outside the grid counts as solid.
+AMCA_HD int brick_count(int ng) { return ((ng - 1) >> 2) + 2; }  // along an axis of ng ghost-inclusive cells
+// Defaults of PlainDevice::warp_sched, mark_split and dec_warps (320^3 at 1, 2,
+// 3, 4, 6, 8 warps of checks: 60.6, 54.0, 52.6, 52.2, 52.5, 54.6 ms; 60^3 does
+// not depend on it up to 6).
 constexpr int kWarpSched = 32;
 constexpr int kMarkSplit = 1024;
-constexpr int kDecWarps = 2;
+constexpr int kDecWarps = 4;
 constexpr int kCompactSlack = 4096;
 constexpr int kMarkBatch = 4;  // ranks per thread whose marks are computed before any is stored
-// Warps per block that start a claim phase with the decrements on teams of
-// at most 64 blocks (the batched launch).
+// Warps per block that start a claim phase with the neighbourhood checks on
+// teams of at most 64 blocks (the batched launch).
 constexpr int kDecWarpsTeam = 4;
 
 // Control block. Between launches it holds the realm's state (step, time,
@@ -89,7 +99,7 @@ struct PlainCtrl {
   long long compact_len;       // live entries after the last compaction
   long long deaths[3];         // entries leaving the active list in step s, in slot s % 3
   long long gen_surv;          // survivors of the last resolved generation
-  unsigned long long zn[2];    // zero-count events of a generation, by generation parity
+  unsigned long long zn[2];    // entries of the zero lists, by generation parity
   double grown;                // growth of the envelopes since the start of the run (sum of dv)
   long long liquid;
   long long gen_n;  // captures of the last resolved generation
@@ -109,8 +119,8 @@ struct PlainCtrl {
   unsigned long long active_grown;     // generation-0 entries processed (woken and nuclei), summed over steps
   unsigned long long grains_processed; // entries processed in every generation, summed
   unsigned long long keys_scanned;     // list positions the wake scan read, summed over steps
-  unsigned long long decrements;       // liquid-count decrements that reached an envelope's cell word
-  unsigned long long zero_events;      // liquid counts that reached zero in a capture generation
+  unsigned long long decrements;       // envelopes next to a nucleus or capture found without a liquid neighbour
+  unsigned long long zero_events;      // envelopes left without a liquid neighbour by a generation's captures
   unsigned long long compactions;      // compactions of the envelope list
   unsigned long long compacted;        // entries moved by them
   // wall time of each phase as block 0 sees it (phase start to barrier exit), ns
@@ -157,12 +167,13 @@ struct PlainDevice {
   int phase_detail; // nonzero: also gather the slowest block's busy time per phase
   int warp_sched;   // ranks per block of the team up to which claims are handed out warp by warp (else block by block)
   int mark_split;   // ranks per block of the team up to which a generation is marked inside the resolve pass
-  int dec_warps;    // warps per block that start a claim phase with the liquid-count decrements (1..kWarps)
+  int dec_warps;    // warps per block that start a claim phase with the neighbourhood checks (1..kWarps)
   int compact_slack;  // the list is compacted when it holds more than 2 x active + this many entries
   // arrays
   uint32_t *orient;
-  uint32_t *solid;    // 1 bit per cell: solid at the start of the current generation (ghosts included)
-  uint32_t *claimed;  // 1 bit per cell: some envelope claimed it (only ever read on cells still liquid)
+  unsigned long long *solid;    // brick map: solid at the start of the current generation (ghosts included)
+  unsigned long long *claimed;  // brick map: some envelope claimed it (only ever read on cells still liquid)
+  int nbx, nbxy, nbricks;       // bricks of a row, a plane and in all
   int64_t ncells;
   const int32_t *site_cell;
   const double *site_dtc;
@@ -176,7 +187,6 @@ struct PlainDevice {
   EnvRec *act[2];
   float *key[2];
   int32_t *lstep[2];
-  int32_t *late;
   uint32_t *cellw;
   int32_t *wlist;
   int32_t *zlist[2];
@@ -215,11 +225,8 @@ cudaError_t plain_barrier_selftest(int blocks, int parties, long long wait_ns, i
 
 // Fill the orientation field: -1 interior, 0 on the ghost layer
 // (CellularAutomataManager.cpp:316-326, CellularAutomataManager_3D.cpp:736-833),
-// the solid bitmap to match, and the cell -> list position map with -1.
+// the solid map to match, and the cell -> list position map with -1.
 cudaError_t plain_init_field(const PlainDevice &d, cudaStream_t s);
-
-// Words of the solid bitmap for `ncells` cells.
-AMCA_HD long long solid_words(long long ncells) { return (ncells + 31) / 32 + 2; }
 
 // Blocks of the persistent kernel that fit on the device at once.
 int plain_persistent_grid(int device);

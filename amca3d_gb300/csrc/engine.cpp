@@ -159,6 +159,8 @@ struct amca_t {
     g.nyg = c.ny + 2;
     g.nzg = c.nz + 2;
     g.nxyg = g.nxg * g.nyg;
+    g.by_x = fast_div(g.nxg);
+    g.by_xy = fast_div(g.nxyg);
     g.x0 = c.x0;
     g.y0 = c.y0;
     g.z0 = c.z0;
@@ -193,7 +195,7 @@ struct amca_t {
     // resolve pass, larger ones in a pass of their own (AMCA_MARK_SPLIT)
     d.mark_split = kMarkSplit;
     if (const char *m = getenv("AMCA_MARK_SPLIT")) d.mark_split = std::max(1, atoi(m));
-    // warps per block that start a claim phase with the decrements on a
+    // warps per block that start a claim phase with the neighbourhood checks on a
     // realm run by the whole GPU (AMCA_DEC_WARPS, 1..8)
     d.dec_warps = kDecWarps;
     if (const char *w = getenv("AMCA_DEC_WARPS")) d.dec_warps = std::min(8, std::max(1, atoi(w)));
@@ -201,6 +203,9 @@ struct amca_t {
     d.compact_slack = kCompactSlack;
     if (const char *cs = getenv("AMCA_COMPACT_SLACK")) d.compact_slack = std::max(0, atoi(cs));
     d.ncells = (int64_t)g.nxyg * g.nzg;
+    d.nbx = brick_count(g.nxg);
+    d.nbxy = d.nbx * brick_count(g.nyg);
+    d.nbricks = d.nbxy * brick_count(g.nzg);
     d.nsites = nsites;
     d.gcap = (int64_t)c.nx * c.ny * c.nz;
     const int64_t ntA = 2 * kStatusWords, ntB = kStatusWords;
@@ -225,7 +230,6 @@ struct amca_t {
         d.lstep[b] = a.take<int32_t>(d.gcap);
         d.zlist[b] = a.take<int32_t>(d.gcap);
       }
-      d.late = a.take<int32_t>(d.gcap);
       d.wlist = a.take<int32_t>(d.gcap);
       d.cellw = a.take<uint32_t>(d.ncells);
       d.dvh = a.take<double>(kDvRing);
@@ -233,8 +237,8 @@ struct amca_t {
       d.cellr = a.take<int32_t>(d.gcap);
       d.con = a.take<uint32_t>(d.gcap);
       d.child = a.take<uint32_t>(d.gcap);
-      d.solid = a.take<uint32_t>(solid_words(d.ncells));
-      d.claimed = a.take<uint32_t>(solid_words(d.ncells));
+      d.solid = a.take<unsigned long long>(d.nbricks);
+      d.claimed = a.take<unsigned long long>(d.nbricks);
       d.scanA = a.take<unsigned long long>(ntA);
       d.scanB = a.take<unsigned long long>(ntB);
       d.scanC = a.take<unsigned long long>(ntA);
@@ -336,14 +340,15 @@ struct amca_t {
   // 24 B per generation-0 entry processed (woken list write + read,
   // half-diagonal write, grow step read + write), 228 B per entry and
   // generation processed (40 B envelope, 26 x 4 B neighbour states, 72 B
-  // matrix, key + cell word), 148 B per capture (cell write, 40 B envelope,
-  // the 26 cell words around it), 8 B per liquid-count decrement, 48 B per
-  // entry moved by a compaction, and the sites and nucleations as above.
+  // matrix, key + cell word), 108 B per capture (cell write, 40 B envelope,
+  // the 8 bricks around it), 8 B per envelope found without a liquid
+  // neighbour, 48 B per entry moved by a compaction, and the sites and
+  // nucleations as above.
   double step_bytes() const {
     const double S = (double)ctrl.sites_scanned, N = (double)ctrl.nucleations, A0 = (double)ctrl.active_grown;
     const double G = (double)ctrl.grains_processed, C = (double)ctrl.captures, K = (double)ctrl.keys_scanned;
     const double D = (double)ctrl.decrements, M = (double)ctrl.compacted;
-    return 12 * S + 48 * N + 4 * K + 24 * A0 + 228 * G + 148 * C + 8 * D + 48 * M;
+    return 12 * S + 48 * N + 4 * K + 24 * A0 + 228 * G + 108 * C + 8 * D + 48 * M;
   }
 
   bool finished() const { return ctrl.done || !(ctrl.time < cfg.final_time); }

@@ -409,6 +409,8 @@ void RemeltRealm::initialize() {
   g.nyg = c.ny + 2;
   g.nzg = c.nz + 2;
   g.nxyg = g.nxg * g.nyg;
+  g.by_x = fast_div(g.nxg);
+  g.by_xy = fast_div(g.nxyg);
   g.x0 = c.x0;
   g.y0 = c.y0;
   g.z0 = c.z0;

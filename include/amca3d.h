@@ -351,8 +351,10 @@ typedef struct {
    * only); block 0's time inside grid barriers [4]. */
   double detail_ms[16];
   /* Plain realm only (zeros otherwise), summed since the last reset: list
-   * positions read by the wake scans, liquid-count decrements, counts that
-   * reached zero in a capture generation, compactions of the envelope list. */
+   * positions read by the wake scans, envelopes found without a liquid
+   * neighbour next to a nucleus or capture (once for each of those), envelopes
+   * that a generation's captures left without one, compactions of the envelope
+   * list. */
   int64_t keys_scanned;
   int64_t decrements;
   int64_t zero_events;

@@ -269,3 +269,27 @@ def test_reused_arena_gives_the_same_fields(amca):
                 assert hashlib.sha256(g.tobytes()).hexdigest() == golden[c.name]["grain_sha256"], (rnd, c.name)
             finally:
                 r.close()
+
+
+@pytest.mark.parametrize("cells", [(1, 1, 2), (2, 3, 5), (4, 4, 4), (5, 9, 6), (7, 4, 13), (17, 2, 11), (6, 21, 34)],
+                         ids=str)
+def test_gpu_grids_across_brick_edges_match_oracle(amca, oracle, cells):
+    """Every place of a neighbourhood in the 4 x 4 x 4-cell bricks of the solid map, edges that end inside and at the
+    end of a brick: with a site on every third cell, counts and fields equal the C restatement's in the middle of the
+    run and at its end, alone and in a batch with small teams."""
+    n = cells[0] * cells[1] * cells[2]
+    case = cases._mixed("bricks", cells, 5, n // 9, max(1, n // 4), t_dot=-120.0)
+    whole = oracle.run_plain(case)
+    for k in (whole["steps"] // 3, whole["steps"] // 2, -1):
+        out = run_gpu(amca, case, max_steps=k)
+        ref = whole if k < 0 else oracle.run_plain(case, max_steps=k)
+        assert out["stats"]["step"] == ref["steps"] and out["stats"]["grains"] == ref["num_grains"], k
+        assert out["stats"]["active"] == ref["active_grains"], k
+        assert out["stats"]["liquid_cells"] == ref["liquid_cells"], k
+        assert np.array_equal(out["orient"], ref["orient"]) and np.array_equal(out["grain"], ref["grain"]), k
+    r = amca.CellularAutomataRealm(case.to_yaml(), seed=case.seed)
+    r.initialize()
+    with amca.Batch([r], team_size=3) as b:
+        b.run()
+    assert np.array_equal(r.field("grain_id"), whole["grain"])
+    r.close()
