@@ -179,8 +179,11 @@ void RemeltRealm::fill_frames(int upto) {
     upto = f;
   } else {
     fill_scan_frames(&scan_, model_, t_liq_, band_, thresh_, avail_, upto - avail_, ring_, slots_, fcount_, stream_);
-    for (int g = avail_; g < upto; ++g)
-      RCK(cudaMemcpyAsync(ftime_ + g % slots_, &frames_.times[g], 8, cudaMemcpyHostToDevice, stream_));
+    for (int g = avail_; g < upto;) {  // the frames' times, one copy up to the ring's end
+      const int run = std::min(upto - g, slots_ - g % slots_);
+      RCK(cudaMemcpyAsync(ftime_ + g % slots_, &frames_.times[g], (size_t)run * 8, cudaMemcpyHostToDevice, stream_));
+      g += run;
+    }
     RCK(cudaStreamSynchronize(stream_));
   }
   produced_ += upto - avail_;
@@ -785,55 +788,74 @@ void RemeltRealm::extend_orientations() {
 // The reference's growth velocity with glibc's pow
 // (ProblemPhysics_RappazGandin1993::compute_growth_velocity_with_temperature_input,
 // CA/src/ProblemPhysics.cpp:142-158), for the arguments the kernel cannot round itself.
+// A zero coefficient's term is that zero (the power is finite and positive for
+// dT below 1e100), without its pow.
+static double velocity_term(double a, double dT, double b) {
+  return a == 0.0 && dT < 1e100 ? a : a * std::pow(dT, b);
+}
 static double reference_velocity(const PlainConfig &c, double T) {
   const double dT = c.Tm - T;
   double v = 0.0;
   if (dT > 0) {
-    v = c.a1 * std::pow(dT, c.b1) + c.a2 * std::pow(dT, c.b2) + c.a3 * std::pow(dT, c.b3);
+    v = velocity_term(c.a1, dT, c.b1) + velocity_term(c.a2, dT, c.b2) + velocity_term(c.a3, dT, c.b3);
     if (v < 0.0) v = 0.0;
   }
   return v;
 }
 
-// Runs beside a kernel launch: answers the kernel's velocity requests.
-void RemeltRealm::serve_velocities(const volatile int *stop, int w, int workers, VelocityJob *job, unsigned last) {
+// The launching thread, while its kernel runs: answers the kernel's velocity
+// requests, with whatever helpers have come to life by then, until the event
+// after the launch has completed (returns its status).
+cudaError_t RemeltRealm::serve_launch(VelocityJob *job) {
   HostVelocity *hv = hostvel_;
-  // worker 0 watches the device's request word and hands each request to all
-  // workers; every worker spins (yielding when idle for long) on the job word.
-  // `last` is what each has served before the launch (read before any thread
-  // starts: a worker that started after the first request was posted would
-  // otherwise take that request as served and never count it off)
-  unsigned idle = 0;
-  while (!*stop) {
-    unsigned r;
-    if (w == 0) {
-      r = __atomic_load_n(&hv->seq_req, __ATOMIC_ACQUIRE);
-      if (r != last) {
-        const unsigned n = std::min(__atomic_load_n(&hv->n, __ATOMIC_ACQUIRE), (unsigned)kHostVelCap);
-        // small requests are not worth waking the others
-        const int use = n >= 64u ? workers : 1;
+  unsigned last = __atomic_load_n(&hv->seq_done, __ATOMIC_ACQUIRE);
+  for (unsigned idle = 1;; ++idle) {
+    const unsigned r = __atomic_load_n(&hv->seq_req, __ATOMIC_ACQUIRE);
+    if (r != last) {
+      const unsigned n = std::min(__atomic_load_n(&hv->n, __ATOMIC_ACQUIRE), (unsigned)kHostVelCap);
+      // small requests are not worth sharing
+      const unsigned use = n >= 64u ? 1u + job->helpers.load(std::memory_order_acquire) : 1u;
+      if (use > 1) {
         job->n.store(n, std::memory_order_relaxed);
-        job->left.store((unsigned)use, std::memory_order_relaxed);
-        if (use > 1) job->seq.store(r, std::memory_order_release);
-        for (unsigned i = 0; i < n; i += (unsigned)use) hv->v[i] = reference_velocity(cfg_.ca, hv->T[i]);
-        if (job->left.fetch_sub(1, std::memory_order_acq_rel) != 1)
-          while (job->left.load(std::memory_order_acquire) != 0 && !*stop) {
-          }
-        __atomic_store_n(&hv->seq_done, r, __ATOMIC_RELEASE);
-        last = r;
-        idle = 0;
-        continue;
+        job->use.store(use, std::memory_order_relaxed);
+        job->left.store(use - 1, std::memory_order_relaxed);
+        job->seq.store(r, std::memory_order_release);
       }
-    } else {
-      r = job->seq.load(std::memory_order_acquire);
-      if (r != last) {
-        const unsigned n = job->n.load(std::memory_order_relaxed);
-        for (unsigned i = (unsigned)w; i < n; i += (unsigned)workers) hv->v[i] = reference_velocity(cfg_.ca, hv->T[i]);
-        job->left.fetch_sub(1, std::memory_order_acq_rel);
-        last = r;
-        idle = 0;
-        continue;
-      }
+      for (unsigned i = 0; i < n; i += use) hv->v[i] = reference_velocity(cfg_.ca, hv->T[i]);
+      if (use > 1)
+        while (job->left.load(std::memory_order_acquire) != 0) {
+        }
+      __atomic_store_n(&hv->seq_done, r, __ATOMIC_RELEASE);
+      last = r;
+      idle = 0;
+      continue;
+    }
+    if (idle % 64u == 0) {
+      const cudaError_t e = cudaEventQuery(ev1_);
+      if (e != cudaErrorNotReady) return e;
+    }
+    if (idle > 4096) std::this_thread::yield();
+  }
+}
+
+// A helper of serve_launch: evaluates its share of the requests made since it
+// came to life, spinning (yielding when idle for long) on the job word.
+void RemeltRealm::help_velocities(VelocityJob *job) {
+  HostVelocity *hv = hostvel_;
+  unsigned last = job->seq.load(std::memory_order_acquire);
+  const unsigned w = 1u + job->helpers.fetch_add(1u, std::memory_order_acq_rel);
+  unsigned idle = 0;
+  while (!job->stop.load(std::memory_order_acquire)) {
+    const unsigned r = job->seq.load(std::memory_order_acquire);
+    if (r != last) {
+      last = r;
+      idle = 0;
+      const unsigned use = job->use.load(std::memory_order_relaxed);
+      if (w >= use) continue;  // made before this helper counted
+      const unsigned n = job->n.load(std::memory_order_relaxed);
+      for (unsigned i = w; i < n; i += use) hv->v[i] = reference_velocity(cfg_.ca, hv->T[i]);
+      job->left.fetch_sub(1, std::memory_order_acq_rel);
+      continue;
     }
     if (++idle > 4096) std::this_thread::yield();
   }
@@ -858,8 +880,9 @@ void RemeltRealm::step_coupled(double dt_cap) {
   const double cap = dt_cap > 0 ? dt_cap : INFINITY;
   if (dev_.external) {
     // the external solver's step is the FE time step of the coupling (dT_FE and the CA's maxTimestep_)
-    h2d(&dev_.ctrl->dT_FE, &cap, sizeof cap);
-    h2d(&dev_.ctrl->max_ts, &cap, sizeof cap);
+    static_assert(offsetof(RemeltCtrl, max_ts) == offsetof(RemeltCtrl, dT_FE) + sizeof(double), "one copy sets both");
+    const double both[2] = {cap, cap};
+    h2d(&dev_.ctrl->dT_FE, both, sizeof both);
   }
   dev_.dt_cap = cap;
   try {
@@ -917,33 +940,47 @@ void RemeltRealm::run(long long max_steps) {
   if (dev_.external) ext_ready_ = false;  // the handed-in node temperatures are used up
 }
 
+// Launches of at least this many steps get helpers for the velocity requests:
+// starting them costs about 50 us each on the host (0.45 ms for the eight of a
+// launch when they started before it, of 0.55 ms for a step driven by an
+// outside solver), a step's few hundred pow calls about 20 us.
+constexpr long long kHelpedSteps = 16;
+
 void RemeltRealm::launch(long long limit) {
-  {
-    const int running = kRemeltRunning;
-    h2d(&dev_.ctrl->status, &running, sizeof running);
-    volatile int stop = 0;
-    // the hard velocities of one step (a few hundred glibc pow calls) are
-    // split over a few spinning host threads
-    const int hw = (int)std::thread::hardware_concurrency();
-    const int workers = std::max(1, std::min(8, hw / 2));
+  static_assert(kRemeltRunning == 0, "the launch clears the status word");
+  RCK(cudaMemsetAsync(&dev_.ctrl->status, 0, sizeof(int), stream_));
+  RCK(cudaEventRecord(ev0_, stream_));
+  cudaError_t le = remelt_run_steps(dev_, limit, blocks_, stream_);
+  if (le == cudaSuccess) le = cudaEventRecord(ev1_, stream_);
+  if (le == cudaSuccess) {
     VelocityJob job;
-    const unsigned done0 = __atomic_load_n(&hostvel_->seq_done, __ATOMIC_ACQUIRE);
-    std::vector<std::thread> servers;
-    for (int w = 0; w < workers; ++w)
-      servers.emplace_back([&, w] { serve_velocities(&stop, w, workers, &job, w == 0 ? done0 : 0u); });
-    RCK(cudaEventRecord(ev0_, stream_));
-    cudaError_t le = remelt_run_steps(dev_, limit, blocks_, stream_);
-    if (le == cudaSuccess) le = cudaEventRecord(ev1_, stream_);
-    if (le == cudaSuccess) le = cudaStreamSynchronize(stream_);
-    stop = 1;
-    for (std::thread &t : servers) t.join();
-    if (le != cudaSuccess) throw CudaError(std::string("remelting kernel: ") + cudaGetErrorString(le));
-    ++launches_;
-    sync_ctrl();
-    float ms = 0.f;
-    RCK(cudaEventElapsedTime(&ms, ev0_, ev1_));
-    kernel_ms_ += ms;
+    std::thread starter;
+    const int hw = (int)std::thread::hardware_concurrency();
+    const int helpers = limit - ctrl_.step >= kHelpedSteps ? std::max(1, std::min(8, hw / 2)) - 1 : 0;
+    if (helpers > 0) {  // started beside the kernel; this thread answers alone until (or unless) they are there
+      try {
+        starter = std::thread([&] {
+          std::vector<std::thread> more;
+          try {
+            for (int k = 1; k < helpers; ++k) more.emplace_back([&] { help_velocities(&job); });
+          } catch (const std::system_error &) {
+          }
+          help_velocities(&job);
+          for (std::thread &t : more) t.join();
+        });
+      } catch (const std::system_error &) {
+      }
+    }
+    le = serve_launch(&job);
+    job.stop.store(true, std::memory_order_release);
+    if (starter.joinable()) starter.join();
   }
+  if (le != cudaSuccess) throw CudaError(std::string("remelting kernel: ") + cudaGetErrorString(le));
+  ++launches_;
+  sync_ctrl();
+  float ms = 0.f;
+  RCK(cudaEventElapsedTime(&ms, ev0_, ev1_));
+  kernel_ms_ += ms;
 }
 
 void RemeltRealm::get_field(int field, void *dst, size_t bytes) {

@@ -73,14 +73,18 @@ class RemeltRealm {
   void sync_ctrl();
   void extend_orientations();
   void upload_initial_state();
-  // Host side of the velocity requests: worker w of `workers` evaluates
-  // entries w, w + workers, ... of each request; the last to finish answers.
+  // Host side of the velocity requests: of a request shared by `use` threads,
+  // thread w (the launching one is 0) evaluates entries w, w + use, ...
   struct VelocityJob {
-    std::atomic<unsigned> seq{0};   // request being served
-    std::atomic<unsigned> n{0};     // its entry count
-    std::atomic<unsigned> left{0};  // workers still evaluating it
+    std::atomic<unsigned> seq{0};      // shared request being served
+    std::atomic<unsigned> n{0};        // its entry count
+    std::atomic<unsigned> use{1};      // threads that share it
+    std::atomic<unsigned> left{0};     // helpers still evaluating it
+    std::atomic<unsigned> helpers{0};  // helpers alive
+    std::atomic<bool> stop{false};
   };
-  void serve_velocities(const volatile int *stop, int w, int workers, VelocityJob *job, unsigned last);
+  cudaError_t serve_launch(VelocityJob *job);
+  void help_velocities(VelocityJob *job);
   void launch(long long limit);
   void write_snapshot();
   // host copies of the output fields of the current state
