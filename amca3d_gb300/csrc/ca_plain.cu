@@ -1566,7 +1566,7 @@ __device__ __forceinline__ void init_field(const PlainDevice &d, long long tid, 
   const Grid &g = d.grid;
   for (long long i = tid; i < d.ncells; i += stride) {
     int I, J, K;
-    cell_ijk(g, (int64_t)i, I, J, K);
+    cell_ijk(g, (int32_t)i, I, J, K);  // (cell ids are 32-bit everywhere)
     const bool ghost = I == 0 || J == 0 || K == 0 || I == g.nxg - 1 || J == g.nyg - 1 || K == g.nzg - 1;
     d.orient[i] = ghost ? 0u : kLiquid;
     d.cellw[i] = kNoEntry;
@@ -1683,18 +1683,27 @@ __global__ void batch_gather_kernel(const PlainDevice *insts, int ninst, PlainCt
   for (int w = threadIdx.x; w < (int)(sizeof(PlainCtrl) / 4); w += blockDim.x) dst[w] = src[w];
 }
 
-__global__ void grain_field_init_kernel(int32_t *out, const uint32_t *orient, Grid g, long long ncells) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ncells; i += (long long)gridDim.x * blockDim.x) {
+__global__ void grain_field_init_kernel(int32_t *out, Grid g, int ncells) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncells; i += gridDim.x * blockDim.x) {
     int I, J, K;
-    cell_ijk(g, (int64_t)i, I, J, K);
+    cell_ijk(g, i, I, J, K);
     const bool ghost = I == 0 || J == 0 || K == 0 || I == g.nxg - 1 || J == g.nyg - 1 || K == g.nzg - 1;
     out[i] = ghost ? 0 : -1;
   }
 }
 
-__global__ void grain_field_scatter_kernel(int32_t *out, const int32_t *gcell, long long ngrains) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ngrains; i += (long long)gridDim.x * blockDim.x)
-    out[gcell[i]] = (int32_t)i;
+// Four envelopes per thread: their cells are loaded at once, before the
+// scattered stores.
+__global__ void grain_field_scatter_kernel(int32_t *out, const int32_t *gcell, int ngrains) {
+  const int n4 = ngrains / 4, stride = gridDim.x * blockDim.x;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += stride) {
+    const int4 c = ((const int4 *)gcell)[q];
+    out[c.x] = 4 * q;
+    out[c.y] = 4 * q + 1;
+    out[c.z] = 4 * q + 2;
+    out[c.w] = 4 * q + 3;
+  }
+  for (int i = 4 * n4 + blockIdx.x * blockDim.x + threadIdx.x; i < ngrains; i += stride) out[gcell[i]] = i;
 }
 
 // One (envelope, cell) pair per thread: the FP64 containment test, the
@@ -2120,8 +2129,8 @@ cudaError_t plain_batch_gather(const PlainDevice *insts, int ninst, PlainCtrl *o
 }
 
 cudaError_t plain_grain_field(const PlainDevice &d, int32_t *out, long long ngrains, cudaStream_t s) {
-  grain_field_init_kernel<<<1024, 256, 0, s>>>(out, d.orient, d.grid, d.ncells);
-  if (ngrains > 0) grain_field_scatter_kernel<<<1024, 256, 0, s>>>(out, d.gcell, ngrains);
+  grain_field_init_kernel<<<152 * 8, 256, 0, s>>>(out, d.grid, (int)d.ncells);
+  if (ngrains > 0) grain_field_scatter_kernel<<<152 * 8, 256, 0, s>>>(out, d.gcell, (int)ngrains);
   return cudaGetLastError();
 }
 
