@@ -1209,7 +1209,7 @@ uint64_t gcd64(uint64_t a, uint64_t b) {
 // and the per-batch buffers of a training step.
 struct ThermalModel {
   using bf16 = __nv_bfloat16;
-  int device = 0;
+  int device = 0, sms = 0;
   cudaStream_t stream = nullptr;
   SurParamLayout L;
   sur::DataSpec data{};
@@ -1224,6 +1224,11 @@ struct ThermalModel {
   int64_t ds_n = 0;
   int64_t adam_t = 0;
   int64_t seen = 0;
+  // evaluation buffers, kept for calls of up to kEvalRows rows (28 bytes each)
+  static constexpr int64_t kEvalRows = 1 << 21;
+  int64_t eval_rows = 0;
+  float *eval_buf = nullptr;
+  CUtensorMap tw[kSurLayers];  // the layers' weights, for the inference kernels
   // batch buffers
   int64_t nb = 0;
   int blocks = 0;                        // of the step kernel
@@ -1253,6 +1258,7 @@ struct ThermalModel {
     if (stream) cudaStreamSynchronize(stream);
     for (void *q : batch_allocs) cudaFree(q);
     for (void *q : allocs) cudaFree(q);
+    cudaFree(eval_buf);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -1334,6 +1340,12 @@ struct ThermalModel {
       const int K = SurParamLayout::in_dim(l);
       Wb[l] = alloc<bf16>((size_t)kSurHid * K);
     }
+    for (int l = 0; l < kSurLayers; ++l) tw[l] = sur::tmap_bf16(Wb[l], kSurHid, SurParamLayout::in_dim(l), 256);
+    SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    SCK(cudaFuncSetAttribute(sur::mlp_infer_kernel<sur::kSrcArray>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sur::kInferSmem));
+    SCK(cudaFuncSetAttribute(sur::mlp_infer_kernel<sur::kSrcFrames>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sur::kInferSmem));
     SCK(cudaFuncSetAttribute(sur::mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sur::kTrainSmem));
     SCK(cudaFuncSetAttribute(sur::mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sur::kWgradSmem));
     err = alloc<int>(1);
@@ -1357,6 +1369,24 @@ struct ThermalModel {
     SCK(cudaStreamSynchronize(stream));
   }
 
+  // Device buffer for an evaluation of n rows (raw inputs, T, error estimate),
+  // kept for the calls after it; null for more than kEvalRows rows.
+  float *eval_buffer(int64_t n) {
+    if (n > kEvalRows) return nullptr;
+    if (n > eval_rows) {
+      SCK(cudaStreamSynchronize(stream));
+      cudaFree(eval_buf);
+      eval_buf = nullptr;
+      eval_rows = 0;
+      const int64_t rows = std::min<int64_t>(kEvalRows, std::max<int64_t>(1024, n + n / 4));
+      void *q = nullptr;
+      SCK(cudaMalloc(&q, (size_t)rows * (kSurIn + 2) * 4));
+      eval_buf = (float *)q;
+      eval_rows = rows;
+    }
+    return eval_buf;
+  }
+
   // Per-batch buffers and tensor maps for batches of n rows (n a multiple of 128).
   void set_batch(int64_t n) {
     if (n == nb) return;
@@ -1370,8 +1400,6 @@ struct ThermalModel {
     pieces = 1;
     while (pieces < 64 && kblocks % (pieces * 2) == 0 && kblocks / (pieces * 2) >= 8) pieces *= 2;
     per = (int)(n / sur::kWgradRows / pieces);
-    int sms = 0;
-    SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     width = kSurHid;
     while (width > 64 && sur::wgrad_items(width) * pieces < sms) width /= 2;
     blocks = (int)std::min<int64_t>(n / 128, sms);
@@ -1527,11 +1555,8 @@ void produce_frames(ThermalModel *model, sur::FrameJob job, cudaStream_t s) {
   if (!job.counters) job.counters = model->counters;
   InferArgs ia{};
   ia.error = model->err;
-  CUtensorMap tw[kSurLayers];
-  for (int l = 0; l < kSurLayers; ++l) tw[l] = tmap_bf16(model->Wb[l], kSurHid, SurParamLayout::in_dim(l), 256);
-  int sms = 0;
-  SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, model->device));
-  SCK(cudaFuncSetAttribute(mlp_infer_kernel<kSrcFrames>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem));
+  const CUtensorMap *tw = model->tw;
+  const int sms = model->sms;
   const int f_end = job.f0 + job.nf;
   for (int f = job.f0; f < f_end; f += kJobFrames) {
     ia.job = job;
@@ -1702,9 +1727,9 @@ int amca_thermal_eval(amca_thermal *h, const float *raw, int64_t n, float *T, fl
     SCK(cudaSetDevice(m.device));
     if (n == 0) return;
     DeviceBuffers tmp;
-    float *d_raw = (float *)tmp.get((size_t)n * amca::kSurIn * 4);
-    float *d_T = (float *)tmp.get((size_t)n * 4);
-    float *d_e = (float *)tmp.get((size_t)n * 4);
+    float *d_raw = m.eval_buffer(n);  // allocating and freeing per call cost a 100,000-row call about a third of its time
+    if (!d_raw) d_raw = (float *)tmp.get((size_t)n * (amca::kSurIn + 2) * 4);
+    float *d_T = d_raw + (size_t)n * amca::kSurIn, *d_e = d_T + n;
     SCK(cudaMemcpyAsync(d_raw, raw, (size_t)n * amca::kSurIn * 4, cudaMemcpyHostToDevice, m.stream));
     SCK(cudaMemsetAsync(m.err, 0, sizeof(int), m.stream));
     InferArgs ia{};
@@ -1713,21 +1738,13 @@ int amca_thermal_eval(amca_thermal *h, const float *raw, int64_t n, float *T, fl
     ia.T = d_T;
     ia.err = d_e;
     ia.error = m.err;
-    CUtensorMap tw[amca::kSurLayers];
-    for (int l = 0; l < amca::kSurLayers; ++l)
-      tw[l] = tmap_bf16(m.Wb[l], amca::kSurHid, amca::SurParamLayout::in_dim(l), 256);
-    int sms = 0;
-    SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device));
-    SCK(cudaFuncSetAttribute(mlp_infer_kernel<kSrcArray>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kInferSmem));
-    const int64_t tiles = (n + 127) / 128;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sms));
-    mlp_infer_kernel<kSrcArray><<<grid, kInferThreads, kInferSmem, m.stream>>>(tw[0], tw[1], tw[2], tw[3], m.dev(), ia);
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 127) / 128, m.sms));
+    mlp_infer_kernel<kSrcArray><<<grid, kInferThreads, kInferSmem, m.stream>>>(m.tw[0], m.tw[1], m.tw[2], m.tw[3],
+                                                                               m.dev(), ia);
     SCK(cudaGetLastError());
     SCK(cudaMemcpyAsync(T, d_T, (size_t)n * 4, cudaMemcpyDeviceToHost, m.stream));
     SCK(cudaMemcpyAsync(err, d_e, (size_t)n * 4, cudaMemcpyDeviceToHost, m.stream));
-    SCK(cudaStreamSynchronize(m.stream));
-    m.check_error();
+    m.check_error();  // waits for the copies too
   });
 }
 
@@ -1745,8 +1762,7 @@ int amca_thermal_gradients(amca_thermal *h, const float *raw, const float *targe
     m.gradients();
     SCK(cudaMemcpyAsync(grad, m.g, (size_t)m.L.total * 4, cudaMemcpyDeviceToHost, m.stream));
     if (pred) SCK(cudaMemcpyAsync(pred, m.pred, (size_t)n * 2 * 4, cudaMemcpyDeviceToHost, m.stream));
-    SCK(cudaStreamSynchronize(m.stream));
-    m.check_error();
+    m.check_error();  // waits for the copies too
   });
 }
 
