@@ -663,6 +663,8 @@ void RemeltRealm::initialize() {
   d.fvel = alloc<double>(N);
   d.hard_idx = alloc<int32_t>(N);
   d.hard_T = alloc<double>(N);
+  d.hard_v = alloc<double>(std::min<size_t>(N, kHostVelCap));  // used while a request fits the mapped buffer
+  d.hard_L = alloc<double>(std::min<size_t>(N, kHostVelCap));
   {
     void *hv = nullptr;
     RCK(cudaHostAlloc(&hv, sizeof(HostVelocity), cudaHostAllocMapped));

@@ -276,6 +276,10 @@ __device__ __forceinline__ double ulp_of(double p) {  // |p| normal
   return e > 52 ? __longlong_as_double((e - 52) << 52) : 4.9406564584124654e-324;
 }
 
+__device__ __forceinline__ bool f64_nan(double x) {
+  return ((unsigned long long)__double_as_longlong(x) << 1) > 0xffe0000000000000ull;
+}
+
 // x^b for b in {1, 2, 3}, correctly rounded (square and cube through exact
 // two-products). `near` is raised when the exact power lies within 0.02 ulp
 // of a rounding midpoint: there glibc's pow, whose error bound is 0.52 ulp,
@@ -303,18 +307,27 @@ __device__ double ipow_checked(double x, int b, bool &near) {
 
 // compute_growth_velocity_with_temperature_input (ProblemPhysics.cpp:142-158).
 // `hard`: a term with a nonzero coefficient could round differently in glibc.
-__device__ double velocity(const RemeltDevice &d, double T, bool &hard) {
+// A zero coefficient's term is that zero (the powers are finite and positive:
+// dT below 1e100), without the dozen FP64 instructions of its power.
+// `near_v`: v itself is within 2^-30 of the host's value all the same (a
+// power is within an ulp of glibc's, the sum's cancellation bounded).
+__device__ double velocity(const RemeltDevice &d, double T, bool &hard, bool &near_v) {
   const double dT = d.Tm - T;
   double v = 0.0;
   hard = false;
+  near_v = false;
   if (dT > 0) {
     bool n1 = false, n2 = false, n3 = false;
-    const double p1 = ipow_checked(dT, d.b1, n1);
-    const double p2 = ipow_checked(dT, d.b2, n2);
-    const double p3 = ipow_checked(dT, d.b3, n3);
+    const bool all = f64_exponent(dT) > 1023 + 332;
+    const double t1 = d.a1 == 0 && !all ? d.a1 : d.a1 * ipow_checked(dT, d.b1, n1);
+    const double t2 = d.a2 == 0 && !all ? d.a2 : d.a2 * ipow_checked(dT, d.b2, n2);
+    const double t3 = d.a3 == 0 && !all ? d.a3 : d.a3 * ipow_checked(dT, d.b3, n3);
     hard = (d.a1 != 0 && n1) || (d.a2 != 0 && n2) || (d.a3 != 0 && n3);
-    v = d.a1 * p1 + d.a2 * p2 + d.a3 * p3;
+    v = t1 + t2 + t3;
     if (v < 0.0) v = 0.0;
+    const float terms = fabsf(f64_to_f32_rz(t1)) + fabsf(f64_to_f32_rz(t2)) + fabsf(f64_to_f32_rz(t3));
+    const float vf = f64_to_f32_rz(v);
+    near_v = vf > 1e-30f && terms < 65536.0f * vf;
   }
   return v;
 }
@@ -423,6 +436,25 @@ __device__ void host_wait_block(const RemeltDevice &d, RemeltCtrl *c) {
   __syncthreads();
 }
 
+// One thread's wait (bounded) for the answer to the block's last request.
+__device__ __noinline__ void host_wait_thread(const RemeltDevice &d, RemeltCtrl *c) {
+  const unsigned long long t0 = now_ns();
+  while (ld_acquire_sys(&d.host->seq_done) != s_host_seq) {
+    if (now_ns() - t0 > kWaitNs) {
+      atomicCAS(&c->error, 0, kRemeltErrHost);
+      return;
+    }
+    __nanosleep(64);
+  }
+}
+
+// The length of a cell whose velocity the host is still working out: a NaN
+// that no computation gives, with the request's slot in its low word.
+constexpr long long kLengthPending = 0x7ff4a11c00000000ll;
+__device__ __forceinline__ bool length_pending(double L) {
+  return (__double_as_longlong(L) & ~0xffffffffll) == kLengthPending;
+}
+
 __device__ __forceinline__ void elem_nodes(const int nn[3], int64_t e, int64_t nid[8]) {
   const int64_t ncx = nn[0] - 1, ncy = nn[1] - 1;
   const int64_t i = e % ncx, j = (e / ncx) % ncy, k = e / (ncx * ncy);
@@ -444,11 +476,13 @@ __device__ bool eval_T(const RemeltDevice &d, const double *th, int64_t c, doubl
   elem_nodes(d.nn, e, nid);
   const double nullMat = d.void_t + 0.00001;
   double t[8];
+  bool below = false;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     t[i] = th[nid[i]];
-    if (t[i] < nullMat) return false;
+    below = below || (f64_less(t[i], nullMat) && !f64_nan(t[i]));
   }
+  if (below) return false;
   T = hex8_interp64(t, d.pc[3 * c], d.pc[3 * c + 1], d.pc[3 * c + 2]);
   return true;
 }
@@ -1404,14 +1438,16 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
           ++exactT;
           eval_T(d, th, cell, T);
           {  // growth velocity of single_integration_step (Remelting.cpp:569-576)
-            bool hard = false;
+            bool hard = false, near_v = false;
             const double Targ = (T < d.Ts) ? d.Ts + 0.01 : T;
-            d.fvel[q] = velocity(d, Targ, hard);
+            const double vel = velocity(d, Targ, hard, near_v);
+            d.fvel[q] = vel;
             if (hard) {
               const unsigned slot = append_slot(&c->n_hard);
               if (slot < d.list_cap) {
                 d.hard_idx[slot] = (int32_t)q;
                 d.hard_T[slot] = Targ;
+                if (slot < (unsigned)kHostVelCap) d.hard_v[slot] = near_v ? vel : -1.0;
                 // the host's answer, slot `slot`, is taken in phase D
                 // (velocities are never negative)
                 d.fvel[q] = -1.0 - (double)slot;
@@ -1486,8 +1522,8 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     __shared__ double s_vmin;
     __shared__ int s_min_hard;
     if (tid == 0) {
-      bool h = false;
-      s_vmin = velocity(d, minT, h);
+      bool h = false, near_v = false;
+      s_vmin = velocity(d, minT, h, near_v);
       s_min_hard = h ? 1 : 0;
     }
     __syncthreads();
@@ -1566,13 +1602,56 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     auto grow_claim = [&](int32_t cell, int I, int J, int K, double vel) {
       grow_finish(grow_load(cell, I, J, K), vel);
     };
-    bool pending = false;  // a hard velocity of this thread waits for the host's answer
+    // A cell whose velocity the host is still working out, slot k of the
+    // request: its claims are made with the device's own value, which is within
+    // 2^-30 of the host's, when the FP32 test decides every candidate (its
+    // margin is 2^-14). The exact length follows in phase E (hard_L keeps the
+    // length before the step, the cell's own names the slot until then), so
+    // the host's 12 us answer time overlaps this phase, its barrier and most of
+    // E instead of standing in this one. False when the exact value is needed.
+    auto grow_early = [&](const GrowPre &p, unsigned k) {
+      const double v = d.hard_v[k];
+      if (v < 0) return false;
+      const double L = p.glen + dT * v;
+      const float L32 = f64_to_f32_rz(L);
+      if (!(L32 > 1e-30f)) return false;
+      const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(p.dx) + fabsf(p.dy) + fabsf(p.dz)) + d.coord_err;
+      uint32_t in = 0;
+      for (uint32_t cand = p.cand; cand; cand &= cand - 1) {
+        const int n = __ffs(cand) - 1;
+        int di, dj, dk;
+        nbr_offset(n, di, dj, dk);
+        ++tests;
+        const int f = captured_f32(p.m32, (float)di * d.h32 - p.dx, (float)dj * d.h32 - p.dy, (float)dk * d.h32 - p.dz,
+                                   errg, L32);
+        if (f < 0) return false;
+        in |= (uint32_t)f << n;
+      }
+      d.hard_L[k] = p.glen;
+      d.glen[p.cell] = __longlong_as_double(kLengthPending | (long long)k);
+      const int32_t mine = INT_MIN + sweep_pos(g, p.I, p.J, p.K);
+      for (; in; in &= in - 1) {
+        const int n = __ffs(in) - 1;
+        int di, dj, dk;
+        nbr_offset(n, di, dj, dk);
+        const int32_t nb = p.cell + dk * g.nxyg + dj * g.nxg + di;
+        if (atomicMin(&d.orient[nb], mine) == -1) {
+          const unsigned slot = append_slot(&c->n_claim);
+          if (slot < d.list_cap) d.claimed[slot] = nb;
+        }
+      }
+      return true;
+    };
+    bool pending = false;  // a hard velocity of this thread waits for the host's answer in this phase
+    bool owing = false;    // ... in phase E
     if (use0) {
       const double vel = d.fvel[q0];  // (the chunked host path rewrites it in the dt phase)
-      if (vel < 0)
-        pending = true;
-      else
+      if (!(vel < 0))
         grow_finish(pre0, vel);
+      else if (grow_early(pre0, (unsigned)(-1.0 - vel)))
+        owing = true;
+      else
+        pending = true;
     }
     for (int64_t q = q0 + spread_stride(0); q < nf && nf <= d.list_cap; q += spread_stride(0)) {
       const int32_t cell = d.flagged[par][q];
@@ -1581,11 +1660,12 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
       if (ghost(g, I, J, K)) continue;
       if (d.grain[cell] < 0) continue;
       const double vel = d.fvel[q];
-      if (vel < 0) {
+      if (!(vel < 0))
+        grow_claim(cell, I, J, K, vel);
+      else if (grow_early(grow_load(cell, I, J, K), (unsigned)(-1.0 - vel)))
+        owing = true;
+      else
         pending = true;
-        continue;
-      }
-      grow_claim(cell, I, J, K, vel);
     }
     if (overlap && __syncthreads_or(pending)) {  // uniform within the block
       host_wait_block(d, c);
@@ -1596,6 +1676,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         int I, J, K;
         cell_ijk(g, cell, I, J, K);
         if (ghost(g, I, J, K) || d.grain[cell] < 0) continue;
+        if (length_pending(d.glen[cell])) continue;  // claimed already
         const double v = ld_volatile(&d.host->v[(unsigned)(-1.0 - vel)]);
         if (q == q0 && use0)
           grow_finish(pre0, v);  // loaded ahead, still current (only this thread grows the cell)
@@ -1624,7 +1705,13 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
           int I, J, K;
           cell_ijk(g, nb, I, J, K);
           const int32_t ori = d.gori[wc];
-          const double px = d.gx[wc], py = d.gy[wc], pz = d.gz[wc], L = d.glen[wc];
+          const double px = d.gx[wc], py = d.gy[wc], pz = d.gz[wc];
+          double L = ld_volatile(&d.glen[wc]);
+          if (length_pending(L)) {  // (its own thread may be writing the same value meanwhile)
+            host_wait_thread(d, c);
+            const unsigned k = (unsigned)__double_as_longlong(L);
+            L = d.hard_L[k] + dT * ld_volatile(&d.host->v[k]);
+          }
           const double ccx = centre_coord(g.x0, g.h, I), ccy = centre_coord(g.y0, g.h, J),
                        ccz = centre_coord(g.z0, g.h, K);
           double out[4];
@@ -1759,6 +1846,18 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
             ++eactive;
           }
         }
+      }
+    }
+    // the lengths that this block's cells still owe
+    if (__syncthreads_or(owing)) {
+      host_wait_block(d, c);
+      for (int64_t q = q0; q < nf; q += spread_stride(0)) {
+        if (!(d.fvel[q] < 0)) continue;
+        const int32_t cell = d.flagged[par][q];
+        const double L = d.glen[cell];
+        if (!length_pending(L)) continue;
+        const unsigned k = (unsigned)__double_as_longlong(L);
+        d.glen[cell] = d.hard_L[k] + dT * ld_volatile(&d.host->v[k]);
       }
     }
     if (gtid == 0) {

@@ -151,7 +151,9 @@ struct RemeltDevice {
   int32_t *newcell;
   double *fvel;              // growth velocity per flagged-list entry
   int32_t *hard_idx;         // flagged-list entries whose velocity the host evaluates
-  double *hard_T;
+  double *hard_T;            // ... their temperatures,
+  double *hard_v;            // the device's own velocities (-1: not near enough to claim with),
+  double *hard_L;            // and the cells' lengths before the step
   HostVelocity *host;        // device view of the mapped host buffer
   int host_cap;              // entries of `host` one request may use (kHostVelCap; smaller in tests)
   int64_t list_cap;
