@@ -662,7 +662,8 @@ __device__ __noinline__ void check_around(const PlainDevice &d, int cur, long lo
 __device__ __noinline__ void flush_zero_buffer(const PlainDevice &d, int zpar) {
   __syncthreads();
   const unsigned nz = s_nz < (unsigned)kZeroBuf ? s_nz : (unsigned)kZeroBuf;
-  if (threadIdx.x == 0 && nz) s_zbase = atomicAdd(&d.ctrl->zn[zpar], (unsigned long long)nz);
+  if (nz == 0) return;
+  if (threadIdx.x == 0) s_zbase = atomicAdd(&d.ctrl->zn[zpar], (unsigned long long)nz);
   __syncthreads();
   for (unsigned i = threadIdx.x; i < nz; i += kBlock) d.zlist[zpar][s_zbase + i] = s_zero[i];
 }
@@ -701,11 +702,12 @@ __device__ __forceinline__ bool site_tiles(const PlainDevice &d) { return d.nsit
 
 // ---------------------------------------------------------------------------
 // Nucleation (CellularAutomataManager.cpp:219-297) in site order.
-// Tiled sites: one pass, nucleus ranks from one block scan plus the look-back
-// over the site tiles. Otherwise pass 1 marks sites (2 = nucleates now, 0 =
+// Tiled sites: part of the wake scan (one block scan and one look-back give
+// both the woken entries' and the nuclei's ranks). Otherwise here: pass 1
+// marks sites (2 = nucleates now, 0 =
 // removed) and pass 2 hands out orientation / envelope ids in site order.
 // The counts that every block tracks itself (orientations, envelope ids,
-// liquid cells) are not read here; the last site tile publishes the active
+// liquid cells) are not read here; the last block publishes the active
 // count in the step's parity slot (a step without envelopes has no barrier
 // before the next nucleation), which every block reads after the barrier.
 // ---------------------------------------------------------------------------
@@ -727,9 +729,26 @@ __device__ __forceinline__ void step_rates(const PlainDevice &d, double time, do
 }
 
 // Nuclei go to the list from position base_pos on.
+// This thread's site of the block's tile: its cell when it nucleates this
+// step, else -1; sites that nucleate or are solid leave the tile.
+__device__ __forceinline__ int tiled_nucleus(const PlainDevice &d, double time, int *s_cell, const double *s_dtc,
+                                             unsigned long long *stat_live) {
+  const int cell = s_cell[threadIdx.x];
+  if (cell < 0) return -1;
+  const double T = d.T0 + d.Tdot * time;  // compute_cell_temperature (ProblemPhysics.cpp:164-169)
+  ++*stat_live;
+  const bool liquid = d.orient[cell] == kLiquid;
+  const bool nuc = liquid && d.Tm - T > s_dtc[threadIdx.x];
+  if (!liquid || nuc) {  // removed from the site list
+    s_cell[threadIdx.x] = -1;
+    d.site_live[(long long)t_b * kBlock + threadIdx.x] = 0;
+  }
+  return nuc ? cell : -1;
+}
+
 __device__ __noinline__ bool nucleation_phase(const PlainDevice &d, int cur, double time, long long step, long long base_pos,
-                                 long long base_orient, long long base_grain, int *s_cell, double *s_dtc,
-                                 unsigned long long *smem, unsigned long long *stat_live) {
+                                 long long base_orient, long long base_grain, unsigned long long *smem,
+                                 unsigned long long *stat_live) {
   PlainCtrl *c = d.ctrl;
   unsigned long long *scan = d.scanA + (step & 1) * kStatusWords;
   const double T = d.T0 + d.Tdot * time;  // compute_cell_temperature (ProblemPhysics.cpp:164-169)
@@ -738,31 +757,6 @@ __device__ __noinline__ bool nucleation_phase(const PlainDevice &d, int cur, dou
   // previous step's nucleation, which every block finished before that
   // phase's barrier
   if (threadIdx.x == 0) d.scanA[((step + 1) & 1) * kStatusWords + t_b] = 0ull;
-  if (site_tiles(d)) {
-    const long long ntiles = (d.nsites + kBlock - 1) / kBlock;
-    if (t_b >= ntiles) {  // no sites in this block
-      if (ntiles == 0 && t_b == 0 && threadIdx.x == 0) c->n_active_nuc[step & 1] = base_pos;
-      return true;
-    }
-    const int cell = s_cell[threadIdx.x];
-    unsigned nuc = 0;
-    if (cell >= 0) {
-      ++*stat_live;
-      const bool liquid = d.orient[cell] == kLiquid;
-      nuc = liquid && dTu > s_dtc[threadIdx.x];
-      if (!liquid || nuc) {  // removed from the site list
-        s_cell[threadIdx.x] = -1;
-        d.site_live[(long long)t_b * kBlock + threadIdx.x] = 0;
-      }
-    }
-    unsigned long long agg;
-    const unsigned long long ex = block_exclusive_scan(nuc, smem, &agg);
-    const unsigned long long pre = block_prefix(scan, agg, smem, c);
-    if (pre == ~0ull) return false;
-    if (nuc) place_nucleus(d, cur, base_pos, base_orient, base_grain, (long long)(pre + ex), cell, step);
-    if (t_b == ntiles - 1 && threadIdx.x == 0) c->n_active_nuc[step & 1] = base_pos + (long long)(pre + agg);
-    return true;
-  }
   long long b, e;
   block_chunk(d.nsites, b, e);
   unsigned long long count = 0;
@@ -837,7 +831,10 @@ __device__ __forceinline__ unsigned woken4(const float4 v, long long p0, long lo
   return (p0 < n && woken(v.x, gf, all) ? 1u : 0u) | (p0 + 1 < n && woken(v.y, gf, all) ? 2u : 0u) |
          (p0 + 2 < n && woken(v.z, gf, all) ? 4u : 0u) | (p0 + 3 < n && woken(v.w, gf, all) ? 8u : 0u);
 }
+// The list positions appended by nuclei follow the n scanned ones; `nuc_cell`:
+// the cell this thread's site nucleates on (tiled sites), or -1.
 __device__ __noinline__ bool wake_scan(const PlainDevice &d, int cur, long long n, long long step, double grown, bool all,
+                                       bool tiled, int nuc_cell, long long base_orient, long long base_grain,
                                        unsigned long long *smem) {
   PlainCtrl *c = d.ctrl;
   // the next step's words start cleared (last read in the previous step)
@@ -858,9 +855,16 @@ __device__ __noinline__ bool wake_scan(const PlainDevice &d, int cur, long long 
     cnt += __popc(woken4(k4[t * (kKeyTile / 4) + lane], p0, n, gf, all));
   }
   cnt = __reduce_add_sync(0xffffffffu, cnt);
-  unsigned long long total = 0;
-  unsigned long long off = warp_offset(cnt, d.scanC + (step & 1) * kStatusWords, smem, &total, c);
-  if (off == ~0ull) return false;
+  // (woken << 32 | nuclei) of the block, and of the threads before
+  unsigned long long agg;
+  const unsigned long long ex = block_exclusive_scan(
+      ((unsigned long long)((threadIdx.x & 31) == 0 ? cnt : 0u) << 32) | (nuc_cell >= 0 ? 1u : 0u), smem, &agg);
+  const unsigned long long pre = block_prefix(d.scanC + (step & 1) * kStatusWords, agg, smem, c);
+  if (pre == ~0ull) return false;
+  const unsigned long long total = pre + agg;
+  unsigned long long off = (pre >> 32) + (__shfl_sync(0xffffffffu, ex, 0) >> 32);
+  if (nuc_cell >= 0)
+    place_nucleus(d, cur, n, base_orient, base_grain, (long long)((pre + ex) & 0xffffffffull), nuc_cell, step);
 #pragma unroll 2
   for (long long t = wb; t < we; ++t) {
     const long long p0 = t * kKeyTile + 4 * lane;
@@ -875,7 +879,10 @@ __device__ __noinline__ bool wake_scan(const PlainDevice &d, int cur, long long 
     for (unsigned bits = f; bits; bits &= bits - 1) d.wlist[at++] = (int32_t)(p0 + __ffs(bits) - 1);
     off += __shfl_sync(0xffffffffu, x, 31);
   }
-  if (t_b == t_nb - 1 && threadIdx.x == 0) c->n_woken[step & 1] = (long long)total;
+  if (t_b == t_nb - 1 && threadIdx.x == 0) {
+    c->n_woken[step & 1] = (long long)(total >> 32);
+    if (tiled) c->n_active_nuc[step & 1] = n + (long long)(total & 0xffffffffull);
+  }
   return true;
 }
 
@@ -936,11 +943,13 @@ __device__ __forceinline__ void flush_departures(PlainCtrl *c, long long step, u
 // one processed this step outlived its turn (it goes next step); a sleeping
 // one goes now if generation 0 emptied it and no capture by a later rank did
 // so too, else next step.
-__device__ __noinline__ void zero_decisions(const PlainDevice &d, int cur, int zpar, int of, long long step,
+__device__ __noinline__ void zero_decisions(const PlainDevice &d, int cur, int zpar, int of, long long step, int threads,
                                             unsigned *now, unsigned *next) {
+  // from the last thread of every block down: the first ones mark their ranks
+  // meanwhile (a chain of five dependent loads, 2 us in front of the marking)
   const unsigned long long nz = ld_volatile(&d.ctrl->zn[zpar]);
-  for (unsigned long long i = (unsigned long long)t_b * kBlock + threadIdx.x; i < nz;
-       i += (unsigned long long)t_nb * kBlock) {
+  for (unsigned long long i = (unsigned long long)(kBlock - 1 - threadIdx.x) * t_nb + t_b; i < nz;
+       i += (unsigned long long)t_nb * threads) {
     const int q = d.zlist[zpar][i];
     const bool processed = d.lstep[cur][q] == (int32_t)step;
     if (of < 0 ? processed : isnan(d.key[cur][q])) continue;
@@ -1184,7 +1193,10 @@ __device__ __noinline__ bool resolve_phase(const PlainDevice &d, int cur, long l
                                            unsigned long long *smem,
                                            unsigned *gone_now, unsigned *gone_next) {
   PlainCtrl *c = d.ctrl;
-  zero_decisions(d, cur, zdec, zof, step, gone_now, gone_next);
+  // (a generation that the blocks' first halves can mark leaves it to the others)
+  const int zthreads = n <= (long long)(kBlock / 2) * t_nb ? kBlock / 2 : kBlock;
+  if (zdec >= 0 && (int)threadIdx.x >= kBlock - zthreads)
+    zero_decisions(d, cur, zdec, zof, step, zthreads, gone_now, gone_next);
   if (t_b == 0 && threadIdx.x == 0) c->zn[zreset] = 0ull;  // last read in the previous resolve phase
   long long b, e;
   block_chunk(n, b, e);
@@ -1266,6 +1278,7 @@ struct RealmState {
   int cur, done;
   // the step in progress
   double da, dn, dv, grown_s;
+  double rate_time, next_vel, next_da, next_dn;  // step_rates of the next step (rate_time: its time, NaN before any)
   int all;
   long long nucs, n, lo, processed, gen_end, caps_all, died;
   unsigned gen;
@@ -1303,6 +1316,7 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
     S.cur = ld_volatile(&c->cur_list);
     S.done = ld_volatile(&c->done) != 0;
     S.t_end = (d.t_stop > 0 && d.t_stop < d.final_time) ? d.t_stop : d.final_time;
+    S.rate_time = __longlong_as_double(0x7ff8000000000000ll);
     S.claim_busy = S.resolve_busy = S.nuc_busy = S.wake_busy = S.compact_busy = 0ull;
     S.t_mark = now_ns();
   }
@@ -1333,7 +1347,13 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
     // --- calculate_time_step (CellularAutomataManager_3D.cpp:441-511) ---
     if (threadIdx.x == 0) {
       double vel;
-      step_rates(d, S.time, vel, S.da, S.dn);
+      if (S.rate_time == S.time) {
+        vel = S.next_vel;
+        S.da = S.next_da;
+        S.dn = S.next_dn;
+      } else {
+        step_rates(d, S.time, vel, S.da, S.dn);
+      }
       // growth of every envelope this step (when there is one); the wake
       // scan compares the keys with the cumulative growth
       S.dv = S.da * vel;
@@ -1342,13 +1362,13 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
       if (t_b == 0) d.dvh[S.step & (kDvRing - 1)] = S.dv;
     }
     __syncthreads();
-    // the wake scan first: every block publishes its part of the scan at
-    // once, while only the blocks holding sites take part in nucleation's.
     const unsigned long long tn0 = threadIdx.x == 0 ? now_ns() : 0ull;
-    if (!(ok = wake_scan(d, S.cur, S.a_len, S.step, S.grown_s, S.all != 0, smem))) break;
-    const unsigned long long tn1 = threadIdx.x == 0 ? now_ns() : 0ull;
-    if (!(ok = nucleation_phase(d, S.cur, S.time, S.step, S.a_len, S.n_orient, S.grain, s_cell, s_dtc, smem, &live)))
+    const bool tiled = site_tiles(d);
+    const int nuc_cell = tiled ? tiled_nucleus(d, S.time, s_cell, s_dtc, &live) : -1;
+    if (!(ok = wake_scan(d, S.cur, S.a_len, S.step, S.grown_s, S.all != 0, tiled, nuc_cell, S.n_orient, S.grain, smem)))
       break;
+    const unsigned long long tn1 = threadIdx.x == 0 ? now_ns() : 0ull;
+    if (!tiled && !(ok = nucleation_phase(d, S.cur, S.time, S.step, S.a_len, S.n_orient, S.grain, smem, &live))) break;
     // the list of generation 0's checks (last read in an earlier step)
     if (timer) c->zn[1] = 0ull;
     if (threadIdx.x == 0) {
@@ -1400,6 +1420,13 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
         S.processed += S.n;
         S.t_work = now_ns();
       }
+      // the next step's time and rates are known by now; the last warp, which
+      // a small generation leaves free, works them out (1.5 us of FP64) beside
+      // the claims instead of at the step's start
+      if (threadIdx.x == kBlock - 1 && S.gen == 0) {
+        S.rate_time = S.time + S.dt;
+        step_rates(d, S.rate_time, S.next_vel, S.next_da, S.next_dn);
+      }
       // (and the envelopes around the previous generation's captures, or the nuclei)
       claim_phase(d, S.cur, S.gen ? 1 : 0, S.lo, S.n, S.gen & 1u, S.list, S.step, S.grown, S.gen ? S.n : S.nucs,
                   (int)((S.gen - 1) & 1u), &tests, &tests64, &dec);
@@ -1436,7 +1463,7 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
         if (threadIdx.x == 0) S.t_work = now_ns();
         __syncthreads();
       }
-      if (!(ok = resolve_phase(d, S.cur, S.n, S.step, S.gen & 1u, S.list, (int)((S.gen - 1) & 1u), (int)S.gen - 1,
+      if (!(ok = resolve_phase(d, S.cur, S.n, S.step, S.gen & 1u, S.list, S.gen || S.nucs ? (int)((S.gen - 1) & 1u) : -1, (int)S.gen - 1,
                                (int)(S.gen & 1u), smem, &gone_now, &gone_next)))
         break;
       flush_departures(c, S.step, gone_now, gone_next);

@@ -39,11 +39,9 @@ namespace {
 
 thread_local std::string g_create_error;
 
-// Interior cells up to which a plain realm runs 2 (kTinyRealmCells) or 3
-// (kSmallRealmCells) blocks per SM instead of the kernel's full occupancy
-// (see initialize).
-constexpr long long kTinyRealmCells = 4200000ll;
-constexpr long long kSmallRealmCells = 8ll << 20;
+// Interior cells up to which a plain realm runs 1, 2 and 3 blocks per SM
+// instead of the kernel's full occupancy (see initialize).
+constexpr long long kRealmCells1 = 1500000ll, kRealmCells2 = 4200000ll, kRealmCells3 = 8ll << 20;
 
 }  // namespace
 
@@ -269,12 +267,14 @@ struct amca_t {
     {
       // Blocks per SM of the persistent launch: a small realm's generations
       // are short, so its steps are set by barrier and look-back latency,
-      // which fall with the number of blocks (GB300, blocks per SM 2 / 3 /
-      // 4: 128^3 17.2 / 17.9 / 19.0 ms, 160^3 21.4 / 21.8, 200^3 29.0 /
-      // 27.8, 256^3 44.6 / 42.4 / 41.9, 320^3 70.8 / 64.6 / 63.0).
+      // which fall with the number of blocks (GB300, blocks per SM 1 / 2 / 3 /
+      // 4: 24^3 6.2 / 6.5 / 7.0 / 7.5 ms, 60^3 12.5 / 13.5 / 14.2 / 15.0, 95^3
+      // 14.7 / 15.3 / 16.0 / 16.9, 128^3 18.5 / 17.9 / 18.2 / 18.9, 160^3 24.5
+      // / 21.9 / 21.8 / 22.3, 200^3 34.0 / 28.3 / 26.9 / 26.9, 256^3 56.1 /
+      // 42.1 / 38.5 / 37.6, 320^3 94.7 / 64.4 / 55.4 / 52.3).
       // AMCA_PLAIN_BLOCKS_PER_SM overrides the choice.
       const long long interior = (long long)c.nx * c.ny * c.nz;
-      int per_sm = interior <= kTinyRealmCells ? 2 : interior <= kSmallRealmCells ? 3 : 0;
+      int per_sm = interior <= kRealmCells1 ? 1 : interior <= kRealmCells2 ? 2 : interior <= kRealmCells3 ? 3 : 0;
       if (const char *e = getenv("AMCA_PLAIN_BLOCKS_PER_SM")) per_sm = std::max(1, atoi(e));
       if (per_sm > 0) {
         int sms = 0;
