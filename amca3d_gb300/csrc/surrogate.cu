@@ -47,23 +47,43 @@ using bf16 = __nv_bfloat16;
 constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s: every mbarrier wait
 constexpr int kErrWait = 1;
 
-// fast reciprocal (MUFU) on an argument kept below 2^126 (z >= -80)
-__device__ __forceinline__ float sigmoid(float z) { return __fdividef(1.0f, 1.0f + __expf(-fmaxf(z, -80.0f))); }
+// 1 / (1 + e^-z) from the MUFU's 2^x and 1/x, e^-z = 2^(-z log2 e), z >= -80 so
+// that every value stays finite. Flushing variants: a 2^x below 2^-126 leaves 1
+// + 2^x at 1 either way, and the denormal and range handling of __expf and
+// __fdividef was a third of the instructions of an epilogue (equal to
+// __fdividef(1, 1 + __expf(-z)) for every float z).
+__device__ __forceinline__ float sigmoid(float z) {
+  float e, s;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * fmaxf(z, -80.0f)));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(1.0f + e));
+  return s;
+}
 __device__ __forceinline__ float silu(float z) { return z * sigmoid(z); }
 __device__ __forceinline__ float silu_grad(float z) {
   const float s = sigmoid(z);
   return s * (1.0f + z * (1.0f - s));
 }
 
-// Phase j of one raw input: sv = sin(2 pi f_j), cv = cos(2 pi f_j),
-// f_j = sum_i B[j][i] u_i (FP32, i ascending), u = (raw - shift) * scale.
-__device__ __forceinline__ void phases(const SurModelDev &m, const float raw[kSurIn], int j, float &sv, float &cv) {
-  float u[kSurIn];
+// Normalised inputs u = (raw - shift) * scale of one raw input.
+__device__ __forceinline__ void normalise(const SurModelDev &m, const float raw[kSurIn], float u[kSurIn]) {
 #pragma unroll
   for (int i = 0; i < kSurIn; ++i) u[i] = (raw[i] - m.in_shift[i]) * m.in_scale[i];
+}
+
+// Fourier matrix in shared memory, a row in 8 floats (two aligned loads).
+constexpr int kFourierPad = 8;
+__device__ __forceinline__ void load_fourier(const SurModelDev &m, float (*B)[kFourierPad]) {
+  for (int i = threadIdx.x; i < kSurFreq * kSurIn; i += blockDim.x) B[i / kSurIn][i % kSurIn] = m.fourier[i];
+}
+
+// Phase of one input: sv = sin(2 pi f), cv = cos(2 pi f), f = sum_i B[i] u_i
+// (FP32, i ascending).
+__device__ __forceinline__ void phases(const float B[kFourierPad], const float u[kSurIn], float &sv, float &cv) {
+  const float4 b = *(const float4 *)B;
+  const float row[kSurIn] = {b.x, b.y, b.z, b.w, B[4]};
   float f = 0.0f;
 #pragma unroll
-  for (int i = 0; i < kSurIn; ++i) f = __fadd_rn(f, __fmul_rn(m.fourier[j * kSurIn + i], u[i]));
+  for (int i = 0; i < kSurIn; ++i) f = __fadd_rn(f, __fmul_rn(row[i], u[i]));
   sincospif(2.0f * f, &sv, &cv);
 }
 
@@ -119,14 +139,13 @@ __device__ __forceinline__ uint64_t sample_of(const StepArgs &a, uint64_t q) {
 // Forward and backward of 128-row tiles, persistent, one block per SM. Shared
 // memory: the tile's current activations or dZ (128 x 256 bf16) and one layer's
 // weights (256 x 256 bf16, streamed by TMA while the previous epilogue runs;
-// the backward pass reads the same [out][in] tiles as MN-major B operands). 512 threads: warp w reads TMEM lanes
-// 32 (w % 4) (its rows) and the 64-column group w / 4. An epilogue is bound by
-// its two MUFU operations per element (2.1 us a tile and layer), a layer's MMAs
-// take 1.35 us.
-// Head gradients: dL/dmu and dL/ds of a row are split into three bf16 terms
-// each, which hold all 24 bits of an FP32 value, so H4^T dpred runs on the
-// tensor cores with exact products and FP32 sums; it accumulates in TMEM over
-// the block's tiles.
+// the backward pass reads the same [out][in] tiles as MN-major B operands). 512
+// threads: warp w reads TMEM lanes 32 (w % 4) (its rows) and the 64-column group
+// w / 4. Bound by instruction issue in the features and epilogues (39% of the
+// slots) and by the MMAs between them (about 1.1 us a layer), which nothing
+// overlaps: 105 us for 32,768 rows with __expf and __fdividef and the Fourier
+// matrix in global memory, 88 with the two MUFU operations of sigmoid() and the
+// matrix in shared memory.
 __global__ void __launch_bounds__(kTrainThreads, 1)
     mlp_step_kernel(const __grid_constant__ TrainMaps tm, SurModelDev md, StepArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -139,7 +158,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   __shared__ __align__(16) float s_wh[kSurOut][kSurHid];
   __shared__ float s_bh[kSurOut];
   __shared__ float s_head[kTrainGroups][128][2];
-  __shared__ float s_raw[128][kSurIn], s_y[128], s_dp[128][2];
+  __shared__ float s_in[128][kSurIn], s_y[128], s_dp[128][2];  // s_in: normalised inputs
+  __shared__ __align__(16) float s_fourier[kSurFreq][kFourierPad];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q4 = warp & 3, grp = warp >> 2, row = q4 * 32 + lane;
@@ -153,6 +173,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     s_abort = 0;
   }
   if (warp == 0) umma::tmem_alloc(umma::smem_u32(&tmem_base), 256);
+  load_fourier(md, s_fourier);
   // the parameters may still be in the making (the previous step's update)
   umma::wait_prerequisites();
   for (int i = threadIdx.x; i < kSurLayers * kSurHid; i += blockDim.x)
@@ -207,22 +228,26 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
     if (grp == 0) {
       const uint64_t i = sample_of(a, (uint64_t)(tile * 128 + row));
+      float raw[kSurIn], u[kSurIn];
 #pragma unroll
-      for (int k = 0; k < kSurIn; ++k) s_raw[row][k] = a.raw[i * kSurIn + k];
+      for (int k = 0; k < kSurIn; ++k) raw[k] = a.raw[i * kSurIn + k];
+      normalise(md, raw, u);
+#pragma unroll
+      for (int k = 0; k < kSurIn; ++k) s_in[row][k] = u[k];
       s_y[row] = a.target[i];
     }
     if (threadIdx.x == 0) umma::bulk_wait_read();  // the previous tile's last store has left H
     __syncthreads();
     {
-      float raw[kSurIn];
+      float u[kSurIn];
 #pragma unroll
-      for (int k = 0; k < kSurIn; ++k) raw[k] = s_raw[row][k];
+      for (int k = 0; k < kSurIn; ++k) u[k] = s_in[row][k];
       for (int j0 = grp * (kSurFreq / kTrainGroups); j0 < (grp + 1) * (kSurFreq / kTrainGroups); j0 += 8) {
         __align__(16) bf16 sb[8], cb[8];
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
           float sv, cv;
-          phases(md, raw, j0 + t, sv, cv);
+          phases(s_fourier[j0 + t], u, sv, cv);
           sb[t] = __float2bfloat16_rn(sv);
           cb[t] = __float2bfloat16_rn(cv);
         }
@@ -892,11 +917,29 @@ __device__ __forceinline__ int64_t frame_query(const FrameJob &j, const FrameBox
 // nodes inside the grid: with all of them evaluated, 1,484 frames took 250 ms,
 // now a few; the whole run of that raster 458 -> 207 ms).
 // Shared memory: activations H (128 x 256 bf16, four 64-column blocks of
-// 16 KB) and one layer's weights (256 x 256 bf16, four blocks of 32 KB).
-// 512 threads: warp w reads TMEM lanes 32 (w % 4) (its rows) and handles the
-// 64-column group w / 4 of every layer's epilogue.
+// 16 KB) and one layer's weights (256 x 256 bf16, four blocks of 64 input
+// columns, 32 KB each).
+// 16 epilogue warps in four groups (warp w reads TMEM lanes 32 (w % 4), its
+// rows; group w / 4 has 64 columns of every layer), a warp that issues the MMAs
+// and one that loads weights. A layer's epilogue is bound by instruction issue
+// (about nine per element, 1.1 us a tile), its MMAs take as long; they overlap:
+//  - the MMAs over the first half of K run as soon as groups 0 and 1 have
+//    written it, while groups 2 and 3 still work on the layer before (into the
+//    other of two accumulators);
+//  - the MMAs over the second half of K finish output columns 0..127 first, so
+//    groups 0 and 1 start while columns 128..255 are still being computed;
+//  - a weight block is replaced by the next layer's as soon as its MMAs are
+//    done, long before it is needed.
+//  - the next tile's features are computed in registers while the second and
+//    third layers' MMAs run.
+// Group 3 also writes a tile's results and fetches the next tile's inputs,
+// behind the first layer's MMAs. Each accumulator still adds
+// its K steps in order. A tile took 19.5 us with everything one after another;
+// now 15.8 (100,003 queries from a cold cache: 117 -> 95 us; a layer's epilogue
+// takes 3.5K cycles of the 5.6K, its exposed MMAs 2K).
 // ---------------------------------------------------------------------------
-constexpr int kInferThreads = 512, kInferGroups = 4, kGroupCols = kSurHid / kInferGroups;
+constexpr int kInferGroups = 4, kGroupCols = kSurHid / kInferGroups, kIoGroup = 3;
+constexpr int kInferEpiWarps = 4 * kInferGroups, kInferThreads = 32 * (kInferEpiWarps + 2);
 enum { kSrcArray = 0, kSrcFrames = 1 };
 
 struct InferArgs {
@@ -917,198 +960,187 @@ __global__ void __launch_bounds__(kInferThreads, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t *H = align1024(smem_raw);
   uint8_t *Wsm = H + 64 * 1024;
-  __shared__ __align__(8) uint64_t wbar, mbar;
+  // weight block loaded / its MMAs done; half of the layer's input written (8
+  // warps); half of the accumulator complete; heads of a tile summed (16
+  // warps); inputs of a tile there (4 warps), by tile parity: a warp that is
+  // slow to look cannot miss one, the next of the parity waits for its heads
+  __shared__ __align__(8) uint64_t wfull[4], wfree[4], hready[2], acc[2], headed, fetched[2], drained;
   __shared__ uint32_t tmem_base;
-  __shared__ int s_abort;
+  __shared__ volatile int s_abort;
   __shared__ __align__(16) float s_bias[kSurLayers][kSurHid];
   __shared__ __align__(16) float s_wh[kSurOut][kSurHid];
   __shared__ float s_bh[kSurOut];
-  __shared__ float s_head[kInferGroups][128][2];
-  __shared__ float s_raw[SRC == kSrcFrames ? 128 : 1][kSurIn];
+  __shared__ float s_head[2][kInferGroups][128][2];  // by tile parity
+  __shared__ float s_in[2][128][kSurIn];             // normalised inputs, by tile parity
+  __shared__ __align__(16) float s_fourier[kSurFreq][kFourierPad];
   __shared__ FrameBox s_box[SRC == kSrcFrames ? kJobFrames : 1];
-  const CUtensorMap *tW[4] = {&tW0, &tW1, &tW2, &tW3};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q4 = warp & 3, grp = warp >> 2, row = q4 * 32 + lane;
   const int64_t nq = SRC == kSrcFrames ? frame_boxes(a.job, s_box) : a.nq;
   const int64_t ntiles = (nq + 127) / 128;
+  const int64_t tile0 = blockIdx.x, dtile = gridDim.x;
   const SurParamLayout L;
 
   for (int i = threadIdx.x; i < kSurLayers * kSurHid; i += blockDim.x)
     s_bias[i / kSurHid][i % kSurHid] = md.p[L.b[i / kSurHid] + i % kSurHid];
   for (int i = threadIdx.x; i < kSurOut * kSurHid; i += blockDim.x) s_wh[i / kSurHid][i % kSurHid] = md.p[L.Wh + i];
   if (threadIdx.x < kSurOut) s_bh[threadIdx.x] = md.p[L.bh + threadIdx.x];
+  load_fourier(md, s_fourier);
   if (threadIdx.x == 0) {
-    umma::mbar_init(umma::smem_u32(&wbar), 1);
-    umma::mbar_init(umma::smem_u32(&mbar), 1);
+    for (int k = 0; k < 4; ++k) {
+      umma::mbar_init(umma::smem_u32(&wfull[k]), 1);
+      umma::mbar_init(umma::smem_u32(&wfree[k]), 1);
+    }
+    for (int k = 0; k < 2; ++k) {
+      umma::mbar_init(umma::smem_u32(&hready[k]), kInferEpiWarps / 2);
+      umma::mbar_init(umma::smem_u32(&acc[k]), 1);
+      umma::mbar_init(umma::smem_u32(&fetched[k]), 4);
+    }
+    umma::mbar_init(umma::smem_u32(&headed), kInferEpiWarps);
+    umma::mbar_init(umma::smem_u32(&drained), 1);
     umma::mbar_fence_init();
     s_abort = 0;
   }
-  if (warp == 0) umma::tmem_alloc(umma::smem_u32(&tmem_base), 256);
+  if (warp == 0) umma::tmem_alloc(umma::smem_u32(&tmem_base), 512);
   umma::tc_fence_before();
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = tmem_base;
-  const uint32_t trow = tmem + ((uint32_t)(q4 * 32) << 16);
-  const uint32_t idesc = umma::idesc_bf16_f32(128, kSurHid);
-
-  auto load_w = [&](int l) {  // thread 0
-    const int kbs = SurParamLayout::in_dim(l) / 64;
-    const uint32_t bar = umma::smem_u32(&wbar);
-    umma::mbar_expect_tx(bar, (uint32_t)kbs * 32u * 1024u);
-    for (int kb = 0; kb < kbs; ++kb) umma::tma_load_2d(umma::smem_u32(Wsm + kb * 32 * 1024), tW[l], bar, kb * 64, 0);
+  auto wait = [&](uint64_t &bar, uint32_t parity) {
+    return umma::mbar_wait_role(umma::smem_u32(&bar), parity, kWaitNs, &s_abort);
   };
-  if (threadIdx.x == 0) {
-    for (int l = 0; l < 4; ++l) umma::tma_prefetch_desc(tW[l]);
-    if ((int64_t)blockIdx.x < ntiles) load_w(0);
-  }
-  uint32_t wph = 0, mph = 0;
-  bool ok = true;
 
-  for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    const int64_t qi = tile * 128 + row;
-    const bool valid = qi < nq;
-    float raw[kSurIn] = {0, 0, 0, 0, 0};
-    int fk = 0;
-    int64_t node = -1;
-    double nx = 0, ny = 0, nz = 0;
-    if (SRC == kSrcArray) {
-      if (valid)
+  if (warp == kInferEpiWarps + 1) {  // ---- weights ----
+    if (lane == 0) {
+      const CUtensorMap *tW[4] = {&tW0, &tW1, &tW2, &tW3};
+      uint32_t uses[4] = {0, 0, 0, 0};
+      bool ok = true;
+      for (int64_t tile = tile0; tile < ntiles && ok; tile += dtile)
+        for (int l = 0; l < kSurLayers && ok; ++l)
+          for (int kb = 0; kb < SurParamLayout::in_dim(l) / 64; ++kb) {
+            if (uses[kb] && !(ok = wait(wfree[kb], (uses[kb] - 1) & 1))) break;
+            const uint32_t bar = umma::smem_u32(&wfull[kb]);
+            umma::mbar_expect_tx(bar, 32u * 1024u);
+            umma::tma_load_2d(umma::smem_u32(Wsm + kb * 32 * 1024), tW[l], bar, kb * 64, 0);
+            ++uses[kb];
+          }
+      if (!ok)  // let the loads in flight land before the block exits
+        for (int kb = 0; kb < 4; ++kb)
+          if (uses[kb]) umma::mbar_wait(umma::smem_u32(&wfull[kb]), (uses[kb] - 1) & 1, kWaitNs);
+    }
+  } else if (warp == kInferEpiWarps) {  // ---- MMAs ----
+    if (lane == 0) {
+      constexpr uint32_t id_all = umma::idesc_bf16_f32(128, kSurHid), id_half = umma::idesc_bf16_f32(128, kSurHid / 2);
+      uint32_t uses[4] = {0, 0, 0, 0}, layers = 0;
+      bool ok = true;
+      // K block kb of the layer into accumulator columns d.. from weight row n0 on
+      auto mma = [&](uint32_t d, int kb, int n0, uint32_t idesc) {
+        const uint32_t ha = umma::smem_u32(H + kb * 16 * 1024), wa = umma::smem_u32(Wsm + kb * 32 * 1024 + n0 * 128);
 #pragma unroll
-        for (int i = 0; i < kSurIn; ++i) raw[i] = a.raw[qi * kSurIn + i];
-    } else {
-      // The first group works out the rows' nodes and raw inputs (along-track
-      // offset from the source, positive ahead of it, lateral offset, depth
-      // below the top surface, in m; power, W; speed, m/s) for all four groups,
-      // with the frame's source position at hand: an FP64 instruction holds its
-      // scheduler for 64 cycles on GB300, and about 110 of them in every one of
-      // the 16 warps (position, window corner and divisions per row) were most
-      // of a tile's 13.6 us.
-      if (grp == 0) {
-        if (valid) {
+        for (int k = 0; k < 4; ++k)
+          umma::mma_bf16(d + n0, umma::sdesc_sw128(ha + 32u * k), umma::sdesc_sw128(wa + 32u * k), idesc,
+                         (kb | k) != 0 ? 1u : 0u);
+      };
+      auto weights = [&](int kb) { return wait(wfull[kb], uses[kb]++ & 1); };
+      for (int64_t tile = tile0; tile < ntiles && ok; tile += dtile)
+        for (int l = 0; l < kSurLayers; ++l, ++layers) {
+          const uint32_t d = tmem + 256u * (l & 1);
+          const int first = l == 0 ? 0 : 2;  // K blocks from here on are computed half by half of the columns
+          if (!(ok = wait(hready[0], layers & 1))) break;
+          for (int kb = 0; kb < first && ok; ++kb) {
+            if (!(ok = weights(kb))) break;
+            umma::tc_fence_after();
+            mma(d, kb, 0, id_all);
+            umma::mma_commit(umma::smem_u32(&wfree[kb]));
+          }
+          if (!ok || !(ok = wait(hready[1], layers & 1) && weights(first) && weights(first + 1))) break;
+          umma::tc_fence_after();
+          for (int half = 0; half < 2; ++half) {
+            mma(d, first, 128 * half, id_half);
+            mma(d, first + 1, 128 * half, id_half);
+            umma::mma_commit(umma::smem_u32(&acc[half]));
+          }
+          umma::mma_commit(umma::smem_u32(&wfree[first]));
+          umma::mma_commit(umma::smem_u32(&wfree[first + 1]));
+        }
+      if (!ok) {  // nothing may still write to the tensor memory when it is given back
+        umma::mma_commit(umma::smem_u32(&drained));
+        umma::mbar_wait(umma::smem_u32(&drained), 0, kWaitNs);
+      }
+    }
+  } else {  // ---- features, epilogues, results ----
+    const int q4 = warp & 3, grp = warp >> 2, row = q4 * 32 + lane, half = grp >> 1;
+    const uint32_t trow = tmem + ((uint32_t)(q4 * 32) << 16);
+    // the io group's row of a tile: whether it is a query, and (frames) its frame's box and node
+    struct Row {
+      int64_t tile, node;
+      int k;
+      bool valid;
+    };
+    auto fetch = [&](int64_t tile, int par) {  // io group: the tile's raw inputs
+      Row r{tile, -1, 0, tile * 128 + row < nq};
+      const int64_t qi = tile * 128 + row;
+      float raw[kSurIn] = {0, 0, 0, 0, 0};
+      if (r.valid) {
+        if (SRC == kSrcArray) {
+#pragma unroll
+          for (int i = 0; i < kSurIn; ++i) raw[i] = a.raw[qi * kSurIn + i];
+        } else {
+          // Along-track offset from the source (positive ahead of it), lateral
+          // offset, depth below the top surface (m), power (W), speed (m/s),
+          // with the frame's source position at hand: an FP64 instruction holds
+          // its scheduler for 64 cycles on GB300, and about 110 of them in
+          // every warp (position, window corner and divisions per row) were
+          // most of a tile's 13.6 us.
           int I, J, K;
-          node = frame_query(a.job, s_box, qi, fk, I, J, K);
-          node_xyz(a.job, I, J, K, nx, ny, nz);
-          const FrameBox &fb = s_box[fk];
-          raw[0] = (float)((nx - fb.xl) * fb.dir);
-          raw[1] = (float)(ny - fb.yl);
-          raw[2] = (float)(a.job.src.z_top - nz);
+          double x, y, z;
+          r.node = frame_query(a.job, s_box, qi, r.k, I, J, K);
+          node_xyz(a.job, I, J, K, x, y, z);
+          const FrameBox &fb = s_box[r.k];
+          raw[0] = (float)((x - fb.xl) * fb.dir);
+          raw[1] = (float)(y - fb.yl);
+          raw[2] = (float)(a.job.src.z_top - z);
           raw[3] = (float)a.job.src.power;
           raw[4] = (float)a.job.src.speed;
         }
-#pragma unroll
-        for (int i = 0; i < kSurIn; ++i) s_raw[row][i] = raw[i];
       }
-      __syncthreads();
+      float u[kSurIn];
+      normalise(md, raw, u);
 #pragma unroll
-      for (int i = 0; i < kSurIn; ++i) raw[i] = s_raw[row][i];
-    }
-    // Fourier features: this group's 16 phases, sines at column j, cosines at 64 + j
-    for (int j0 = grp * (kSurFreq / kInferGroups); j0 < (grp + 1) * (kSurFreq / kInferGroups); j0 += 8) {
-      __align__(16) bf16 sb[8], cb[8];
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        float sv, cv;
-        phases(md, raw, j0 + t, sv, cv);
-        sb[t] = __float2bfloat16_rn(sv);
-        cb[t] = __float2bfloat16_rn(cv);
-      }
-      *(uint4 *)(H + umma::sw128_offset(row, j0, 128)) = *(const uint4 *)sb;
-      *(uint4 *)(H + umma::sw128_offset(row, kSurFreq + j0, 128)) = *(const uint4 *)cb;
-    }
-    umma::fence_async_smem();
-    umma::tc_fence_before();
-    __syncthreads();
-    float mu = 0.0f, sl = 0.0f;
-    for (int l = 0; l < kSurLayers; ++l) {
-      if (threadIdx.x == 0) {
-        const bool wok = umma::mbar_wait(umma::smem_u32(&wbar), wph, kWaitNs);
-        if (!wok) {
-          s_abort = 1;
-        } else {
-          umma::tc_fence_after();
-          const int kbs = SurParamLayout::in_dim(l) / 64;
-          for (int kb = 0; kb < kbs; ++kb) {
-            const uint32_t ha = umma::smem_u32(H + kb * 16 * 1024), wa = umma::smem_u32(Wsm + kb * 32 * 1024);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma::mma_bf16(tmem, umma::sdesc_sw128(ha + 32u * k), umma::sdesc_sw128(wa + 32u * k), idesc,
-                             (kb | k) != 0 ? 1u : 0u);
-          }
-        }
-        umma::mma_commit(umma::smem_u32(&mbar));
-      }
-      wph ^= 1u;
-      const bool mok = umma::mbar_wait(umma::smem_u32(&mbar), mph, kWaitNs);
-      mph ^= 1u;
-      ok = __syncthreads_and(mok ? 1 : 0) != 0 && !s_abort;
-      if (!ok) break;
-      umma::tc_fence_after();
-      // the weights are free again: stream in the next layer's (or the next tile's first) while the epilogue runs
-      if (threadIdx.x == 0 && (l < kSurLayers - 1 || tile + gridDim.x < ntiles)) load_w((l + 1) % kSurLayers);
-      for (int c0 = grp * kGroupCols; c0 < (grp + 1) * kGroupCols; c0 += 32) {
-        float v[32];
-        umma::tmem_ld32(trow + c0, v);
-        const float4 *b4 = reinterpret_cast<const float4 *>(&s_bias[l][c0]);
-        if (l < kSurLayers - 1) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            const float4 ba = b4[j / 4], bb = b4[j / 4 + 1];
-            const float b[8] = {ba.x, ba.y, ba.z, ba.w, bb.x, bb.y, bb.z, bb.w};
-            __align__(16) bf16 hb[8];
-#pragma unroll
-            for (int t = 0; t < 8; ++t) hb[t] = __float2bfloat16_rn(silu(v[j + t] + b[t]));
-            *(uint4 *)(H + umma::sw128_offset(row, c0 + j, 128)) = *(const uint4 *)hb;
-          }
-        } else {
-          const float4 *w0 = reinterpret_cast<const float4 *>(&s_wh[0][c0]);
-          const float4 *w1 = reinterpret_cast<const float4 *>(&s_wh[1][c0]);
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const float4 bq = b4[j / 4], m0 = w0[j / 4], m1 = w1[j / 4];
-            const float b[4] = {bq.x, bq.y, bq.z, bq.w}, x0[4] = {m0.x, m0.y, m0.z, m0.w},
-                        x1[4] = {m1.x, m1.y, m1.z, m1.w};
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const float h = silu(v[j + t] + b[t]);
-              mu = fmaf(h, x0[t], mu);
-              sl = fmaf(h, x1[t], sl);
-            }
-          }
-        }
-      }
-      if (l < kSurLayers - 1) umma::fence_async_smem();
-      umma::tc_fence_before();
-      __syncthreads();
-    }
-    if (!ok) break;
-    s_head[grp][row][0] = mu;
-    s_head[grp][row][1] = sl;
-    __syncthreads();
-    if (grp == 0) {  // whole warps
+      for (int i = 0; i < kSurIn; ++i) s_in[par][row][i] = u[i];
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(umma::smem_u32(&fetched[par]));
+      return r;
+    };
+    auto results = [&](const Row &r, int par) {  // io group (whole warps)
       float m = s_bh[0], s = s_bh[1];
 #pragma unroll
       for (int k = 0; k < kInferGroups; ++k) {
-        m += s_head[k][row][0];
-        s += s_head[k][row][1];
+        m += s_head[par][k][row][0];
+        s += s_head[par][k][row][1];
       }
       s = fminf(fmaxf(s, -12.0f), 4.0f);
       const float T = md.log_out ? md.t_shift + md.t_scale * expf(m) : md.t_shift + md.t_scale * m;
       const float e = md.log_out ? 2.0f * (T - md.t_shift) * expf(s) : 2.0f * md.t_scale * expf(s);
       if (SRC == kSrcArray) {
-        if (valid) {
-          a.T[qi] = T;
-          a.err[qi] = e;
+        if (r.valid) {
+          a.T[r.tile * 128 + row] = T;
+          a.err[r.tile * 128 + row] = e;
         }
       } else {
-        const bool near = valid && fabsf(T - a.job.t_liq) < a.job.band;
+        const bool near = r.valid && fabsf(T - a.job.t_liq) < a.job.band;
         const bool fb = near && e > a.job.thresh;
-        if (valid) {
+        if (r.valid) {
           double out = (double)T;
-          if (fb) out = scan_field(a.job.src, nx, ny, nz, s_box[fk].t);
-          a.job.ring[(int64_t)((a.job.f0 + fk) % a.job.slots) * a.job.nnodes + node] = out;
+          if (fb) {
+            double x, y, z;
+            const int64_t nx = a.job.nodes[0], ny = a.job.nodes[1];
+            node_xyz(a.job, r.node % nx, r.node / nx % ny, r.node / (nx * ny), x, y, z);
+            out = scan_field(a.job.src, x, y, z, s_box[r.k].t);
+          }
+          a.job.ring[(int64_t)((a.job.f0 + r.k) % a.job.slots) * a.job.nnodes + r.node] = out;
         }
-        const unsigned nv = __popc(__ballot_sync(0xffffffffu, valid));
+        const unsigned nv = __popc(__ballot_sync(0xffffffffu, r.valid));
         const unsigned nn = __popc(__ballot_sync(0xffffffffu, near));
         const unsigned nfb = __popc(__ballot_sync(0xffffffffu, fb));
         if (lane == 0) {
@@ -1117,13 +1149,116 @@ __global__ void __launch_bounds__(kInferThreads, 1)
           if (nfb) atomicAdd(&a.job.counters[2], (unsigned long long)nfb);
         }
       }
+    };
+    // this warp's part of the layer's input is written (and its TMEM reads are done)
+    auto written = [&]() {
+      umma::fence_async_smem();
+      umma::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(umma::smem_u32(&hready[half]));
+    };
+    // Fourier features of a tile's row: half h of this group's 16 phases (sines
+    // at column j, cosines at 64 + j), held in registers until H is free
+    uint4 fs[2], fc[2];
+    auto features = [&](int par, int h) {
+      float u[kSurIn];
+#pragma unroll
+      for (int i = 0; i < kSurIn; ++i) u[i] = s_in[par][row][i];
+      __align__(16) bf16 sb[8], cb[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        float sv, cv;
+        phases(s_fourier[grp * (kSurFreq / kInferGroups) + 8 * h + t], u, sv, cv);
+        sb[t] = __float2bfloat16_rn(sv);
+        cb[t] = __float2bfloat16_rn(cv);
+      }
+      fs[h] = *(const uint4 *)sb;
+      fc[h] = *(const uint4 *)cb;
+    };
+    Row cur{}, last{};
+    if (grp == kIoGroup && tile0 < ntiles) cur = fetch(tile0, 0);
+    uint32_t tiles = 0, layers = 0;
+    bool ok = true;
+    for (int64_t tile = tile0; tile < ntiles; tile += dtile, ++tiles) {
+      const int par = tiles & 1;
+      if (tiles == 0) {
+        if (!(ok = wait(fetched[0], 0))) break;
+        features(0, 0);
+        features(0, 1);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j0 = grp * (kSurFreq / kInferGroups) + 8 * h;
+        *(uint4 *)(H + umma::sw128_offset(row, j0, 128)) = fs[h];
+        *(uint4 *)(H + umma::sw128_offset(row, kSurFreq + j0, 128)) = fc[h];
+      }
+      written();
+      if (grp == kIoGroup) {
+        if (tiles > 0) {
+          if (!(ok = wait(headed, par ^ 1))) break;
+          results(last, par ^ 1);
+        }
+        last = cur;
+        // (every warp has read the inputs of the tile before: it has its heads)
+        if (tile + dtile < ntiles) cur = fetch(tile + dtile, par ^ 1);
+      }
+      float mu = 0.0f, sl = 0.0f;
+      for (int l = 0; l < kSurLayers; ++l, ++layers) {
+        const uint32_t dcol = trow + 256u * (l & 1);
+        // the next tile's features, while this layer's MMAs run
+        if ((l == 1 || l == 2) && tile + dtile < ntiles) {
+          if (l == 1 && !(ok = wait(fetched[par ^ 1], (tiles + 1) >> 1 & 1))) break;
+          if (l == 1) features(par ^ 1, 0);
+          else features(par ^ 1, 1);
+        }
+        // the first layer's input, which is overwritten below, is read for both halves
+        if (!(ok = wait(acc[half], layers & 1) && (l > 0 || wait(acc[half ^ 1], layers & 1)))) break;
+        umma::tc_fence_after();
+        for (int c0 = grp * kGroupCols; c0 < (grp + 1) * kGroupCols; c0 += 32) {
+          float v[32];
+          umma::tmem_ld32(dcol + c0, v);
+          const float4 *b4 = reinterpret_cast<const float4 *>(&s_bias[l][c0]);
+          if (l < kSurLayers - 1) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+              const float4 ba = b4[j / 4], bb = b4[j / 4 + 1];
+              const float b[8] = {ba.x, ba.y, ba.z, ba.w, bb.x, bb.y, bb.z, bb.w};
+              __align__(16) bf16 hb[8];
+#pragma unroll
+              for (int t = 0; t < 8; ++t) hb[t] = __float2bfloat16_rn(silu(v[j + t] + b[t]));
+              *(uint4 *)(H + umma::sw128_offset(row, c0 + j, 128)) = *(const uint4 *)hb;
+            }
+          } else {
+            const float4 *w0 = reinterpret_cast<const float4 *>(&s_wh[0][c0]);
+            const float4 *w1 = reinterpret_cast<const float4 *>(&s_wh[1][c0]);
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const float4 bq = b4[j / 4], m0 = w0[j / 4], m1 = w1[j / 4];
+              const float b[4] = {bq.x, bq.y, bq.z, bq.w}, x0[4] = {m0.x, m0.y, m0.z, m0.w},
+                          x1[4] = {m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+              for (int t = 0; t < 4; ++t) {
+                const float h = silu(v[j + t] + b[t]);
+                mu = fmaf(h, x0[t], mu);
+                sl = fmaf(h, x1[t], sl);
+              }
+            }
+          }
+        }
+        if (l < kSurLayers - 1) written();
+      }
+      if (!ok) break;
+      s_head[par][grp][row][0] = mu;
+      s_head[par][grp][row][1] = sl;
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(umma::smem_u32(&headed));
     }
-    __syncthreads();
+    if (ok && tiles > 0 && grp == kIoGroup && wait(headed, (tiles - 1) & 1)) results(last, (tiles - 1) & 1);
   }
-  if (!ok && threadIdx.x == 0) atomicCAS(a.error, 0, kErrWait);
   umma::tc_fence_before();
   __syncthreads();
-  if (warp == 0) umma::tmem_free(tmem, 256);
+  if (threadIdx.x == 0 && s_abort) atomicCAS(a.error, 0, kErrWait);
+  if (warp == 0) umma::tmem_free(tmem, 512);
 }
 
 }  // namespace sur

@@ -39,6 +39,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -58,6 +62,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
   const unsigned long long t0 = global_ns();
   while (!mbar_test(bar, parity))
     if (global_ns() - t0 > limit_ns) return false;
+  return true;
+}
+
+// The same for blocks whose warps have separate roles: a wait that runs out
+// sets *abort, and every wait ends (false) once it is set.
+__device__ __forceinline__ bool mbar_wait_role(uint32_t bar, uint32_t parity, unsigned long long limit_ns,
+                                               volatile int *abort) {
+  if (mbar_test(bar, parity)) return true;
+  const unsigned long long t0 = global_ns();
+  while (!mbar_test(bar, parity)) {
+    if (*abort) return false;
+    if (global_ns() - t0 > limit_ns) {
+      *abort = 1;
+      return false;
+    }
+  }
   return true;
 }
 
