@@ -66,11 +66,14 @@ namespace amca {
 
 namespace {
 
-constexpr int kBlock = 256;
-constexpr int kWarps = kBlock / 32;
-#ifndef AMCA_MIN_BLOCKS
+// ca_batch_wide*.cu compile this file again with wider blocks, for the batched
+// kernel alone (AMCA_BATCH_WIDE names the wrapper they define).
+#ifndef AMCA_BLOCK
+#define AMCA_BLOCK 256
 #define AMCA_MIN_BLOCKS 4
 #endif
+constexpr int kBlock = AMCA_BLOCK;
+constexpr int kWarps = kBlock / 32;
 constexpr int kMinBlocks = AMCA_MIN_BLOCKS;  // co-resident blocks per SM the register budget is sized for
 constexpr unsigned long long kWaitNs = 5000000000ull;  // 5 s bound on any spin
 constexpr long long kClaimBatch = 2 * kBlock;           // ranks a block takes per grab in the claim phase
@@ -992,9 +995,10 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
     __syncthreads();
   }
   RankSched sched(n, &d.ctrl->claim_next, &d.ctrl->error, d.warp_sched);
-  // teams of the batched launch (at most 64 blocks) give the checks more of
-  // their warps
-  const int dw = t_nb <= 64 ? kDecWarpsTeam : d.dec_warps;
+  // teams of the batched launch (at most 64 blocks) give the checks half of
+  // their warps (eight blocks of 256 threads on 24 realms of 32 to 96 cells an
+  // edge: 59.2 ms at two warps, 54.4 at four, 59.1 at eight)
+  const int dw = t_nb <= 64 ? kWarps / 2 : d.dec_warps;
   const int cw = (int)(threadIdx.x >> 5) - (kWarps - dw);
   if (checks && cw >= 0)
     check_around(d, cur, checks, kind == 0 ? list.base : -1, zpar,
@@ -1569,6 +1573,7 @@ __device__ void run_realm(const PlainDevice &d, long long step_limit, unsigned l
   }
 }
 
+#ifndef AMCA_BATCH_WIDE
 __global__ void __launch_bounds__(kBlock, kMinBlocks) plain_persistent_kernel(PlainDevice d, long long step_limit) {
   __shared__ unsigned long long smem[kWarps + 2];
   // the descriptor in shared memory: the phases take it by reference, and a
@@ -1619,6 +1624,7 @@ __device__ __forceinline__ void init_field(const PlainDevice &d, long long tid, 
 __global__ void init_field_kernel(PlainDevice d) {
   init_field(d, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
+#endif  // AMCA_BATCH_WIDE
 
 // ---------------------------------------------------------------------------
 // Batched launch: many independent realms in one cooperative launch. The
@@ -1669,6 +1675,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
   }
 }
 
+#ifndef AMCA_BATCH_WIDE
 // Every realm of a batch back to its state right after initialize (site
 // flags, look-back words, control block, field), and the queue and team
 // words to zero. blockIdx.y is the realm.
@@ -2126,6 +2133,11 @@ int plain_batched_grid(int device) {
   return sms * per_sm;
 }
 
+int plain_batched_threads(int device, int grid_blocks, long long cells_per_block) {
+  if (cells_per_block >= 96000 && grid_blocks <= plain_batched_grid_1024(device)) return 1024;
+  return cells_per_block >= 24000 && grid_blocks <= plain_batched_grid_512(device) ? 512 : kBlock;
+}
+
 cudaError_t plain_batch_reset(const PlainDevice *insts, int ninst, unsigned *queues, int nclasses, BatchTeam *teams,
                               int nteams, int *error, cudaStream_t s) {
   if (ninst <= 0) return cudaSuccess;
@@ -2134,8 +2146,8 @@ cudaError_t plain_batch_reset(const PlainDevice *insts, int ninst, unsigned *que
 }
 
 cudaError_t plain_batched_run(const PlainDevice *insts, const int *order, int ninst, const BatchPlanDev &plan,
-                              int grid_blocks, unsigned *queues, BatchTeam *teams, int *error, long long step_limit,
-                              cudaStream_t s) {
+                              int grid_blocks, int threads, unsigned *queues, BatchTeam *teams, int *error,
+                              long long step_limit, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid_blocks);
   cfg.blockDim = dim3(kBlock);
@@ -2146,6 +2158,9 @@ cudaError_t plain_batched_run(const PlainDevice *insts, const int *order, int ni
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (threads == 1024)
+    return plain_batched_launch_1024(cfg, insts, order, ninst, plan, queues, teams, error, step_limit);
+  if (threads == 512) return plain_batched_launch_512(cfg, insts, order, ninst, plan, queues, teams, error, step_limit);
   return cudaLaunchKernelEx(&cfg, plain_batched_kernel, insts, order, ninst, plan, queues, teams, error, step_limit);
 }
 
@@ -2162,3 +2177,25 @@ cudaError_t plain_grain_field(const PlainDevice &d, int32_t *out, long long ngra
 }
 
 }  // namespace amca
+
+#else  // AMCA_BATCH_WIDE
+
+}  // namespace
+
+int AMCA_BATCH_WIDE_GRID(int device) {
+  int sms = 0, per_sm = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plain_batched_kernel, kBlock, 0) != cudaSuccess) return 0;
+  return sms * per_sm;
+}
+
+cudaError_t AMCA_BATCH_WIDE(const cudaLaunchConfig_t &cfg, const PlainDevice *insts, const int *order, int ninst,
+                            const BatchPlanDev &plan, unsigned *queues, BatchTeam *teams, int *error,
+                            long long step_limit) {
+  cudaLaunchConfig_t c = cfg;
+  c.blockDim = dim3(kBlock);
+  return cudaLaunchKernelEx(&c, plain_batched_kernel, insts, order, ninst, plan, queues, teams, error, step_limit);
+}
+
+}  // namespace amca
+#endif  // AMCA_BATCH_WIDE

@@ -76,9 +76,6 @@ constexpr int kMarkSplit = 1024;
 constexpr int kDecWarps = 4;
 constexpr int kCompactSlack = 4096;
 constexpr int kMarkBatch = 4;  // ranks per thread whose marks are computed before any is stored
-// Warps per block that start a claim phase with the neighbourhood checks on
-// teams of at most 64 blocks (the batched launch).
-constexpr int kDecWarpsTeam = 4;
 
 // Control block. Between launches it holds the realm's state (step, time,
 // active count, ...). Inside a launch every block keeps the per-step values
@@ -238,20 +235,41 @@ cudaError_t plain_run_steps(const PlainDevice &d, long long step_limit, int grid
 // Blocks of the batched kernel that fit on the device at once.
 int plain_batched_grid(int device);
 
+// Threads per block of a batched launch of grid_blocks blocks whose busiest
+// team has cells_per_block interior cells a block: few blocks would leave most
+// of every SM idle, so where they are co-resident all the same and have enough
+// to do they are wider. A realm's result does not depend on it. Eight blocks a
+// realm, 256 / 512 / 1,024 threads: 19 realms of 32 to 48 cells an edge 18.3 /
+// 19.7 / 21.4 ms (14,000 cells a block), 19 of 48 to 80 30.0 / 25.3 / 26.1
+// (64,000), 24 of 32 to 96 41.9 / 33.0 / (too many blocks), 16 of 40 to 104
+// 49.7 / 37.1 / 33.1 (140,000), 4 of 90 to 112 60.4 / 47.5 / 43.1.
+int plain_batched_threads(int device, int grid_blocks, long long cells_per_block);
+
+// The batched kernel with wider blocks: co-resident blocks, launch.
+int plain_batched_grid_512(int device);
+int plain_batched_grid_1024(int device);
+cudaError_t plain_batched_launch_512(const cudaLaunchConfig_t &cfg, const PlainDevice *insts, const int *order,
+                                     int ninst, const BatchPlanDev &plan, unsigned *queues, BatchTeam *teams,
+                                     int *error, long long step_limit);
+cudaError_t plain_batched_launch_1024(const cudaLaunchConfig_t &cfg, const PlainDevice *insts, const int *order,
+                                      int ninst, const BatchPlanDev &plan, unsigned *queues, BatchTeam *teams,
+                                      int *error, long long step_limit);
+
 // Every realm of insts[0..ninst) (a device array) back to its state right
 // after initialize; the nclasses queues, the error word and the nteams team
 // records to zero.
 cudaError_t plain_batch_reset(const PlainDevice *insts, int ninst, unsigned *queues, int nclasses, BatchTeam *teams,
                               int nteams, int *error, cudaStream_t s);
 
-// One cooperative launch of grid_blocks blocks laid out by `plan`: the teams
+// One cooperative launch of grid_blocks blocks (of `threads` threads: 256, 512
+// or 1,024) laid out by `plan`: the teams
 // of each class take that class's realms, in order, from the class's queue
 // and run each to solid, final_time or step_limit, as plain_run_steps would.
 // A team barrier that ran out sets *error; a realm's own failures go to its
 // control block.
 cudaError_t plain_batched_run(const PlainDevice *insts, const int *order, int ninst, const BatchPlanDev &plan,
-                              int grid_blocks, unsigned *queues, BatchTeam *teams, int *error, long long step_limit,
-                              cudaStream_t s);
+                              int grid_blocks, int threads, unsigned *queues, BatchTeam *teams, int *error,
+                              long long step_limit, cudaStream_t s);
 
 // out[r] (device) = realm r's control block.
 cudaError_t plain_batch_gather(const PlainDevice *insts, int ninst, PlainCtrl *out, cudaStream_t s);

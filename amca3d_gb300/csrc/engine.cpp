@@ -573,7 +573,7 @@ struct amca_batch {
   int *h_error = nullptr;        // pinned
   int max_blocks = 0;
   Plan plan;
-  int grid = 0;
+  int grid = 0, threads = 256;  // blocks of the launch, their width
   std::vector<int> order;  // realms by measured time, longest first
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -669,6 +669,10 @@ struct amca_batch {
     CK(cudaStreamSynchronize(stream));
     plan = p;
     grid = (int)blk.size();
+    long long busiest = 0;  // interior cells a block of its team has of a realm, at most
+    for (int t = 0; t < nt; ++t)
+      for (int r : p.classes[p.tclass[t]]) busiest = std::max(busiest, (long long)(realms[r]->dev.gcap / p.tsize[t]));
+    threads = plain_batched_threads(device, grid, busiest);
     graph_stale = true;
   }
 
@@ -677,7 +681,7 @@ struct amca_batch {
     const BatchPlanDev pd{d_blk, d_tsize, d_tclass, d_crange};
     CK(plain_batch_reset(d_insts, nr, d_queues, (int)plan.classes.size(), d_teams, (int)plan.tsize.size(), d_error,
                          stream));
-    CK(plain_batched_run(d_insts, d_order, nr, pd, grid, d_queues, d_teams, d_error, 1ll << 60, stream));
+    CK(plain_batched_run(d_insts, d_order, nr, pd, grid, threads, d_queues, d_teams, d_error, 1ll << 60, stream));
     CK(plain_batch_gather(d_insts, nr, d_ctrls, stream));
     CK(cudaMemcpyAsync(h_ctrls, d_ctrls, nr * sizeof(PlainCtrl), cudaMemcpyDeviceToHost, stream));
     CK(cudaMemcpyAsync(h_error, d_error, sizeof(int), cudaMemcpyDeviceToHost, stream));

@@ -168,3 +168,32 @@ def test_batched_64_full_size_matches_reference(amca):
     finally:
         for r in realms:
             r.close()
+
+
+@pytest.mark.parametrize("edge,team,count", [
+    (58, 8, 3),    # 24,389 cells a block: 512 threads
+    (57, 8, 3),    # 23,149: 256
+    (92, 8, 2),    # 97,336: 1,024
+    (46, 1, 5),    # a block of its own per realm: 1,024
+    (60, 3, 120),  # 360 blocks: too many for wider ones
+])
+def test_batch_block_widths_give_the_same_fields(amca, edge, team, count):
+    """The widths a launch's blocks can have, at the edges of the rule that picks them: every realm's fields and steps
+    equal its own run's."""
+    case = cases._mixed("wide", (edge, edge - 1, edge + 1), 3, 40, 200, t_dot=-200.0)
+    realms = [amca.CellularAutomataRealm(case.to_yaml(), seed=3 + k % 3) for k in range(count)]
+    for r in realms:
+        r.initialize()
+    want = []
+    for r in realms[:3]:
+        r.run()
+        want.append((r.field("grain_id"), r.field("orientation_id"), r.stats()["step"]))
+    with amca.Batch(realms, team_size=team) as b:
+        b.run()
+        for k in (0, 1, 2, count - 1):
+            if k < count:
+                g, o, n = want[k % 3] if k % 3 < len(want) else want[0]
+                assert np.array_equal(realms[k].field("grain_id"), g)
+                assert np.array_equal(realms[k].field("orientation_id"), o) and realms[k].stats()["step"] == n
+    for r in realms:
+        r.close()
