@@ -279,6 +279,11 @@ __device__ __forceinline__ double ulp_of(double p) {  // |p| normal
 __device__ __forceinline__ bool f64_nan(double x) {
   return ((unsigned long long)__double_as_longlong(x) << 1) > 0xffe0000000000000ull;
 }
+// x < y by the bits (NaN and zeros of either sign included): an FP64
+// comparison takes 64 cycles whatever the number of lanes.
+__device__ __forceinline__ bool f64_below(double x, double y) {
+  return f64_less(plus_zero(x), plus_zero(y)) && !f64_nan(x) && !f64_nan(y);
+}
 
 // x^b for b in {1, 2, 3}, correctly rounded (square and cube through exact
 // two-products). `near` is raised when the exact power lies within 0.02 ulp
@@ -480,7 +485,7 @@ __device__ bool eval_T(const RemeltDevice &d, const double *th, int64_t c, doubl
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     t[i] = th[nid[i]];
-    below = below || (f64_less(t[i], nullMat) && !f64_nan(t[i]));
+    below = below || f64_below(t[i], nullMat);
   }
   if (below) return false;
   T = hex8_interp64(t, d.pc[3 * c], d.pc[3 * c + 1], d.pc[3 * c + 2]);
@@ -505,8 +510,9 @@ __device__ float eval_T32(const RemeltDevice &d, const float *th32, int64_t c, i
 
 // thetaArray_ update of pseudo_single_integration_step (LoadDataFromFile.cpp:281-290)
 __device__ __forceinline__ double lerp_node(double th0, double th1, double ratio, double null_mat) {
-  if (th0 <= null_mat) return null_mat;
-  if (th1 <= null_mat) return th0;
+  // th0 <= null_mat, th1 <= null_mat, by the bits (false for NaN)
+  if (!f64_below(null_mat, th0) && !f64_nan(th0)) return null_mat;
+  if (!f64_below(null_mat, th1) && !f64_nan(th1)) return th0;
   return ratio * (th0 - th1) + th1;
 }
 
@@ -555,15 +561,23 @@ __device__ void frame_extrema(const RemeltDevice &d, const int64_t nid[8], int f
   }
   const double *fr = d.frames + (int64_t)(f % d.frame_slots) * d.nnodes;
   const double V = d.void_t + 0.00001;
+  // Comparisons by the bits (an FP64 one takes 64 cycles, and a rebuild made
+  // about 60 FP64 instructions per element). A node clear of `above`, which
+  // exceeds V by 2^-40 of |V|, is not near V unless it is 2^8 times as large;
+  // the exact test decides the others.
+  const double above = V + ldexp(fabs(V), -40);
+  double v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = fr[nid[i]];
   mx = -INFINITY;
   mn = INFINITY;
   near = false;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const double v = fr[nid[i]];
-    if (!(v >= V + ldexp(fmax(fabs(v), fabs(V)), -48))) near = true;
-    mx = v > mx ? v : mx;
-    mn = v < mn ? v : mn;
+    if (!(f64_below(above, v[i]) && f64_exponent(v[i]) < f64_exponent(V) + 7))
+      if (!(v[i] >= V + ldexp(fmax(fabs(v[i]), fabs(V)), -48))) near = true;
+    mx = f64_below(mx, v[i]) ? v[i] : mx;
+    mn = f64_below(v[i], mn) ? v[i] : mn;
   }
   d.fmax[sl][e] = mx;
   d.fmin[sl][e] = mn;
@@ -573,6 +587,11 @@ __device__ void frame_extrema(const RemeltDevice &d, const int64_t nid[8], int f
 // nullMatTemp_ + 0.01: below it a cell counts as without material in the
 // liquid-neighbour pass (Remelting.cpp:504-507)
 __device__ __forceinline__ double null_plus() { return -1.0 + 0.01; }
+
+// mx < Tm && mn >= null_plus() for an element's bounds (never NaN), by the bits
+__device__ __forceinline__ bool quiet(double mx, double mn, double Tm) {
+  return f64_below(mx, Tm) && !f64_below(mn, null_plus());
+}
 
 }  // namespace
 
@@ -936,6 +955,76 @@ __device__ StepScalars read_scalars(const RemeltCtrl *c) {
   return s;
 }
 
+// The next step's scalars and what this step's frame replay decides, worked
+// out by one thread of every block (the same operations on the same values
+// everywhere) and read by all from shared memory: read from the control block
+// by every thread they cost 3.4 us at the start of each step, recomputed by
+// every thread about 2 us of FP64 in phases D and E. With the bit compares of
+// the rebuild and the site conditions ahead of the flags: 47.1 to 40.2 us a
+// step on a track over 75x50x30 cells, 68.7 to 60.9 us over 500x250x100.
+struct Replay {
+  double ratio;
+  bool exhausted, bad, unloaded;
+};
+
+// Why no step may start with these scalars (kRemeltRunning: one may).
+__device__ int stop_reason(const RemeltDevice &d, const StepScalars &S, long long limit) {
+  // --- loop condition of time_integration_weak_coupling (CafeSolver.cpp:188) and launch limits ---
+  if (!(S.time < d.final_time)) return kRemeltFinalTime;
+  if (!(S.time < d.t_stop)) return kRemeltTimeStop;
+  if (S.step >= limit) return kRemeltStepLimit;
+  if (d.nsites > 0 && S.n_orient + d.nsites > d.orient_cap) return kRemeltNeedOrient;
+  // the step's frame replay reads frame f_next (and f_next + 1 when two frames share a time): both loaded,
+  // unless the frames end before them
+  if (!d.external && S.f_next + 1 >= d.frames_avail && d.frames_avail < d.nframes) return kRemeltNeedFrames;
+  return kRemeltRunning;
+}
+
+// The step's dt from the velocity at the minimum temperature (Remelting.cpp:706-726, CafeSolver.cpp:195-199).
+__device__ double step_dt(const RemeltDevice &d, const StepScalars &S, double vmin) {
+  const double maxV = vmin > 0 ? vmin : 0;
+  const double a = d.tsf_ca * d.h / maxV;
+  const double dtLoc = (S.max_ts < a) ? S.max_ts : a;
+  const double dT_ = (S.dT_FE < dtLoc) ? S.dT_FE : dtLoc;
+  return (d.dt_cap < dT_) ? d.dt_cap : dT_;  // setup_time_step_for_coupling of an external solver
+}
+
+// The scalars after a step of dT, and its frame replay (LoadDataFromFile.cpp:207-313).
+__device__ void next_scalars(const RemeltDevice &d, const StepScalars &S, double dT, unsigned nuclei, StepScalars &N,
+                             Replay &R) {
+  N = S;
+  N.step = S.step + 1;
+  N.time = S.time + dT;
+  N.dt = dT;
+  N.n_orient = S.n_orient + nuclei;
+  R.ratio = 0.0;
+  R.exhausted = R.bad = R.unloaded = false;
+  // an external FE solver hands in the next node temperatures and element bounds between
+  // steps (amca_set_nodal_temperatures): no replay then
+  if (d.external) return;
+  if (N.fe_time == 0) N.fe_time = N.ts1;
+  N.fe_time += dT;
+  while (N.fe_time >= N.ts0) {
+    if (N.f_next >= d.nframes) {
+      R.exhausted = true;
+      R.bad = (d.bad_frame == N.f_next);
+      break;
+    }
+    if (N.f_next >= d.frames_avail) {  // cannot happen after the check at the step's start
+      R.unloaded = true;
+      R.exhausted = true;
+      break;
+    }
+    N.ts1 = N.ts0;
+    N.ts0 = d.frame_time[N.f_next % d.frame_slots];
+    N.f_new = N.f_next;
+    N.f_next++;
+  }
+  if (!R.exhausted) R.ratio = (N.fe_time - N.ts1) / (N.ts0 - N.ts1);
+  N.dT_FE = N.ts0 - N.fe_time;
+  N.max_ts = N.ts0 - N.fe_time;
+}
+
 // Sweep position of a cell in the reference's i-outer, j, k-inner order.
 __device__ __forceinline__ int32_t sweep_pos(const Grid &g, int I, int J, int K) {
   return (int32_t)(((int64_t)I * g.nyg + J) * g.nzg + K);
@@ -1010,7 +1099,7 @@ __device__ __forceinline__ ElemView elem_view(const RemeltDevice &d, const float
     if (lane == i) mine = nid[i];
   const float tl = lane < 8 ? th32[mine] : 0.0f;
   v.void_ = d.evoid[e] != 0;
-  v.quiet = d.emax[e] < d.Tm && d.emin[e] >= null_plus();
+  v.quiet = quiet(d.emax[e], d.emin[e], d.Tm);
 #pragma unroll
   for (int i = 0; i < 8; ++i) v.t[i] = __shfl_sync(0xffffffffu, tl, i);
   v.err = hex8_err32(v.t);
@@ -1050,7 +1139,7 @@ __device__ __forceinline__ float eval_T32_view(const RemeltDevice &d, int64_t c,
 // (the cell's tag is then ev->e), or nullptr; `pre`: the cell's values
 // loaded by the caller, or nullptr.
 __device__ __forceinline__ void phase_update(const RemeltDevice &d, RemeltCtrl *c, int64_t cell, const double *th,
-                                             const float *th32, const StepScalars &S, bool count_all,
+                                             const float *th32, bool settled, bool count_all,
                                              unsigned long long &exactT, unsigned long long &melts,
                                              const ElemView *ev = nullptr, const CellPre *pre = nullptr) {
   int32_t o = pre ? pre->o : d.orient[cell];
@@ -1141,7 +1230,7 @@ __device__ __forceinline__ void phase_update(const RemeltDevice &d, RemeltCtrl *
   }
   const uint8_t m0 = pre ? mel : d.melted[cell];
   uint8_t m1 = m0;
-  if (wm2 && S.time >= S.max_ts) m1 = 1;
+  if (wm2 && settled) m1 = 1;
   if (!wm2) m1 = 0;
   if (m1 != m0) d.melted[cell] = m1;
   d.tcls[cell] = (uint8_t)((flags ? kTlt : 0) | (le ? kTle : 0) | (gtn ? kTgtNull : 0) | (wm2 ? kTgeNullPlus : 0));
@@ -1169,19 +1258,24 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     for (int i = 0; i < kClkN; ++i) s_clk[i] = 0ull;
     s_host_seq = ld_volatile(&c->host_seq);
   }
-  for (;;) {
-    const StepScalars S = read_scalars(c);
-    // --- loop condition of time_integration_weak_coupling (CafeSolver.cpp:188) and launch limits ---
-    int stop = kRemeltRunning;
-    if (!(S.time < d.final_time)) stop = kRemeltFinalTime;
-    else if (!(S.time < d.t_stop)) stop = kRemeltTimeStop;
-    else if (S.step >= limit) stop = kRemeltStepLimit;
-    else if (d.nsites > 0 && S.n_orient + d.nsites > d.orient_cap) stop = kRemeltNeedOrient;
-    // the step's frame replay reads frame f_next (and f_next + 1 when two frames share a time): both loaded,
-    // unless the frames end before them
-    else if (!d.external && S.f_next + 1 >= d.frames_avail && d.frames_avail < d.nframes) stop = kRemeltNeedFrames;
-    if (stop != kRemeltRunning) {
-      if (gtid == 0) c->status = stop;
+  // this step's scalars and the next one's, by step parity of the launch
+  __shared__ StepScalars s_S[2];
+  __shared__ Replay s_R;
+  __shared__ int s_stop;
+  __shared__ double s_dT, s_minT;
+  __shared__ unsigned s_nh;
+  __shared__ int s_min_hard;
+  const bool lead = tid == kBlock - 32;  // the last warp has the least else to do in phase D
+  if (lead) {
+    s_S[0] = read_scalars(c);
+    s_stop = stop_reason(d, s_S[0], limit);
+  }
+  __syncthreads();
+  for (unsigned turn = 0;; ++turn) {
+    const StepScalars &S = s_S[turn & 1];
+    StepScalars &N = s_S[(turn & 1) ^ 1];
+    if (s_stop != kRemeltRunning) {
+      if (gtid == 0) c->status = s_stop;
       break;
     }
     const int par = (int)(S.step & 1);
@@ -1210,12 +1304,13 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
       // elements in the update below)
       for (int64_t q = nthr - 1 - gtid; q < nprev; q += nthr) d.flagbits[fl[q] >> 5] = 0u;
     }
+    const bool settled = S.time >= S.max_ts;
     if (S.step == 0) {  // every interior cell; the liquid count per element starts here
       for (int64_t q = gtid; q < M; q += nthr) {
         const int I = (int)(q % g.nx) + 1;
         const int J = (int)((q / g.nx) % g.ny) + 1;
         const int K = (int)(q / ((int64_t)g.nx * g.ny)) + 1;
-        phase_update(d, c, (int64_t)K * g.nxyg + (int64_t)J * g.nxg + I, th, th32, S, true, exactT, melts);
+        phase_update(d, c, (int64_t)K * g.nxyg + (int64_t)J * g.nxg + I, th, th32, settled, true, exactT, melts);
       }
       visited += (M + nthr - 1 - gtid) / nthr;
     } else {  // the cells of the active elements (a warp per element)
@@ -1245,7 +1340,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
 #pragma unroll
           for (int j = 0; j < kCellPre; ++j) {
             if (cl[j] < 0) continue;
-            phase_update(d, c, cl[j], th, th32, S, false, exactT, melts, &ev, &pre[j]);
+            phase_update(d, c, cl[j], th, th32, settled, false, exactT, melts, &ev, &pre[j]);
             ++visited;
           }
         }
@@ -1263,6 +1358,32 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     if (tid == 0 && blockIdx.x == 0 && d.detail) {
       s_clk[kClkFlagsMax] += ld_volatile(&c->flags_scratch);  // last step's maximum: every block added it before the A barrier
       c->flags_scratch = 0ull;
+    }
+    // site conditions of nucleate_at_nucleation_sites (Remelting.cpp:946-960), all blocks, from their last threads
+    // down: the first warps flag meanwhile (5 us of FP64 behind the flag pass of a block with a liquid site)
+    // (only a liquid, melted cell can nucleate: the temperatures are
+    // evaluated for those alone)
+    for (int64_t sidx = (int64_t)(kBlock - 1 - tid) * gridDim.x + blockIdx.x; sidx < d.nsites; sidx += nthr) {
+      const int32_t cell = d.site_cell[sidx];
+      uint8_t f = 0;
+      if (d.orient[cell] == -1 && d.melted[cell]) {
+        double T = -1.0, Told = -1.0;
+        const bool withMat = eval_T(d, th, cell, T);
+        bool cooling = false;
+        if (S.step > 0) {  // cooling_ of this step's phase update (Remelting.cpp:362-373)
+          eval_T(d, thp, cell, Told);
+          double rate = 410;
+          if (Told > 0) rate = (T - Told) / S.dt;
+          if (T <= 0) rate = 0;
+          cooling = withMat ? (rate < 0) : false;
+        }
+        if (cooling && T > d.Tnuc) {
+          const double dT = d.Tm - T;
+          if (dT > d.site_dtc[sidx]) f = d.grain[cell] == -1 ? 2 : 1;
+        }
+      }
+      d.snuc[sidx] = f;
+      if (f) atomicAdd(&c->n_nuc_sites[par], 1u);
     }
     const unsigned long long tfl = tid == 0 ? now_ns() : 0ull;
     {
@@ -1340,31 +1461,6 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     if (tid == 0) {
       const unsigned long long w = now_ns() - tfl;
       if (d.detail && w > ld_volatile(&c->flags_scratch)) atomicMax(&c->flags_scratch, w);
-    }
-    // site conditions of nucleate_at_nucleation_sites (Remelting.cpp:946-960), all blocks
-    // (only a liquid, melted cell can nucleate: the temperatures are
-    // evaluated for those alone)
-    for (int64_t sidx = spread_begin(0); sidx < d.nsites; sidx += spread_stride(0)) {
-      const int32_t cell = d.site_cell[sidx];
-      uint8_t f = 0;
-      if (d.orient[cell] == -1 && d.melted[cell]) {
-        double T = -1.0, Told = -1.0;
-        const bool withMat = eval_T(d, th, cell, T);
-        bool cooling = false;
-        if (S.step > 0) {  // cooling_ of this step's phase update (Remelting.cpp:362-373)
-          eval_T(d, thp, cell, Told);
-          double rate = 410;
-          if (Told > 0) rate = (T - Told) / S.dt;
-          if (T <= 0) rate = 0;
-          cooling = withMat ? (rate < 0) : false;
-        }
-        if (cooling && T > d.Tnuc) {
-          const double dT = d.Tm - T;
-          if (dT > d.site_dtc[sidx]) f = d.grain[cell] == -1 ? 2 : 1;
-        }
-      }
-      d.snuc[sidx] = f;
-      if (f) atomicAdd(&c->n_nuc_sites[par], 1u);
     }
     if (gtid == 0) {
       const unsigned long long t1 = now_ns();
@@ -1503,6 +1599,19 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
       p.cand = cand;
       return p;
     };
+    // ===== dt (Remelting.cpp:706-726, CafeSolver.cpp:195-199), by one thread beside those loads =====
+    if (lead) {
+      s_nh = ld_volatile(&c->n_hard);  // uniform: every block reads the same counter and key
+      s_minT = dkey_inv(ld_volatile(&c->minT_key));
+      bool h = false, near_v = false;
+      const double v = velocity(d, s_minT, h, near_v);
+      s_min_hard = h ? 1 : 0;
+      if (!h) {
+        s_dT = step_dt(d, S, v);
+        next_scalars(d, S, s_dT, ld_volatile(&c->n_nuc_sites[par]), N, s_R);
+        s_stop = stop_reason(d, N, limit);
+      }
+    }
     const int64_t q0 = spread_begin(0);
     GrowPre pre0{};
     bool use0 = false;
@@ -1515,47 +1624,35 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         use0 = true;
       }
     }
-
-    // ===== dt (Remelting.cpp:706-726, CafeSolver.cpp:195-199) =====
-    const double minT = dkey_inv(ld_volatile(&c->minT_key));
-    // the same FP64 velocity for every thread: one thread per block computes it
-    __shared__ double s_vmin;
-    __shared__ int s_min_hard;
-    if (tid == 0) {
-      bool h = false, near_v = false;
-      s_vmin = velocity(d, minT, h, near_v);
-      s_min_hard = h ? 1 : 0;
-    }
     __syncthreads();
     const bool min_hard = s_min_hard != 0;
-    double vmin = s_vmin;
     // The host evaluates the hard velocities while the blocks grow and claim
     // with the others: block 0 posts the request, every block counts it, and
     // a block waits for the answer only before its own hard cells (or before
     // dt, when the velocity at the minimum temperature is one of them). A
     // request larger than the mapped buffer goes in chunks, behind a barrier.
-    const unsigned nh = ld_volatile(&c->n_hard);  // uniform: every block read the same counter and key
+    const unsigned nh = s_nh;
     const bool ask = nh > 0 || min_hard;
     const bool overlap = ask && nh + 1u <= (unsigned)d.host_cap;
     if (ask && !overlap) {
-      if (blockIdx.x == 0 && !host_velocities(d, c, nh, min_hard, minT)) atomicCAS(&c->error, 0, kRemeltErrHost);
+      if (blockIdx.x == 0 && !host_velocities(d, c, nh, min_hard, s_minT)) atomicCAS(&c->error, 0, kRemeltErrHost);
       if (!(ok = grid_barrier(d, 5))) break;
       // block 0's requests, one per chunk, counted by the others
       if (tid == 0 && blockIdx.x != 0) s_host_seq += (nh + (min_hard ? 1u : 0u) + d.host_cap - 1u) / d.host_cap;
-      if (min_hard) vmin = ld_volatile(&c->vmin);
     }
     if (overlap) {
-      host_post(d, nh, min_hard, minT);
-      if (min_hard) {
-        host_wait_block(d, c);
-        vmin = ld_volatile(&d.host->v[nh]);
-      }
+      host_post(d, nh, min_hard, s_minT);
+      if (min_hard) host_wait_block(d, c);
     }
-    const double maxV = vmin > 0 ? vmin : 0;
-    const double a = d.tsf_ca * d.h / maxV;
-    const double dtLoc = (S.max_ts < a) ? S.max_ts : a;
-    const double dT_ = (S.dT_FE < dtLoc) ? S.dT_FE : dtLoc;
-    const double dT = (d.dt_cap < dT_) ? d.dt_cap : dT_;  // setup_time_step_for_coupling of an external solver
+    if (min_hard) {  // uniform
+      if (lead) {
+        s_dT = step_dt(d, S, overlap ? ld_volatile(&d.host->v[nh]) : ld_volatile(&c->vmin));
+        next_scalars(d, S, s_dT, ld_volatile(&c->n_nuc_sites[par]), N, s_R);
+        s_stop = stop_reason(d, N, limit);
+      }
+      __syncthreads();
+    }
+    const double dT = s_dT;
 
     // ===== D: grow and claim (Remelting.cpp:545-622) =====
     // one flagged cell: growth by dT * vel and its claims (atomicMin of the
@@ -1745,34 +1842,12 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         }
       }
     }
-    // FE replay (uniform in every thread)
-    double fe_time = S.fe_time, ts0 = S.ts0, ts1 = S.ts1;
-    int f_new = S.f_new, f_next = S.f_next;
-    bool exhausted = false, bad = false, unloaded = false;
-    double ratio = 0.0;
-    // an external FE solver hands in the next node temperatures and element bounds between
-    // steps (amca_set_nodal_temperatures): no replay then
+    // FE replay
+    const bool exhausted = s_R.exhausted;
+    const int f_new = N.f_new;
     if (!d.external) {
-      if (fe_time == 0) fe_time = ts1;
-      fe_time += dT;
-      while (fe_time >= ts0) {
-        if (f_next >= d.nframes) {
-          exhausted = true;
-          bad = (d.bad_frame == f_next);
-          break;
-        }
-        if (f_next >= d.frames_avail) {  // cannot happen after the check at the step's start
-          unloaded = true;
-          exhausted = true;
-          break;
-        }
-        ts1 = ts0;
-        ts0 = d.frame_time[f_next % d.frame_slots];
-        f_new = f_next;
-        f_next++;
-      }
       if (!exhausted) {
-        ratio = (fe_time - ts1) / (ts0 - ts1);
+        const double ratio = s_R.ratio;
         if (ratio < 0.0 && gtid == 0) atomicCAS(&c->error, 0, kRemeltErrRatio);
         const double *f0 = d.frames + (int64_t)(f_new % d.frame_slots) * d.nnodes;
         const double *f1 = d.frames + (int64_t)((f_new - 1) % d.frame_slots) * d.nnodes;
@@ -1827,18 +1902,18 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
             for (int i = 0; i < 8; ++i) t[i] = lerp_node(f0[nid[i]], f1[nid[i]], ratio, d.void_t);
             element_bounds(d, e, t);
           } else {
-            const double mx = mx0 > mx1 ? mx0 : mx1, mn = mn0 < mn1 ? mn0 : mn1;
-            const double mg = fmax(fabs(mx), fabs(mn));
+            const double mx = f64_below(mx1, mx0) ? mx0 : mx1, mn = f64_below(mn0, mn1) ? mn0 : mn1;
+            const double margin = ldexp(f64_below(fabs(mn), fabs(mx)) ? fabs(mx) : fabs(mn), -44);
             d.evoid[e] = 0;
-            d.emax[e] = mx + ldexp(mg, -44);
-            d.emin[e] = mn - ldexp(mg, -44);
+            d.emax[e] = mx + margin;
+            d.emin[e] = mn - margin;
           }
           // the next phase update visits this element's cells when some may change: hot enough to
           // melt or below nullMatTemp_ + 0.01, void status changed, or holding liquid with material
           // (cells of a cold element are solid except those counted in eliq; a void element's cells
           // are all liquid without material once it has been visited)
           const bool v = d.evoid[e] != 0;
-          const bool active = (!v && !(d.emax[e] < d.Tm && d.emin[e] >= null_plus())) || (v != (void_before != 0)) ||
+          const bool active = (!v && !quiet(d.emax[e], d.emin[e], d.Tm)) || (v != (void_before != 0)) ||
                               (!v && ld_volatile(&d.eliq[e]) > 0);
           if (active) {
             const unsigned slot = append_slot(&c->n_eact[par ^ 1]);
@@ -1861,24 +1936,24 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
       }
     }
     if (gtid == 0) {
-      if (bad) atomicCAS(&c->error, 0, kRemeltErrFrame);
-      if (unloaded) atomicCAS(&c->error, 0, kRemeltErrRing);
+      if (s_R.bad) atomicCAS(&c->error, 0, kRemeltErrFrame);
+      if (s_R.unloaded) atomicCAS(&c->error, 0, kRemeltErrRing);
       if (!d.external) {
         if (!exhausted) {
           c->fstat_frame[f_new & 1] = f_new;
           c->fstat_frame[(f_new - 1) & 1] = f_new - 1;
         }
-        c->fe_time = fe_time;
-        c->ts0 = ts0;
-        c->ts1 = ts1;
+        c->fe_time = N.fe_time;
+        c->ts0 = N.ts0;
+        c->ts1 = N.ts1;
         c->f_new = f_new;
-        c->f_next = f_next;
-        c->ratio = ratio;
-        c->dT_FE = ts0 - fe_time;
-        c->max_ts = ts0 - fe_time;
+        c->f_next = N.f_next;
+        c->ratio = s_R.ratio;
+        c->dT_FE = N.dT_FE;
+        c->max_ts = N.max_ts;
       }
-      c->step = S.step + 1;
-      c->time = S.time + dT;
+      c->step = N.step;
+      c->time = N.time;
       c->dt_prev = S.dt;
       c->dt = dT;
       c->theta_init = 0;
