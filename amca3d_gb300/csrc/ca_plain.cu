@@ -67,7 +67,9 @@ namespace amca {
 namespace {
 
 // ca_batch_wide*.cu compile this file again with wider blocks, for the batched
-// kernel alone (AMCA_BATCH_WIDE names the wrapper they define).
+// kernel alone (AMCA_BATCH_WIDE names the wrapper they define), and
+// ca_realm_few.cu for the kernel that runs one realm with at most two blocks
+// per SM (AMCA_REALM_FEW): registers for two blocks, lanes that share a rank.
 #ifndef AMCA_BLOCK
 #define AMCA_BLOCK 256
 #define AMCA_MIN_BLOCKS 4
@@ -971,48 +973,42 @@ __device__ __noinline__ void zero_decisions(const PlainDevice &d, int cur, int z
 // (generation >= 1), neighbour tests, atomicMin claims and the entry's next
 // wake key.
 // ---------------------------------------------------------------------------
-// With `checks` > 0 the neighbourhoods of that many newly solid cells are
-// checked in the same phase (check_around: the previous generation's captures,
-// or in generation 0 the nuclei, the last ranks): the last dec_warps warps of
-// every block do that first and then join the claims, whose dynamic hand-out
-// balances the difference (a generation of at most 32 ranks per block keeps
-// its claims on the blocks' first warps).
-__device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind, long long lo, long long n, unsigned par,
-                            const GenList &list, long long step, double grown, long long checks,
-                            int zpar, unsigned long long *stat_tests, unsigned long long *stat_tests64,
-                            unsigned long long *stat_dec) {
+#ifdef AMCA_REALM_FEW
+// The lanes (as a power of two) that share a rank of a generation of n. A claim
+// lasts as long as the warp's rank with the most liquid neighbours (17 tests
+// of 130 ns behind the capture's 2.5 us), so a generation that leaves most
+// lanes without a rank gives each rank up to eight, as long as every scheduler
+// of the SMs has one warp: the capture's FP64 instructions take a scheduler's
+// unit 64 cycles a warp whatever the lanes (without that bound, 3 blocks per SM on
+// 320^3: 2% slower). One, 4, 8, 16 lanes on 60^3: 15.4, 13.7, 13.5, 13.7 ms.
+__device__ __forceinline__ int lane_shift(const PlainDevice &d, long long n) {
+  int sh = 0;
+  while (sh < 3 && n << (sh + 1) <= (long long)d.claim_lanes * t_nb) ++sh;
+  return sh;
+}
+#endif
+// The neighbours of lane 0 of 2^sh: every 2^sh-th.
+__device__ __forceinline__ uint32_t lane_neighbours(int sh) {
+  return sh == 0 ? 0xffffffffu : sh == 1 ? 0x55555555u : sh == 2 ? 0x11111111u : 0x01010101u;
+}
+
+// One rank, by 2^sh lanes that all hold it (`valid`: it exists): each tests
+// and claims the neighbours numbered its `sub` modulo 2^sh. Every lane of the
+// warp calls it with the same sh.
+__device__ __forceinline__ void claim_rank(const PlainDevice &d, int cur, int kind, long long lo, long long r, bool valid,
+                                           int sh, int sub, unsigned par, const GenList &list, long long step,
+                                           double grown, float gf, unsigned &tests, unsigned &tests64) {
   const Grid &g = d.grid;
-  if (threadIdx.x == 0) d.scanB[t_b] = 0ull;  // this block's look-back word of the resolve phase
   EnvRec *act = d.act[cur];
   int32_t *lstep = d.lstep[cur];
-  const float gf = wake_bound(grown);
-  unsigned tests = 0, tests64 = 0;  // this phase's, added to the launch totals at its end
-  // Claims need no order: warps or blocks take chunks of consecutive ranks
-  // from a shared counter until none is left, so those that drew cheap
-  // envelopes (few liquid neighbours) take more chunks.
-  if (checks) {
-    if (threadIdx.x == 0) s_nz = 0u;
-    __syncthreads();
-  }
-  RankSched sched(n, &d.ctrl->claim_next, &d.ctrl->error, d.warp_sched);
-  // teams of the batched launch (at most 64 blocks) give the checks half of
-  // their warps (eight blocks of 256 threads on 24 realms of 32 to 96 cells an
-  // edge: 59.2 ms at two warps, 54.4 at four, 59.1 at eight)
-  const int dw = t_nb <= 64 ? kWarps / 2 : d.dec_warps;
-  const int cw = (int)(threadIdx.x >> 5) - (kWarps - dw);
-  if (checks && cw >= 0)
-    check_around(d, cur, checks, kind == 0 ? list.base : -1, zpar,
-                 ((long long)cw * t_nb + t_b) * 32 + (threadIdx.x & 31), (long long)t_nb * dw * 32, stat_dec);
-  const int first = sched.first(), stride = sched.stride();
-  long long b, e;
-  while (sched.next(b, e)) {
-  for (long long r = b + first; r < e; r += stride) {
-    EnvRec en;
-    double gxd = 0, gyd = 0, gzd = 0;
-    bool have_centre = false;
-    uint32_t liq = 0;
-    const long long p = list.at(r);
-    int I, J, K;
+  EnvRec en{};
+  double gxd = 0, gyd = 0, gzd = 0;
+  bool have_centre = false;
+  uint32_t liq = 0;
+  long long p = 0;
+  int I = 0, J = 0, K = 0;
+  if (valid) {
+    p = list.at(r);
     if (kind == 0) {
       en = act[p];
       cell_ijk(g, en.cell, I, J, K);
@@ -1020,8 +1016,6 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
       // Grain::grow (Grain.h:27) for every step since the record was last
       // grown: L + dt * vel, the product rounded once per step
       en.L = replay_growth(d.dvh, en.L, (long long)lstep[p], step);
-      act[p].L = en.L;
-      lstep[p] = (int32_t)step;
     } else {
       // CellularAutomataManager_3D::capture_cell (:677-707) for the capture
       // recorded by the parent: decentred envelope from the parent's
@@ -1049,68 +1043,77 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
       en.dy = f64_to_f32_rz(gyd - ccy);
       en.dz = f64_to_f32_rz(gzd - ccz);
       have_centre = true;
-      act[p] = en;
-      lstep[p] = (int32_t)step;
-      d.gx[en.id] = gxd;
-      d.gy[en.id] = gyd;
-      d.gz[en.id] = gzd;
-      d.gori[en.id] = en.ori;
-      d.gcell[en.id] = en.cell;
-      d.orient[en.cell] = (uint32_t)en.ori;  // the claim word of last generation becomes the orientation id
+      if (sub == 0) {
+        act[p] = en;
+        d.gx[en.id] = gxd;
+        d.gy[en.id] = gyd;
+        d.gz[en.id] = gzd;
+        d.gori[en.id] = en.ori;
+        d.gcell[en.id] = en.cell;
+        d.orient[en.cell] = (uint32_t)en.ori;  // the claim word of last generation becomes the orientation id
+      }
     }
-    const int cell = en.cell, ori = en.ori, id = en.id;
-    const double L = en.L;
-    uint32_t con = 0;
-    // lower bound of |c'|_1 over the liquid neighbours it does not contain
-    float t_lb = INFINITY;
-    // cell_is_captured is false for a zero half-diagonal (tested on the bits:
-    // an integer compare instead of one on the narrow FP64 pipe); such an
-    // entry is looked at again next step
-    if (liq && (__double_as_longlong(L) << 1) == 0) t_lb = -INFINITY;
-    if (liq && (__double_as_longlong(L) << 1) != 0) {
-      const float dxf = en.dx, dyf = en.dy, dzf = en.dz;
-      const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(dxf) + fabsf(dyf) + fabsf(dzf)) + d.coord_err;
-      const float L32 = f64_to_f32_rz(L);  // the pre-test's margin is 2^-14 of it
-      float m32[9];
+  }
+  const int cell = en.cell, ori = en.ori, id = en.id;
+  const double L = en.L;
+  uint32_t con = 0;
+  // lower bound of |c'|_1 over the liquid neighbours it does not contain
+  float t_lb = INFINITY;
+  // cell_is_captured is false for a zero half-diagonal (tested on the bits:
+  // an integer compare instead of one on the narrow FP64 pipe); such an
+  // entry is looked at again next step
+  if (liq && (__double_as_longlong(L) << 1) == 0) t_lb = -INFINITY;
+  if (liq && (__double_as_longlong(L) << 1) != 0) {
+    const float dxf = en.dx, dyf = en.dy, dzf = en.dz;
+    const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(dxf) + fabsf(dyf) + fabsf(dzf)) + d.coord_err;
+    const float L32 = f64_to_f32_rz(L);  // the pre-test's margin is 2^-14 of it
+    float m32[9];
 #pragma unroll
-      for (int q = 0; q < 9; ++q) m32[q] = __ldg(d.omat32 + 9 * ori + q);
-      uint32_t bits = liq;
-      while (bits) {
-        const int nb = __ffs(bits) - 1;
-        bits &= bits - 1;
-        int di, dj, dk;
-        nbr_offset(nb, di, dj, dk);
-        ++tests;
-        float lower;
-        int f = captured_f32_lb(m32, (float)di * d.h32 - dxf, (float)dj * d.h32 - dyf, (float)dk * d.h32 - dzf, errg,
-                                L32, &lower);
-        if (f < 0) {
-          ++tests64;
-          if (!have_centre) {
-            gxd = d.gx[id];
-            gyd = d.gy[id];
-            gzd = d.gz[id];
-            have_centre = true;
-          }
-          const double ccx = centre_coord(g.x0, g.h, I + di);
-          const double ccy = centre_coord(g.y0, g.h, J + dj);
-          const double ccz = centre_coord(g.z0, g.h, K + dk);
-          f = is_captured_f64(d.omat + 9 * ori, ccx - gxd, ccy - gyd, ccz - gzd, L) ? 1 : 0;
+    for (int q = 0; q < 9; ++q) m32[q] = __ldg(d.omat32 + 9 * ori + q);
+    uint32_t bits = liq & (lane_neighbours(sh) << sub);
+    while (bits) {
+      const int nb = __ffs(bits) - 1;
+      bits &= bits - 1;
+      int di, dj, dk;
+      nbr_offset(nb, di, dj, dk);
+      ++tests;
+      float lower;
+      int f = captured_f32_lb(m32, (float)di * d.h32 - dxf, (float)dj * d.h32 - dyf, (float)dk * d.h32 - dzf, errg, L32,
+                              &lower);
+      if (f < 0) {
+        ++tests64;
+        if (!have_centre) {
+          gxd = d.gx[id];
+          gyd = d.gy[id];
+          gzd = d.gz[id];
+          have_centre = true;
         }
-        con |= (f ? 1u : 0u) << nb;
-        if (!f) t_lb = fminf(t_lb, lower);
+        const double ccx = centre_coord(g.x0, g.h, I + di);
+        const double ccy = centre_coord(g.y0, g.h, J + dj);
+        const double ccz = centre_coord(g.z0, g.h, K + dk);
+        f = is_captured_f64(d.omat + 9 * ori, ccx - gxd, ccy - gyd, ccz - gzd, L) ? 1 : 0;
       }
-      const uint32_t mine = claim_word(par, (uint32_t)r);
-      bits = con;
-      while (bits) {
-        const int nb = __ffs(bits) - 1;
-        bits &= bits - 1;
-        int di, dj, dk;
-        const int nc = cell + nbr_delta(g, nb, di, dj, dk);
-        atomicMin(d.orient + nc, mine);
-        set_bit(d, d.claimed, I + di, J + dj, K + dk);
-      }
+      con |= (f ? 1u : 0u) << nb;
+      if (!f) t_lb = fminf(t_lb, lower);
     }
+    const uint32_t mine = claim_word(par, (uint32_t)r);
+    bits = con;
+    while (bits) {
+      const int nb = __ffs(bits) - 1;
+      bits &= bits - 1;
+      int di, dj, dk;
+      const int nc = cell + nbr_delta(g, nb, di, dj, dk);
+      atomicMin(d.orient + nc, mine);
+      set_bit(d, d.claimed, I + di, J + dj, K + dk);
+    }
+  }
+  for (int o = 1; o < 1 << sh; o <<= 1) {
+    con |= __shfl_xor_sync(0xffffffffu, con, o);
+    t_lb = fminf(t_lb, __shfl_xor_sync(0xffffffffu, t_lb, o));
+  }
+  if (valid && sub == 0) {
+    if (kind == 0) act[p].L = L;
+    lstep[p] = (int32_t)step;
     // growth is uniform: the entry can contain one of the neighbours left
     // only once the run's cumulative growth reaches this key
     d.key[cur][p] = t_lb == -INFINITY ? gf : wake_key(t_lb, L, grown, gf);
@@ -1118,7 +1121,66 @@ __device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind
     d.con[r] = con;
     d.cellr[r] = cell;
   }
+}
+
+// With `checks` > 0 the neighbourhoods of that many newly solid cells are
+// checked in the same phase (check_around: the previous generation's captures,
+// or in generation 0 the nuclei, the last ranks): the last dec_warps warps of
+// every block do that first and then join the claims, whose dynamic hand-out
+// balances the difference (a generation of at most 32 ranks per block keeps
+// its claims on the blocks' first warps).
+__device__ __noinline__ void claim_phase(const PlainDevice &d, int cur, int kind, long long lo, long long n, unsigned par,
+                            const GenList &list, long long step, double grown, long long checks,
+                            int zpar, unsigned long long *stat_tests, unsigned long long *stat_tests64,
+                            unsigned long long *stat_dec) {
+  if (threadIdx.x == 0) d.scanB[t_b] = 0ull;  // this block's look-back word of the resolve phase
+  const float gf = wake_bound(grown);
+  unsigned tests = 0, tests64 = 0;  // this phase's, added to the launch totals at its end
+  // Claims need no order: warps or blocks take chunks of consecutive ranks
+  // from a shared counter until none is left, so those that drew cheap
+  // envelopes (few liquid neighbours) take more chunks.
+  if (checks) {
+    if (threadIdx.x == 0) s_nz = 0u;
+    __syncthreads();
   }
+  // (its block barrier comes before the checks: the warps without any go on)
+#ifdef AMCA_REALM_FEW
+  const int sh = lane_shift(d, n), lane = threadIdx.x & 31;
+  RankSched sched(sh ? 0 : n, &d.ctrl->claim_next, &d.ctrl->error, d.warp_sched);
+#else
+  RankSched sched(n, &d.ctrl->claim_next, &d.ctrl->error, d.warp_sched);
+#endif
+  // teams of the batched launch (at most 64 blocks) give the checks half of
+  // their warps (eight blocks of 256 threads on 24 realms of 32 to 96 cells an
+  // edge: 59.2 ms at two warps, 54.4 at four, 59.1 at eight)
+  const int dw = t_nb <= 64 ? kWarps / 2 : d.dec_warps;
+  const int cw = (int)(threadIdx.x >> 5) - (kWarps - dw);
+  if (checks && cw >= 0)
+    check_around(d, cur, checks, kind == 0 ? list.base : -1, zpar,
+                 ((long long)cw * t_nb + t_b) * 32 + (threadIdx.x & 31), (long long)t_nb * dw * 32, stat_dec);
+#ifdef AMCA_REALM_FEW
+  const int first = sh ? lane >> sh : sched.first(), stride = sched.stride();
+  long long b, e;
+  bool more;
+  if (sh) {  // one piece per warp, warps numbered across blocks first
+    b = ((long long)(threadIdx.x >> 5) * t_nb + t_b) * (32 >> sh);
+    e = b + (32 >> sh) < n ? b + (32 >> sh) : n;
+    more = b < n;
+  } else
+    more = sched.next(b, e);
+  while (more) {
+    for (long long r0 = b; r0 < e; r0 += stride)
+      claim_rank(d, cur, kind, lo, r0 + first, r0 + first < e, sh, lane & ((1 << sh) - 1), par, list, step, grown, gf,
+                 tests, tests64);
+    more = sh == 0 && sched.next(b, e);
+  }
+#else
+  const int first = sched.first(), stride = sched.stride();
+  long long b, e;
+  while (sched.next(b, e))
+    for (long long r = b + first; r < e; r += stride)
+      claim_rank(d, cur, kind, lo, r, true, 0, 0, par, list, step, grown, gf, tests, tests64);
+#endif
   *stat_tests += tests;
   *stat_tests64 += tests64;
   if (checks) flush_zero_buffer(d, zpar);
@@ -1590,7 +1652,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) plain_persistent_kernel(Pl
   __syncthreads();
   run_realm(sd, step_limit, smem);
 }
+#endif  // AMCA_BATCH_WIDE
 
+#if !defined(AMCA_BATCH_WIDE) && !defined(AMCA_REALM_FEW)
 // The initial field, maps and cell words, by the threads numbered tid + k *
 // stride. A brick row is solid where its y or z lies outside the interior, else
 // in the cells whose x does.
@@ -1624,8 +1688,9 @@ __device__ __forceinline__ void init_field(const PlainDevice &d, long long tid, 
 __global__ void init_field_kernel(PlainDevice d) {
   init_field(d, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
-#endif  // AMCA_BATCH_WIDE
+#endif
 
+#ifndef AMCA_REALM_FEW
 // ---------------------------------------------------------------------------
 // Batched launch: many independent realms in one cooperative launch. The
 // grid is cut into teams of consecutive blocks (plan.blk gives each block
@@ -1674,8 +1739,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
     __syncthreads();  // sd and s_idx are rewritten in the next round
   }
 }
+#endif  // AMCA_REALM_FEW
 
-#ifndef AMCA_BATCH_WIDE
+#if !defined(AMCA_BATCH_WIDE) && !defined(AMCA_REALM_FEW)
 // Every realm of a batch back to its state right after initialize (site
 // flags, look-back words, control block, field), and the queue and team
 // words to zero. blockIdx.y is the realm.
@@ -2121,6 +2187,12 @@ cudaError_t plain_run_steps(const PlainDevice &d, long long step_limit, int grid
   // the barrier's arrival counter starts every launch at zero
   const cudaError_t e = cudaMemsetAsync(d.ctrl, 0, 2 * sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) == cudaSuccess &&
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && grid_blocks <= 2 * sms) {
+    dd.claim_lanes = grid_blocks <= sms ? 128 : 64;
+    return plain_few_launch(dd, step_limit, grid_blocks, s);
+  }
   return cudaLaunchCooperativeKernel((const void *)plain_persistent_kernel, dim3(grid_blocks), dim3(kBlock), args, 0,
                                      s);
 }
@@ -2178,9 +2250,20 @@ cudaError_t plain_grain_field(const PlainDevice &d, int32_t *out, long long ngra
 
 }  // namespace amca
 
-#else  // AMCA_BATCH_WIDE
+#else
 
 }  // namespace
+
+#ifdef AMCA_REALM_FEW
+
+cudaError_t plain_few_launch(const PlainDevice &d, long long step_limit, int grid_blocks, cudaStream_t s) {
+  void *args[] = {(void *)&d, (void *)&step_limit};
+  return cudaLaunchCooperativeKernel((const void *)plain_persistent_kernel, dim3(grid_blocks), dim3(kBlock), args, 0,
+                                     s);
+}
+
+}  // namespace amca
+#else  // AMCA_BATCH_WIDE
 
 int AMCA_BATCH_WIDE_GRID(int device) {
   int sms = 0, per_sm = 0;
@@ -2198,4 +2281,5 @@ cudaError_t AMCA_BATCH_WIDE(const cudaLaunchConfig_t &cfg, const PlainDevice *in
 }
 
 }  // namespace amca
-#endif  // AMCA_BATCH_WIDE
+#endif  // AMCA_REALM_FEW
+#endif  // AMCA_BATCH_WIDE || AMCA_REALM_FEW

@@ -39,9 +39,9 @@ namespace {
 
 thread_local std::string g_create_error;
 
-// Interior cells up to which a plain realm runs 1, 2 and 3 blocks per SM
-// instead of the kernel's full occupancy (see initialize).
-constexpr long long kRealmCells1 = 1500000ll, kRealmCells2 = 4200000ll, kRealmCells3 = 8ll << 20;
+// Interior cells up to which a plain realm runs 1 and 2 blocks per SM instead
+// of the kernel's full occupancy (see initialize).
+constexpr long long kRealmCells1 = 1500000ll, kRealmCells2 = 8ll << 20;
 
 }  // namespace
 
@@ -267,14 +267,14 @@ struct amca_t {
     {
       // Blocks per SM of the persistent launch: a small realm's generations
       // are short, so its steps are set by barrier and look-back latency,
-      // which fall with the number of blocks (GB300, blocks per SM 1 / 2 / 3 /
-      // 4: 24^3 6.2 / 6.5 / 7.0 / 7.5 ms, 60^3 12.5 / 13.5 / 14.2 / 15.0, 95^3
-      // 14.7 / 15.3 / 16.0 / 16.9, 128^3 18.5 / 17.9 / 18.2 / 18.9, 160^3 24.5
-      // / 21.9 / 21.8 / 22.3, 200^3 34.0 / 28.3 / 26.9 / 26.9, 256^3 56.1 /
-      // 42.1 / 38.5 / 37.6, 320^3 94.7 / 64.4 / 55.4 / 52.3).
+      // which fall with the number of blocks (GB300, blocks per SM 1 / 2 / 3:
+      // 24^3 5.07 / 5.39 / 6.5 ms, 60^3 11.09 / 11.70 / 13.7, 95^3 12.86 /
+      // 13.52 / 15.4, 128^3 16.57 / 15.93 / 17.4, 160^3 22.5 / 19.9 / 21.2,
+      // 200^3 31.6 / 26.0 / 26.6, 256^3 52.6 / 39.2 / 38.3 and 37.6 at 4, 320^3
+      // 89.3 / 60.6 / 55.8 and 52.3).
       // AMCA_PLAIN_BLOCKS_PER_SM overrides the choice.
       const long long interior = (long long)c.nx * c.ny * c.nz;
-      int per_sm = interior <= kRealmCells1 ? 1 : interior <= kRealmCells2 ? 2 : interior <= kRealmCells3 ? 3 : 0;
+      int per_sm = interior <= kRealmCells1 ? 1 : interior <= kRealmCells2 ? 2 : 0;
       if (const char *e = getenv("AMCA_PLAIN_BLOCKS_PER_SM")) per_sm = std::max(1, atoi(e));
       if (per_sm > 0) {
         int sms = 0;

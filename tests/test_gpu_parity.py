@@ -293,3 +293,20 @@ def test_gpu_grids_across_brick_edges_match_oracle(amca, oracle, cells):
         b.run()
     assert np.array_equal(r.field("grain_id"), whole["grain"])
     r.close()
+
+
+@pytest.mark.parametrize("per_sm", [1, 2, 3])
+@pytest.mark.parametrize("sites", [4700, 24000])
+def test_gpu_generations_around_the_shared_lane_sizes_match_oracle(amca, oracle, monkeypatch, per_sm, sites):
+    """Claims by eight, four, two and one lane a rank (up to 2,432, 4,864, 9,728 entries on 152 blocks of one per SM,
+    and the same on 304) and by the kernel without: sites that nucleate within a few steps of one another, counts and
+    fields equal to the C restatement's in the middle of the run and at its end."""
+    monkeypatch.setenv("AMCA_PLAIN_BLOCKS_PER_SM", str(per_sm))
+    case = cases._mixed("lanes", (46, 41, 37), 11, 40, sites, t_dot=-900.0)
+    whole = oracle.run_plain(case)
+    for k in (whole["steps"] // 2, -1):
+        out = run_gpu(amca, case, max_steps=k)
+        ref = whole if k < 0 else oracle.run_plain(case, max_steps=k)
+        assert out["stats"]["step"] == ref["steps"] and out["stats"]["grains"] == ref["num_grains"], k
+        assert out["stats"]["active"] == ref["active_grains"], k
+        assert np.array_equal(out["orient"], ref["orient"]) and np.array_equal(out["grain"], ref["grain"]), k
