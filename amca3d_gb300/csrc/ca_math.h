@@ -520,10 +520,14 @@ AMCA_HD double hex8_interp64(const double t[8], double xi, double eta, double ze
 }
 
 // FP32 estimate of hex8_interp64 from the node values and parametric
-// coordinates rounded to float. The shape functions are convex weights
-// (coordinates in [-1, 1]), so its error stays below 2e-6 of the largest node
-// magnitude; hex8_err32 gives the bound the kernels decide with: 2^-16 of that
-// magnitude plus 2^-16 absolute.
+// coordinates rounded to float, and a bound on its error to decide with. With
+// u = 2^-24 and M the largest node magnitude: a factor 1 +- x errs by 1.5 u (x
+// rounded, then the sum), which over the eight nodes and three directions
+// comes to 36 u M (the other two factors sum to 4); node values rounded 8 u M;
+// three roundings per product 24 u M (the weights times 8 sum to 8); seven sums
+// 56 u M; times 1/8: 15.5 u M < 2^-20 M. The bound is 2^-19 of M (plus 2^-16
+// absolute, for underflow); FP64 decides closer to a threshold. A margin of
+// 2^-16 sent a lane of every other warp of a melt pool's elements there.
 AMCA_HD float hex8_interp32(const float t[8], float xi, float eta, float zeta) {
   const float a0 = 1.0f - eta, a1 = 1.0f + eta, b0 = 1.0f - xi, b1 = 1.0f + xi, c0 = 1.0f - zeta, c1 = 1.0f + zeta;
   return 0.125f * (a0 * b0 * c0 * t[0] + a0 * b1 * c0 * t[1] + a1 * b1 * c0 * t[2] + a1 * b0 * c0 * t[3] +
@@ -532,7 +536,7 @@ AMCA_HD float hex8_interp32(const float t[8], float xi, float eta, float zeta) {
 AMCA_HD float hex8_err32(const float t[8]) {
   float mg = 0.0f;
   for (int i = 0; i < 8; ++i) mg = fmaxf(mg, fabsf(t[i]));
-  return ldexpf(mg, -16) + 1.52587890625e-05f;
+  return ldexpf(mg, -19) + 1.52587890625e-05f;
 }
 
 // ProblemPhysics_RappazGandin1993::compute_growth_velocity for a uniform field

@@ -372,6 +372,7 @@ void RemeltRealm::upload_initial_state() {
   RCK(cudaMemsetAsync(dev_.gdz, 0, N * 4, stream_));
   RCK(cudaMemsetAsync(dev_.flagbits, 0, ((N + 31) / 32) * 4, stream_));
   RCK(cudaMemsetAsync(dev_.eliq, 0, std::max<int64_t>(dev_.nelem, 1) * 4, stream_));
+  RCK(cudaMemsetAsync(dev_.emolten, 0, std::max<int64_t>(dev_.nelem, 1), stream_));
   RCK(remelt_init_theta(dev_, stream_));
   hostvel_->seq_req = 0;
   hostvel_->seq_done = 0;
@@ -449,6 +450,9 @@ void RemeltRealm::initialize() {
   }
   // --- FE -> CA map (MapVoxelManager::execute_with_focus_on_CA_region) ---
   for (int a = 0; a < 3; ++a) d.nn[a] = frames_.nn[a];
+  d.e_xy = (d.nn[0] - 1) * (d.nn[1] - 1);
+  d.e_by_x = fast_div(std::max(1, d.nn[0] - 1));
+  d.e_by_xy = fast_div(std::max(1, d.e_xy));
   d.nnodes = frames_.nnodes;
   d.nelem = frames_.nelem();
   int32_t *tag = alloc<int32_t>(N);
@@ -632,6 +636,7 @@ void RemeltRealm::initialize() {
   d.emin = alloc<double>(d.nelem);
   d.evoid = alloc<uint8_t>(d.nelem);
   d.eliq = alloc<int32_t>(d.nelem);
+  d.emolten = alloc<uint8_t>(d.nelem);
   for (int sl = 0; sl < 2; ++sl) {
     d.fmax[sl] = alloc<double>(d.nelem);
     d.fmin[sl] = alloc<double>(d.nelem);
@@ -664,6 +669,7 @@ void RemeltRealm::initialize() {
   d.hard_idx = alloc<int32_t>(N);
   d.hard_T = alloc<double>(N);
   d.hard_v = alloc<double>(std::min<size_t>(N, kHostVelCap));  // used while a request fits the mapped buffer
+  d.hard_other = alloc<double>(std::min<size_t>(N, kHostVelCap));
   d.hard_L = alloc<double>(std::min<size_t>(N, kHostVelCap));
   {
     void *hv = nullptr;

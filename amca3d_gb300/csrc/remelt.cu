@@ -16,25 +16,25 @@
 //
 // GB300 design: one persistent cooperative kernel runs whole steps, five
 // phases per step separated by bounded grid barriers.
-//   A  full-grid pass over interior cells. A cell's temperature is a pure
-//      function of the node temperatures, so it is computed in FP64 only where
-//      a decision depends on it: liquid cells, and solid cells whose element's
-//      node maximum (plus a rounding margin) reaches the liquidus. Every other
-//      solid cell costs two 4-byte loads and an L2-resident element lookup.
-//      (GB300's FP64 rate is ~1/64 of its FP32 rate; this keeps the step
-//      bandwidth-bound.) Liquid cells that can flag neighbours go to a list.
+//   A  the cells of the active elements, a warp per element: those that may
+//      melt or change class (not below the liquidus as a whole, nor above it
+//      with every cell molten). A cell's temperature is a pure function of the
+//      node temperatures; FP32 with an error bound decides, FP64 where it does
+//      not (the FP64 rate is ~1/64 of FP32's). Liquid cells that can flag
+//      neighbours go to a list; lengths that waited for the host settle.
 //   B  listed liquid cells set the flag bits of their solid neighbours; each
 //      newly flagged cell is appended to the flagged list.
 //   C  block 0 nucleates (sites in ascending order, block scan for ids);
 //      the other blocks apply the grain-length cutoff and take the minimum
 //      temperature over flagged cells (atomicMin on an ordered key).
-//   D  dt (uniform); every flagged cell grows its grain and tests its liquid
-//      neighbours; a containment claims the neighbour with atomicMin of
+//   D  dt (one thread per block); every flagged cell, by one to eight lanes,
+//      grows its grain and tests its liquid neighbours; a containment claims the neighbour with atomicMin of
 //      INT_MIN + sweep position, so the smallest claim is the first capturing
 //      cell of the reference's sweep (captures do not cascade within a step).
 //   E  claimed cells take the winner's orientation and decentred envelope
-//      (FP64, reference operation order); the FE replay advances and the next
-//      step's node temperatures and element bounds are computed.
+//      (FP64, reference operation order) on the blocks' last warps; beside
+//      them the FE replay advances and the next step's node temperatures,
+//      element bounds and active list are computed.
 // New grain objects (cells without one) get ids in sweep order: events
 // (sweep position, neighbour index) are sorted by block 0 after the step.
 #include <cooperative_groups.h>
@@ -226,9 +226,7 @@ __device__ void stage_flush(unsigned *count, int32_t *list, unsigned cap) {
   __syncthreads();
   for (unsigned i = threadIdx.x; i < n; i += blockDim.x)
     if (s_base + i < cap) list[s_base + i] = s_stage[i];
-  __syncthreads();
-  if (threadIdx.x == 0) s_stage_n = 0u;
-  __syncthreads();
+  if (threadIdx.x == 0) s_stage_n = 0u;  // (the grid barrier comes before the next push)
 }
 
 // `cnt` consecutive list slots for each thread that reaches it together: one
@@ -254,11 +252,11 @@ __device__ __forceinline__ int64_t spread_begin(int first_block) {
 __device__ __forceinline__ int64_t spread_stride(int first_block) {
   return (int64_t)(gridDim.x - first_block) * blockDim.x;
 }
-// The same spread over all blocks, last block first: for short lists whose
-// items are heavy, so that they meet the blocks with the least other work in
-// the phase (those past the ends of the thread-ordered loops).
+// The same spread over all blocks, last block and last thread first: for short
+// lists whose items are heavy, so that they meet the blocks and warps with the
+// least other work in the phase.
 __device__ __forceinline__ int64_t spread_begin_last() {
-  return (int64_t)threadIdx.x * gridDim.x + (gridDim.x - 1 - blockIdx.x);
+  return (int64_t)(kBlock - 1 - threadIdx.x) * gridDim.x + (gridDim.x - 1 - blockIdx.x);
 }
 
 // Order-preserving key of a double (for atomicMin); NaN never reaches it.
@@ -285,17 +283,24 @@ __device__ __forceinline__ bool f64_below(double x, double y) {
   return f64_less(plus_zero(x), plus_zero(y)) && !f64_nan(x) && !f64_nan(y);
 }
 
+// The double next to x > 0 on the side of r.
+__device__ __forceinline__ double toward(double x, double r) {
+  return __longlong_as_double(__double_as_longlong(x) + (__double_as_longlong(r) < 0 ? -1 : 1));
+}
+
 // x^b for b in {1, 2, 3}, correctly rounded (square and cube through exact
 // two-products). `near` is raised when the exact power lies within 0.02 ulp
 // of a rounding midpoint: there glibc's pow, whose error bound is 0.52 ulp,
-// may round to the other neighbour. pow(x, 1) == x holds for every double.
-__device__ double ipow_checked(double x, int b, bool &near) {
+// may round to the other neighbour (`other`). pow(x, 1) == x holds for every
+// double.
+__device__ double ipow_checked(double x, int b, bool &near, double &other) {
   if (b == 1) return x;
   const double p = x * x;
   const double e = __fma_rn(x, x, -p);
   if (b == 2) {
     const double u = ulp_of(p);
     near = near || fabs(fabs(e) - 0.5 * u) <= 0.02 * u;
+    other = toward(p, e);
     return p;
   }
   const double q1 = p * x;
@@ -307,6 +312,7 @@ __device__ double ipow_checked(double x, int b, bool &near) {
   const double rem = (q1 - c) + t;
   const double u = ulp_of(c);
   near = near || fabs(fabs(rem) - 0.5 * u) <= 0.02 * u;
+  other = toward(c, rem);
   return c;
 }
 
@@ -316,23 +322,36 @@ __device__ double ipow_checked(double x, int b, bool &near) {
 // dT below 1e100), without the dozen FP64 instructions of its power.
 // `near_v`: v itself is within 2^-30 of the host's value all the same (a
 // power is within an ulp of glibc's, the sum's cancellation bounded).
-__device__ double velocity(const RemeltDevice &d, double T, bool &hard, bool &near_v) {
+// `other`: with one such term, v with the power's other neighbour (the host's
+// velocity is one of the two), else -1.
+__device__ double velocity(const RemeltDevice &d, double T, bool &hard, bool &near_v, double &other) {
   const double dT = d.Tm - T;
   double v = 0.0;
   hard = false;
   near_v = false;
+  other = -1.0;
   if (dT > 0) {
     bool n1 = false, n2 = false, n3 = false;
+    double p1 = 0, p2 = 0, p3 = 0;
     const bool all = f64_exponent(dT) > 1023 + 332;
-    const double t1 = d.a1 == 0 && !all ? d.a1 : d.a1 * ipow_checked(dT, d.b1, n1);
-    const double t2 = d.a2 == 0 && !all ? d.a2 : d.a2 * ipow_checked(dT, d.b2, n2);
-    const double t3 = d.a3 == 0 && !all ? d.a3 : d.a3 * ipow_checked(dT, d.b3, n3);
-    hard = (d.a1 != 0 && n1) || (d.a2 != 0 && n2) || (d.a3 != 0 && n3);
+    const double t1 = d.a1 == 0 && !all ? d.a1 : d.a1 * ipow_checked(dT, d.b1, n1, p1);
+    const double t2 = d.a2 == 0 && !all ? d.a2 : d.a2 * ipow_checked(dT, d.b2, n2, p2);
+    const double t3 = d.a3 == 0 && !all ? d.a3 : d.a3 * ipow_checked(dT, d.b3, n3, p3);
+    n1 = n1 && d.a1 != 0;
+    n2 = n2 && d.a2 != 0;
+    n3 = n3 && d.a3 != 0;
+    hard = n1 || n2 || n3;
     v = t1 + t2 + t3;
     if (v < 0.0) v = 0.0;
     const float terms = fabsf(f64_to_f32_rz(t1)) + fabsf(f64_to_f32_rz(t2)) + fabsf(f64_to_f32_rz(t3));
     const float vf = f64_to_f32_rz(v);
     near_v = vf > 1e-30f && terms < 65536.0f * vf;
+    if (hard && (int)n1 + (int)n2 + (int)n3 == 1) {
+      const double a = n1 ? d.a1 : (n2 ? d.a2 : d.a3), p = n1 ? p1 : (n2 ? p2 : p3);
+      const double t = a * p;
+      other = (n1 ? t : t1) + (n2 ? t : t2) + (n3 ? t : t3);
+      if (other < 0.0) other = 0.0;
+    }
   }
   return v;
 }
@@ -400,23 +419,32 @@ __device__ bool host_velocities(const RemeltDevice &d, RemeltCtrl *c, unsigned n
 }
 
 // The overlapped form of host_velocities for a request that fits the mapped
-// buffer: block 0 writes the temperatures and posts the request without
-// waiting; every block counts it (its s_host_seq names the answer it waits
-// for). Called by every block, uniformly.
+// buffer: the last four warps of block 0 write the temperatures and post the
+// request without waiting (a short flagged list is on its first warps, which
+// grow meanwhile: 2.4 us that the phase waited for); every block counts it (its
+// s_host_seq names the answer it waits for, from the next block barrier on).
+// Called by every block, uniformly.
+constexpr int kPostThreads = 128;
 __device__ void host_post(const RemeltDevice &d, unsigned nh, bool min_hard, double minT) {
   const unsigned total = nh + (min_hard ? 1u : 0u);
-  if (blockIdx.x == 0 && d.host != nullptr) {
-    for (unsigned k = threadIdx.x; k < total; k += blockDim.x) d.host->T[k] = k < nh ? d.hard_T[k] : minT;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      d.host->n = total;
-      __threadfence_system();
-      st_release_sys(&d.host->seq_req, s_host_seq + 1);
-      s_clk[kClkHostCalls] += 1;
-      s_clk[kClkHostVel] += total;
+  const int t = (int)threadIdx.x - (kBlock - kPostThreads);
+  if (blockIdx.x == 0 && t >= 0) {
+    const unsigned seq = s_host_seq + 1;
+    if (d.host != nullptr)
+      for (unsigned k = t; k < total; k += kPostThreads) d.host->T[k] = k < nh ? d.hard_T[k] : minT;
+    asm volatile("bar.sync 1, %0;" ::"n"(kPostThreads) : "memory");
+    if (t == 0) {
+      if (d.host != nullptr) {
+        d.host->n = total;
+        __threadfence_system();
+        st_release_sys(&d.host->seq_req, seq);
+        s_clk[kClkHostCalls] += 1;
+        s_clk[kClkHostVel] += total;
+      }
+      s_host_seq = seq;
     }
   }
-  if (threadIdx.x == 0) s_host_seq += 1;
+  if (blockIdx.x != 0 && threadIdx.x == 0) s_host_seq += 1;
 }
 
 // Thread 0 waits (bounded) for the answer to the block's last request; the
@@ -472,13 +500,25 @@ __device__ __forceinline__ void elem_nodes(const int nn[3], int64_t e, int64_t n
   for (int l = 4; l < 8; l++) nid[l] = nid[l - 4] + nxy;
 }
 
+// The same of the device's element grid, without 64-bit divisions.
+__device__ __forceinline__ void elem_nodes(const RemeltDevice &d, int32_t e, int64_t nid[8]) {
+  const int k = quotient(e, d.e_by_xy), r = e - k * d.e_xy, j = quotient(r, d.e_by_x), i = r - j * (d.nn[0] - 1);
+  const int64_t nxy = (int64_t)d.nn[0] * d.nn[1];
+  nid[0] = nxy * k + (int64_t)d.nn[0] * j + i;
+  nid[1] = nid[0] + 1;
+  nid[2] = nid[1] + d.nn[0];
+  nid[3] = nid[2] - 1;
+#pragma unroll
+  for (int l = 4; l < 8; l++) nid[l] = nid[l - 4] + nxy;
+}
+
 // MapVoxelManager::evaluate_temperature (MapVoxelManager.cpp:746-799):
 // false (T untouched) without an element or next to a void node.
-__device__ bool eval_T(const RemeltDevice &d, const double *th, int64_t c, double &T) {
-  const int32_t e = d.tag[c];
+__device__ bool eval_T(const RemeltDevice &d, const double *th, int32_t e, double xi, double eta, double zeta,
+                       double &T) {
   if (e < 0) return false;
   int64_t nid[8];
-  elem_nodes(d.nn, e, nid);
+  elem_nodes(d, (int32_t)e, nid);
   const double nullMat = d.void_t + 0.00001;
   double t[8];
   bool below = false;
@@ -488,8 +528,11 @@ __device__ bool eval_T(const RemeltDevice &d, const double *th, int64_t c, doubl
     below = below || f64_below(t[i], nullMat);
   }
   if (below) return false;
-  T = hex8_interp64(t, d.pc[3 * c], d.pc[3 * c + 1], d.pc[3 * c + 2]);
+  T = hex8_interp64(t, xi, eta, zeta);
   return true;
+}
+__device__ __forceinline__ bool eval_T(const RemeltDevice &d, const double *th, int64_t c, double &T) {
+  return eval_T(d, th, d.tag[c], d.pc[3 * c], d.pc[3 * c + 1], d.pc[3 * c + 2], T);
 }
 
 // FP32 estimate of evaluate_temperature's value for a cell with material,
@@ -500,12 +543,25 @@ __device__ bool eval_T(const RemeltDevice &d, const double *th, int64_t c, doubl
 // 2^-16 of it (plus 2^-16 absolute).
 __device__ float eval_T32(const RemeltDevice &d, const float *th32, int64_t c, int32_t e, float &err) {
   int64_t nid[8];
-  elem_nodes(d.nn, e, nid);
+  elem_nodes(d, (int32_t)e, nid);
   float t[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) t[i] = th32[nid[i]];
   err = hex8_err32(t);
   return hex8_interp32(t, d.pc32[3 * c], d.pc32[3 * c + 1], d.pc32[3 * c + 2]);
+}
+
+// Whether FP32 shows that a site's cell is not undercooled by more than dtc:
+// above Tm - dtc its T has Tm - T <= dtc, also rounded. Two FP64 instructions
+// in place of two exact temperatures (the last blocks of phase B worked on those
+// of the sites inside the melt pool: 3 us of 9).
+__device__ __forceinline__ bool too_hot_to_nucleate(const RemeltDevice &d, const float *th32, int32_t cell, double dtc) {
+  const int32_t e = d.tag[cell];
+  if (e < 0 || d.evoid[e]) return false;
+  float err;
+  const float T = eval_T32(d, th32, cell, e, err);
+  const float thr = __double2float_ru(d.Tm - dtc);
+  return __fsub_rd(T, err) > __fadd_ru(thr, 2.4e-7f * fabsf(thr));  // (Tm - dtc itself rounded)
 }
 
 // thetaArray_ update of pseudo_single_integration_step (LoadDataFromFile.cpp:281-290)
@@ -587,6 +643,11 @@ __device__ void frame_extrema(const RemeltDevice &d, const int64_t nid[8], int f
 // nullMatTemp_ + 0.01: below it a cell counts as without material in the
 // liquid-neighbour pass (Remelting.cpp:504-507)
 __device__ __forceinline__ double null_plus() { return -1.0 + 0.01; }
+
+// Every cell of an element above the liquidus (and above nullMatTemp_ + 0.01).
+__device__ __forceinline__ bool hot(bool void_, double mn, double Tm) {
+  return !void_ && f64_below(Tm, mn) && f64_below(null_plus(), Tm);
+}
 
 // mx < Tm && mn >= null_plus() for an element's bounds (never NaN), by the bits
 __device__ __forceinline__ bool quiet(double mx, double mn, double Tm) {
@@ -829,7 +890,7 @@ __global__ void init_theta_kernel(RemeltDevice d) {
   }
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < d.nelem; e += stride) {
     int64_t nid[8];
-    elem_nodes(d.nn, e, nid);
+    elem_nodes(d, (int32_t)e, nid);
     double t[8];
     for (int i = 0; i < 8; ++i) t[i] = d.frames[nid[i]];
     element_bounds(d, e, t);
@@ -850,7 +911,7 @@ __global__ void external_theta_kernel(RemeltDevice d, long long step, const doub
   }
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < d.nelem; e += stride) {
     int64_t nid[8];
-    elem_nodes(d.nn, e, nid);
+    elem_nodes(d, (int32_t)e, nid);
     double t[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) t[i] = theta[nid[i]];
@@ -1081,27 +1142,48 @@ __device__ void assign_new_grains(const RemeltDevice &d, RemeltCtrl *c) {
 struct ElemView {
   int32_t e;
   bool void_;
-  bool quiet;
+  bool quiet, hot;
   float t[8];
   float err;
 };
 
-// Warp-collective: the view of element e (every lane gets it).
-__device__ __forceinline__ ElemView elem_view(const RemeltDevice &d, const float *th32, int32_t e) {
-  ElemView v;
+// What a warp loads of an element before it looks at it (each of lanes 0 to 7
+// a node's temperature).
+struct ElemLoad {
+  int32_t e;
+  int64_t begin, end;  // its cells
+  float t;
+  bool void_, molten;
+  double mx, mn;
+};
+__device__ __forceinline__ ElemLoad elem_load(const RemeltDevice &d, const float *th32, int32_t e) {
+  ElemLoad v;
   v.e = e;
   const int lane = threadIdx.x & 31;
+  v.begin = d.ecell_start[e];
+  v.end = d.ecell_start[e + 1];
   int64_t nid[8];
-  elem_nodes(d.nn, e, nid);
+  elem_nodes(d, (int32_t)e, nid);
   int64_t mine = nid[0];
 #pragma unroll
   for (int i = 1; i < 8; ++i)
     if (lane == i) mine = nid[i];
-  const float tl = lane < 8 ? th32[mine] : 0.0f;
+  v.t = lane < 8 ? th32[mine] : 0.0f;
   v.void_ = d.evoid[e] != 0;
-  v.quiet = quiet(d.emax[e], d.emin[e], d.Tm);
+  v.molten = d.emolten[e] != 0;
+  v.mx = d.emax[e];
+  v.mn = d.emin[e];
+  return v;
+}
+// Warp-collective: the view of the element (every lane gets it).
+__device__ __forceinline__ ElemView elem_view(const RemeltDevice &d, const ElemLoad &l) {
+  ElemView v;
+  v.e = l.e;
+  v.void_ = l.void_;
+  v.quiet = quiet(l.mx, l.mn, d.Tm);
+  v.hot = hot(l.void_, l.mn, d.Tm);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v.t[i] = __shfl_sync(0xffffffffu, tl, i);
+  for (int i = 0; i < 8; ++i) v.t[i] = __shfl_sync(0xffffffffu, l.t, i);
   v.err = hex8_err32(v.t);
   return v;
 }
@@ -1138,7 +1220,8 @@ __device__ __forceinline__ float eval_T32_view(const RemeltDevice &d, int64_t c,
 // `ev`: the cell's element view when the caller walks an element's cells
 // (the cell's tag is then ev->e), or nullptr; `pre`: the cell's values
 // loaded by the caller, or nullptr.
-__device__ __forceinline__ void phase_update(const RemeltDevice &d, RemeltCtrl *c, int64_t cell, const double *th,
+// Returns whether the cell ends liquid and melted.
+__device__ __forceinline__ bool phase_update(const RemeltDevice &d, RemeltCtrl *c, int64_t cell, const double *th,
                                              const float *th32, bool settled, bool count_all,
                                              unsigned long long &exactT, unsigned long long &melts,
                                              const ElemView *ev = nullptr, const CellPre *pre = nullptr) {
@@ -1173,7 +1256,7 @@ __device__ __forceinline__ void phase_update(const RemeltDevice &d, RemeltCtrl *
   if (o > -1) {
     if (withMat) {
       // certainly below the liquidus and above nullMatTemp_ + 0.01: nothing changes
-      if (ev ? ev->quiet : (d.emax[e] < d.Tm && d.emin[e] >= np)) return;
+      if (ev ? ev->quiet : (d.emax[e] < d.Tm && d.emin[e] >= np)) return false;
       T32 = ev ? eval_T32_view(d, cell, *ev, err, pre) : eval_T32(d, th32, cell, e, err);
       have32 = true;
       int b = below(d.Tm, d.tm_lo, d.tm_hi);
@@ -1188,7 +1271,7 @@ __device__ __forceinline__ void phase_update(const RemeltDevice &d, RemeltCtrl *
           bn = below(np, d.np_lo, d.np_hi);
         }
         if (bn == 1 && (pre ? mel : d.melted[cell])) d.melted[cell] = 0;
-        return;
+        return false;
       }
     }
     d.orient[cell] = -1;  // melt
@@ -1235,11 +1318,14 @@ __device__ __forceinline__ void phase_update(const RemeltDevice &d, RemeltCtrl *
   if (m1 != m0) d.melted[cell] = m1;
   d.tcls[cell] = (uint8_t)((flags ? kTlt : 0) | (le ? kTle : 0) | (gtn ? kTgtNull : 0) | (wm2 ? kTgeNullPlus : 0));
   if (wm2 && flags) stage_push((int32_t)cell, &c->n_liq, d.liq, d.list_cap);  // the cell flags its solid neighbours
+  return m1 != 0;
 }
 
 // Register budget of two blocks per SM (128 per thread), run with one block
-// per SM: on pbf_500 that is faster than the unconstrained 186 registers, two
-// blocks per SM, or 512-thread blocks (740 against 768, 793 and 801 ms per run).
+// per SM: two realms fit on the device together, and 236 registers without
+// spills gave the same times (500 x 250 x 100 cells: 463 against 460 ms).
+// 512-thread blocks: 48.3 against 49.6 us a step there, 37.2 against 35.5 on
+// 75 x 50 x 30.
 __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long long limit) {
   __shared__ unsigned smem[kWarps + 2];
   RemeltCtrl *c = d.ctrl;
@@ -1248,7 +1334,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
   const int64_t gtid = blockIdx.x * (int64_t)blockDim.x + tid;
   const int64_t nthr = (int64_t)gridDim.x * blockDim.x;
   const int64_t M = (int64_t)g.nx * g.ny * g.nz;
-  const int64_t nyzg = (int64_t)g.nyg * g.nzg;
+  const int nyzg = g.nyg * g.nzg;
   unsigned long long tests = 0, tests64 = 0, caps = 0, exactT = 0, melts = 0, visited = 0, eactive = 0;
   bool ok = true;
   if (tid == 0) {
@@ -1271,6 +1357,22 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     s_stop = stop_reason(d, s_S[0], limit);
   }
   __syncthreads();
+  // The exact lengths of the last step's cells whose velocity the host worked
+  // out (entries of its flagged list, parity lp), by the blocks' last warps: dt
+  // is still the last step's.
+  unsigned owed = 0;  // its hard velocities
+  auto settle = [&](int lp) {
+    for (int64_t k = spread_begin_last(); k < owed; k += spread_stride(0)) {
+      const int32_t cell = d.flagged[lp][d.hard_idx[k]];
+      const double L = d.glen[cell];
+      if (!length_pending(L)) continue;
+      const unsigned slot = (unsigned)__double_as_longlong(L);
+      host_wait_thread(d, c);
+      d.glen[cell] = d.hard_L[slot] + s_dT * ld_volatile(&d.host->v[slot]);
+    }
+    owed = 0;
+  };
+  int last_par = 0;
   for (unsigned turn = 0;; ++turn) {
     const StepScalars &S = s_S[turn & 1];
     StepScalars &N = s_S[(turn & 1) ^ 1];
@@ -1316,11 +1418,28 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     } else {  // the cells of the active elements (a warp per element)
       const unsigned na = ld_volatile(&c->n_eact[par]);
       const int lane = tid & 31;
-      const int64_t gw = gtid >> 5, nw = nthr >> 5;
+      // (elements that come second on a warp are dealt over all blocks, block 0 last)
+      const int64_t gw = (int64_t)(tid >> 5) * gridDim.x + (gridDim.x - 1 - blockIdx.x), nw = nthr >> 5;
+      // the warp's next element is loaded while it works on this one (its id one element earlier still)
+      ElemLoad el{};
+      int32_t e1 = -1;
+      if (gw < na) {
+        const int32_t e0 = d.eact[par][gw];
+        if (gw + nw < na) e1 = d.eact[par][gw + nw];
+        el = elem_load(d, th32, e0);
+      }
       for (int64_t w = gw; w < na; w += nw) {
-        const int32_t e = d.eact[par][w];
-        const int64_t b = d.ecell_start[e], en = d.ecell_start[e + 1];
-        const ElemView ev = elem_view(d, th32, e);
+        const int64_t b = el.begin, en = el.end;
+        const ElemView ev = elem_view(d, el);
+        const bool was_molten = el.molten;
+        if (e1 >= 0) {
+          el = elem_load(d, th32, e1);
+          e1 = w + 2 * nw < na ? d.eact[par][w + 2 * nw] : -1;
+        }
+        // An element above the liquidus whose cells the last visit left liquid, melted and classed as such has nothing
+        // to change (a cell that nucleates takes the mark away); lists made by the host's temperatures hold them
+        if (ev.hot && was_molten) continue;
+        bool molten = true;
         // kCellPre cells per lane at a time: their ids, then everything the
         // update reads of them, each set of loads in flight together
         for (int64_t k0 = b + lane; k0 < en; k0 += 32 * kCellPre) {
@@ -1340,12 +1459,16 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
 #pragma unroll
           for (int j = 0; j < kCellPre; ++j) {
             if (cl[j] < 0) continue;
-            phase_update(d, c, cl[j], th, th32, settled, false, exactT, melts, &ev, &pre[j]);
+            if (!phase_update(d, c, cl[j], th, th32, settled, false, exactT, melts, &ev, &pre[j])) molten = false;
             ++visited;
           }
         }
+        molten = __all_sync(0xffffffffu, molten) && ev.hot;
+        if (lane == 0 && molten != was_molten) d.emolten[ev.e] = molten ? 1 : 0;
       }
     }
+    settle(par ^ 1);
+    last_par = par;
     stage_flush(&c->n_liq, d.liq, d.list_cap);
     if (gtid == 0) {
       const unsigned long long t1 = now_ns();
@@ -1366,7 +1489,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     for (int64_t sidx = (int64_t)(kBlock - 1 - tid) * gridDim.x + blockIdx.x; sidx < d.nsites; sidx += nthr) {
       const int32_t cell = d.site_cell[sidx];
       uint8_t f = 0;
-      if (d.orient[cell] == -1 && d.melted[cell]) {
+      if (d.orient[cell] == -1 && d.melted[cell] && !too_hot_to_nucleate(d, th32, cell, d.site_dtc[sidx])) {
         double T = -1.0, Told = -1.0;
         const bool withMat = eval_T(d, th, cell, T);
         bool cooling = false;
@@ -1504,7 +1627,10 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
           if (newg) d.grain[cell] = (int32_t)(n_grains + done_g + r_g);
           d.orient[cell] = oid;
           const int32_t e = d.tag[cell];
-          if (e >= 0) atomicSub(&d.eliq[e], 1);
+          if (e >= 0) {
+            atomicSub(&d.eliq[e], 1);
+            d.emolten[e] = 0;
+          }
         }
         done_o += tot_o;
         done_g += tot_g;
@@ -1527,24 +1653,32 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
           const int32_t cell = d.flagged[par][q];
           int I, J, K;
           cell_ijk(g, cell, I, J, K);
+          // all it reads by cell in flight at once
+          const int32_t gid = d.grain[cell], e = d.tag[cell];
+          const double len = d.glen[cell], xi = d.pc[3 * (int64_t)cell], eta = d.pc[3 * (int64_t)cell + 1],
+                       zeta = d.pc[3 * (int64_t)cell + 2];
           if (ghost(g, I, J, K)) continue;
-          if (d.grain[cell] < 0) continue;
-          if (!(d.glen[cell] < d.cutoff)) d.glen[cell] = d.h;  // length reset (:688-694)
+          if (gid < 0) continue;
+          if (!(len < d.cutoff)) d.glen[cell] = d.h;  // length reset (:688-694)
           double T = -1.0;
           ++exactT;
-          eval_T(d, th, cell, T);
+          eval_T(d, th, e, xi, eta, zeta, T);
           {  // growth velocity of single_integration_step (Remelting.cpp:569-576)
             bool hard = false, near_v = false;
             const double Targ = (T < d.Ts) ? d.Ts + 0.01 : T;
-            const double vel = velocity(d, Targ, hard, near_v);
+            double other;
+            const double vel = velocity(d, Targ, hard, near_v, other);
             d.fvel[q] = vel;
             if (hard) {
               const unsigned slot = append_slot(&c->n_hard);
               if (slot < d.list_cap) {
                 d.hard_idx[slot] = (int32_t)q;
                 d.hard_T[slot] = Targ;
-                if (slot < (unsigned)kHostVelCap) d.hard_v[slot] = near_v ? vel : -1.0;
-                // the host's answer, slot `slot`, is taken in phase D
+                if (slot < (unsigned)kHostVelCap) {
+                  d.hard_v[slot] = near_v ? vel : -1.0;
+                  d.hard_other[slot] = near_v ? other : -1.0;
+                }
+                // the host's answer, slot `slot`, is taken later
                 // (velocities are never negative)
                 d.fvel[q] = -1.0 - (double)slot;
               }
@@ -1572,7 +1706,9 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     // states loaded at once). Neither the dt phase nor another cell's growth
     // changes any of it (a claim leaves a candidate a candidate), so this
     // thread's first flagged cell is loaded while dt is found.
-    auto grow_load = [&](int32_t cell, int I, int J, int K) {
+    // (by `lanes` lanes that share the cell: each looks at the neighbours
+    // numbered its `sub` modulo that)
+    auto grow_load = [&](int32_t cell, int I, int J, int K, int sub, int lanes) {
       GrowPre p;
       p.cell = cell;
       p.I = I;
@@ -1583,11 +1719,8 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
       p.dx = d.gdx[cell];
       p.dy = d.gdy[cell];
       p.dz = d.gdz[cell];
-#pragma unroll
-      for (int qq = 0; qq < 9; ++qq) p.m32[qq] = d.omat32[9 * (int64_t)p.ori + qq];
       uint32_t cand = 0;
-#pragma unroll
-      for (int n = 0; n < 26; ++n) {
+      auto look = [&](int n) {
         int di, dj, dk;
         nbr_offset(n, di, dj, dk);
         const int32_t nb = cell + dk * g.nxyg + dj * g.nxg + di;
@@ -1595,7 +1728,16 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         const int32_t o = in ? d.orient[nb] : 0;
         const uint8_t cls = in ? d.tcls[nb] : 0;  // a liquid neighbour's classes are this step's
         cand |= (in && o <= -1 && (cls & kTle) && (cls & kTgtNull) ? 1u : 0u) << n;
+      };
+      if (lanes == 1) {
+#pragma unroll
+        for (int n = 0; n < 26; ++n) look(n);
+      } else {
+#pragma unroll 4
+        for (int n = sub; n < 26; n += lanes) look(n);
       }
+#pragma unroll
+      for (int qq = 0; qq < 9; ++qq) p.m32[qq] = d.omat32[9 * (int64_t)p.ori + qq];
       p.cand = cand;
       return p;
     };
@@ -1604,15 +1746,29 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
       s_nh = ld_volatile(&c->n_hard);  // uniform: every block reads the same counter and key
       s_minT = dkey_inv(ld_volatile(&c->minT_key));
       bool h = false, near_v = false;
-      const double v = velocity(d, s_minT, h, near_v);
+      double other;
+      const double v = velocity(d, s_minT, h, near_v, other);
+      const double dt_v = step_dt(d, S, v);
+      // (where something else bounds dt, either velocity will do)
+      if (h && other >= 0 && __double_as_longlong(step_dt(d, S, other)) == __double_as_longlong(dt_v)) h = false;
       s_min_hard = h ? 1 : 0;
       if (!h) {
-        s_dT = step_dt(d, S, v);
-        next_scalars(d, S, s_dT, ld_volatile(&c->n_nuc_sites[par]), N, s_R);
-        s_stop = stop_reason(d, N, limit);
+        s_dT = dt_v;
       }
     }
-    const int64_t q0 = spread_begin(0);
+    // A list that leaves most threads without an entry gives each entry eight,
+    // four or two lanes, the last warp's left out (dt is found there), as long as
+    // that takes one turn. One lane per entry has the block's 26 neighbour states
+    // and tests in one or two warps, each load in sectors of its own: at 60
+    // entries a block 3.9 us of loads and 2.1 us of tests, with two lanes 2.4 and
+    // 1.2; the phase 13.2 us, with four lanes in two turns 13.2, with two 9.4.
+    const int64_t nshare = (int64_t)gridDim.x * (kBlock - 32);
+    const int lsh = nf * 8ll <= nshare ? 3 : nf * 4ll <= nshare ? 2 : nf * 2ll <= nshare ? 1 : 0, lanes = 1 << lsh, sub = tid & (lanes - 1);
+    // this thread's entries: q0, then every qn-th; the first of its warp's
+    const int lt = lsh ? kBlock - 32 : kBlock;
+    const int64_t q0 = tid < lt ? (int64_t)(tid >> lsh) * gridDim.x + blockIdx.x : INT64_MAX / 2;
+    const int64_t w0 = tid < lt ? (int64_t)((tid & ~31) >> lsh) * gridDim.x + blockIdx.x : INT64_MAX / 2;
+    const int64_t qn = (int64_t)(lt >> lsh) * gridDim.x;
     GrowPre pre0{};
     bool use0 = false;
     if (q0 < nf && nf <= d.list_cap) {
@@ -1620,7 +1776,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
       int I, J, K;
       cell_ijk(g, cell, I, J, K);
       if (!ghost(g, I, J, K) && d.grain[cell] >= 0) {
-        pre0 = grow_load(cell, I, J, K);
+        pre0 = grow_load(cell, I, J, K, sub, lanes);
         use0 = true;
       }
     }
@@ -1642,90 +1798,62 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     }
     if (overlap) {
       host_post(d, nh, min_hard, s_minT);
-      if (min_hard) host_wait_block(d, c);
+      if (min_hard) {
+        __syncthreads();  // (block 0's thread 0 waits by the count that another of its threads raises)
+        host_wait_block(d, c);
+      }
     }
     if (min_hard) {  // uniform
-      if (lead) {
-        s_dT = step_dt(d, S, overlap ? ld_volatile(&d.host->v[nh]) : ld_volatile(&c->vmin));
-        next_scalars(d, S, s_dT, ld_volatile(&c->n_nuc_sites[par]), N, s_R);
-        s_stop = stop_reason(d, N, limit);
-      }
+      if (lead) s_dT = step_dt(d, S, overlap ? ld_volatile(&d.host->v[nh]) : ld_volatile(&c->vmin));
       __syncthreads();
     }
     const double dT = s_dT;
+    if (lead) {  // beside the growth, read from phase E on
+      next_scalars(d, S, dT, ld_volatile(&c->n_nuc_sites[par]), N, s_R);
+      s_stop = stop_reason(d, N, limit);
+    }
+    owed = overlap ? nh : 0u;
 
     // ===== D: grow and claim (Remelting.cpp:545-622) =====
-    // one flagged cell: growth by dT * vel and its claims (atomicMin of the
-    // sweep position: the order cells are taken in does not matter)
-    auto grow_finish = [&](const GrowPre &p, double vel) {
-      const int32_t cell = p.cell;
-      const int I = p.I, J = p.J, K = p.K;
-      const double L = p.glen + dT * vel;
-      d.glen[cell] = L;
-      if (L == 0) return;  // Octahedron::cell_is_captured: a zero half-diagonal captures nothing
-      const int32_t ori = p.ori;
-      const int32_t mine = INT_MIN + sweep_pos(g, I, J, K);
-      const float dxf = p.dx, dyf = p.dy, dzf = p.dz;
-      const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(dxf) + fabsf(dyf) + fabsf(dzf)) + d.coord_err;
-      const float L32 = f64_to_f32_rz(L);  // the pre-test's margin is 2^-14 of it
-      const float *m32 = p.m32;
-      uint32_t cand = p.cand;
-      while (cand) {
-        const int n = __ffs(cand) - 1;
-        cand &= cand - 1;
-        int di, dj, dk;
-        nbr_offset(n, di, dj, dk);
-        const int32_t nb = cell + dk * g.nxyg + dj * g.nxg + di;
-        ++tests;
-        int f = captured_f32(m32, (float)di * d.h32 - dxf, (float)dj * d.h32 - dyf, (float)dk * d.h32 - dzf, errg,
-                             L32);
-        if (f < 0) {
-          ++tests64;
-          const double ccx = centre_coord(g.x0, g.h, I + di);
-          const double ccy = centre_coord(g.y0, g.h, J + dj);
-          const double ccz = centre_coord(g.z0, g.h, K + dk);
-          f = is_captured_f64(d.omat + 9 * (int64_t)ori, ccx - d.gx[cell], ccy - d.gy[cell], ccz - d.gz[cell], L) ? 1
-                                                                                                                  : 0;
-        }
-        if (f) {
-          const int32_t old = atomicMin(&d.orient[nb], mine);
-          if (old == -1) {
-            const unsigned slot = append_slot(&c->n_claim);
-            if (slot < d.list_cap) d.claimed[slot] = nb;
-          }
-        }
-      }
+    auto captured_exact = [&](const GrowPre &p, int n, double L) {
+      int di, dj, dk;
+      nbr_offset(n, di, dj, dk);
+      const double ccx = centre_coord(g.x0, g.h, p.I + di);
+      const double ccy = centre_coord(g.y0, g.h, p.J + dj);
+      const double ccz = centre_coord(g.z0, g.h, p.K + dk);
+      return is_captured_f64(d.omat + 9 * (int64_t)p.ori, ccx - d.gx[p.cell], ccy - d.gy[p.cell], ccz - d.gz[p.cell], L)
+                 ? 1
+                 : 0;
     };
-    auto grow_claim = [&](int32_t cell, int I, int J, int K, double vel) {
-      grow_finish(grow_load(cell, I, J, K), vel);
-    };
-    // A cell whose velocity the host is still working out, slot k of the
-    // request: its claims are made with the device's own value, which is within
-    // 2^-30 of the host's, when the FP32 test decides every candidate (its
-    // margin is 2^-14). The exact length follows in phase E (hard_L keeps the
-    // length before the step, the cell's own names the slot until then), so
-    // the host's 12 us answer time overlaps this phase, its barrier and most of
-    // E instead of standing in this one. False when the exact value is needed.
-    auto grow_early = [&](const GrowPre &p, unsigned k) {
-      const double v = d.hard_v[k];
-      if (v < 0) return false;
-      const double L = p.glen + dT * v;
-      const float L32 = f64_to_f32_rz(L);
-      if (!(L32 > 1e-30f)) return false;
-      const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(p.dx) + fabsf(p.dy) + fabsf(p.dz)) + d.coord_err;
+    // the candidates that a length of L contains; `undecided` (given for a length
+    // that is not exact): stops where FP32 does not decide
+    auto contained = [&](const GrowPre &p, double L, float L32, bool *undecided) {
       uint32_t in = 0;
+      // Octahedron::cell_is_captured: a zero half-diagonal captures nothing
+      if ((__double_as_longlong(L) << 1) == 0) return in;
+      const float errg = 4.76837158203125e-07f * (d.h32 + fabsf(p.dx) + fabsf(p.dy) + fabsf(p.dz)) + d.coord_err;
       for (uint32_t cand = p.cand; cand; cand &= cand - 1) {
         const int n = __ffs(cand) - 1;
         int di, dj, dk;
         nbr_offset(n, di, dj, dk);
         ++tests;
-        const int f = captured_f32(p.m32, (float)di * d.h32 - p.dx, (float)dj * d.h32 - p.dy, (float)dk * d.h32 - p.dz,
-                                   errg, L32);
-        if (f < 0) return false;
+        int f = captured_f32(p.m32, (float)di * d.h32 - p.dx, (float)dj * d.h32 - p.dy, (float)dk * d.h32 - p.dz, errg,
+                             L32);
+        if (f < 0) {
+          if (undecided) {
+            *undecided = true;
+            return in;
+          }
+          ++tests64;
+          f = captured_exact(p, n, L);
+        }
         in |= (uint32_t)f << n;
       }
-      d.hard_L[k] = p.glen;
-      d.glen[p.cell] = __longlong_as_double(kLengthPending | (long long)k);
+      return in;
+    };
+    // claims of the neighbours in `in`: atomicMin of the sweep position, so the
+    // order cells are taken in does not matter
+    auto claim = [&](const GrowPre &p, uint32_t in) {
       const int32_t mine = INT_MIN + sweep_pos(g, p.I, p.J, p.K);
       for (; in; in &= in - 1) {
         const int n = __ffs(in) - 1;
@@ -1737,36 +1865,78 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
           if (slot < d.list_cap) d.claimed[slot] = nb;
         }
       }
-      return true;
+    };
+    // one flagged cell: growth by dT * vel and its claims
+    auto grow_finish = [&](const GrowPre &p, double vel) {
+      const double L = p.glen + dT * vel;
+      d.glen[p.cell] = L;
+      claim(p, contained(p, L, f64_to_f32_rz(L), nullptr));
+    };
+    // The velocity that entry q grows with: the host's value is the device's or
+    // the one with the power's other neighbour, and mostly both give the same
+    // length (the growth of a step is a small part of it), so that the entry
+    // need not wait. Negative: it does.
+    auto usable_velocity = [&](int64_t q, double glen) {
+      const double vel = d.fvel[q];  // (the chunked host path rewrites it in the dt phase)
+      if (!(vel < 0)) return vel;
+      const unsigned k = (unsigned)(-1.0 - vel);
+      const double v = d.hard_v[k], w = d.hard_other[k];
+      if (!(v >= 0 && w >= 0) || __double_as_longlong(glen + dT * w) != __double_as_longlong(glen + dT * v)) return vel;
+      d.fvel[q] = v;
+      return v;
+    };
+    // An entry's growth and claims, by the lanes that share it, the whole warp
+    // together (`use`: the lanes have one). One that waits for slot k of the
+    // request claims with the device's own value, which is within 2^-30 of the
+    // host's, when the FP32 test decides every candidate (its margin is 2^-14).
+    // The exact length follows in the next step's phase A (hard_L keeps the
+    // length before the step, the cell's own names the slot until then), so that
+    // no phase stands in the host's 12 to 17 us answer time, except for a capture
+    // by such a cell in E. True when the exact value is needed here.
+    auto grow_entry = [&](int64_t q, const GrowPre &p, bool use) {
+      const double vel = use ? usable_velocity(q, p.glen) : 0.0;
+      const bool early = vel < 0;
+      const unsigned k = early ? (unsigned)(-1.0 - vel) : 0u;
+      const double v = early ? d.hard_v[k] : vel;
+      const double L = p.glen + dT * v;
+      const float L32 = f64_to_f32_rz(L);  // the pre-test's margin is 2^-14 of it
+      bool wait = early && (v < 0 || !(L32 > 1e-30f));
+      const uint32_t in = use && !wait ? contained(p, L, L32, early ? &wait : nullptr) : 0u;
+      const unsigned mates = ((1u << lanes) - 1u) << (tid & 31 & ~(lanes - 1));
+      wait = (__ballot_sync(0xffffffffu, wait) & mates) != 0;
+      if (!use || wait) return wait;
+      if (sub == 0) {
+        if (early) {
+          d.hard_L[k] = p.glen;
+          d.glen[p.cell] = __longlong_as_double(kLengthPending | (long long)k);
+        } else {
+          d.glen[p.cell] = L;
+        }
+      }
+      claim(p, in);
+      return false;
     };
     bool pending = false;  // a hard velocity of this thread waits for the host's answer in this phase
-    bool owing = false;    // ... in phase E
-    if (use0) {
-      const double vel = d.fvel[q0];  // (the chunked host path rewrites it in the dt phase)
-      if (!(vel < 0))
-        grow_finish(pre0, vel);
-      else if (grow_early(pre0, (unsigned)(-1.0 - vel)))
-        owing = true;
-      else
-        pending = true;
-    }
-    for (int64_t q = q0 + spread_stride(0); q < nf && nf <= d.list_cap; q += spread_stride(0)) {
-      const int32_t cell = d.flagged[par][q];
-      int I, J, K;
-      cell_ijk(g, cell, I, J, K);
-      if (ghost(g, I, J, K)) continue;
-      if (d.grain[cell] < 0) continue;
-      const double vel = d.fvel[q];
-      if (!(vel < 0))
-        grow_claim(cell, I, J, K, vel);
-      else if (grow_early(grow_load(cell, I, J, K), (unsigned)(-1.0 - vel)))
-        owing = true;
-      else
-        pending = true;
-    }
+    if (nf <= d.list_cap)
+      for (int64_t q = q0, w = w0; w < nf; q += qn, w += qn) {
+        bool use = use0;
+        if (q != q0) {
+          use = false;
+          if (q < nf) {
+            const int32_t cell = d.flagged[par][q];
+            int I, J, K;
+            cell_ijk(g, cell, I, J, K);
+            if (!ghost(g, I, J, K) && d.grain[cell] >= 0) {
+              pre0 = grow_load(cell, I, J, K, sub, lanes);
+              use = true;
+            }
+          }
+        }
+        if (grow_entry(q, pre0, use) && sub == 0) pending = true;
+      }
     if (overlap && __syncthreads_or(pending)) {  // uniform within the block
       host_wait_block(d, c);
-      for (int64_t q = spread_begin(0); q < nf && nf <= d.list_cap; q += spread_stride(0)) {
+      for (int64_t q = q0; sub == 0 && q < nf && nf <= d.list_cap; q += qn) {
         const double vel = d.fvel[q];
         if (!(vel < 0)) continue;
         const int32_t cell = d.flagged[par][q];
@@ -1774,11 +1944,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         cell_ijk(g, cell, I, J, K);
         if (ghost(g, I, J, K) || d.grain[cell] < 0) continue;
         if (length_pending(d.glen[cell])) continue;  // claimed already
-        const double v = ld_volatile(&d.host->v[(unsigned)(-1.0 - vel)]);
-        if (q == q0 && use0)
-          grow_finish(pre0, v);  // loaded ahead, still current (only this thread grows the cell)
-        else
-          grow_claim(cell, I, J, K, v);
+        grow_finish(grow_load(cell, I, J, K, 0, 1), ld_volatile(&d.host->v[(unsigned)(-1.0 - vel)]));
       }
     }
     if (gtid == 0) {
@@ -1789,22 +1955,23 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     if (!(ok = grid_barrier(d, 3))) break;
 
     // ===== E: captures (Remelting.cpp:807-847) and the FE replay step (LoadDataFromFile.cpp:207-313) =====
+    // (captures by the blocks' last warps, the replay by the others)
+    const unsigned nc = ld_volatile(&c->n_claim);
     {
-      const unsigned nc = ld_volatile(&c->n_claim);
       if (nc > d.list_cap) {
         if (gtid == 0) atomicCAS(&c->error, 0, kRemeltErrList);
       } else {
         for (int64_t q = spread_begin_last(); q < nc; q += spread_stride(0)) {
           const int32_t nb = d.claimed[q];
           const int32_t w = d.orient[nb] - INT_MIN;
-          const int wi = (int)(w / nyzg), wj = (int)((w / g.nzg) % g.nyg), wk = (int)(w % g.nzg);
+          const int wi = w / nyzg, wr = w - wi * nyzg, wj = wr / g.nzg, wk = wr - wj * g.nzg;
           const int64_t wc = (int64_t)wk * g.nxyg + (int64_t)wj * g.nxg + wi;
           int I, J, K;
           cell_ijk(g, nb, I, J, K);
           const int32_t ori = d.gori[wc];
           const double px = d.gx[wc], py = d.gy[wc], pz = d.gz[wc];
           double L = ld_volatile(&d.glen[wc]);
-          if (length_pending(L)) {  // (its own thread may be writing the same value meanwhile)
+          if (length_pending(L)) {
             host_wait_thread(d, c);
             const unsigned k = (unsigned)__double_as_longlong(L);
             L = d.hard_L[k] + dT * ld_volatile(&d.host->v[k]);
@@ -1837,7 +2004,10 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
           }
           d.orient[nb] = ori;
           const int32_t e = d.tag[nb];
-          if (e >= 0) atomicSub(&d.eliq[e], 1);
+          if (e >= 0) {
+            atomicSub(&d.eliq[e], 1);
+            d.emolten[e] = 0;
+          }
           ++caps;
         }
       }
@@ -1856,17 +2026,20 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         // four nodes per thread at a time: their frame values are loaded
         // before any interpolated value is stored (a store could alias the
         // next node's loads and would keep them one after another)
-        for (int64_t n0 = gtid; n0 < d.nnodes; n0 += 4 * nthr) {
+        // a block's last warp is still at its first capture when the others are through here
+        const int rt = nc > 0 ? kBlock - 32 : kBlock;
+        const int64_t rid = tid < rt ? blockIdx.x * (int64_t)rt + tid : INT64_MAX / 2, rn = gridDim.x * (int64_t)rt;
+        for (int64_t n0 = rid; n0 < d.nnodes; n0 += 4 * rn) {
           double a[4], b[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const int64_t n = n0 + j * nthr;
+            const int64_t n = n0 + j * rn;
             a[j] = n < d.nnodes ? f0[n] : 0.0;
             b[j] = n < d.nnodes ? f1[n] : 0.0;
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const int64_t n = n0 + j * nthr;
+            const int64_t n = n0 + j * rn;
             if (n >= d.nnodes) continue;
             const double v = lerp_node(a[j], b[j], ratio, d.void_t);
             tn[n] = v;
@@ -1876,20 +2049,26 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         // Element bounds depend on the frame pair only (every interpolated node value lies between
         // its two frame values), so the active list is rebuilt when the pair changes; elements near
         // the void threshold need the exact interpolation and force a rebuild every step.
-        const bool rebuild = S.step == 0 || f_new != S.f_new || ld_volatile(&c->any_near) || d.force_exact;
+        // An element above the liquidus with every cell molten is left out: it has nothing to change until a cell
+        // nucleates in it (another rebuild; a cell above the liquidus is never captured) or its bounds do. Of 1,990
+        // active elements on a 500 x 250 x 100 track 1,150 are such, and more than one per warp were left: phase A
+        // 11.8 to 9.1 us.
+        const bool rebuild = S.step == 0 || f_new != S.f_new || N.n_orient != S.n_orient ||
+                             ld_volatile(&c->any_near) || d.force_exact;
         if (!rebuild) {
           const unsigned na = ld_volatile(&c->n_eact[par]);
-          for (int64_t q = gtid; q < na; q += nthr) d.eact[par ^ 1][q] = d.eact[par][q];
-          if (gtid == 0) {
-            c->n_eact[par ^ 1] = na;
-            eactive += na;
+          for (int64_t q = rid; q < na; q += rn) {
+            const int32_t e = d.eact[par][q];
+            if (d.emolten[e]) continue;
+            d.eact[par ^ 1][append_slot(&c->n_eact[par ^ 1])] = e;
+            ++eactive;
           }
         }
         const bool st0 = ld_volatile(&c->fstat_frame[f_new & 1]) == f_new;
         const bool st1 = ld_volatile(&c->fstat_frame[(f_new - 1) & 1]) == f_new - 1;
-        for (int64_t e = gtid; e < d.nelem && rebuild; e += nthr) {
+        for (int64_t e = rid; e < d.nelem && rebuild; e += rn) {
           int64_t nid[8];
-          elem_nodes(d.nn, e, nid);
+          elem_nodes(d, (int32_t)e, nid);
           const uint8_t void_before = d.evoid[e];
           double mx0, mn0, mx1, mn1;
           bool near0, near1;
@@ -1915,24 +2094,12 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
           const bool v = d.evoid[e] != 0;
           const bool active = (!v && !quiet(d.emax[e], d.emin[e], d.Tm)) || (v != (void_before != 0)) ||
                               (!v && ld_volatile(&d.eliq[e]) > 0);
-          if (active) {
+          if (active && !(d.emolten[e] && hot(v, d.emin[e], d.Tm))) {
             const unsigned slot = append_slot(&c->n_eact[par ^ 1]);
             if (slot < (unsigned)d.nelem) d.eact[par ^ 1][slot] = (int32_t)e;
             ++eactive;
           }
         }
-      }
-    }
-    // the lengths that this block's cells still owe
-    if (__syncthreads_or(owing)) {
-      host_wait_block(d, c);
-      for (int64_t q = q0; q < nf; q += spread_stride(0)) {
-        if (!(d.fvel[q] < 0)) continue;
-        const int32_t cell = d.flagged[par][q];
-        const double L = d.glen[cell];
-        if (!length_pending(L)) continue;
-        const unsigned k = (unsigned)__double_as_longlong(L);
-        d.glen[cell] = d.hard_L[k] + dT * ld_volatile(&d.host->v[k]);
       }
     }
     if (gtid == 0) {
@@ -1970,6 +2137,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     if (!(ok = grid_barrier(d, 4))) break;
     if (exhausted) break;  // uniform; block 0 recorded kRemeltFramesEnd
   }
+  if (ok) settle(last_par);
   if (ok && blockIdx.x == 0) assign_new_grains(d, c);
   if (tid == 0)
     for (int i = 0; i < 6; ++i)

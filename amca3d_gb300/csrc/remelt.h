@@ -119,6 +119,8 @@ struct RemeltDevice {
   int nsites;
   // FE replay
   int nn[3];
+  int e_xy;                  // elements of an x-y layer
+  FastDiv e_by_x, e_by_xy;   // of a row's and a layer's elements
   int64_t nnodes, nelem;
   const double *frames;      // ring of frame_slots frames (frame f in slot f % frame_slots), nnodes each
   const double *frame_time;  // per frame, scaled (every frame)
@@ -135,6 +137,7 @@ struct RemeltDevice {
   double *emax, *emin;       // per element bounds on the interpolated temperature (current step)
   int force_exact;           // some parametric coordinate is not finite: no bound shortcuts
   int detail;                // nonzero: also gather the slowest block's busy time per barrier
+  uint8_t *emolten;          // per element: above the liquidus at its last visit, every cell left liquid and melted
   uint8_t *evoid;            // per element: some node below void_temperature + 1e-5
   int32_t *eliq;             // per element: interior liquid cells it holds
   double *fmax[2], *fmin[2]; // per element: node extrema of a frame (slot = frame index & 1)
@@ -153,6 +156,7 @@ struct RemeltDevice {
   int32_t *hard_idx;         // flagged-list entries whose velocity the host evaluates
   double *hard_T;            // ... their temperatures,
   double *hard_v;            // the device's own velocities (-1: not near enough to claim with),
+  double *hard_other;        // the other value the host's may have (-1: not known),
   double *hard_L;            // and the cells' lengths before the step
   HostVelocity *host;        // device view of the mapped host buffer
   int host_cap;              // entries of `host` one request may use (kHostVelCap; smaller in tests)

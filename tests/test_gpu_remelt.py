@@ -7,6 +7,7 @@ and compared, after every CA step, with the reference's per-step state
 liquid-neighbour fields — bit for bit. The synthetic-frame generator on the
 GPU and frames passed from memory must give the same run as the text file.
 """
+import dataclasses
 import os
 import sys
 
@@ -99,6 +100,43 @@ def test_remelt_gpu_host_velocities_in_chunks(amca, tmp_path, monkeypatch, name)
         d = digests(r)
         assert not [k for k in STATE if d[k] != g["digests"][i][fields.index(k)]], f"step {i + 1}"
     assert r.stats()["reserved"] > calls > 0
+    r.close()
+
+
+@pytest.mark.parametrize("stride", [2, 9])
+@pytest.mark.parametrize("name", ["remelt_random", "remelt_scaled", "remelt_new_grains"])
+def test_remelt_gpu_launches_of_several_steps_match_the_reference(amca, tmp_path, name, stride):
+    """Lengths whose velocity came from the host settle in the next step of a launch, or at the launch's end: state,
+    time and dt equal the reference's after launches of two and nine steps."""
+    fx = FIX[name]
+    r = make_realm(amca, fx, str(tmp_path))
+    g = np.load(os.path.join(HERE, "golden", f"{name}.npz"))
+    fields = [str(f) for f in g["fields"]]
+    for i in range(stride - 1, len(g["digests"]), stride):
+        r.run(stride)
+        st = r.stats()
+        assert st["step"] == i + 1 and st["time"] == g["time"][i] and st["dt"] == g["dt"][i]
+        d = digests(r)
+        assert not [k for k in STATE if d[k] != g["digests"][i][fields.index(k)]], f"step {i + 1}"
+    r.close()
+
+
+@pytest.mark.parametrize("mean", [20.0, -400.0])
+def test_remelt_gpu_sites_that_nucleate_above_the_liquidus(amca, oracle, tmp_path, mean):
+    """Elements above the liquidus whose cells are all molten are not visited again, unless a cell nucleates in one (a
+    site with a negative undercooling does so while it cools and melts again): state, time and dt equal the C
+    restatement's along the run, in launches of several steps."""
+    fx = dataclasses.replace(FIX["remelt_nucleation"],
+                             case=dataclasses.replace(FIX["remelt_nucleation"].case, bulk=(4.0e14, mean, 30.0)))
+    r = make_realm(amca, fx, str(tmp_path))
+    whole = oracle.run_remelt(fx.case, str(tmp_path))
+    for k in list(range(50, whole["steps"], 100)) + [whole["steps"]]:
+        r.run(k - r.stats()["step"])
+        o = oracle.run_remelt(fx.case, str(tmp_path), max_steps=k)
+        st = r.stats()
+        assert st["step"] == o["steps"] == k and st["time"] == o["time"] and st["dt"] == o["last_dt"]
+        for name in ("orient", "grain", "melted", "cooling", "flag", "T"):
+            assert np.array_equal(r.field(FIELD_OF[name]).astype(o[name].dtype), o[name]), (k, name)
     r.close()
 
 
