@@ -299,8 +299,9 @@ def test_gpu_grids_across_brick_edges_match_oracle(amca, oracle, cells):
 @pytest.mark.parametrize("sites", [4700, 24000])
 def test_gpu_generations_around_the_shared_lane_sizes_match_oracle(amca, oracle, monkeypatch, per_sm, sites):
     """Claims by eight, four, two and one lane a rank (up to 2,432, 4,864, 9,728 entries on 152 blocks of one per SM,
-    and the same on 304), by the kernel without, and neighbourhood checks by as many lanes a cell: sites that nucleate within a few steps of one another, counts and
-    fields equal to the C restatement's in the middle of the run and at its end."""
+    and the same on 304) and by the kernel without; neighbourhood checks and marks by as many lanes a cell or rank:
+    sites that nucleate within a few steps of one another, counts and fields equal to the C restatement's in the middle
+    of the run and at its end."""
     monkeypatch.setenv("AMCA_PLAIN_BLOCKS_PER_SM", str(per_sm))
     case = cases._mixed("lanes", (46, 41, 37), 11, 40, sites, t_dot=-900.0)
     whole = oracle.run_plain(case)
