@@ -1863,7 +1863,11 @@ __global__ void grain_field_scatter_kernel(int32_t *out, const int32_t *gcell, i
 // captured, the decentred new envelope.
 __global__ void envelope_eval_kernel(long long n, const double *l2g, const double *gc, const double *len, double h,
                                      const double *trunc, int32_t *cap64, int32_t *capfast, double *info) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+  // four lanes per envelope: capture_f64 in each of them, capture_f64_quad in all together; capfast is -1 where a bit
+  // of the two differs
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < 4 * n; t += (long long)gridDim.x * blockDim.x) {
+    const long long i = t >> 2;
+    const int lane = threadIdx.x & 31, base = lane & ~3, a = (lane & 3) < 2 ? lane & 3 : 2;
     const double *m = l2g + 9 * i;
     const double gx = gc[3 * i], gy = gc[3 * i + 1], gz = gc[3 * i + 2], L = len[i];
     const bool c64 = is_captured_f64(m, gx, gy, gz, L);
@@ -1873,11 +1877,22 @@ __global__ void envelope_eval_kernel(long long n, const double *l2g, const doubl
     const float err = 5.9604645e-08f * (fabsf(fx) + fabsf(fy) + fabsf(fz));  // conversion rounding of gc
     int f = L == 0 ? 0 : captured_f32(m32, fx, fy, fz, err, (float)L);
     if (f < 0) f = c64 ? 1 : 0;
-    cap64[i] = c64 ? 1 : 0;
-    capfast[i] = f;
+    if ((lane & 3) == 3) {
+      cap64[i] = c64 ? 1 : 0;
+      capfast[i] = f;
+    }
+    __syncwarp(15u << base);
     double out[4] = {0.0, 0.0, 0.0, 0.0};
-    if (c64) capture_f64(m, gx, gy, gz, L, h, trunc[i], out);
-    for (int q = 0; q < 4; ++q) info[4 * i + q] = out[q];
+    if (c64) {
+      capture_f64(m, gx, gy, gz, L, h, trunc[i], out);
+      double len;
+      const double o = capture_f64_quad(m, a, 15u << base, base, a == 0 ? gx : (a == 1 ? gy : gz), L, h, trunc[i], len);
+      const bool same = (f64_bits(o) == f64_bits(out[a]) || (isnan(o) && isnan(out[a]))) &&
+                        (f64_bits(len) == f64_bits(out[3]) || (isnan(len) && isnan(out[3])));
+      if (!same) capfast[i] = -1;
+    }
+    info[4 * i + a] = out[a];
+    if ((lane & 3) == 3) info[4 * i + 3] = out[3];
   }
 }
 

@@ -142,6 +142,32 @@ def test_gpu_envelope_kat(amca):
     assert info[m].tobytes() == k["info"][m].tobytes()
 
 
+@pytest.mark.parametrize("kind", ["random", "tied", "on_axis", "tiny", "huge"])
+def test_gpu_decentring_by_four_lanes_equals_one(amca, kind):
+    """envelope_eval decentres every envelope by one lane and by four, and gives -1 as its fast verdict where a bit
+    differs: points anywhere inside, at equal distances from two or three corners, on an axis, and at magnitudes that
+    leave the fast path's range of exponents (where squares overflow, both give NaN)."""
+    rng = np.random.default_rng(7)
+    n, h = 4000, 2.0e-6
+    q = np.linalg.qr(rng.normal(size=(n, 3, 3)))[0]
+    scale = {"tiny": 1e-160, "huge": 1e160}.get(kind, h)
+    c = rng.uniform(0.0, 1.0, (n, 3)) * rng.choice([-1.0, 1.0], (n, 3))
+    if kind == "tied":
+        q[:] = np.eye(3)
+        c[: n // 2] = c[: n // 2, :1] * np.sign(c[: n // 2])
+        c[n // 2:, 1] = c[n // 2:, 0]
+    if kind == "on_axis":
+        q[:] = np.eye(3)
+        c[np.arange(n), rng.integers(0, 3, n)] = 0.0
+    length = (np.abs(c).sum(1) + rng.uniform(0.0, 1.0, n)) * scale
+    gc = np.einsum("nij,nj->ni", q, c * scale)
+    l2g = np.ascontiguousarray(q.reshape(n, 9))
+    trunc = np.full(n, float(np.float32(np.sqrt(np.float32(3.0)))))
+    cap64, fast, _ = amca.envelope_eval(l2g, gc, length, scale, trunc)
+    assert (cap64 == 1).sum() > n // 2
+    assert (fast >= 0).all()
+
+
 def test_gpu_outputs_byte_identical(amca):
     case = cases.output_case()
     ref_dir = os.path.join(GOLD, "outputs_tiny")
