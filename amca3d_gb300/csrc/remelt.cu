@@ -14,7 +14,7 @@
 //   5. advances the FE replay and interpolates nodal temperatures between two
 //      frames (LoadDataFromFile.cpp:207-313).
 //
-// GB300 design: one persistent cooperative kernel runs whole steps, five
+// GB300 design: one persistent cooperative kernel runs whole steps, four
 // phases per step separated by bounded grid barriers.
 //   A  the cells of the active elements, a warp per element: those that may
 //      melt or change class (not below the liquidus as a whole, nor above it
@@ -23,10 +23,12 @@
 //      not (the FP64 rate is ~1/64 of FP32's). Liquid cells that can flag
 //      neighbours go to a list; lengths that waited for the host settle.
 //   B  listed liquid cells set the flag bits of their solid neighbours; each
-//      newly flagged cell is appended to the flagged list.
-//   C  block 0 nucleates (sites in ascending order, block scan for ids);
-//      the other blocks apply the grain-length cutoff and take the minimum
-//      temperature over flagged cells (atomicMin on an ordered key).
+//      newly flagged cell is appended to the flagged list, and its block
+//      applies the grain-length cutoff, works out its growth velocity and
+//      takes the minimum temperature (atomicMin on an ordered key). The site
+//      conditions, on the blocks' last warps.
+//   C  block 0 nucleates (sites in ascending order, block scan for ids), in
+//      front of its part of D.
 //   D  dt (one thread per block); every flagged cell, by one to eight lanes,
 //      grows its grain and tests its liquid neighbours; a containment claims the neighbour with atomicMin of
 //      INT_MIN + sweep position, so the smallest claim is the first capturing
@@ -204,6 +206,11 @@ __device__ __forceinline__ unsigned append_slot(unsigned *counter) {
 // global atomicAdd when the phase ends (stage_flush, every thread) — one
 // same-address global atomic per block instead of one per warp and
 // iteration. Entries beyond the buffer go to the global list directly.
+// Cells that a block's first kFlagWarps warps flag in a step, with their list entries.
+constexpr int kFlagWarps = kWarps - 1;
+__shared__ unsigned s_fresh_n;
+__shared__ int32_t s_fresh[kFresh], s_fresh_slot[kFresh];
+
 constexpr unsigned kStage = 1024;
 __shared__ unsigned s_stage_n;
 __shared__ int32_t s_stage[kStage];
@@ -242,19 +249,11 @@ __device__ __forceinline__ unsigned append_slots(unsigned *counter, unsigned cnt
 }
 
 // Short lists whose items carry FP64 work or long load chains are dealt
-// across blocks first: item q goes to block first_block + q % nb (thread
-// q / nb of it), so the work spreads over every SM instead of filling the
-// first few. Visit q = spread_begin(...), then q += spread_stride(...).
-__device__ __forceinline__ int64_t spread_begin(int first_block) {
-  const int64_t nb = gridDim.x - first_block;
-  return (int64_t)threadIdx.x * nb + (blockIdx.x - first_block);
-}
-__device__ __forceinline__ int64_t spread_stride(int first_block) {
-  return (int64_t)(gridDim.x - first_block) * blockDim.x;
-}
-// The same spread over all blocks, last block and last thread first: for short
-// lists whose items are heavy, so that they meet the blocks and warps with the
-// least other work in the phase.
+// across blocks first, so that the work spreads over every SM instead of
+// filling the first few; here from the last block and thread down, so that they
+// meet the blocks and warps with the least other work in the phase. Visit
+// q = spread_begin_last(), then q += spread_stride().
+__device__ __forceinline__ int64_t spread_stride() { return (int64_t)gridDim.x * blockDim.x; }
 __device__ __forceinline__ int64_t spread_begin_last() {
   return (int64_t)(kBlock - 1 - threadIdx.x) * gridDim.x + (gridDim.x - 1 - blockIdx.x);
 }
@@ -1341,6 +1340,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     s_left = now_ns();
     for (int i = 0; i < 6; ++i) s_busy[i] = 0ull;
     s_stage_n = 0u;
+    s_fresh_n = 0u;
     for (int i = 0; i < kClkN; ++i) s_clk[i] = 0ull;
     s_host_seq = ld_volatile(&c->host_seq);
   }
@@ -1362,7 +1362,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
   // is still the last step's.
   unsigned owed = 0;  // its hard velocities
   auto settle = [&](int lp) {
-    for (int64_t k = spread_begin_last(); k < owed; k += spread_stride(0)) {
+    for (int64_t k = spread_begin_last(); k < owed; k += spread_stride()) {
       const int32_t cell = d.flagged[lp][d.hard_idx[k]];
       const double L = d.glen[cell];
       if (!length_pending(L)) continue;
@@ -1506,9 +1506,52 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         }
       }
       d.snuc[sidx] = f;
-      if (f) atomicAdd(&c->n_nuc_sites[par], 1u);
+      if (f) {
+        atomicAdd(&c->n_nuc_sites[par], 1u);
+        d.tcls[cell] &= (uint8_t)~kTle;  // solid to the growth phase (block 0 nucleates it meanwhile)
+      }
     }
     const unsigned long long tfl = tid == 0 ? now_ns() : 0ull;
+    // Length cutoff and minimum temperature (Remelting.cpp:656-705) of the flagged cell of list entry q, and its growth
+    // velocity, by the block that flagged it (a phase of its own cost another barrier and the list's way through
+    // memory: B and C 13.6 us, now 12.2, on a 500 x 250 x 100 track). Without room in the block's buffer: at once.
+    unsigned long long best = dkey(d.Tm);
+    auto coldest = [&](int32_t cell, unsigned q) {
+      int I, J, K;
+      cell_ijk(g, cell, I, J, K);
+      // all it reads by cell in flight at once
+      const int32_t gid = d.grain[cell], e = d.tag[cell];
+      const double len = d.glen[cell], xi = d.pc[3 * (int64_t)cell], eta = d.pc[3 * (int64_t)cell + 1],
+                   zeta = d.pc[3 * (int64_t)cell + 2];
+      if (ghost(g, I, J, K) || gid < 0) return;
+      if (!(len < d.cutoff)) d.glen[cell] = d.h;  // length reset (:688-694)
+      double T = -1.0;
+      ++exactT;
+      eval_T(d, th, e, xi, eta, zeta, T);
+      // growth velocity of single_integration_step (Remelting.cpp:569-576)
+      bool hard = false, near_v = false;
+      const double Targ = (T < d.Ts) ? d.Ts + 0.01 : T;
+      double other;
+      const double vel = velocity(d, Targ, hard, near_v, other);
+      d.fvel[q] = vel;
+      if (hard) {
+        const unsigned slot = append_slot(&c->n_hard);
+        if (slot < d.list_cap) {
+          d.hard_idx[slot] = (int32_t)q;
+          d.hard_T[slot] = Targ;
+          if (slot < (unsigned)kHostVelCap) {
+            d.hard_v[slot] = near_v ? vel : -1.0;
+            d.hard_other[slot] = near_v ? other : -1.0;
+          }
+          // the host's answer, slot `slot`, is taken later
+          // (velocities are never negative)
+          d.fvel[q] = -1.0 - (double)slot;
+        }
+      }
+      if (T <= d.Ts || !(T == T)) return;
+      const unsigned long long k = dkey(T);
+      best = k < best ? k : best;
+    };
     {
       const unsigned nl = ld_volatile(&c->n_liq);
       if (nl > d.list_cap) {
@@ -1518,8 +1561,8 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         // warp): the list holds the cells of an element together, and their
         // flag bits share bitmap words, so neighbouring entries go to
         // different warps rather than into one warp's same-word atomics
-        const int64_t nw = nthr >> 5, wid = gtid >> 5, lane = tid & 31;
-        for (int64_t q = lane * nw + wid; q < nl; q += nthr) {
+        const int64_t nw = (int64_t)gridDim.x * kFlagWarps, wid = blockIdx.x * (int64_t)kFlagWarps + (tid >> 5), lane = tid & 31;
+        for (int64_t q = tid < 32 * kFlagWarps ? lane * nw + wid : INT64_MAX / 2; q < nl; q += 32 * nw) {
           const int32_t cell = d.liq[q];
           // all 26 neighbour states, then all flag updates, in flight at once
           uint32_t solid = 0;
@@ -1574,14 +1617,32 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
             fresh &= fresh - 1;
             int di, dj, dk;
             nbr_offset(n, di, dj, dk);
-            if (slot < d.list_cap) d.flagged[par][slot] = cell + dk * g.nxyg + dj * g.nxg + di;
+            const int32_t fc = cell + dk * g.nxyg + dj * g.nxg + di;
+            if (slot < d.list_cap) {
+              d.flagged[par][slot] = fc;
+              const unsigned k = atomicAdd(&s_fresh_n, 1u);
+              if (k < (unsigned)d.fresh_cap) {
+                s_fresh[k] = fc;
+                s_fresh_slot[k] = (int32_t)slot;
+              } else {
+                coldest(fc, slot);
+              }
+            }
             ++slot;
           }
         }
       }
     }
+    // the cells that this block's warps flagged first
+    if (tid < 32 * kFlagWarps) {
+      asm volatile("bar.sync 2, %0;" ::"n"(32 * kFlagWarps) : "memory");
+      const unsigned n = min(s_fresh_n, (unsigned)d.fresh_cap);
+      for (unsigned k = tid; k < n; k += 32 * kFlagWarps) coldest(s_fresh[k], (unsigned)s_fresh_slot[k]);
+      if (best < dkey(d.Tm) && best < ld_volatile(&c->minT_key)) atomicMin(&c->minT_key, best);
+    }
     __syncthreads();
     if (tid == 0) {
+      s_fresh_n = 0u;
       const unsigned long long w = now_ns() - tfl;
       if (d.detail && w > ld_volatile(&c->flags_scratch)) atomicMax(&c->flags_scratch, w);
     }
@@ -1592,7 +1653,8 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     }
     if (!(ok = grid_barrier(d, 1))) break;
 
-    // ===== C: nucleation (block 0) | cutoff + minimum temperature (Remelting.cpp:656-705) =====
+    // ===== C: nucleation (block 0; Remelting.cpp:936-999) =====
+    // Beside the others' growth: the sites' cells were taken from the candidates in phase B.
     const unsigned nf = ld_volatile(&c->n_flag[par]);
     if (nf > d.list_cap) {
       if (gtid == 0) atomicCAS(&c->error, 0, kRemeltErrList);
@@ -1642,63 +1704,11 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
         s_clk[kClkNucleation] += now_ns() - tn;
       }
     }
-    {
-      const bool solo = gridDim.x == 1;
-      const int64_t g0 = spread_begin(solo ? 0 : 1);
-      const int64_t gn = spread_stride(solo ? 0 : 1);
-      if (nf <= d.list_cap && (solo || blockIdx.x > 0)) {
-        const unsigned long long key_tm = dkey(d.Tm);
-        unsigned long long best = key_tm;
-        for (int64_t q = g0; q < nf; q += gn) {
-          const int32_t cell = d.flagged[par][q];
-          int I, J, K;
-          cell_ijk(g, cell, I, J, K);
-          // all it reads by cell in flight at once
-          const int32_t gid = d.grain[cell], e = d.tag[cell];
-          const double len = d.glen[cell], xi = d.pc[3 * (int64_t)cell], eta = d.pc[3 * (int64_t)cell + 1],
-                       zeta = d.pc[3 * (int64_t)cell + 2];
-          if (ghost(g, I, J, K)) continue;
-          if (gid < 0) continue;
-          if (!(len < d.cutoff)) d.glen[cell] = d.h;  // length reset (:688-694)
-          double T = -1.0;
-          ++exactT;
-          eval_T(d, th, e, xi, eta, zeta, T);
-          {  // growth velocity of single_integration_step (Remelting.cpp:569-576)
-            bool hard = false, near_v = false;
-            const double Targ = (T < d.Ts) ? d.Ts + 0.01 : T;
-            double other;
-            const double vel = velocity(d, Targ, hard, near_v, other);
-            d.fvel[q] = vel;
-            if (hard) {
-              const unsigned slot = append_slot(&c->n_hard);
-              if (slot < d.list_cap) {
-                d.hard_idx[slot] = (int32_t)q;
-                d.hard_T[slot] = Targ;
-                if (slot < (unsigned)kHostVelCap) {
-                  d.hard_v[slot] = near_v ? vel : -1.0;
-                  d.hard_other[slot] = near_v ? other : -1.0;
-                }
-                // the host's answer, slot `slot`, is taken later
-                // (velocities are never negative)
-                d.fvel[q] = -1.0 - (double)slot;
-              }
-            }
-          }
-          if (T <= d.Ts) continue;
-          if (T == T) {
-            const unsigned long long k = dkey(T);
-            best = k < best ? k : best;
-          }
-        }
-        if (best < key_tm && best < ld_volatile(&c->minT_key)) atomicMin(&c->minT_key, best);
-      }
-    }
     if (gtid == 0) {
       const unsigned long long t1 = now_ns();
       s_clk[kClkPhase + 2] += t1 - t_phase;
       t_phase = t1;
     }
-    if (!(ok = grid_barrier(d, 2))) break;
 
     // What the growth of a flagged cell reads besides dt and its velocity:
     // its state, orientation matrix and candidate neighbours (non-ghost

@@ -29,6 +29,8 @@ constexpr int kRemeltRunning = 0, kRemeltFinalTime = 1, kRemeltFramesEnd = 2, kR
 // temperatures in this mapped, page-locked buffer and waits (bounded) for
 // the host service thread to answer.
 constexpr int kHostVelCap = 1 << 16;
+// Flagged cells that a block of the step kernel buffers (see remelt.cu, phase B).
+constexpr int kFresh = 2048;
 struct HostVelocity {
   unsigned int seq_req, seq_done, n, pad;
   double T[kHostVelCap];
@@ -159,6 +161,7 @@ struct RemeltDevice {
   double *hard_other;        // the other value the host's may have (-1: not known),
   double *hard_L;            // and the cells' lengths before the step
   HostVelocity *host;        // device view of the mapped host buffer
+  int fresh_cap;             // flagged cells a block keeps for its own turn at them (kFresh; smaller in tests)
   int host_cap;              // entries of `host` one request may use (kHostVelCap; smaller in tests)
   int64_t list_cap;
   RemeltCtrl *ctrl;

@@ -104,8 +104,8 @@ __device__ __forceinline__ uint8_t *align1024(uint8_t *p) {
 // copy of an activation or a weight exists. Before (a GEMM per layer and
 // direction, each epilogue storing a row-major and a transposed copy, the
 // transposed one 2 bytes at a time, one-block-per-column bias and head sums):
-// 505 us for a step of 32,768 rows; now 188 us (alone and from a cold cache:
-// 105, 32, 32 and 22 us; the chains run beside the weight gradients, a step's
+// 505 us for a step of 32,768 rows; now 168 us (alone and from a cold cache:
+// 88, 32, 31 and 22 us; the chains run beside the weight gradients, a step's
 // set-up beside the update before it). Every sum keeps its order: the trained
 // parameters are the same bits.
 // ---------------------------------------------------------------------------

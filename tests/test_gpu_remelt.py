@@ -121,6 +121,25 @@ def test_remelt_gpu_launches_of_several_steps_match_the_reference(amca, tmp_path
     r.close()
 
 
+@pytest.mark.parametrize("cap", [0, 1, 3])
+@pytest.mark.parametrize("name", ["remelt_random", "remelt_new_grains"])
+def test_remelt_gpu_flagged_cells_beyond_the_block_buffer(amca, tmp_path, monkeypatch, name, cap):
+    """A block takes the temperature and velocity of the cells it flags from its buffer, or at once when that is full
+    (here after no, one or three cells): state, time and dt equal the reference's."""
+    monkeypatch.setenv("AMCA_FRESH_CAP", str(cap))
+    fx = FIX[name]
+    r = make_realm(amca, fx, str(tmp_path))
+    g = np.load(os.path.join(HERE, "golden", f"{name}.npz"))
+    fields = [str(f) for f in g["fields"]]
+    for i in range(19, len(g["digests"]), 20):
+        r.run(20)
+        st = r.stats()
+        assert st["step"] == i + 1 and st["time"] == g["time"][i] and st["dt"] == g["dt"][i]
+        d = digests(r)
+        assert not [k for k in STATE if d[k] != g["digests"][i][fields.index(k)]], f"step {i + 1}"
+    r.close()
+
+
 @pytest.mark.parametrize("mean", [20.0, -400.0])
 def test_remelt_gpu_sites_that_nucleate_above_the_liquidus(amca, oracle, tmp_path, mean):
     """Elements above the liquidus whose cells are all molten are not visited again, unless a cell nucleates in one (a
