@@ -235,9 +235,10 @@ cudaError_t plain_run_steps(const PlainDevice &d, long long step_limit, int grid
 
 // The same kernel with registers for two blocks per SM (128 instead of 64,
 // which spill) and lanes that share a rank; plain_run_steps takes it for grids
-// of at most two blocks per SM. Before / with it: 24^3 5.79 / 5.07 ms, 60^3
+// of at most two blocks per SM. Without / with it: 24^3 5.79 / 5.07 ms, 60^3
 // 12.31 / 11.09, 95^3 14.07 / 12.86 (one block per SM), 128^3 17.25 / 15.93,
-// 160^3 21.4 / 19.9, 200^3 28.2 / 26.0 (two).
+// 160^3 21.4 / 19.9, 200^3 28.2 / 26.0 (two), when checks and marks still took
+// neighbours one by one (now 4.4, 9.2, 10.3, 13.1, 16.4 and 21.3 ms with it).
 cudaError_t plain_few_launch(const PlainDevice &d, long long step_limit, int grid_blocks, cudaStream_t s);
 
 // Blocks of the batched kernel that fit on the device at once.

@@ -267,11 +267,11 @@ struct amca_t {
     {
       // Blocks per SM of the persistent launch: a small realm's generations
       // are short, so its steps are set by barrier and look-back latency,
-      // which fall with the number of blocks (GB300, blocks per SM 1 / 2 / 3:
-      // 24^3 5.07 / 5.39 / 6.5 ms, 60^3 11.09 / 11.70 / 13.7, 95^3 12.86 /
-      // 13.52 / 15.4, 128^3 16.57 / 15.93 / 17.4, 160^3 22.5 / 19.9 / 21.2,
-      // 200^3 31.6 / 26.0 / 26.6, 256^3 52.6 / 39.2 / 38.3 and 37.6 at 4, 320^3
-      // 89.3 / 60.6 / 55.8 and 52.3).
+      // which fall with the number of blocks (GB300, blocks per SM 1 / 2 / 3 / 4:
+      // 24^3 4.42 / 4.78 / 5.93 / 6.36 ms, 60^3 9.15 / 9.91 / 12.0 / 12.9, 95^3
+      // 10.3 / 11.0 / 12.9 / 13.8, 128^3 13.4 / 13.1 / 14.6 / 15.5, 160^3 18.4 /
+      // 16.4 / 18.0 / 18.7, 200^3 26.0 / 21.3 / 22.1 / 22.7, 256^3 43.8 / 33.2 /
+      // 33.1 / 32.3, 320^3 75.6 / 52.4 / 49.3 / 46.9).
       // AMCA_PLAIN_BLOCKS_PER_SM overrides the choice.
       const long long interior = (long long)c.nx * c.ny * c.nz;
       int per_sm = interior <= kRealmCells1 ? 1 : interior <= kRealmCells2 ? 2 : 0;

@@ -679,10 +679,10 @@ void RemeltRealm::initialize() {
     void *dv = nullptr;
     RCK(cudaHostGetDevicePointer(&dv, hv, 0));
     d.host = (HostVelocity *)dv;
+    d.fresh_cap = kFresh;  // (AMCA_FRESH_CAP: tests make it small to run the path beyond it)
+    if (const char *e = getenv("AMCA_FRESH_CAP")) d.fresh_cap = std::min(kFresh, std::max(0, atoi(e)));
     // entries one request may use; AMCA_HOST_VEL_CAP (tests) makes it small
     // so that steps take the chunked path
-    d.fresh_cap = kFresh;
-    if (const char *e = getenv("AMCA_FRESH_CAP")) d.fresh_cap = std::min(kFresh, std::max(0, atoi(e)));
     d.host_cap = kHostVelCap;
     if (const char *e = getenv("AMCA_HOST_VEL_CAP")) d.host_cap = std::min(kHostVelCap, std::max(2, atoi(e)));
   }

@@ -342,8 +342,8 @@ typedef struct {
   double phase_ms[9];
   /* Remelting realm only (zeros otherwise), ms summed over steps: per-block
    * busy time between grid barriers, mean over blocks [0..5] and slowest
-   * block [6..11], for the work closed by the barrier after phase A, B, C,
-   * D, E and after the host velocity answers; block 0's new-grain ids [12]
+   * block [6..11], for the work closed by the barrier after phase A, B, C
+   * (0: it has none), D, E and after the host velocity answers; block 0's new-grain ids [12]
    * and nucleation [13]; the slowest block's liquid-neighbour flag pass in
    * phase B [14]. Plain realm: per-block busy time, mean over blocks, of
    * nucleation [0], the wake scan [1] and list compactions [2]; the slowest
