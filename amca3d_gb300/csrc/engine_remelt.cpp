@@ -815,59 +815,27 @@ static double reference_velocity(const PlainConfig &c, double T) {
 
 // The launching thread, while its kernel runs: answers the kernel's velocity
 // requests, with whatever helpers have come to life by then, until the event
-// after the launch has completed (returns its status).
-cudaError_t RemeltRealm::serve_launch(VelocityJob *job) {
+// after the launch has completed (returns its status). The launch ends by
+// itself, its own waits being bounded, so the event also bounds the wait for
+// the helpers.
+cudaError_t RemeltRealm::serve_launch(VelocityShare *share) {
   HostVelocity *hv = hostvel_;
   unsigned last = __atomic_load_n(&hv->seq_done, __ATOMIC_ACQUIRE);
+  cudaError_t e = cudaErrorNotReady;
+  const auto ended = [&] { return (e = cudaEventQuery(ev1_)) != cudaErrorNotReady; };
+  const auto eval = [&](unsigned i) { hv->v[i] = reference_velocity(cfg_.ca, hv->T[i]); };
   for (unsigned idle = 1;; ++idle) {
     const unsigned r = __atomic_load_n(&hv->seq_req, __ATOMIC_ACQUIRE);
     if (r != last) {
       const unsigned n = std::min(__atomic_load_n(&hv->n, __ATOMIC_ACQUIRE), (unsigned)kHostVelCap);
-      // small requests are not worth sharing
-      const unsigned use = n >= 64u ? 1u + job->helpers.load(std::memory_order_acquire) : 1u;
-      if (use > 1) {
-        job->n.store(n, std::memory_order_relaxed);
-        job->use.store(use, std::memory_order_relaxed);
-        job->left.store(use - 1, std::memory_order_relaxed);
-        job->seq.store(r, std::memory_order_release);
-      }
-      for (unsigned i = 0; i < n; i += use) hv->v[i] = reference_velocity(cfg_.ca, hv->T[i]);
-      if (use > 1)
-        while (job->left.load(std::memory_order_acquire) != 0) {
-        }
+      if (!share->serve(r, n, eval, ended)) return e;
       __atomic_store_n(&hv->seq_done, r, __ATOMIC_RELEASE);
       last = r;
       idle = 0;
       continue;
     }
-    if (idle % 64u == 0) {
-      const cudaError_t e = cudaEventQuery(ev1_);
-      if (e != cudaErrorNotReady) return e;
-    }
+    if (idle % 64u == 0 && ended()) return e;
     if (idle > 4096) std::this_thread::yield();
-  }
-}
-
-// A helper of serve_launch: evaluates its share of the requests made since it
-// came to life, spinning (yielding when idle for long) on the job word.
-void RemeltRealm::help_velocities(VelocityJob *job) {
-  HostVelocity *hv = hostvel_;
-  unsigned last = job->seq.load(std::memory_order_acquire);
-  const unsigned w = 1u + job->helpers.fetch_add(1u, std::memory_order_acq_rel);
-  unsigned idle = 0;
-  while (!job->stop.load(std::memory_order_acquire)) {
-    const unsigned r = job->seq.load(std::memory_order_acquire);
-    if (r != last) {
-      last = r;
-      idle = 0;
-      const unsigned use = job->use.load(std::memory_order_relaxed);
-      if (w >= use) continue;  // made before this helper counted
-      const unsigned n = job->n.load(std::memory_order_relaxed);
-      for (unsigned i = w; i < n; i += use) hv->v[i] = reference_velocity(cfg_.ca, hv->T[i]);
-      job->left.fetch_sub(1, std::memory_order_acq_rel);
-      continue;
-    }
-    if (++idle > 4096) std::this_thread::yield();
   }
 }
 
@@ -963,26 +931,28 @@ void RemeltRealm::launch(long long limit) {
   cudaError_t le = remelt_run_steps(dev_, limit, blocks_, stream_);
   if (le == cudaSuccess) le = cudaEventRecord(ev1_, stream_);
   if (le == cudaSuccess) {
-    VelocityJob job;
+    VelocityShare share;
+    const auto help = [&] { share.help([&](unsigned i) { hostvel_->v[i] = reference_velocity(cfg_.ca, hostvel_->T[i]); }); };
     std::thread starter;
     const int hw = (int)std::thread::hardware_concurrency();
+    static_assert(kHostVelCap <= VelocityShare::kMaxEntries && 8 <= VelocityShare::kMaxThreads, "a request's word holds both");
     const int helpers = limit - ctrl_.step >= kHelpedSteps ? std::max(1, std::min(8, hw / 2)) - 1 : 0;
     if (helpers > 0) {  // started beside the kernel; this thread answers alone until (or unless) they are there
       try {
         starter = std::thread([&] {
           std::vector<std::thread> more;
           try {
-            for (int k = 1; k < helpers; ++k) more.emplace_back([&] { help_velocities(&job); });
+            for (int k = 1; k < helpers; ++k) more.emplace_back(help);
           } catch (const std::system_error &) {
           }
-          help_velocities(&job);
+          help();
           for (std::thread &t : more) t.join();
         });
       } catch (const std::system_error &) {
       }
     }
-    le = serve_launch(&job);
-    job.stop.store(true, std::memory_order_release);
+    le = serve_launch(&share);
+    share.stop();
     if (starter.joinable()) starter.join();
   }
   if (le != cudaSuccess) throw CudaError(std::string("remelting kernel: ") + cudaGetErrorString(le));

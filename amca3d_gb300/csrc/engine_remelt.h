@@ -9,7 +9,6 @@
 
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <memory>
 #include <string>
 #include <utility>
@@ -21,6 +20,7 @@
 #include "host_init.h"
 #include "remelt.h"
 #include "surrogate.h"
+#include "velocity_share.h"
 #include "writers.h"
 
 namespace amca {
@@ -73,18 +73,7 @@ class RemeltRealm {
   void sync_ctrl();
   void extend_orientations();
   void upload_initial_state();
-  // Host side of the velocity requests: of a request shared by `use` threads,
-  // thread w (the launching one is 0) evaluates entries w, w + use, ...
-  struct VelocityJob {
-    std::atomic<unsigned> seq{0};      // shared request being served
-    std::atomic<unsigned> n{0};        // its entry count
-    std::atomic<unsigned> use{1};      // threads that share it
-    std::atomic<unsigned> left{0};     // helpers still evaluating it
-    std::atomic<unsigned> helpers{0};  // helpers alive
-    std::atomic<bool> stop{false};
-  };
-  cudaError_t serve_launch(VelocityJob *job);
-  void help_velocities(VelocityJob *job);
+  cudaError_t serve_launch(VelocityShare *share);
   void launch(long long limit);
   void write_snapshot();
   // host copies of the output fields of the current state
