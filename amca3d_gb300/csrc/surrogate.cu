@@ -1009,6 +1009,9 @@ __global__ void __launch_bounds__(kInferThreads, 1)
   auto wait = [&](uint64_t &bar, uint32_t parity) {
     return umma::mbar_wait_role(umma::smem_u32(&bar), parity, kWaitNs, &s_abort);
   };
+  auto wait_warp = [&](uint64_t &bar, uint32_t parity) {
+    return umma::mbar_wait_warp(umma::smem_u32(&bar), parity, kWaitNs, &s_abort);
+  };
 
   if (warp == kInferEpiWarps + 1) {  // ---- weights ----
     if (lane == 0) {
@@ -1182,7 +1185,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     for (int64_t tile = tile0; tile < ntiles; tile += dtile, ++tiles) {
       const int par = tiles & 1;
       if (tiles == 0) {
-        if (!(ok = wait(fetched[0], 0))) break;
+        if (!(ok = wait_warp(fetched[0], 0))) break;
         features(0, 0);
         features(0, 1);
       }
@@ -1195,7 +1198,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
       written();
       if (grp == kIoGroup) {
         if (tiles > 0) {
-          if (!(ok = wait(headed, par ^ 1))) break;
+          if (!(ok = wait_warp(headed, par ^ 1))) break;
           results(last, par ^ 1);
         }
         last = cur;
@@ -1207,12 +1210,12 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         const uint32_t dcol = trow + 256u * (l & 1);
         // the next tile's features, while this layer's MMAs run
         if ((l == 1 || l == 2) && tile + dtile < ntiles) {
-          if (l == 1 && !(ok = wait(fetched[par ^ 1], (tiles + 1) >> 1 & 1))) break;
+          if (l == 1 && !(ok = wait_warp(fetched[par ^ 1], (tiles + 1) >> 1 & 1))) break;
           if (l == 1) features(par ^ 1, 0);
           else features(par ^ 1, 1);
         }
         // the first layer's input, which is overwritten below, is read for both halves
-        if (!(ok = wait(acc[half], layers & 1) && (l > 0 || wait(acc[half ^ 1], layers & 1)))) break;
+        if (!(ok = wait_warp(acc[half], layers & 1) && (l > 0 || wait_warp(acc[half ^ 1], layers & 1)))) break;
         umma::tc_fence_after();
         for (int c0 = grp * kGroupCols; c0 < (grp + 1) * kGroupCols; c0 += 32) {
           float v[32];
@@ -1253,7 +1256,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
       __syncwarp();
       if (lane == 0) umma::mbar_arrive(umma::smem_u32(&headed));
     }
-    if (ok && tiles > 0 && grp == kIoGroup && wait(headed, (tiles - 1) & 1)) results(last, (tiles - 1) & 1);
+    if (ok && tiles > 0 && grp == kIoGroup && wait_warp(headed, (tiles - 1) & 1)) results(last, (tiles - 1) & 1);
   }
   umma::tc_fence_before();
   __syncthreads();

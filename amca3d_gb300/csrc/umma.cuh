@@ -12,6 +12,8 @@
 
 #include <stdint.h>
 
+#include "bounded_wait.h"
+
 namespace amca {
 namespace umma {
 
@@ -66,19 +68,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
 }
 
 // The same for blocks whose warps have separate roles: a wait that runs out
-// sets *abort, and every wait ends (false) once it is set.
+// sets *abort, and every wait ends (false) once it is set. For a role that is
+// one thread; a role of whole warps waits by mbar_wait_warp, whose verdict is
+// the same in every lane.
 __device__ __forceinline__ bool mbar_wait_role(uint32_t bar, uint32_t parity, unsigned long long limit_ns,
                                                volatile int *abort) {
-  if (mbar_test(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  while (!mbar_test(bar, parity)) {
-    if (*abort) return false;
-    if (global_ns() - t0 > limit_ns) {
-      *abort = 1;
-      return false;
-    }
-  }
-  return true;
+  return wait_or_abort([&] { return mbar_test(bar, parity); }, [] { return global_ns(); }, limit_ns, abort);
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, unsigned long long limit_ns,
+                                               volatile int *abort) {
+  return wait_or_abort_together([&] { return mbar_test(bar, parity); }, [] { return global_ns(); }, limit_ns, abort,
+                                [](bool ok) { return __all_sync(0xffffffffu, ok) != 0; });
 }
 
 // ---- TMA ------------------------------------------------------------------
