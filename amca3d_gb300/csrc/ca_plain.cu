@@ -68,8 +68,8 @@ namespace {
 
 // ca_batch_wide*.cu compile this file again with wider blocks, for the batched
 // kernel alone (AMCA_BATCH_WIDE names the wrapper they define), and
-// ca_realm_few.cu for the kernel that runs one realm with at most two blocks
-// per SM (AMCA_REALM_FEW): registers for two blocks, lanes that share a rank.
+// ca_realm_few.cu for the kernel that runs one realm with at most one block
+// per SM (AMCA_REALM_FEW): registers for two, lanes that share a rank.
 #ifndef AMCA_BLOCK
 #define AMCA_BLOCK 256
 #define AMCA_MIN_BLOCKS 4
@@ -998,6 +998,7 @@ __device__ __noinline__ void zero_decisions(const PlainDevice &d, int cur, int z
 // wake key.
 // ---------------------------------------------------------------------------
 #ifdef AMCA_REALM_FEW
+constexpr int kClaimLanes = 128;  // lanes of a block that share the ranks of a small generation
 // The lanes (as a power of two) that share a rank of a generation of n. A claim
 // lasts as long as the warp's rank with the most liquid neighbours (17 tests
 // of 130 ns behind the capture's 2.5 us), so a generation that leaves most
@@ -1007,7 +1008,7 @@ __device__ __noinline__ void zero_decisions(const PlainDevice &d, int cur, int z
 // 320^3: 2% slower). One, 4, 8, 16 lanes on 60^3: 15.4, 13.7, 13.5, 13.7 ms.
 __device__ __forceinline__ int lane_shift(const PlainDevice &d, long long n) {
   int sh = 0;
-  while (sh < 3 && n << (sh + 1) <= (long long)d.claim_lanes * t_nb) ++sh;
+  while (sh < 3 && n << (sh + 1) <= (long long)kClaimLanes * t_nb) ++sh;
   return sh;
 }
 #endif
@@ -2256,10 +2257,8 @@ cudaError_t plain_run_steps(const PlainDevice &d, long long step_limit, int grid
   if (e != cudaSuccess) return e;
   int device = 0, sms = 0;
   if (cudaGetDevice(&device) == cudaSuccess &&
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && grid_blocks <= 2 * sms) {
-    dd.claim_lanes = grid_blocks <= sms ? 128 : 64;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && grid_blocks <= sms)
     return plain_few_launch(dd, step_limit, grid_blocks, s);
-  }
   return cudaLaunchCooperativeKernel((const void *)plain_persistent_kernel, dim3(grid_blocks), dim3(kBlock), args, 0,
                                      s);
 }

@@ -165,7 +165,6 @@ struct PlainDevice {
   int warp_sched;   // ranks per block of the team up to which claims are handed out warp by warp (else block by block)
   int mark_split;   // ranks per block of the team up to which a generation is marked inside the resolve pass
   int dec_warps;    // warps per block that start a claim phase with the neighbourhood checks (1..kWarps)
-  int claim_lanes;  // set for the launch: lanes per block that share the ranks of a small generation (plain_run_steps)
   int compact_slack;  // the list is compacted when it holds more than 2 x active + this many entries
   // arrays
   uint32_t *orient;
@@ -233,12 +232,12 @@ int plain_persistent_grid(int device);
 // One cooperative launch; every phase boundary is a bounded grid barrier.
 cudaError_t plain_run_steps(const PlainDevice &d, long long step_limit, int grid_blocks, cudaStream_t s);
 
-// The same kernel with registers for two blocks per SM (128 instead of 64,
-// which spill) and lanes that share a rank; plain_run_steps takes it for grids
-// of at most two blocks per SM. Without / with it: 24^3 5.79 / 5.07 ms, 60^3
-// 12.31 / 11.09, 95^3 14.07 / 12.86 (one block per SM), 128^3 17.25 / 15.93,
-// 160^3 21.4 / 19.9, 200^3 28.2 / 26.0 (two), when checks and marks still took
-// neighbours one by one (now 4.4, 9.2, 10.3, 13.1, 16.4 and 21.3 ms with it).
+// The same kernel with 128 registers instead of 64, which spill, and lanes that
+// share a rank; plain_run_steps takes it for grids of at most one block per SM,
+// so that half of every SM's registers stay free for other launches. At one block per SM,
+// without / with it: 24^3 5.79 / 5.07 ms, 60^3 12.31 / 11.09, 95^3 14.07 /
+// 12.86, when checks and marks still took neighbours one by one (now 4.4, 9.2
+// and 10.3 ms with it).
 cudaError_t plain_few_launch(const PlainDevice &d, long long step_limit, int grid_blocks, cudaStream_t s);
 
 // Blocks of the batched kernel that fit on the device at once.

@@ -39,9 +39,9 @@ namespace {
 
 thread_local std::string g_create_error;
 
-// Interior cells up to which a plain realm runs 1 and 2 blocks per SM instead
-// of the kernel's full occupancy (see initialize).
-constexpr long long kRealmCells1 = 1500000ll, kRealmCells2 = 8ll << 20;
+// Interior cells up to which a plain realm runs 1, 2 and 3 blocks per SM
+// instead of the kernel's full occupancy (see initialize).
+constexpr long long kRealmCells1 = 3200000ll, kRealmCells2 = 4200000ll, kRealmCells3 = 8ll << 20;
 
 }  // namespace
 
@@ -267,14 +267,21 @@ struct amca_t {
     {
       // Blocks per SM of the persistent launch: a small realm's generations
       // are short, so its steps are set by barrier and look-back latency,
-      // which fall with the number of blocks (GB300, blocks per SM 1 / 2 / 3 / 4:
-      // 24^3 4.42 / 4.78 / 5.93 / 6.36 ms, 60^3 9.15 / 9.91 / 12.0 / 12.9, 95^3
-      // 10.3 / 11.0 / 12.9 / 13.8, 128^3 13.4 / 13.1 / 14.6 / 15.5, 160^3 18.4 /
-      // 16.4 / 18.0 / 18.7, 200^3 26.0 / 21.3 / 22.1 / 22.7, 256^3 43.8 / 33.2 /
-      // 33.1 / 32.3, 320^3 75.6 / 52.4 / 49.3 / 46.9).
+      // which fall with the number of blocks (GB300, blocks per SM 1 (128
+      // registers, see plain_few_launch) / 2 / 3 / 4 (64 registers): 24^3 4.4 /
+      // - / 5.9 / 6.4 ms, 60^3 9.2 / - / 12.0 / 12.9, 95^3 10.3 / - / 12.9 /
+      // 13.8, 128^3 14.2 / 15.1 / 15.7 / 17.0, 144^3 16.1 / 16.4 / 17.0 / 17.9,
+      // 152^3 16.2 / 16.1 / 16.6 / 17.1, 160^3 18.2 / 17.5 / 17.9 / 18.6, 180^3
+      // 21.9 / 19.9 / 19.8 / 20.6, 200^3 25.4 / 22.1 / 21.1 / 21.7, 256^3 43.8 / - /
+      // 33.1 / 32.3, 320^3 75.6 / - / 49.3 / 46.9).
+      // Up to 8M cells none of these takes all the registers of an SM, so that
+      // kernels of other threads' realms and batches run beside it. Two blocks of
+      // 128 registers per SM (128^3 13.9, 160^3 16.2, 180^3 18.5 ms) do: two 128^3
+      // realms on two threads took 27.3 ms instead of 20.7, and a small realm's
+      // grain field beside a 180^3 run 14.5 instead of 0.13.
       // AMCA_PLAIN_BLOCKS_PER_SM overrides the choice.
       const long long interior = (long long)c.nx * c.ny * c.nz;
-      int per_sm = interior <= kRealmCells1 ? 1 : interior <= kRealmCells2 ? 2 : 0;
+      int per_sm = interior <= kRealmCells1 ? 1 : interior <= kRealmCells2 ? 2 : interior <= kRealmCells3 ? 3 : 0;
       if (const char *e = getenv("AMCA_PLAIN_BLOCKS_PER_SM")) per_sm = std::max(1, atoi(e));
       if (per_sm > 0) {
         int sms = 0;

@@ -9,6 +9,8 @@ import json
 import os
 import sys
 import tempfile
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -337,3 +339,71 @@ def test_gpu_generations_around_the_shared_lane_sizes_match_oracle(amca, oracle,
         assert out["stats"]["step"] == ref["steps"] and out["stats"]["grains"] == ref["num_grains"], k
         assert out["stats"]["active"] == ref["active_grains"], k
         assert np.array_equal(out["orient"], ref["orient"]) and np.array_equal(out["grain"], ref["grain"]), k
+
+
+def _wide_realm(amca, edge, seed):
+    case = cases._mixed("beside", (edge, edge, edge), seed, 100, edge ** 3 // 1700, t_dot=-50.0)
+    r = amca.CellularAutomataRealm(case.to_yaml(), seed=case.seed)
+    r.initialize()
+    return r
+
+
+def _rerun(r):
+    r.reset()
+    r.run()
+
+
+def _timed(*calls):
+    """Seconds until every call, each on a thread of its own, has returned."""
+    gate = threading.Barrier(len(calls) + 1)
+
+    def go(call):
+        gate.wait()
+        call()
+
+    threads = [threading.Thread(target=go, args=(c,)) for c in calls]
+    for t in threads:
+        t.start()
+    gate.wait()
+    t0 = time.perf_counter()
+    for t in threads:
+        t.join()
+    return time.perf_counter() - t0
+
+
+@pytest.mark.parametrize("edge", [110, 130, 147, 150, 159])
+def test_gpu_two_threads_realms_run_beside_one_another(amca, edge):
+    """Realms of up to 4.2M cells leave room for one another: two of them on two threads take far less than twice the
+    time of one (a fifth longer where they run together, 1.95 times where they take turns)."""
+    a, b = _wide_realm(amca, edge, 3), _wide_realm(amca, edge, 4)
+    for r in (a, b):
+        r.run()
+    one = np.median([_timed(lambda: _rerun(a)) for _ in range(7)])
+    two = np.median([_timed(lambda: _rerun(a), lambda: _rerun(b)) for _ in range(7)])
+    a.close()
+    b.close()
+    assert two < 1.6 * one, (one, two)
+
+
+@pytest.mark.parametrize("edge", [130, 150, 165, 200])
+def test_gpu_other_threads_kernels_run_beside_a_realm(amca, edge):
+    """Realms of up to 8M cells leave room for other threads' kernels: a small realm's grain field is there long before
+    the run beside it ends (0.1 ms of its 15 to 25; it waited for the end where the run took every register)."""
+    big, small = _wide_realm(amca, edge, 3), _wide_realm(amca, 40, 4)
+    big.run()
+    small.run()
+    out = small.field("grain_id")
+    run, wait = [], []
+
+    def late_field():
+        time.sleep(0.003)
+        t0 = time.perf_counter()
+        small.field("grain_id", out=out)
+        wait.append(time.perf_counter() - t0)
+
+    for _ in range(9):
+        run.append(_timed(lambda: _rerun(big)))
+        _timed(lambda: _rerun(big), late_field)
+    big.close()
+    small.close()
+    assert np.median(wait) < 0.25 * np.median(run), (np.median(wait), np.median(run))
