@@ -438,8 +438,9 @@ inline void capture_f64_slow(const double *l2g, double gcx, double gcy, double g
 //  - the edge products share S1A's term, and a sum of two terms accumulated
 //    from +0.0 is plus_zero of one plus the other in either order;
 //  - both edge quotients divide by the same n12, a float.
-// A point outside the envelope, corners too near a tie and magnitudes near the
-// ends of the exponent range go the general way.
+// A point outside the envelope, corners too near a tie, magnitudes near the
+// ends of the exponent range and a truncation with a sign or NaN go the general
+// way.
 AMCA_HD void capture_f64(const double *l2g, double gcx, double gcy, double gcz, double length, double h,
                          double trunc_coeff, double out[4]) {
   double c[3];
@@ -448,8 +449,11 @@ AMCA_HD void capture_f64(const double *l2g, double gcx, double gcy, double gcz, 
   const int quad = quadrant(c[0], c[1], c[2]);
   const double perp = length - interception;
   const int ep = f64_exponent(perp), el = f64_exponent(length);
-  // lengths between 2^-50 and 2^50; perp positive (or +0) and not vanishing
-  bool general = el - 973u > 100u || f64_bits(perp) < 0 || (ep < 400 && f64_bits(perp) != 0);
+  const double tv = trunc_coeff * h;
+  // lengths between 2^-50 and 2^50; perp positive (or +0) and not vanishing;
+  // a truncation that compares by its bits (no sign, no NaN)
+  bool general = el - 973u > 100u || f64_bits(perp) < 0 || (ep < 400 && f64_bits(perp) != 0) ||
+                 (unsigned long long)f64_bits(tv) > 0x7ff0000000000000ull;
   const double third = f64_third(perp);
   double pA[3];
   for (int i = 0; i < 3; i++) pA[i] = c[i] + (nonneg(c[i]) ? third : -third);  // the face normal's signs are c's
@@ -485,7 +489,6 @@ AMCA_HD void capture_f64(const double *l2g, double gcx, double gcy, double gcz, 
   const double y = recip_of_f32(n12f, n12);
   double I0 = div_by_f32(d12, n12, y), I1 = n12 - I0;
   const double J0 = div_by_f32(d13, n12, y), J1 = n12 - J0;
-  const double tv = trunc_coeff * h;
   if (f64_less(I0, tv) && f64_less(I1, tv)) {
     I0 = f64_half(n12);  // == n12 / 2
     I1 = I0;
@@ -517,7 +520,9 @@ __device__ __forceinline__ double capture_f64_quad(const double *l2g, int a, uns
   const int quad = quadrant(c0, c1, c2);
   const double perp = length - interception;
   const int ep = f64_exponent(perp), el = f64_exponent(length);
-  bool general = el - 973u > 100u || f64_bits(perp) < 0 || (ep < 400 && f64_bits(perp) != 0);
+  const double tv = trunc_coeff * h;
+  bool general = el - 973u > 100u || f64_bits(perp) < 0 || (ep < 400 && f64_bits(perp) != 0) ||
+                 (unsigned long long)f64_bits(tv) > 0x7ff0000000000000ull;
   const double third = f64_third(perp);
   const double pA = c + (nonneg(c) ? third : -third);
   const float mag = fabsf(f64_to_f32_rz(pA));
@@ -553,7 +558,6 @@ __device__ __forceinline__ double capture_f64_quad(const double *l2g, int a, uns
   const double n12 = pos_f32_to_f64(n12f);
   const double y = recip_of_f32(n12f, n12);
   double I0 = div_by_f32(de, n12, y), I1 = n12 - I0;
-  const double tv = trunc_coeff * h;
   if (a == 0 && f64_less(I0, tv) && f64_less(I1, tv)) {
     I0 = f64_half(n12);  // == n12 / 2
     I1 = I0;

@@ -45,3 +45,14 @@ def test_capture_equals_the_general_path_and_helpers_the_fp64_operations(tmp_pat
     out = subprocess.run([exe, "200000", "7"], check=True, capture_output=True, text=True).stdout.split("\n")
     rows = [line.split() for line in out if line]
     assert len(rows) == 13 and all(int(n) == 200000 and int(wrong) == 0 for _, n, wrong in rows), rows
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_capture_with_any_truncation_equals_the_general_path(tmp_path):
+    """Truncations with a sign, NaN, infinities and products that underflow (an envelope evaluation takes any):
+    capture_f64 returns capture_f64_general's bits."""
+    exe = str(tmp_path / "truncation")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", os.path.join(HERE, "capture_truncation.cpp"), "-o", exe],
+                   check=True)
+    rows = [line.split() for line in subprocess.run([exe], check=True, capture_output=True, text=True).stdout.splitlines()]
+    assert len(rows) == 13 and all(int(wrong) == 0 for _, _, wrong in rows), rows

@@ -170,6 +170,21 @@ def test_gpu_decentring_by_four_lanes_equals_one(amca, kind):
     assert (fast >= 0).all()
 
 
+@pytest.mark.parametrize("trunc", [np.nan, -np.nan, -0.0, -1.0, -5e-324, np.inf])
+def test_gpu_decentring_with_any_truncation(amca, trunc):
+    """One lane and four decentre alike with truncations that have a sign, are NaN or infinite."""
+    rng = np.random.default_rng(11)
+    n, h = 2000, 2.0e-6
+    q = np.linalg.qr(rng.normal(size=(n, 3, 3)))[0]
+    c = rng.uniform(-0.6, 0.6, (n, 3)) * h
+    q[: n // 4] = np.eye(3)
+    c[: n // 4, 1:] = 0.0
+    length = np.abs(c).sum(1) * rng.choice([1.0, 1.25, 1.7], n)
+    cap64, fast, _ = amca.envelope_eval(np.ascontiguousarray(q.reshape(n, 9)), np.einsum("nij,nj->ni", q, c), length, h,
+                                        np.full(n, trunc))
+    assert (cap64 == 1).sum() > n // 2 and (fast >= 0).all()
+
+
 def test_gpu_outputs_byte_identical(amca):
     case = cases.output_case()
     ref_dir = os.path.join(GOLD, "outputs_tiny")
