@@ -534,12 +534,10 @@ __device__ __forceinline__ bool eval_T(const RemeltDevice &d, const double *th, 
   return eval_T(d, th, d.tag[c], d.pc[3 * c], d.pc[3 * c + 1], d.pc[3 * c + 2], T);
 }
 
-// FP32 estimate of evaluate_temperature's value for a cell with material,
-// with a bound on its error: the shape functions are convex weights
-// (parametric coordinates in [-1, 1]), so the FP32 evaluation of the
-// weighted sum, with the coordinates and node values rounded to float, errs
-// by less than 2e-6 of the largest node magnitude; the bound returned is
-// 2^-16 of it (plus 2^-16 absolute).
+// FP32 estimate of evaluate_temperature's value for a cell with material, and
+// the bound on its error that decisions are made with: hex8_err32's 2^-19 of
+// the largest node magnitude (plus 2^-16 absolute), twice what the derivation
+// at hex8_interp32 gives.
 __device__ float eval_T32(const RemeltDevice &d, const float *th32, int64_t c, int32_t e, float &err) {
   int64_t nid[8];
   elem_nodes(d, (int32_t)e, nid);
