@@ -47,11 +47,13 @@ using bf16 = __nv_bfloat16;
 constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s: every mbarrier wait
 constexpr int kErrWait = 1;
 
-// 1 / (1 + e^-z) from the MUFU's 2^x and 1/x, e^-z = 2^(-z log2 e), z >= -80 so
-// that every value stays finite. Flushing variants: a 2^x below 2^-126 leaves 1
-// + 2^x at 1 either way, and the denormal and range handling of __expf and
-// __fdividef was a third of the instructions of an epilogue (equal to
-// __fdividef(1, 1 + __expf(-z)) for every float z).
+// 1 / (1 + e^-z), with e^-z = 2^(-z log2 e), by the approximate 2^x and 1/x
+// instructions in their flushing form: a 2^x below 2^-126 leaves 1 + 2^x at 1
+// either way. The instructions are specified to a relative error of 2^-22 and to
+// 1 ulp; the rounded constant and product add |z| 2^-23 to that of e^-z, of which
+// the result takes the part e^-z / (1 + e^-z). z below -80 counts as -80, so
+// that every value stays finite: the result is then 1.8e-35, where the true one
+// is between that and 0.
 __device__ __forceinline__ float sigmoid(float z) {
   float e, s;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * fmaxf(z, -80.0f)));

@@ -265,3 +265,46 @@ def test_gradients_at_the_edges_of_the_batch_pieces(A, n):
     moved = m.params() - before
     assert np.max(np.abs(moved)) <= 1e-3 * (1 + 1e-4) + 1e-7 and np.mean(np.abs(moved) > 0.9e-3) > 0.5
     m.close()
+
+
+def silu_through(A, z):
+    """z * sigmoid(z) as the inference kernel and the training forward pass work it out: a model whose last hidden layer
+    is its biases, of which the head takes one, and whose temperature is the head's value."""
+    spec = dict(decks.thermal_spec(), t_shift=0.0, t_scale=1.0)
+    m = A.ThermalModel(**spec)
+    raw = window_inputs(spec, 128, seed=1)
+    p = np.zeros(A.ThermalModel.param_count(), np.float32)
+    lay = TO.layout()
+    last, head = lay["b3"][0], lay["Wh"][0]
+    infer, train = np.empty(len(z), np.float32), np.empty(len(z), np.float32)
+    for i, v in enumerate(z):
+        col = (37 * i) % TO.N_HID
+        p[:] = 0.0
+        p[last + col], p[head + col] = v, 1.0
+        m.set_params(p)
+        T, _ = m.eval(raw)
+        _, pred = m.gradients(raw, np.zeros(128, np.float32))
+        assert (T == T[0]).all() and (pred[:, 0] == pred[0, 0]).all()
+        infer[i], train[i] = T[0], pred[0, 0]
+    m.close()
+    return infer, train
+
+
+def test_sigmoid_error_against_fp64(A):
+    """The activation's sigmoid over all its range, the part below -80 included where its argument is held: within the
+    bound that its instructions' specified errors give (relative: 2^-22 and |z| 2^-23 of e^-z, weighted by e^-z / (1 +
+    e^-z), 2^-23 of the reciprocal and 2^-24 each of the sum and of the product with z)."""
+    z = np.concatenate([np.geomspace(1e-30, 1.0, 40), np.linspace(0.03, 20.0, 150), np.linspace(20.5, 100.0, 60),
+                        [79.999, 80.0, 80.00001, 87.3, 87.4, 88.0, 126.0, 1000.0, 1e30]])
+    z = np.concatenate([-z, z, [0.0, -0.0]]).astype(np.float32)
+    infer, train = silu_through(A, z)
+    assert np.array_equal(infer, train)
+    zd = z.astype(np.float64)
+    held = np.maximum(zd, -80.0)
+    e = np.exp(-held)
+    want = zd / (1.0 + e)
+    rel = (e / (1.0 + e)) * (2.0 ** -22 + np.abs(held) * 2.0 ** -23) + 2.0 ** -23 + 2.0 ** -24 + 2.0 ** -24
+    assert (np.abs(infer - want) <= np.abs(want) * rel * (1 + 1e-5) + 2.0 ** -126).all()
+    # against the sigmoid itself, whose argument nothing holds
+    true = zd * np.exp(np.minimum(zd, 0.0)) / (1.0 + np.exp(-np.abs(zd)))
+    assert (np.abs(infer - true)[zd < -80.0] <= np.abs(zd[zd < -80.0]) * 1.81e-35).all()
