@@ -78,7 +78,7 @@ EXPORTS = ("amca_create", "amca_get_grid", "amca_prepare", "amca_get_sites", "am
            "amca_thermal_get_params", "amca_thermal_set_params", "amca_thermal_get_encoding", "amca_thermal_frames",
            "amca_thermal_last_error", "amca_thermal_destroy",
            "amca_batch_create", "amca_batch_run", "amca_batch_tune", "amca_batch_set_layout", "amca_batch_get_layout",
-           "amca_batch_get_stats",
+           "amca_batch_get_stats", "amca_batch_block_threads",
            "amca_batch_last_error",
            "amca_batch_destroy", "amca_last_error", "amca_destroy")
 
@@ -228,6 +228,8 @@ def load_library(path: Optional[str] = None) -> ctypes.CDLL:
     lib.amca_batch_get_layout.restype = i
     lib.amca_batch_get_stats.argtypes = [vp, ctypes.POINTER(BatchStats)]
     lib.amca_batch_get_stats.restype = i
+    lib.amca_batch_block_threads.argtypes = [vp, ctypes.POINTER(ctypes.c_int32)]
+    lib.amca_batch_block_threads.restype = i
     lib.amca_batch_last_error.argtypes = [vp]
     lib.amca_batch_last_error.restype = cp
     lib.amca_batch_destroy.argtypes = [vp]
@@ -599,6 +601,12 @@ class Batch:
         s = BatchStats()
         self._check(self._lib.amca_batch_get_stats(self._b, ctypes.byref(s)))
         return s.as_dict()
+
+    def block_threads(self) -> int:
+        """Threads per block of the present layout's launch."""
+        n = ctypes.c_int32()
+        self._check(self._lib.amca_batch_block_threads(self._b, ctypes.byref(n)))
+        return n.value
 
     def close(self) -> None:
         if self._b:

@@ -1521,6 +1521,12 @@ int amca_batch_get_stats(const amca_batch *b, amca_batch_stats *s) {
   return AMCA_OK;
 }
 
+int amca_batch_block_threads(const amca_batch *b, int32_t *threads) {
+  if (!b || !threads) return AMCA_ERR_ARG;
+  *threads = b->threads;
+  return AMCA_OK;
+}
+
 const char *amca_batch_last_error(const amca_batch *b) {
   if (!b) return g_create_error.c_str();
   return b->err.c_str();

@@ -556,6 +556,10 @@ typedef struct {
 
 int amca_batch_get_stats(const amca_batch *b, amca_batch_stats *out);
 
+/* Threads per block of the present layout's launch: 256, 512 or 1,024, chosen
+ * from the layout. A realm's result does not depend on it. */
+int amca_batch_block_threads(const amca_batch *b, int32_t *threads);
+
 /* Message of the last failing call on b (or of the last failing
  * amca_batch_create when b is NULL). Never NULL. */
 const char *amca_batch_last_error(const amca_batch *b);

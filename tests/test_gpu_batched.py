@@ -197,3 +197,36 @@ def test_batch_block_widths_give_the_same_fields(amca, edge, team, count):
                 assert np.array_equal(realms[k].field("orientation_id"), o) and realms[k].stats()["step"] == n
     for r in realms:
         r.close()
+
+
+@pytest.mark.parametrize("cells,team,count,width", [
+    ((26, 13, 71), 1, 3, 256),    # 23,998 cells a block: below the first line
+    ((30, 32, 25), 1, 3, 512),    # 24,000: on it
+    ((29, 10, 331), 1, 3, 512),   # 95,990
+    ((40, 48, 50), 1, 3, 1024),   # 96,000
+    ((58, 57, 59), 8, 3, 512),    # 24,381 of a block of a team
+    ((57, 56, 58), 8, 3, 256),    # 23,142
+    ((92, 91, 93), 8, 2, 1024),   # 97,324
+    ((60, 59, 61), 3, 120, 256),  # 360 blocks: too many for wider ones
+])
+def test_batch_launch_takes_the_width_of_its_rule(amca, cells, team, count, width):
+    """The widths of blocks on both sides of each line of the rule, as the launch has them, and the fields of its first
+    and last realm against their own runs."""
+    case = cases._mixed("width", cells, 3, 40, 200, t_dot=-200.0)
+    realms = [amca.CellularAutomataRealm(case.to_yaml(), seed=3 + k % 3) for k in range(count)]
+    for r in realms:
+        r.initialize()
+    with amca.Batch(realms, team_size=team) as b:
+        assert b.block_threads() == width
+        b.run()
+        assert b.block_threads() == width
+        got = [(realms[k].field("grain_id"), realms[k].stats()["step"]) for k in (0, count - 1)]
+        # the width follows the layout
+        b.set_layout([64], [1], [0] * count)
+        assert b.block_threads() == (512 if np.prod(cells) // 64 >= 24000 else 256)
+    for k, (grain, step) in zip((0, count - 1), got):
+        realms[k].reset()
+        realms[k].run()
+        assert np.array_equal(realms[k].field("grain_id"), grain) and realms[k].stats()["step"] == step
+    for r in realms:
+        r.close()
