@@ -2272,8 +2272,9 @@ int plain_batched_grid(int device) {
 }
 
 int plain_batched_threads(int device, int grid_blocks, long long cells_per_block) {
-  if (cells_per_block >= 96000 && grid_blocks <= plain_batched_grid_1024(device)) return 1024;
-  return cells_per_block >= 24000 && grid_blocks <= plain_batched_grid_512(device) ? 512 : kBlock;
+  const auto leaves_room = [&](int resident) { return 16ll * grid_blocks <= 15ll * resident; };
+  if (cells_per_block >= 96000 && leaves_room(plain_batched_grid_1024(device))) return 1024;
+  return cells_per_block >= 24000 && leaves_room(plain_batched_grid_512(device)) ? 512 : kBlock;
 }
 
 cudaError_t plain_batch_reset(const PlainDevice *insts, int ninst, unsigned *queues, int nclasses, BatchTeam *teams,

@@ -251,6 +251,11 @@ int plain_batched_grid(int device);
 // 19.7 / 21.4 ms (14,000 cells a block), 19 of 48 to 80 30.0 / 25.3 / 26.1
 // (64,000), 24 of 32 to 96 41.9 / 33.0 / (too many blocks), 16 of 40 to 104
 // 49.7 / 37.1 / 33.1 (140,000), 4 of 90 to 112 60.4 / 47.5 / 43.1.
+// The wider blocks leave a sixteenth of the SMs' registers to what other threads
+// launch meanwhile (256 threads would leave half or more): 19 realms of 64 to 112
+// cells an edge (152 blocks) 52.5 / 48.4 ms with 512 / 1,024 threads, but a small
+// realm's grain field beside them 0.05 / 8.0 ms, two such batches on two threads
+// 60 / 90 ms and four 116 / 180.
 int plain_batched_threads(int device, int grid_blocks, long long cells_per_block);
 
 // The batched kernel with wider blocks: co-resident blocks, launch.

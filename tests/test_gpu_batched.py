@@ -12,6 +12,8 @@ import hashlib
 import json
 import os
 import sys
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -229,4 +231,46 @@ def test_batch_launch_takes_the_width_of_its_rule(amca, cells, team, count, widt
         realms[k].run()
         assert np.array_equal(realms[k].field("grain_id"), grain) and realms[k].stats()["step"] == step
     for r in realms:
+        r.close()
+
+
+@pytest.mark.parametrize("cells", [(30, 32, 25), (40, 48, 50)])
+def test_batch_of_wide_blocks_leaves_room_for_other_threads(amca, cells):
+    """On both sides of the launch that would take nearly all of the SMs' registers: the width gives way before it does,
+    and a small realm's grain field comes while the batch runs (it waited for the batch's first teams to end)."""
+    case = cases._mixed("room", cells, 3, 40, 60, t_dot=-20.0)
+    small = amca.CellularAutomataRealm(cases._mixed("small", (40, 40, 40), 3, 40, 60).to_yaml(), seed=3)
+    small.initialize()
+    small.run()
+    out = small.field("grain_id")
+    realms = [amca.CellularAutomataRealm(case.to_yaml(), seed=3 + k % 3) for k in range(3)]
+    for r in realms:
+        r.initialize()
+    wide = 1024 if np.prod(cells) >= 96000 else 512
+    with amca.Batch(realms, team_size=1) as b:
+        assert b.block_threads() == wide
+        most = 15 * (b.stats()["max_blocks"] * 256 // wide) // 16  # (512 and 1,024 threads: as many registers a thread)
+    for r in realms:
+        r.close()
+    realms = []
+    for count, width in ((most, wide), (most + 1, wide // 2)):
+        while len(realms) < count:
+            realms.append(amca.CellularAutomataRealm(case.to_yaml(), seed=3 + len(realms) % 3))
+            realms[-1].initialize()
+        with amca.Batch(realms, team_size=1) as b:
+            assert b.stats()["grid_blocks"] == count and b.block_threads() == width
+            b.run()
+            run, wait = [], []
+            for _ in range(7):
+                t0 = time.perf_counter()
+                th = threading.Thread(target=b.run)
+                th.start()
+                time.sleep(0.003)
+                t1 = time.perf_counter()
+                small.field("grain_id", out=out)
+                wait.append(time.perf_counter() - t1)
+                th.join()
+                run.append(time.perf_counter() - t0)
+        assert np.median(wait) < 0.1 * np.median(run), (count, wait, run)
+    for r in realms + [small]:
         r.close()
