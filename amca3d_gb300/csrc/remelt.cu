@@ -201,6 +201,16 @@ __device__ __forceinline__ unsigned append_slot(unsigned *counter) {
   return grp.shfl(base, 0) + grp.thread_rank();
 }
 
+// Barrier number ID of the warps of a block that hold its N participating
+// threads. The instruction is one of whole warps, and a warp comes here from a
+// loop that its lanes leave after different numbers of turns: they meet first.
+template <int ID, int N>
+__device__ __forceinline__ void part_barrier() {
+  static_assert(ID > 0 && N % 32 == 0, "barrier 0 is the block's; whole warps take part");
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+
 // Block-staged list appends: entries go to a shared-memory buffer (shared
 // atomic), and the block moves the buffer to the global list with one
 // global atomicAdd when the phase ends (stage_flush, every thread) — one
@@ -431,7 +441,7 @@ __device__ void host_post(const RemeltDevice &d, unsigned nh, bool min_hard, dou
     const unsigned seq = s_host_seq + 1;
     if (d.host != nullptr)
       for (unsigned k = t; k < total; k += kPostThreads) d.host->T[k] = k < nh ? d.hard_T[k] : minT;
-    asm volatile("bar.sync 1, %0;" ::"n"(kPostThreads) : "memory");
+    part_barrier<1, kPostThreads>();
     if (t == 0) {
       if (d.host != nullptr) {
         d.host->n = total;
@@ -1633,7 +1643,7 @@ __global__ void __launch_bounds__(kBlock, 2) remelt_kernel(RemeltDevice d, long 
     }
     // the cells that this block's warps flagged first
     if (tid < 32 * kFlagWarps) {
-      asm volatile("bar.sync 2, %0;" ::"n"(32 * kFlagWarps) : "memory");
+      part_barrier<2, 32 * kFlagWarps>();
       const unsigned n = min(s_fresh_n, (unsigned)d.fresh_cap);
       for (unsigned k = tid; k < n; k += 32 * kFlagWarps) coldest(s_fresh[k], (unsigned)s_fresh_slot[k]);
       if (best < dkey(d.Tm) && best < ld_volatile(&c->minT_key)) atomicMin(&c->minT_key, best);
