@@ -454,11 +454,13 @@ typedef struct {
  * per site, as amca_get_orientations' angles give through the reference's
  * Bunge formula with the host's libm), and the int32 orientation field
  * ((nx+2)(ny+2)(nz+2) cells, filled by this call). The run's other state
- * lives in one static device array of 32 MiB, which every GPU that loads the
- * library holds until the process exits; grids that need more (about
- * 148 bytes per interior cell plus 37 per site and 300 KB, i.e. roughly
+ * lives in one static device array of 36 MiB, which every GPU that loads the
+ * library holds until the process exits; grids that need more than 32 MiB by
+ * a count of about
+ * 148 bytes per interior cell plus 37 per site and 300 KB (roughly
  * 225,000 interior cells, a 61^3 cube) are rejected with AMCA_ERR_ARG and a
- * message.
+ * message; the rest is for thin grids, whose maps take more than they are
+ * counted with.
  *
  * The site list is checked on the GPU before the run (every site cell an
  * interior cell, ids strictly ascending, at most one site per interior cell);
