@@ -255,7 +255,9 @@ int plain_batched_grid(int device);
 // launch meanwhile (256 threads would leave half or more): 19 realms of 64 to 112
 // cells an edge (152 blocks) 52.5 / 48.4 ms with 512 / 1,024 threads, but a small
 // realm's grain field beside them 0.05 / 8.0 ms, two such batches on two threads
-// 60 / 90 ms and four 116 / 180.
+// 60 / 90 ms and four 116 / 180. More than two batches of wide blocks take turns
+// all the same (four of 16 realms of 40 to 104 cells an edge 109 ms, 77 before there
+// were wide blocks): one batch of all realms is the way to run them.
 int plain_batched_threads(int device, int grid_blocks, long long cells_per_block);
 
 // The batched kernel with wider blocks: co-resident blocks, launch.
